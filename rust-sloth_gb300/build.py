@@ -18,7 +18,7 @@ INCLUDE = HERE.parent / "include"
 OUT_DIR = HERE / "_build"
 LIB = OUT_DIR / "libsloth_gpu.so"
 
-SOURCES = ["setup.cu", "bin.cu", "raster.cu", "resolve.cu", "sloth_api.cu", "noalloc.cu", "batch.cu",
+SOURCES = ["setup.cu", "bin.cu", "raster.cu", "fold.cu", "resolve.cu", "sloth_api.cu", "noalloc.cu", "batch.cu",
            "batch_api.cu", "diff.cu", "flush.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ARCH + [

@@ -53,41 +53,42 @@ constexpr int kDirectStageWords = kDirectFields * 32;
 // per warp).  Indexing the array itself keeps the accesses 32-bit shared ones.
 extern __shared__ uint32_t setup_smem[];
 
-__device__ __forceinline__ uint32_t direct_raster_warp(bool mine, const TriRecord &r, uint32_t gtri, int w, int pitch,
-                                                      int tw, unsigned long long *keys, int xend, uint32_t exit_mask,
-                                                      uint32_t stage)
+// Stages this lane's triangle (mine false: none) and returns the samples to walk.
+__device__ __forceinline__ int direct_stage(bool mine, const TriRecord &r, uint32_t gtri, int xend, uint32_t exit_mask,
+                                            uint32_t stage)
 {
     const int lane = threadIdx.x & 31;
     float *sf = reinterpret_cast<float *>(setup_smem + stage);
     int *si = reinterpret_cast<int *>(setup_smem + stage);
-    int n = 0;
-    if (mine) {
-        const bool probe = exit_mask != 0u && r.xe < xend;   // r.xe <= xend always
-        const int xs = probe ? r.xe + 1 : xend;
-        const int cols = xs - r.x0;
-        n = cols * (r.y1 - r.y0);
-        const float v[16] = {r.v1x, r.v1y, r.v2x, r.v2y, r.v3x, r.v3y, r.dx0, r.dy0,
-                             r.dx1, r.dy1, r.dx2, r.dy2, r.v1z, r.dz2, r.dz3, r.a};
+    if (!mine) return 0;
+    const bool probe = exit_mask != 0u && r.xe < xend;   // r.xe <= xend always
+    const int xs = probe ? r.xe + 1 : xend;
+    const int cols = xs - r.x0;
+    const float v[16] = {r.v1x, r.v1y, r.v2x, r.v2y, r.v3x, r.v3y, r.dx0, r.dy0,
+                         r.dx1, r.dy1, r.dx2, r.dy2, r.v1z, r.dz2, r.dz3, r.a};
 #pragma unroll
-        for (int f = 0; f < 16; ++f) sf[f * 32 + lane] = v[f];
-        si[16 * 32 + lane] = r.x0;
-        si[17 * 32 + lane] = r.y0;
-        si[18 * 32 + lane] = cols;
-        si[19 * 32 + lane] = probe ? r.xe : INT_MAX;
-        si[20 * 32 + lane] = xend;
-        si[21 * 32 + lane] = (int)exit_mask;
-        si[22 * 32 + lane] = (int)gtri;
-    }
-    int end = n;   // running end of the samples up to this lane's triangle
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int o = __shfl_up_sync(0xffffffffu, end, d);
-        if (lane >= d) end += o;
-    }
-    const int total = __shfl_sync(0xffffffffu, end, 31), first = end - n;
-    __syncwarp();
+    for (int f = 0; f < 16; ++f) sf[f * 32 + lane] = v[f];
+    si[16 * 32 + lane] = r.x0;
+    si[17 * 32 + lane] = r.y0;
+    si[18 * 32 + lane] = cols;
+    si[19 * 32 + lane] = probe ? r.xe : INT_MAX;
+    si[20 * 32 + lane] = xend;
+    si[21 * 32 + lane] = (int)exit_mask;
+    si[22 * 32 + lane] = (int)gtri;
+    return cols * (r.y1 - r.y0);
+}
+
+// Walks samples k0, k0 + kstep, ... (32 from each) of a stage's triangles: `end` holds the
+// running end of the samples up to the lane's triangle, `first` their running start and
+// `total` the last end.  Returns the lane's covered samples.
+__device__ __forceinline__ uint32_t direct_walk(int end, int first, int total, int k0, int kstep, int w, int pitch,
+                                                int tw, unsigned long long *keys, uint32_t stage)
+{
+    const int lane = threadIdx.x & 31;
+    const float *sf = reinterpret_cast<const float *>(setup_smem + stage);
+    const int *si = reinterpret_cast<const int *>(setup_smem + stage);
     uint32_t frags = 0;
-    for (int base = 0; base < total; base += 32) {
+    for (int base = k0; base < total; base += kstep) {
         const int k = base + lane;
         // the triangle of sample k: the number of lanes whose samples end at or before k
         int src = 0;
@@ -139,6 +140,24 @@ __device__ __forceinline__ uint32_t direct_raster_warp(bool mine, const TriRecor
             }
         }
     }
+    return frags;
+}
+
+__device__ __forceinline__ uint32_t direct_raster_warp(bool mine, const TriRecord &r, uint32_t gtri, int w, int pitch,
+                                                      int tw, unsigned long long *keys, int xend, uint32_t exit_mask,
+                                                      uint32_t stage)
+{
+    const int lane = threadIdx.x & 31;
+    const int n = direct_stage(mine, r, gtri, xend, exit_mask, stage);
+    int end = n;   // running end of the samples up to this lane's triangle
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, end, d);
+        if (lane >= d) end += o;
+    }
+    const int total = __shfl_sync(0xffffffffu, end, 31);
+    __syncwarp();
+    const uint32_t frags = direct_walk(end, end - n, total, 0, 32, w, pitch, tw, keys, stage);
     __syncwarp();   // the stage is reused by the warp's next call
     return frags;
 }

@@ -1,0 +1,220 @@
+// fold.cuh -- drawing without tiles: every triangle's samples folded straight into the
+// frame's global depth keys.
+//
+// The tile raster (raster_common.cuh) pays for itself when the samples are many: a tile
+// count, a scan, an entry per triangle and tile, a sort and a walk per tile, in nine
+// launches that each wait for the one before.  A draw of a few thousand triangles over few
+// samples is all launches.  Here it takes two: fold_triangles sets up 32 triangles per
+// block and walks their samples (direct.cuh) with every warp of the block, and queues the
+// triangles of more than kFoldQueueSamples samples; fold_large_part walks those with the
+// warps of the whole GPU.  The minimum of a cell's keys does not depend on the order of
+// the folds, so the frame is the tile raster's bit for bit.  The newline rows go straight
+// into the frame's segment tree, whose nodes are maxima.
+//
+// Every tile's keys must be current (cleared or written since the clear) before the folds.
+#pragma once
+
+#include "raster_common.cuh"
+#include "record.cuh"
+
+namespace sloth {
+
+// Triangles a block sets up (one per lane of its first warp).
+constexpr int kFoldTris = 32;
+// Triangles of more samples than this (rows times walked columns) are queued: the block
+// that set one up would walk it alone while the rest of the GPU is idle.  1024 samples are
+// eight steps of a block of four warps.
+constexpr uint32_t kFoldQueueSamples = 1024;
+// A queued triangle is kFoldParts warp items; item i takes the groups of kFoldRows rows
+// i, i + kFoldParts, ... (a frame of 360 rows gives each item at most three groups).
+constexpr uint32_t kFoldParts = 16;
+constexpr int kFoldRows = 8;
+
+// Dynamic shared memory of a fold block: one direct stage and the samples' running ends.
+constexpr size_t kFoldSmemBytes = (kDirectStageWords + 32) * 4;
+
+// Triangles too large for their block: draw index and frame (batches; null otherwise).
+struct FoldQueue {
+    uint32_t *tri;
+    uint32_t *frame;
+    uint32_t *count;
+};
+
+// Newline rows [y0, y1) of draw index v into the frame's tree (nltree_update with
+// reductions, which return nothing to wait for).
+__device__ __forceinline__ void nltree_reduce(int32_t *tree, int n, int y0, int y1, int32_t v)
+{
+    auto put = [&](int i) { asm volatile("red.global.max.s32 [%0], %1;" ::"l"(tree + i), "r"(v) : "memory"); };
+    int l = y0 + n, r = y1 + n;
+    while (l < r) {
+        if (l & 1) put(l++);
+        if (r & 1) put(--r);
+        l >>= 1;
+        r >>= 1;
+    }
+}
+
+// Positions p0 .. p0+31 of setup's order of the mesh, by a block of kWarps warps: records,
+// newline rows, samples folded or the triangle queued.  base: draw index of the mesh's
+// first triangle.  Bound by latency at the sizes it serves (the first warp's chain index ->
+// vertex -> record, then the walk), so the samples of 32 triangles are spread over kWarps
+// warps instead of one.
+template <int kWarps>
+__device__ __forceinline__ void fold_triangles(const MeshDev &mesh, const Mat4 &M, uint32_t p0, uint32_t base,
+                                               const FrameGeom &g, const FrameBuffers &fb, const FoldQueue &queue,
+                                               uint32_t frame)
+{
+    int *ends = reinterpret_cast<int *>(setup_smem + kDirectStageWords);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (wid == 0) {
+        const uint32_t p = p0 + lane;
+        bool mine = false, big = false;
+        uint32_t gtri = 0;
+        int n = 0;
+        DirectWalk dw{false, 0, 0u};
+        TriRecord r;
+        if (p < mesh.ntri) {
+            const uint32_t t = mesh_triangle(mesh, p);
+            gtri = base + t;
+            uint32_t i1, i2, i3;
+            mesh_corners(mesh, p, t, i1, i2, i3);
+            const float4 p1 = transform_vertex(mesh, M, i1), p2 = transform_vertex(mesh, M, i2),
+                         p3 = transform_vertex(mesh, M, i3);
+            const uint32_t rgb = load_rgb(mesh.rgb, t);
+            int4 row4;
+            const bool keep = needs_setup(p1, p2, p3, g.w, g.h, row4);
+            if (g.image) nltree_reduce(fb.nltree, g.nl_size, row4.z, row4.w, (int32_t)gtri);
+            if (keep) {
+                r = build_record(p1, p2, p3, rgb, g.w, g.h, INT_MAX, &dw);
+                if (r.x0 < r.xe) {
+                    // a triangle the direct walk does not size (none of dy > 0, non-finite, or
+                    // more than 2^31 samples) is left to the row walk
+                    const uint64_t walked = (uint64_t)(r.xe + 1 - r.x0) * (uint32_t)(r.y1 - r.y0);
+                    big = !dw.direct || walked > kFoldQueueSamples;
+                    mine = !big;
+                    store_record(fb.records + gtri, r, 1u, true);
+                }
+            }
+        }
+        if (mine) n = direct_stage(true, r, gtri, dw.xend, dw.exit_mask, 0u);
+        const unsigned bm = __ballot_sync(0xffffffffu, big);
+        if (bm) {
+            uint32_t q0 = 0;
+            if (lane == 0) q0 = atomicAdd(queue.count, (uint32_t)__popc(bm));
+            q0 = __shfl_sync(0xffffffffu, q0, 0) + __popc(bm & ((1u << lane) - 1u));
+            if (big) {
+                queue.tri[q0] = gtri;
+                if (queue.frame) queue.frame[q0] = frame;
+            }
+        }
+        int end = n;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, end, d);
+            if (lane >= d) end += o;
+        }
+        ends[lane] = end;
+    }
+    if (kWarps > 1) block_sync();
+    else __syncwarp();
+    const int end = ends[lane], prev = lane ? ends[lane - 1] : 0;
+    const int total = __shfl_sync(0xffffffffu, end, 31);
+    const uint32_t frags = direct_walk(end, prev, total, wid * 32, kWarps * 32, g.w, g.pitch, g.tw,
+                                       reinterpret_cast<unsigned long long *>(fb.keys), 0u);
+    add_frags_warp(frags, fb.fragments);
+}
+
+// One edge's columns on one row, as edge_row_span, for rows as wide as the frame: past a
+// few steps from the estimate (edges of huge coordinates, whose real-valued crossing is
+// only a guess) the first column that fails is found by bisection, since the columns that
+// pass are a prefix (dy > 0) or a suffix (dy < 0) of the row.
+__device__ __forceinline__ void fold_row_span(float dx, float dy, float ax, float ay, float py, int &lo, int &hi)
+{
+    if (lo >= hi) return;
+    auto pass = [&](int x) { return edge_eval(dx, dy, ax, ay, (float)x, py) >= 0.0f; };
+    if (dy == 0.0f) {
+        if (!pass(lo)) hi = lo;
+        return;
+    }
+    const float cross = ax + __fdividef(fmul(dx, fsub(py, ay)), dy);   // estimate only
+    if (dy > 0.0f) {
+        int t = (int)fminf(fmaxf(floorf(cross), (float)(lo - 1)), (float)(hi - 1)) + 1;
+        for (int k = 0; k < 3 && t < hi && pass(t); ++k) ++t;
+        if (t < hi && pass(t)) t = first_true(t + 1, hi, [&](int x) { return !pass(x); });
+        hi = t;
+    } else {
+        int t = (int)fminf(fmaxf(ceilf(cross), (float)lo), (float)hi) - 1;
+        for (int k = 0; k < 3 && t >= lo && pass(t); ++k) --t;
+        if (t >= lo && pass(t)) t = first_true(lo, t, [&](int x) { return pass(x); }) - 1;
+        lo = t + 1;
+    }
+}
+
+// Warp item `part` of a queued triangle: its groups of rows, each row cut to the columns
+// that can pass all three edges, the spans of a group walked 32 samples at a time with the
+// exact test for every sample.  A covered sample whose cell already holds a nearer key is
+// dropped before the reduction: the plain load may be older than the key in L2, and keys
+// only fall, so it can only keep a sample that was not needed.
+__device__ __forceinline__ uint32_t fold_large_part(uint32_t gtri, uint32_t part, const FrameGeom &g,
+                                                    const FrameBuffers &fb)
+{
+    const int lane = threadIdx.x & 31;
+    const float4 *rp = reinterpret_cast<const float4 *>(fb.records + gtri);
+    const int4 xr = *(reinterpret_cast<const int4 *>(rp) + 4);
+    if (xr.z + (int)part * kFoldRows >= xr.w) return 0;
+    const float4 q0 = rp[0], q1 = rp[1], q5 = rp[5];
+    TriRecord r;
+    r.v1x = q0.x; r.v1y = q0.y; r.v2x = q0.z; r.v2y = q0.w; r.v3x = q1.x; r.v3y = q1.y;
+    r.dx0 = fsub(r.v3x, r.v2x); r.dy0 = fsub(r.v3y, r.v2y);
+    r.dx1 = fsub(r.v1x, r.v3x); r.dy1 = fsub(r.v1y, r.v3y);
+    r.dx2 = fsub(r.v2x, r.v1x); r.dy2 = fsub(r.v2y, r.v1y);
+    r.v1z = q5.x; r.dz2 = q5.y; r.dz3 = q5.z; r.a = q5.w;
+    // the reference's right end (row 4 may hold the shorter end the walk was sized by)
+    const int x1 = sat_hi(ceilf(fminf(fmul(fmaxf(r.v1x, fmaxf(r.v2x, r.v3x)), 2.0f), (float)(g.w - 1))));
+    const float big = 1e18f;
+    const bool finite = fabsf(r.v1x) < big && fabsf(r.v1y) < big && fabsf(r.v2x) < big && fabsf(r.v2y) < big &&
+                        fabsf(r.v3x) < big && fabsf(r.v3y) < big;
+    unsigned long long *keys = reinterpret_cast<unsigned long long *>(fb.keys);
+    uint32_t frags = 0;
+    for (int ya = xr.z + (int)part * kFoldRows; ya < xr.w; ya += (int)(kFoldParts * kFoldRows)) {
+        int lo = xr.x, hi = lane < kFoldRows && ya + lane < xr.w ? x1 : xr.x;
+        if (finite) {
+            const float py = (float)(ya + lane);
+            fold_row_span(r.dx0, r.dy0, r.v2x, r.v2y, py, lo, hi);
+            fold_row_span(r.dx1, r.dy1, r.v3x, r.v3y, py, lo, hi);
+            fold_row_span(r.dx2, r.dy2, r.v1x, r.v1y, py, lo, hi);
+        }
+        const int len = max(hi - lo, 0);
+        int end = len;
+#pragma unroll
+        for (int d = 1; d < kFoldRows; d <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, end, d);
+            if (lane >= d) end += o;
+        }
+        const int total = __shfl_sync(0xffffffffu, end, kFoldRows - 1), xoff = lo - (end - len);
+        for (int base = 0; base < total; base += 32) {
+            const int k = base + lane;
+            int row = 0;   // the rows whose spans end at or before k
+#pragma unroll
+            for (int step = kFoldRows / 2; step > 0; step >>= 1)
+                if (__shfl_sync(0xffffffffu, end, row + step - 1) <= k) row += step;
+            const int x = k + __shfl_sync(0xffffffffu, xoff, row), y = ya + row;
+            if (k >= total) continue;
+            const EdgeVals e = eval_edges(r, (float)x, (float)y);
+            if (e.w0 >= 0.0f && e.w1 >= 0.0f && e.w2 >= 0.0f) {
+                ++frags;
+                const float z = interp_z(r.v1z, r.dz2, r.dz3, r.a, e.w1, e.w2);
+                if (z < kFltMax) {
+                    const uint32_t nw = 2 * x < g.w ? 1u : 0u;
+                    unsigned long long *kp = keys + (size_t)(nw ? y : y + 1) * g.pitch +
+                                             key_col(nw ? 2 * x : 2 * x - g.w, g.tw);
+                    const unsigned long long key = make_key(z, gtri, nw);
+                    if (key < *kp) red_min_u64(kp, key);
+                }
+            }
+        }
+    }
+    return frags;
+}
+
+}  // namespace sloth

@@ -1,0 +1,43 @@
+// launch.cuh -- programmatic dependent launches: a kernel launched with launch_pdl may be
+// scheduled while the kernel before it on the stream still runs, and waits in pdl_wait()
+// until that one has completed and its writes are visible.  What is saved is the launch
+// latency between two short kernels.
+#pragma once
+
+#include <cstdint>
+#include <cuda_runtime.h>
+
+namespace sloth {
+
+// Waits for the kernels this one depends on (returns at once after an ordinary launch).
+// Every kernel launched with launch_pdl calls it before its first access to global memory,
+// so that "the kernel before" always covers everything before that one too.  The zero it
+// returns is added to the indices of the loads that follow: read-only loads (__ldg) are not
+// ordered by the memory clobber, and this makes their addresses depend on the wait.
+__device__ __forceinline__ uint32_t pdl_wait()
+{
+    uint32_t zero;
+    asm volatile("griddepcontrol.wait;\nmov.u32 %0, 0;" : "=r"(zero)::"memory");
+    return zero;
+}
+
+// Lets the dependents of this kernel be scheduled once every block has called it or left.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... K, class... A>
+cudaError_t launch_pdl(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+
+}  // namespace sloth

@@ -14,9 +14,10 @@
 //
 // Scratch layout (byte offsets into g_noalloc_scratch):
 //   records   kMaxTri x 96 B          per-triangle setup records
-//   rows      kMaxTri x 4 B           per-triangle packed sample rows (setup -> newline)
+//   (free)    kMaxTri x 4 B           unused, as are the tile counts below: the header states
+//                                     the array's size
 //   keys      kMaxCells x 8 B         depth keys (tiles padded to 64x32 cells)
-//   bins      tile counts/offsets/cursors, the large-triangle queue and its counter
+//   queue     kMaxTri x 4 B + 8 B     triangles too large for their block, and two counters
 //   tile_gen  kMaxTiles x 4 B         tile generations (cleared every call)
 //   nltree    2*kMaxNl x 4 B          newline segment tree (cleared every call)
 //   frags     8 B                     fragment counter (cleared every call)
@@ -53,75 +54,6 @@ static_assert(kScratchBytes == SLOTH_NOALLOC_SCRATCH_BYTES, "header states the s
 // device symbol; its device address comes from cudaGetSymbolAddress (scratch_on()), with
 // the device the caller made current.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
-
-// Raster variant without binning: one CTA per tile tests every triangle of the draw
-// against the tile (the soup is bounded by kMaxTri) and folds covered samples' depth
-// keys into a shared-memory tile with the same 64-bit atomicMin as raster_kernel.
-__global__ void __launch_bounds__(256)
-noalloc_raster_kernel(uint32_t ntri, FrameGeom g, FrameBuffers fb)
-{
-    constexpr int TW = kTileW, TH = kTileH;
-    __shared__ unsigned long long skeys[TH * TW];
-    __shared__ uint32_t s_next, s_frags[8];
-    const int tile = blockIdx.x;
-    const int tr = tile / g.ntx, tc = tile - tr * g.ntx;
-    const int R0 = tr * TH, C0 = tc * TW;
-    for (int i = threadIdx.x; i < TH * TW; i += blockDim.x) skeys[i] = kEmptyKey;
-    if (threadIdx.x == 0) s_next = 0;
-    block_sync();
-    const int lane = threadIdx.x & 31;
-    const Viewport vp{g.w, g.h, g.image, g.tw, g.th, g.ntx, g.nty, g.pitch};
-    uint32_t frags = 0;
-    for (;;) {
-        uint32_t t = 0;
-        if (lane == 0) t = atomicAdd(&s_next, 1u);
-        t = __shfl_sync(0xffffffffu, t, 0);
-        if (t >= ntri) break;
-        const TriRecord r = fb.records[t];
-        const Rect U = unwrapped_part(vp, r.x0, r.xe, r.y0, r.y1);
-        const Rect W = wrapped_part(vp, r.x0, r.xe, r.y0, r.y1);
-        const Rect cu = U.empty() ? Rect{0, 0, 0, 0} : clip_unwrapped(vp, U, tr, tc);
-        const Rect cw = W.empty() ? Rect{0, 0, 0, 0} : clip_wrapped(vp, W, tr, tc);
-        const bool exact = (r.flags & kFlagFiniteXY) != 0;
-        for (int part = 0; part < 2; ++part) {
-            const Rect c = part == 0 ? cu : cw;
-            if (c.empty() || (exact && !rect_may_cover(r, c))) continue;
-            const int bw = c.xb - c.xa, area = bw * (c.yb - c.ya);
-            for (int k = lane; k < area; k += 32) {
-                const int x = c.xa + k % bw, y = c.ya + k / bw;
-                const EdgeVals e = eval_edges(r, (float)x, (float)y);
-                if (e.w0 >= 0.0f && e.w1 >= 0.0f && e.w2 >= 0.0f) {
-                    ++frags;
-                    const float z = interp_z(r.v1z, r.dz2, r.dz3, r.a, e.w1, e.w2);
-                    if (z < kFltMax) {
-                        const uint32_t nw = part == 0 ? 1u : 0u;
-                        const unsigned long long key = make_key(z, t, nw);
-                        const int row = nw ? (y - R0) : (y + 1 - R0);
-                        const int col = nw ? (2 * x - C0) : (2 * x - g.w - C0);
-                        unsigned long long *p = &skeys[row * TW + key_col(col, TW)];
-                        if (key < *(volatile unsigned long long *)p) atomicMin(p, key);
-                    }
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) frags += __shfl_xor_sync(0xffffffffu, frags, d);
-    if (lane == 0) s_frags[threadIdx.x >> 5] = frags;
-    block_sync();
-    unsigned long long *gk = reinterpret_cast<unsigned long long *>(fb.keys) + (size_t)R0 * g.pitch + C0;
-    // shared and global keys share the layout (key_col): slot i of tile row rr is slot i globally
-    for (int i = threadIdx.x; i < TH * TW; i += blockDim.x) {
-        const int rr = i / TW, cc = i - rr * TW;
-        gk[(size_t)rr * g.pitch + cc] = skeys[i];
-    }
-    if (threadIdx.x == 0) {
-        uint32_t tot = 0;
-        for (int k = 0; k < 8; ++k) tot += s_frags[k];
-        atomicAdd(fb.fragments, (unsigned long long)tot);
-        fb.tile_gen[tile] = fb.gen;
-    }
-}
 
 namespace {
 
@@ -166,7 +98,6 @@ extern "C" sloth_status sloth_render_noalloc(const float *x, const float *y, con
     while (g.nl_size < g.h) g.nl_size <<= 1;
     const uint64_t padded = (uint64_t)g.pitch * g.nty * g.th;
     if (padded > kMaxCells) return SLOTH_ERR_LIMIT;
-    const uint32_t ntiles = (uint32_t)(g.ntx * g.nty);
 
     unsigned char *base = nullptr;
     if (scratch_on(&base) != cudaSuccess) return SLOTH_ERR_CUDA;
@@ -174,7 +105,6 @@ extern "C" sloth_status sloth_render_noalloc(const float *x, const float *y, con
 
     FrameBuffers fb{};
     fb.records = reinterpret_cast<TriRecord *>(base + kOffRecords);
-    fb.rows = reinterpret_cast<uint32_t *>(base + kOffRows);
     fb.keys = reinterpret_cast<uint64_t *>(base + kOffKeys);
     fb.tile_gen = reinterpret_cast<uint32_t *>(base + kOffGen);
     fb.nltree = reinterpret_cast<int32_t *>(base + kOffNl);
@@ -183,33 +113,17 @@ extern "C" sloth_status sloth_render_noalloc(const float *x, const float *y, con
     fb.cells_out = cells;
     fb.winner_out = winner;
     fb.gen = 1;
-    BinBuffers bb{};
-    bb.tile_count = reinterpret_cast<uint32_t *>(base + kOffCount);
-    bb.tile_offset = reinterpret_cast<uint32_t *>(base + kOffOffset);
-    bb.tile_cursor = reinterpret_cast<uint32_t *>(base + kOffCursor);
-    bb.large_queue = reinterpret_cast<uint32_t *>(base + kOffQueue);
-    bb.large_count = reinterpret_cast<uint32_t *>(base + kOffQCount);
-    bb.large_cap = kMaxTri;
-    bb.entries = nullptr;
-    bb.capacity = 0;
-
-    // The array keeps the previous call's contents: reset what must start empty.
-    cudaError_t e;
-    if ((e = cudaMemsetAsync(fb.tile_gen, 0, ntiles * sizeof(uint32_t), s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(fb.nltree, 0xff, 2 * (size_t)g.nl_size * sizeof(int32_t), s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(fb.fragments, 0, sizeof(unsigned long long), s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(bb.tile_count, 0, ntiles * sizeof(uint32_t), s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(bb.large_count, 0, 2 * sizeof(uint32_t), s)) != cudaSuccess)
-        return SLOTH_ERR_CUDA;
+    // The array keeps the previous call's contents: every tile's keys and the frame's
+    // counters are reset first.  The draw goes without tiles (fold.cuh): a raster of one CTA
+    // per tile over the whole soup took 1323 us for 20,000 triangles at 640x360, all of it
+    // record loads of triangles that miss the tile; this takes 53 us.
+    uint32_t *queue = reinterpret_cast<uint32_t *>(base + kOffQueue);
+    uint32_t *queue_counts = reinterpret_cast<uint32_t *>(base + kOffQCount);
+    if (launch_fold_begin(g, fb, true, true, queue_counts, s) != cudaSuccess) return SLOTH_ERR_CUDA;
     Mat4 M;
     for (int i = 0; i < 16; ++i) M.m[i] = m[i];
-    MeshDev md{x, y, z, nullptr, rgb, 3 * ntri, ntri};
-    if (launch_setup(md, nullptr, M, 0, g, fb, bb, s) != cudaSuccess) return SLOTH_ERR_CUDA;
-    if (launch_newline(ntri, nullptr, 0, g, fb, s) != cudaSuccess) return SLOTH_ERR_CUDA;
-    if (ntri) {
-        noalloc_raster_kernel<<<ntiles, 256, 0, s>>>(ntri, g, fb);
-        if (cudaGetLastError() != cudaSuccess) return SLOTH_ERR_CUDA;
-    }
+    const MeshDev md{x, y, z, nullptr, rgb, 3 * ntri, ntri};
+    if (launch_fold_draw(md, M, 0, g, fb, queue, queue_counts, 0, s) != cudaSuccess) return SLOTH_ERR_CUDA;
     if (launch_resolve(g, fb, s) != cudaSuccess) return SLOTH_ERR_CUDA;
     return SLOTH_OK;
 }
