@@ -53,11 +53,12 @@ fold_large_kernel(FrameGeom g, FrameBuffers fb, FoldQueue queue, uint32_t *next)
     pdl_trigger();
     const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x + pdl_wait()) >> 5;
     if (blockIdx.x == 0 && threadIdx.x == 0) *next = 0u;
-    const uint32_t items = *queue.count * kFoldParts;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t queued = *queue.count, nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t parts = fold_parts(queued, nwarps), items = queued * parts;
+    const bool filter = queued > kFoldFilterMin;
     uint32_t frags = 0;
     for (uint32_t it = first; it < items; it += nwarps)
-        frags += fold_large_part(queue.tri[it / kFoldParts], it % kFoldParts, g, fb);
+        frags += fold_large_part(queue.tri[it / parts], it % parts, parts, filter, g, fb);
     add_frags_warp(frags, fb.fragments);
 }
 
@@ -78,7 +79,7 @@ cudaError_t launch_fold_draw(const MeshDev &mesh, const Mat4 &M, uint32_t tri_ba
     cudaError_t e = launch_pdl(fold_setup_kernel<4>, dim3(blocks), dim3(128), kFoldSmemBytes, s, mesh, M, tri_base, g,
                                fb, q);
     if (e != cudaSuccess) return e;
-    return launch_pdl(fold_large_kernel, dim3(2u * (unsigned)device_sm_count()), dim3(256), 0, s, g, fb, q,
+    return launch_pdl(fold_large_kernel, dim3(4u * (unsigned)device_sm_count()), dim3(256), 0, s, g, fb, q,
                       queue_counts + (parity ^ 1));
 }
 

@@ -25,10 +25,20 @@ constexpr int kFoldTris = 32;
 // that set one up would walk it alone while the rest of the GPU is idle.  1024 samples are
 // eight steps of a block of four warps.
 constexpr uint32_t kFoldQueueSamples = 1024;
-// A queued triangle is kFoldParts warp items; item i takes the groups of kFoldRows rows
-// i, i + kFoldParts, ... (a frame of 360 rows gives each item at most three groups).
-constexpr uint32_t kFoldParts = 16;
+// A queued triangle is `parts` warp items; item i takes the groups of kFoldRows rows i,
+// i + parts, ...  A few queued triangles are cut finely enough to occupy every warp of the
+// grid (64 parts: one group each up to 512 rows), many of them coarsely, so that the items
+// past a triangle's last row stay few (20,000 triangles at 640x360, 40 of them queued: 32 us
+// in 16 parts with the filter below, 15 us as here).
 constexpr int kFoldRows = 8;
+__device__ __forceinline__ uint32_t fold_parts(uint32_t queued, uint32_t nwarps)
+{
+    return min(64u, max(8u, nwarps / max(queued, 1u)));
+}
+// With more queued triangles than this, cells that already hold a nearer key are left out
+// before the reduction (they may overdraw each other many times); with fewer, the load
+// would only lengthen each step.
+constexpr uint32_t kFoldFilterMin = 512;
 
 // Dynamic shared memory of a fold block: one direct stage and the samples' running ends.
 constexpr size_t kFoldSmemBytes = (kDirectStageWords + 32) * 4;
@@ -152,11 +162,11 @@ __device__ __forceinline__ void fold_row_span(float dx, float dy, float ax, floa
 
 // Warp item `part` of a queued triangle: its groups of rows, each row cut to the columns
 // that can pass all three edges, the spans of a group walked 32 samples at a time with the
-// exact test for every sample.  A covered sample whose cell already holds a nearer key is
-// dropped before the reduction: the plain load may be older than the key in L2, and keys
+// exact test for every sample.  With filter, a covered sample whose cell already holds a
+// nearer key is dropped before the reduction: the plain load may be older than the key in L2, and keys
 // only fall, so it can only keep a sample that was not needed.
-__device__ __forceinline__ uint32_t fold_large_part(uint32_t gtri, uint32_t part, const FrameGeom &g,
-                                                    const FrameBuffers &fb)
+__device__ __forceinline__ uint32_t fold_large_part(uint32_t gtri, uint32_t part, uint32_t parts, bool filter,
+                                                    const FrameGeom &g, const FrameBuffers &fb)
 {
     const int lane = threadIdx.x & 31;
     const float4 *rp = reinterpret_cast<const float4 *>(fb.records + gtri);
@@ -176,7 +186,7 @@ __device__ __forceinline__ uint32_t fold_large_part(uint32_t gtri, uint32_t part
                         fabsf(r.v3x) < big && fabsf(r.v3y) < big;
     unsigned long long *keys = reinterpret_cast<unsigned long long *>(fb.keys);
     uint32_t frags = 0;
-    for (int ya = xr.z + (int)part * kFoldRows; ya < xr.w; ya += (int)(kFoldParts * kFoldRows)) {
+    for (int ya = xr.z + (int)part * kFoldRows; ya < xr.w; ya += (int)parts * kFoldRows) {
         int lo = xr.x, hi = lane < kFoldRows && ya + lane < xr.w ? x1 : xr.x;
         if (finite) {
             const float py = (float)(ya + lane);
@@ -209,7 +219,7 @@ __device__ __forceinline__ uint32_t fold_large_part(uint32_t gtri, uint32_t part
                     unsigned long long *kp = keys + (size_t)(nw ? y : y + 1) * g.pitch +
                                              key_col(nw ? 2 * x : 2 * x - g.w, g.tw);
                     const unsigned long long key = make_key(z, gtri, nw);
-                    if (key < *kp) red_min_u64(kp, key);
+                    if (!filter || key < *kp) red_min_u64(kp, key);
                 }
             }
         }
