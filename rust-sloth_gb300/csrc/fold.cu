@@ -17,7 +17,7 @@ fold_begin_kernel(FrameGeom g, FrameBuffers fb, uint32_t nl_nodes, int frame, in
     if (frame)
         for (uint32_t i = t * blockDim.x + threadIdx.x; i < nl_nodes; i += gridDim.x * blockDim.x) fb.nltree[i] = -1;
     if (t == 0 && threadIdx.x == 0) {
-        queue_counts[0] = queue_counts[1] = 0u;
+        queue_counts[0] = queue_counts[1] = queue_counts[2] = queue_counts[3] = 0u;
         if (frame) {
             if (fb.error) *fb.error = 0u;
             *fb.fragments = 0ull;
@@ -45,20 +45,22 @@ fold_setup_kernel(MeshDev mesh, Mat4 M, uint32_t tri_base, FrameGeom g, FrameBuf
     fold_triangles<kWarps>(mesh, M, blockIdx.x * kFoldTris + pdl_wait(), tri_base, g, fb, queue, 0u);
 }
 
-// The queued triangles' items over the warps of the grid.  next: the counter the frame's
-// next draw queues with, emptied here (the draw after that reuses this one's).
+// The queued triangles' items over the warps of the grid, the large ones' first.  next: the
+// counters the frame's next draw queues with, emptied here (the draw after that reuses
+// this one's).
 __global__ void __launch_bounds__(256)
 fold_large_kernel(FrameGeom g, FrameBuffers fb, FoldQueue queue, uint32_t *next)
 {
     pdl_trigger();
     const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x + pdl_wait()) >> 5;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *next = 0u;
-    const uint32_t queued = *queue.count, nwarps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t parts = fold_parts(queued, nwarps), items = queued * parts;
-    const bool filter = queued > kFoldFilterMin;
+    if (blockIdx.x == 0 && threadIdx.x < 2) next[threadIdx.x] = 0u;
+    const uint32_t large = queue.count[0], mid = queue.count[1], nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t parts = fold_parts(large, nwarps), cut = large * parts, items = cut + mid;
+    const bool filter = large + mid > kFoldFilterMin;
     uint32_t frags = 0;
     for (uint32_t it = first; it < items; it += nwarps)
-        frags += fold_large_part(queue.tri[it / parts], it % parts, parts, filter, g, fb);
+        frags += it < cut ? fold_queued<kFoldRows>(queue.tri[it / parts], it % parts, parts, filter, g, fb)
+                          : fold_queued<32>(queue.tri[queue.cap - 1u - (it - cut)], 0u, 1u, filter, g, fb);
     add_frags_warp(frags, fb.fragments);
 }
 
@@ -69,18 +71,22 @@ cudaError_t launch_fold_begin(const FrameGeom &g, const FrameBuffers &fb, bool f
                       2u * (uint32_t)g.nl_size, frame ? 1 : 0, all ? 1 : 0, queue_counts);
 }
 
-cudaError_t launch_fold_draw(const MeshDev &mesh, const Mat4 &M, uint32_t tri_base, const FrameGeom &g,
-                             const FrameBuffers &fb, uint32_t *queue, uint32_t *queue_counts, int parity,
-                             cudaStream_t s)
+cudaError_t launch_fold_setup(const MeshDev &mesh, const Mat4 &M, uint32_t tri_base, const FrameGeom &g,
+                              const FrameBuffers &fb, uint32_t *queue, uint32_t cap, uint32_t *queue_counts,
+                              int parity, cudaStream_t s)
 {
     if (mesh.ntri == 0) return cudaSuccess;
-    const FoldQueue q{queue, nullptr, queue_counts + parity};
+    const FoldQueue q{queue, nullptr, queue_counts + 2 * parity, cap};
     const uint32_t blocks = (mesh.ntri + kFoldTris - 1) / kFoldTris;
-    cudaError_t e = launch_pdl(fold_setup_kernel<4>, dim3(blocks), dim3(128), kFoldSmemBytes, s, mesh, M, tri_base, g,
-                               fb, q);
-    if (e != cudaSuccess) return e;
+    return launch_pdl(fold_setup_kernel<4>, dim3(blocks), dim3(128), kFoldSmemBytes, s, mesh, M, tri_base, g, fb, q);
+}
+
+cudaError_t launch_fold_large(const FrameGeom &g, const FrameBuffers &fb, uint32_t *queue, uint32_t cap,
+                              uint32_t *queue_counts, int parity, cudaStream_t s)
+{
+    const FoldQueue q{queue, nullptr, queue_counts + 2 * parity, cap};
     return launch_pdl(fold_large_kernel, dim3(4u * (unsigned)device_sm_count()), dim3(256), 0, s, g, fb, q,
-                      queue_counts + (parity ^ 1));
+                      queue_counts + 2 * (parity ^ 1));
 }
 
 }  // namespace sloth

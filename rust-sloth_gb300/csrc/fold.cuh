@@ -22,18 +22,17 @@ namespace sloth {
 // Triangles a block sets up (one per lane of its first warp).
 constexpr int kFoldTris = 32;
 // Triangles of more samples than this (rows times walked columns) are queued: the block
-// that set one up would walk it alone while the rest of the GPU is idle.  1024 samples are
-// eight steps of a block of four warps.
-constexpr uint32_t kFoldQueueSamples = 1024;
-// A queued triangle is `parts` warp items; item i takes the groups of kFoldRows rows i,
-// i + parts, ...  A few queued triangles are cut finely enough to occupy every warp of the
-// grid (64 parts: one group each up to 512 rows), many of them coarsely, so that the items
-// past a triangle's last row stay few (20,000 triangles at 640x360, 40 of them queued: 32 us
-// in 16 parts with the filter below, 15 us as here).
+// that set one up would walk it alone while the rest of the GPU is idle.
+constexpr uint32_t kFoldBlockSamples = 128;
+// Of the queued ones, those of at most this many samples are one warp item each, 32 rows at
+// a time; larger ones are cut into `parts` items of every parts-th group of kFoldRows rows.
+// Few large triangles are cut finely, so that they occupy every warp of the grid, many
+// coarsely, so that the items past a triangle's last row stay few.
+constexpr uint32_t kFoldWarpSamples = 4096;
 constexpr int kFoldRows = 8;
-__device__ __forceinline__ uint32_t fold_parts(uint32_t queued, uint32_t nwarps)
+__device__ __forceinline__ uint32_t fold_parts(uint32_t large, uint32_t nwarps)
 {
-    return min(64u, max(8u, nwarps / max(queued, 1u)));
+    return min(256u, max(16u, 2u * nwarps / max(large, 1u)));
 }
 // With more queued triangles than this, cells that already hold a nearer key are left out
 // before the reduction (they may overdraw each other many times); with fewer, the load
@@ -43,12 +42,34 @@ constexpr uint32_t kFoldFilterMin = 512;
 // Dynamic shared memory of a fold block: one direct stage and the samples' running ends.
 constexpr size_t kFoldSmemBytes = (kDirectStageWords + 32) * 4;
 
-// Triangles too large for their block: draw index and frame (batches; null otherwise).
+// Triangles too large for their block: draw index and frame (batches; null otherwise), the
+// large ones from the front of the cap entries, the others from the back; count[0] and
+// count[1] are their numbers.
 struct FoldQueue {
     uint32_t *tri;
     uint32_t *frame;
     uint32_t *count;
+    uint32_t cap;
 };
+
+// Queue slot of a lane's triangle (called by all 32 lanes; -1 for lanes without one).
+__device__ __forceinline__ int fold_queue_slot(const FoldQueue &q, bool mid, bool large)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned ml = __ballot_sync(0xffffffffu, large), mm = __ballot_sync(0xffffffffu, mid);
+    if (!(ml | mm)) return -1;
+    uint32_t l0 = 0, m0 = 0;
+    if (lane == 0) {
+        if (ml) l0 = atomicAdd(&q.count[0], (uint32_t)__popc(ml));
+        if (mm) m0 = atomicAdd(&q.count[1], (uint32_t)__popc(mm));
+    }
+    l0 = __shfl_sync(0xffffffffu, l0, 0);
+    m0 = __shfl_sync(0xffffffffu, m0, 0);
+    const unsigned lt = (1u << lane) - 1u;
+    if (large) return (int)(l0 + __popc(ml & lt));
+    if (mid) return (int)(q.cap - 1u - (m0 + __popc(mm & lt)));
+    return -1;
+}
 
 // Newline rows [y0, y1) of draw index v into the frame's tree (nltree_update with
 // reductions, which return nothing to wait for).
@@ -78,7 +99,7 @@ __device__ __forceinline__ void fold_triangles(const MeshDev &mesh, const Mat4 &
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (wid == 0) {
         const uint32_t p = p0 + lane;
-        bool mine = false, big = false;
+        bool mine = false, mid = false, large = false;
         uint32_t gtri = 0;
         int n = 0;
         DirectWalk dw{false, 0, 0u};
@@ -100,22 +121,18 @@ __device__ __forceinline__ void fold_triangles(const MeshDev &mesh, const Mat4 &
                     // a triangle the direct walk does not size (none of dy > 0, non-finite, or
                     // more than 2^31 samples) is left to the row walk
                     const uint64_t walked = (uint64_t)(r.xe + 1 - r.x0) * (uint32_t)(r.y1 - r.y0);
-                    big = !dw.direct || walked > kFoldQueueSamples;
-                    mine = !big;
+                    mine = dw.direct && walked <= kFoldBlockSamples;
+                    mid = !mine && walked <= kFoldWarpSamples;
+                    large = !mine && !mid;
                     store_record(fb.records + gtri, r, 1u, true);
                 }
             }
         }
         if (mine) n = direct_stage(true, r, gtri, dw.xend, dw.exit_mask, 0u);
-        const unsigned bm = __ballot_sync(0xffffffffu, big);
-        if (bm) {
-            uint32_t q0 = 0;
-            if (lane == 0) q0 = atomicAdd(queue.count, (uint32_t)__popc(bm));
-            q0 = __shfl_sync(0xffffffffu, q0, 0) + __popc(bm & ((1u << lane) - 1u));
-            if (big) {
-                queue.tri[q0] = gtri;
-                if (queue.frame) queue.frame[q0] = frame;
-            }
+        const int q = fold_queue_slot(queue, mid, large);
+        if (q >= 0) {
+            queue.tri[q] = gtri;
+            if (queue.frame) queue.frame[q] = frame;
         }
         int end = n;
 #pragma unroll
@@ -160,18 +177,20 @@ __device__ __forceinline__ void fold_row_span(float dx, float dy, float ax, floa
     }
 }
 
-// Warp item `part` of a queued triangle: its groups of rows, each row cut to the columns
-// that can pass all three edges, the spans of a group walked 32 samples at a time with the
-// exact test for every sample.  With filter, a covered sample whose cell already holds a
-// nearer key is dropped before the reduction: the plain load may be older than the key in L2, and keys
-// only fall, so it can only keep a sample that was not needed.
-__device__ __forceinline__ uint32_t fold_large_part(uint32_t gtri, uint32_t part, uint32_t parts, bool filter,
-                                                    const FrameGeom &g, const FrameBuffers &fb)
+// One warp's share of a queued triangle: the groups of kRows rows part, part + parts, ...,
+// each row cut to the columns that can pass all three edges, the spans of a group walked 32
+// samples at a time with the exact test for every sample.  With filter, a covered sample
+// whose cell already holds a nearer key is dropped before the reduction: the plain load may
+// be older than the key in L2, and keys only fall, so it can only keep a sample that was not
+// needed.
+template <int kRows>
+__device__ __forceinline__ uint32_t fold_queued(uint32_t gtri, uint32_t part, uint32_t parts, bool filter,
+                                                const FrameGeom &g, const FrameBuffers &fb)
 {
     const int lane = threadIdx.x & 31;
     const float4 *rp = reinterpret_cast<const float4 *>(fb.records + gtri);
     const int4 xr = *(reinterpret_cast<const int4 *>(rp) + 4);
-    if (xr.z + (int)part * kFoldRows >= xr.w) return 0;
+    if (xr.z + (int)part * kRows >= xr.w) return 0;
     const float4 q0 = rp[0], q1 = rp[1], q5 = rp[5];
     TriRecord r;
     r.v1x = q0.x; r.v1y = q0.y; r.v2x = q0.z; r.v2y = q0.w; r.v3x = q1.x; r.v3y = q1.y;
@@ -186,8 +205,8 @@ __device__ __forceinline__ uint32_t fold_large_part(uint32_t gtri, uint32_t part
                         fabsf(r.v3x) < big && fabsf(r.v3y) < big;
     unsigned long long *keys = reinterpret_cast<unsigned long long *>(fb.keys);
     uint32_t frags = 0;
-    for (int ya = xr.z + (int)part * kFoldRows; ya < xr.w; ya += (int)parts * kFoldRows) {
-        int lo = xr.x, hi = lane < kFoldRows && ya + lane < xr.w ? x1 : xr.x;
+    for (int ya = xr.z + (int)part * kRows; ya < xr.w; ya += (int)parts * kRows) {
+        int lo = xr.x, hi = lane < kRows && ya + lane < xr.w ? x1 : xr.x;
         if (finite) {
             const float py = (float)(ya + lane);
             fold_row_span(r.dx0, r.dy0, r.v2x, r.v2y, py, lo, hi);
@@ -197,16 +216,16 @@ __device__ __forceinline__ uint32_t fold_large_part(uint32_t gtri, uint32_t part
         const int len = max(hi - lo, 0);
         int end = len;
 #pragma unroll
-        for (int d = 1; d < kFoldRows; d <<= 1) {
+        for (int d = 1; d < kRows; d <<= 1) {
             const int o = __shfl_up_sync(0xffffffffu, end, d);
             if (lane >= d) end += o;
         }
-        const int total = __shfl_sync(0xffffffffu, end, kFoldRows - 1), xoff = lo - (end - len);
+        const int total = __shfl_sync(0xffffffffu, end, kRows - 1), xoff = lo - (end - len);
         for (int base = 0; base < total; base += 32) {
             const int k = base + lane;
             int row = 0;   // the rows whose spans end at or before k
 #pragma unroll
-            for (int step = kFoldRows / 2; step > 0; step >>= 1)
+            for (int step = kRows / 2; step > 0; step >>= 1)
                 if (__shfl_sync(0xffffffffu, end, row + step - 1) <= k) row += step;
             const int x = k + __shfl_sync(0xffffffffu, xoff, row), y = ya + row;
             if (k >= total) continue;

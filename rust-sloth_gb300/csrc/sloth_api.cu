@@ -51,6 +51,7 @@ struct sloth_mesh {
     uint32_t nvert = 0, ntri = 0;
     float bbox_max[3] = {0, 0, 0};
     uint32_t *order = nullptr, *oidx = nullptr;   // setup's order of an indexed mesh (spatial_order)
+    float span2 = 0.0f;   // sum over the triangles of their longest edge squared, when made (mesh_span2)
 };
 
 struct sloth_ctx {
@@ -100,6 +101,8 @@ struct sloth_ctx {
     int direct_max = 0;            // SLOTH_OPTION_DIRECT_SAMPLES (applied at the next clear)
     int tpb = kDefaultTrianglesPerBlock;   // SLOTH_OPTION_TRIANGLES_PER_BLOCK
     bool keys_current = false;     // every tile's keys cleared for the current generation
+    uint32_t *fold_counts = nullptr;   // queue counters of the draws without tiles (launch_fold_setup)
+    int fold_parity = 0;               // the counter the frame's next such draw uses
     bool timing = false;
     std::map<std::string, KernelClock> clocks;
     uint64_t launches = 0;
@@ -535,6 +538,7 @@ void sloth_ctx_destroy(sloth_ctx *ctx)
     dfree(ctx->bb.large_queue);
     dfree(ctx->bb.fill_list);
     dfree(ctx->bb.large_count);
+    dfree(ctx->fold_counts);
     dfree(ctx->bb.items);
     dfree(ctx->tv);
     if (ctx->h_total) cudaFreeHost(ctx->h_total);
@@ -808,6 +812,27 @@ static void spatial_order(const float *x, const float *y, const float *z, const 
     order.swap(src);
 }
 
+// Sum over the triangles of the longest edge squared, from at most 4096 of them spread over
+// the mesh: what draws_without_tiles estimates a draw's samples from.
+static float mesh_span2(const float *x, const float *y, const float *z, const uint32_t *idx, uint32_t ntri)
+{
+    const uint32_t step = ntri / 4096 + 1;
+    double sum = 0.0;
+    uint32_t n = 0;
+    for (uint64_t t = 0; t < ntri; t += step, ++n) {
+        uint64_t v[3];
+        for (int k = 0; k < 3; ++k) v[k] = idx ? idx[3 * t + k] : 3 * t + k;
+        double e2 = 0.0;
+        for (int k = 0; k < 3; ++k) {
+            const uint64_t a = v[k], b = v[(k + 1) % 3];
+            const double dx = (double)x[a] - x[b], dy = (double)y[a] - y[b], dz = (double)z[a] - z[b];
+            e2 = std::fmax(e2, dx * dx + dy * dy + dz * dz);
+        }
+        if (std::isfinite(e2)) sum += e2;
+    }
+    return n ? (float)(sum * ((double)ntri / n)) : 0.0f;
+}
+
 sloth_status sloth_spatial_order(const float *x, const float *y, const float *z, uint32_t nvert, const uint32_t *idx,
                                  uint32_t ntri, uint32_t *order)
 {
@@ -847,6 +872,7 @@ sloth_status sloth_mesh_create(sloth_ctx *ctx, const float *x, const float *y, c
     m->device = ctx->device;
     m->nvert = nvert;
     m->ntri = ntri;
+    m->span2 = mesh_span2(x, y, z, idx, ntri);
     auto cleanup = [&](sloth_status st) {
         sloth_mesh_destroy(m);
         return st;
@@ -975,6 +1001,60 @@ static sloth_status poll_entry_max(sloth_ctx *ctx)
     return SLOTH_OK;
 }
 
+// Whether a draw goes without tiles (fold.cuh).  The samples it will walk are estimated
+// from the mesh's edges as it was made and the matrix's scale; a mesh of no extent says
+// nothing.  Up to kFoldMaxSamples the tile raster's launches cost more than its culling
+// saves (us a frame, tiles / fold: 960 triangles at 160x48, 3e4 samples, 68 / 15; 82k at
+// 640x360, 8e5, 84 / 28; 5k at 1920x1080, 7e6, 78 / 35; 8k with 16 large ones at 1920x1080,
+// 1.5e7, 88 / 108; 32k at 1920x1080, 6e7, 104 / 119; at 640x360 the fold stays ahead up to
+// 1.5e8).  Above kFoldMaxTriangles the estimate is not trusted with the whole draw
+// (positions may have been updated since), and the tiles bound what a wrong one costs.
+// With culling off a caller counts or compares the tile raster's fragments, and the wait
+// test needs its tile loads: both keep it.
+constexpr uint32_t kFoldMaxTriangles = 131072;
+constexpr float kFoldMaxSamples = 1e7f;
+static bool draws_without_tiles(const sloth_ctx *ctx, const sloth_mesh *mesh, const Mat4 &M)
+{
+    if (!ctx->depth_cull || ctx->fb.wait_test || mesh->ntri > kFoldMaxTriangles || !(mesh->span2 > 0.0f)) return false;
+    const float *m = M.m;
+    const float sx = std::sqrt(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
+    const float sy = std::sqrt(m[4] * m[4] + m[5] * m[5] + m[6] * m[6]);
+    const float cells = (float)ctx->g.w * (float)ctx->g.h;
+    return std::fmin(mesh->span2 * sx * sy, (float)mesh->ntri * cells) <= kFoldMaxSamples;   // false for NaN
+}
+
+// One draw without tiles: every tile's keys made current first (once a frame).
+static sloth_status draw_folded(sloth_ctx *ctx, const sloth_mesh *mesh, const Mat4 &M)
+{
+    sloth_status st;
+    cudaStream_t s = ctx->stream;
+    if (!ctx->fold_counts) CU(ctx, dalloc(&ctx->fold_counts, 4));
+    if (ctx->reset_pending || !ctx->keys_current) {
+        if ((st = join_newline(ctx)) != SLOTH_OK) return st;   // the last frame's fold into the tree
+        const bool frame = ctx->reset_pending;
+        CU(ctx, timed(ctx, "reset", [&] {
+               return launch_fold_begin(ctx->g, ctx->fb, frame, false, ctx->fold_counts, s);
+           }));
+        ctx->reset_pending = false;
+        ctx->keys_current = true;
+        ctx->fold_parity = 0;
+    }
+    const MeshDev md{mesh->x, mesh->y, mesh->z, mesh->idx, mesh->rgb, mesh->nvert, mesh->ntri, mesh->order, mesh->oidx};
+    const int parity = ctx->fold_parity;
+    const uint32_t cap = (uint32_t)std::min<size_t>(ctx->large_cap, 0x7fffffffu);
+    CU(ctx, timed(ctx, "fold", [&] {
+           return launch_fold_setup(md, M, ctx->tri_base, ctx->g, ctx->fb, ctx->bb.large_queue, cap, ctx->fold_counts, parity,
+                                    s);
+       }));
+    CU(ctx, timed(ctx, "fold_large", [&] {
+           return launch_fold_large(ctx->g, ctx->fb, ctx->bb.large_queue, cap, ctx->fold_counts, parity, s);
+       }));
+    ctx->fold_parity ^= 1;
+    ctx->tri_base += mesh->ntri;
+    ctx->dirty = true;
+    return SLOTH_OK;
+}
+
 sloth_status sloth_draw_mesh(sloth_ctx *ctx, const sloth_mesh *mesh, const float transform[16])
 {
     if (!ctx) return SLOTH_ERR_INVALID_ARGUMENT;
@@ -986,6 +1066,13 @@ sloth_status sloth_draw_mesh(sloth_ctx *ctx, const sloth_mesh *mesh, const float
         return fail(ctx, SLOTH_ERR_LIMIT, "more than %u triangles since the last clear", SLOTH_MAX_TRIANGLES);
     CU(ctx, cudaSetDevice(ctx->device));
     sloth_status st;
+    Mat4 M;
+    sloth_mat4_mul(ctx->U, transform, M.m);
+    if (draws_without_tiles(ctx, mesh, M)) {
+        if ((st = ensure_records(ctx, (size_t)ctx->tri_base + mesh->ntri)) != SLOTH_OK) return st;
+        if ((st = ensure_scratch(ctx, &ctx->bb.large_queue, &ctx->large_cap, mesh->ntri)) != SLOTH_OK) return st;
+        return draw_folded(ctx, mesh, M);
+    }
     if ((st = poll_entry_max(ctx)) != SLOTH_OK) return st;
     if ((st = ensure_records(ctx, (size_t)ctx->tri_base + mesh->ntri)) != SLOTH_OK) return st;
     if (mesh->idx && (st = ensure_scratch(ctx, &ctx->tv, &ctx->tv_cap, mesh->nvert)) != SLOTH_OK) return st;
@@ -994,8 +1081,6 @@ sloth_status sloth_draw_mesh(sloth_ctx *ctx, const sloth_mesh *mesh, const float
     if (!ctx->bb.large_count) CU(ctx, dalloc(&ctx->bb.large_count, 3));
     ctx->bb.large_cap = mesh->ntri;
 
-    Mat4 M;
-    sloth_mat4_mul(ctx->U, transform, M.m);
     MeshDev md{mesh->x, mesh->y, mesh->z, mesh->idx, mesh->rgb, mesh->nvert, mesh->ntri, mesh->order, mesh->oidx};
     const FrameGeom &g = ctx->g;
     const uint32_t ntiles = (uint32_t)(g.ntx * g.nty);

@@ -57,3 +57,53 @@ def test_noalloc_hostile(seed, w, h, image):
     R = O.euler_rotation(*W.cli_rotation(yaw=0.4 + seed))
     U = O.viewport_transform(w, h, O.scene_extent([m["bbox_max"]]))
     check(noalloc(m, O.mat4_mul(U, R), w, h, image), oracle_render([m], R, w, h, image, U=U), f"hostile {seed}")
+
+
+@pytest.mark.parametrize("w,h,image", [(160, 48, True), (161, 47, False)])
+def test_context_mixes_fold_and_tiles(w, h, image):
+    """Draws of one frame with and without tiles, in both orders, over frames and a resize:
+    each keeps the keys of the ones before it.  A draw goes without tiles by its estimated
+    samples, so the big soup (its triangles cover the frame) takes the tiles."""
+    small, ico = W.soup(100, seed=3, sigma=0.05), W.displaced_icosphere(2, seed=5)
+    big = W.soup(6000, seed=4, n_large=400, sigma=0.8)
+    R = O.euler_rotation(*W.cli_rotation(yaw=0.6, pitch=0.2))
+    with S.Context(0) as c:
+        dev = {id(m): S.Mesh(c, m["x"], m["y"], m["z"], m["rgb"], m["idx"], m["bbox_max"]) for m in (small, ico, big)}
+        for k, (order, scale) in enumerate([((small, big, ico), 40.0), ((big, small, ico, small), 40.0),
+                                            ((ico, ico, small), 1.0), ((small, big, big), 40.0)]):
+            ww, hh = (w, h) if k < 3 else (w + 64, h + 32)
+            U = O.viewport_transform(ww, hh, O.scene_extent([m["bbox_max"] for m in order]))
+            Rs = [R * np.float32(scale) if m is big else R for m in order]
+            c.set_viewport(ww, hh, image)
+            c.set_utransform(U)
+            c.clear()
+            for m, Rm in zip(order, Rs):
+                c.draw_mesh(dev[id(m)], Rm)
+            check([a.view(np.int32) if a.dtype == np.float32 else a for a in c.read()],
+                  oracle_render(list(order), Rs, ww, hh, image, U=U), f"mix {k} {ww}x{hh}")
+
+
+@pytest.mark.parametrize("side", [3, 60, 130])
+def test_context_fold_queue_classes(side):
+    """A grid of right triangles of `side` samples a side: walked by their block (up to 128
+    samples), by one warp (up to 4096) and by many; enough of them for the filter."""
+    rng = np.random.default_rng(side)
+    n = 700
+    c = rng.uniform([0, 0], [256, 200], (n, 2))
+    t = np.zeros((n, 3, 3), np.float32)
+    t[:, :, :2] = c[:, None, :] + np.array([[0, 0], [0, side], [side, 0]])
+    t[:, :, 2] = rng.uniform(-1, 1, (n, 3))
+    t[::3] = t[::3, ::-1]
+    v = t.reshape(-1, 3)
+    m = {"x": v[:, 0].copy(), "y": v[:, 1].copy(), "z": v[:, 2].copy(), "idx": None,
+         "rgb": rng.integers(0, 256, (n, 3), dtype=np.uint8), "bbox_max": np.ones(3, np.float32)}
+    eye = np.eye(4, dtype=np.float32)
+    with S.Context(0) as ctx:
+        dm = S.Mesh(ctx, m["x"], m["y"], m["z"], m["rgb"])
+        for w, h, image in ((512, 256, True), (513, 255, False)):
+            ctx.set_viewport(w, h, image)
+            ctx.set_utransform(eye)
+            ctx.clear()
+            ctx.draw_mesh(dm, eye)
+            check([a.view(np.int32) if a.dtype == np.float32 else a for a in ctx.read()],
+                  oracle_render([m], eye, w, h, image, U=eye), f"side {side} {w}x{h}")
