@@ -55,7 +55,7 @@ fold_large_kernel(FrameGeom g, FrameBuffers fb, FoldQueue queue, uint32_t *next)
     const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x + pdl_wait()) >> 5;
     if (blockIdx.x == 0 && threadIdx.x < 2) next[threadIdx.x] = 0u;
     const uint32_t large = queue.count[0], mid = queue.count[1], nwarps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t parts = fold_parts(large, nwarps), cut = large * parts, items = cut + mid;
+    const uint32_t parts = fold_parts(large), cut = large * parts, items = cut + mid;
     const bool filter = large + mid > kFoldFilterMin;
     uint32_t frags = 0;
     for (uint32_t it = first; it < items; it += nwarps)

@@ -24,16 +24,16 @@ constexpr int kFoldTris = 32;
 // Triangles of more samples than this (rows times walked columns) are queued: the block
 // that set one up would walk it alone while the rest of the GPU is idle.
 constexpr uint32_t kFoldBlockSamples = 128;
-// Of the queued ones, those of at most this many samples are one warp item each, 32 rows at
-// a time; larger ones are cut into `parts` items of every parts-th group of kFoldRows rows.
-// Few large triangles are cut finely, so that they occupy every warp of the grid, many
-// coarsely, so that the items past a triangle's last row stay few.
+// Of the queued ones, those of at most kFoldWarpSamples samples are one warp item each, 32
+// rows at a time; larger ones are cut into `parts` items of every parts-th group of
+// kFoldRows rows: 64 items take a triangle of 512 rows in one group each, and an item past
+// the last row costs one cached load.  Thousands of them fill the grid at a quarter of that.
+// A warp walks kFoldUnroll steps of 32 samples at once: the row searches, edge values and
+// key loads of a step are one chain, and the walk waits on its latency.
 constexpr uint32_t kFoldWarpSamples = 4096;
 constexpr int kFoldRows = 8;
-__device__ __forceinline__ uint32_t fold_parts(uint32_t large, uint32_t nwarps)
-{
-    return min(256u, max(16u, 2u * nwarps / max(large, 1u)));
-}
+constexpr int kFoldUnroll = 4;
+__device__ __forceinline__ uint32_t fold_parts(uint32_t large) { return large > 2048u ? 16u : 64u; }
 // With more queued triangles than this, cells that already hold a nearer key are left out
 // before the reduction (they may overdraw each other many times); with fewer, the load
 // would only lengthen each step.
@@ -221,26 +221,45 @@ __device__ __forceinline__ uint32_t fold_queued(uint32_t gtri, uint32_t part, ui
             if (lane >= d) end += o;
         }
         const int total = __shfl_sync(0xffffffffu, end, kRows - 1), xoff = lo - (end - len);
-        for (int base = 0; base < total; base += 32) {
-            const int k = base + lane;
-            int row = 0;   // the rows whose spans end at or before k
+        for (int base = 0; base < total; base += 32 * kFoldUnroll) {
+            int row[kFoldUnroll];   // the rows whose spans end at or before the sample
+#pragma unroll
+            for (int u = 0; u < kFoldUnroll; ++u) row[u] = 0;
 #pragma unroll
             for (int step = kRows / 2; step > 0; step >>= 1)
-                if (__shfl_sync(0xffffffffu, end, row + step - 1) <= k) row += step;
-            const int x = k + __shfl_sync(0xffffffffu, xoff, row), y = ya + row;
-            if (k >= total) continue;
-            const EdgeVals e = eval_edges(r, (float)x, (float)y);
-            if (e.w0 >= 0.0f && e.w1 >= 0.0f && e.w2 >= 0.0f) {
-                ++frags;
-                const float z = interp_z(r.v1z, r.dz2, r.dz3, r.a, e.w1, e.w2);
-                if (z < kFltMax) {
-                    const uint32_t nw = 2 * x < g.w ? 1u : 0u;
-                    unsigned long long *kp = keys + (size_t)(nw ? y : y + 1) * g.pitch +
-                                             key_col(nw ? 2 * x : 2 * x - g.w, g.tw);
-                    const unsigned long long key = make_key(z, gtri, nw);
-                    if (!filter || key < *kp) red_min_u64(kp, key);
+#pragma unroll
+                for (int u = 0; u < kFoldUnroll; ++u)
+                    if (__shfl_sync(0xffffffffu, end, row[u] + step - 1) <= base + 32 * u + lane) row[u] += step;
+            unsigned long long *kp[kFoldUnroll], key[kFoldUnroll];
+#pragma unroll
+            for (int u = 0; u < kFoldUnroll; ++u) {
+                const int k = base + 32 * u + lane, y = ya + row[u];
+                const int x = k + __shfl_sync(0xffffffffu, xoff, row[u]);
+                key[u] = kEmptyKey;
+                kp[u] = keys;
+                if (k >= total) continue;
+                const EdgeVals e = eval_edges(r, (float)x, (float)y);
+                if (e.w0 >= 0.0f && e.w1 >= 0.0f && e.w2 >= 0.0f) {
+                    ++frags;
+                    const float z = interp_z(r.v1z, r.dz2, r.dz3, r.a, e.w1, e.w2);
+                    if (z < kFltMax) {
+                        const uint32_t nw = 2 * x < g.w ? 1u : 0u;
+                        kp[u] = keys + (size_t)(nw ? y : y + 1) * g.pitch + key_col(nw ? 2 * x : 2 * x - g.w, g.tw);
+                        key[u] = make_key(z, gtri, nw);
+                    }
                 }
             }
+            if (filter) {
+                unsigned long long cur[kFoldUnroll];
+#pragma unroll
+                for (int u = 0; u < kFoldUnroll; ++u) cur[u] = key[u] != kEmptyKey ? *kp[u] : 0ull;
+#pragma unroll
+                for (int u = 0; u < kFoldUnroll; ++u)
+                    if (key[u] >= cur[u]) key[u] = kEmptyKey;
+            }
+#pragma unroll
+            for (int u = 0; u < kFoldUnroll; ++u)
+                if (key[u] != kEmptyKey) red_min_u64(kp[u], key[u]);
         }
     }
     return frags;

@@ -1004,15 +1004,15 @@ static sloth_status poll_entry_max(sloth_ctx *ctx)
 // Whether a draw goes without tiles (fold.cuh).  The samples it will walk are estimated
 // from the mesh's edges as it was made and the matrix's scale; a mesh of no extent says
 // nothing.  Up to kFoldMaxSamples the tile raster's launches cost more than its culling
-// saves (us a frame, tiles / fold: 960 triangles at 160x48, 3e4 samples, 68 / 15; 82k at
-// 640x360, 8e5, 84 / 28; 5k at 1920x1080, 7e6, 78 / 35; 8k with 16 large ones at 1920x1080,
-// 1.5e7, 88 / 108; 32k at 1920x1080, 6e7, 104 / 119; at 640x360 the fold stays ahead up to
+// saves (us a frame, tiles / fold: 960 triangles at 160x48, 3e4 samples, 68 / 14; 82k at
+// 640x360, 8e5, 84 / 28; 5k at 1920x1080, 7e6, 78 / 32; 8k with 16 large ones at 1920x1080,
+// 1.5e7, 88 / 75; 8k at 1920x1080, 1e8, 111 / 127; at 640x360 the fold stays ahead up to
 // 1.5e8).  Above kFoldMaxTriangles the estimate is not trusted with the whole draw
 // (positions may have been updated since), and the tiles bound what a wrong one costs.
 // With culling off a caller counts or compares the tile raster's fragments, and the wait
 // test needs its tile loads: both keep it.
 constexpr uint32_t kFoldMaxTriangles = 131072;
-constexpr float kFoldMaxSamples = 1e7f;
+constexpr float kFoldMaxSamples = 16777216.0f;
 static bool draws_without_tiles(const sloth_ctx *ctx, const sloth_mesh *mesh, const Mat4 &M)
 {
     if (!ctx->depth_cull || ctx->fb.wait_test || mesh->ntri > kFoldMaxTriangles || !(mesh->span2 > 0.0f)) return false;
