@@ -3,9 +3,13 @@
 // work queue.  Every per-triangle, per-tile and per-cell step is the single-frame one
 // (record.cuh, bin_common.cuh, raster_common.cuh, resolve_common.cuh) applied to the
 // item's frame, so each frame is bit-identical to drawing it alone.
+#include <algorithm>
+
 #include "batch_kernels.h"
 #include "bin_common.cuh"
 #include "direct.cuh"
+#include "fold.cuh"
+#include "launch.cuh"
 #include "raster_common.cuh"
 #include "record.cuh"
 #include "resolve_common.cuh"
@@ -113,10 +117,41 @@ __device__ __forceinline__ void batch_setup_triangle(const BatchDev &b, const Ba
     }
 }
 
+// batch_setup_triangle for a frame drawn without tiles (fold.cuh): the record, the samples
+// of a small triangle folded by the warp, a larger one queued.
+__device__ __forceinline__ void batch_fold_triangle(const BatchDev &b, const BatchDraw &d, const BatchFrame &f,
+                                                    bool live, uint32_t t, float4 p1, float4 p2, float4 p3,
+                                                    uint32_t rgb, uint32_t stage)
+{
+    FoldClass c{false, false, false};
+    DirectWalk dw{false, 0, 0u};
+    TriRecord r;
+    if (live) {
+        r = build_record(p1, p2, p3, rgb, f.g.w, f.g.h, INT_MAX, &dw);
+        if (r.x0 < r.xe) {
+            c = fold_class(r, dw);
+            store_record(f.fb.records + d.local_base + t, r, 1u, true);
+        }
+    }
+    const FoldQueue queue{b.bb.large_queue, b.large_frame, b.bb.large_count, b.bb.large_cap};
+    const int q = fold_queue_slot(queue, c.mid, c.large);
+    if (q >= 0) {
+        queue.tri[q] = d.local_base + t;
+        queue.frame[q] = d.frame;
+    }
+    if (__any_sync(0xffffffffu, c.mine)) {
+        const uint32_t frags = direct_raster_warp(c.mine, r, d.local_base + t, f.g.w, f.g.pitch, f.g.tw,
+                                                  reinterpret_cast<unsigned long long *>(f.fb.keys), dw.xend,
+                                                  dw.exit_mask, stage);
+        add_frags_warp(frags, f.fb.fragments);
+    }
+}
+
 // blocks[i] = (draw, first triangle): b.tpb triangles of the draw in the single-frame
 // setup's chunks and two phases (setup.cu): the range and the back-face proof for every
 // triangle, the rest of the setup for the ones queued in shared memory with their vertices.
-template <bool kDirect, bool kChunks>
+// kFold: every frame is drawn without tiles.
+template <bool kDirect, bool kChunks, bool kFold = false>
 __global__ void __launch_bounds__(kSetupThreads, kDirect ? kSetupMinBlocks : kFillMinBlocks) batch_setup_kernel(BatchDev b, const int2 *__restrict__ blocks)
 {
     __shared__ uint32_t sq_n;
@@ -174,13 +209,81 @@ __global__ void __launch_bounds__(kSetupThreads, kDirect ? kSetupMinBlocks : kFi
             float4 p1, p2, p3;
             uint32_t rgb = 0, t = 0;
             if (q < nq) t = st.get(q, p1, p2, p3, rgb);
-            batch_setup_triangle<kDirect>(b, d, f, q < nq, t, p1, p2, p3, rgb,
-                                          11u * cap + (threadIdx.x >> 5) * (uint32_t)kDirectStageWords);
+            const uint32_t stage = 11u * cap + (threadIdx.x >> 5) * (uint32_t)kDirectStageWords;
+            if constexpr (kFold) batch_fold_triangle(b, d, f, q < nq, t, p1, p2, p3, rgb, stage);
+            else batch_setup_triangle<kDirect>(b, d, f, q < nq, t, p1, p2, p3, rgb, stage);
         }
         if (!kChunks) break;
         base = total;
         if (c0 + cap < t_end) block_sync();   // the next chunk refills the stash
     }
+}
+
+// blocks[i] = (draw, first triangle): 32 triangles of a draw by a block of kWarps warps
+// (fold_triangles; few triangles in all, where the spread over blocks counts).
+template <int kWarps>
+__global__ void __launch_bounds__(32 * kWarps) batch_fold_setup_kernel(BatchDev b, const int2 *__restrict__ blocks)
+{
+    __shared__ BatchDraw sd;
+    __shared__ BatchFrame sf;
+    __shared__ Mat4 sm;
+    pdl_trigger();
+    const uint32_t zero = pdl_wait();
+    const int2 blk = blocks[blockIdx.x + zero];
+    if (threadIdx.x < 16) sm.m[threadIdx.x] = b.mats[blk.x].m[threadIdx.x];
+    if (threadIdx.x == 0) {
+        sd = b.draws[blk.x];
+        sf = b.frames[sd.frame];
+    }
+    block_sync();
+    const FoldQueue queue{b.bb.large_queue, b.large_frame, b.bb.large_count, b.bb.large_cap};
+    fold_triangles<kWarps>(sd.mesh, sm, (uint32_t)blk.y, sd.local_base, sf.g, sf.fb, queue, sd.frame);
+}
+
+// The queued triangles of every frame (fold_large_kernel).
+__global__ void __launch_bounds__(256) batch_fold_large_kernel(BatchDev b)
+{
+    pdl_trigger();
+    const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x + pdl_wait()) >> 5;
+    const uint32_t large = b.bb.large_count[0], mid = b.bb.large_count[1], nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t parts = fold_parts(large), cut = large * parts, items = cut + mid;
+    const bool filter = large + mid > kFoldFilterMin;
+    unsigned long long *counter = b.frames[0].fb.fragments;   // the batch's one counter
+    uint32_t frags = 0;
+    for (uint32_t it = first; it < items; it += nwarps) {
+        const uint32_t q = it < cut ? it / parts : b.bb.large_cap - 1u - (it - cut);
+        const BatchFrame &f = b.frames[b.large_frame[q]];
+        const FrameGeom g = f.g;
+        const FrameBuffers fb = f.fb;
+        frags += it < cut ? fold_queued<kFoldRows>(b.bb.large_queue[q], it % parts, parts, filter, g, fb)
+                          : fold_queued<32>(b.bb.large_queue[q], 0u, 1u, filter, g, fb);
+    }
+    add_frags_warp(frags, counter);
+}
+
+// Everything a render starts from: counters, tile counts and generations, the newline
+// trees, the matrices, and the keys when the setup folds into them.  One launch instead of
+// nine memsets and a copy, each of them a node of the graph that the next one waited for.
+__global__ void __launch_bounds__(256) batch_reset_kernel(BatchReset r)
+{
+    const uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    pdl_trigger();
+    const uint64_t mask = r.half_shift < 63u ? (1ull << r.half_shift) - 1ull : ~0ull;
+    const uint4 empty = make_uint4(~0u, ~0u, ~0u, ~0u);
+    for (uint64_t i = i0 + pdl_wait(); i < r.nmats; i += step) r.mats[i] = r.mats_host[i];
+    if (i0 == 0) {
+        r.large_count[0] = r.large_count[1] = 0u;
+        *r.fill_count = 0u;
+        *r.overflow = 0u;
+        *r.fragments = 0ull;
+    }
+    for (uint64_t i = i0; i < r.ntiles; i += step) {
+        r.tile_count[i] = r.tile_cursor[i] = 0u;
+        r.tile_gen[i] = r.gen;
+    }
+    for (uint64_t i = i0; i < r.nnl; i += step) r.nltree[i] = -1;
+    for (uint64_t v = i0; v < r.n4; v += step)
+        r.keys[r.half_shift < 63u ? ((v >> r.half_shift) << (r.half_shift + 1)) | (v & mask) : v] = empty;
 }
 
 // blocks[i] = (draw, first triangle of a chunk): newline segment tree of the draw's frame.
@@ -345,20 +448,23 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterMinBlocks) batch_raster
 // blocks per SM (64 registers, no spills): the winners' record loads are latency-bound, and
 // the fourth block's loads in flight took config 3 from 3.33 to 3.22 ms.
 constexpr int kBatchRun = 2;
-static_assert(kBatchResolveChunk % (kBatchRun * 256) == 0, "whole runs, the same trip count in every warp");
+static_assert(kFoldBlockTris == kFoldTris, "the host's table steps by the block's triangles");
+static_assert(kBatchResolveChunk % (kBatchRun * 256) == 0 && kBatchResolveSmall % (kBatchRun * 256) == 0,
+              "whole runs, the same trip count in every warp");
 
 __global__ void __launch_bounds__(256, 4) batch_resolve_kernel(BatchDev b, const int2 *__restrict__ blocks)
 {
     // the frame's descriptor in shared memory: read there, its fields are not reloaded
     // from global memory after each of the block's output stores
     __shared__ BatchFrame sf;
-    const int2 blk = blocks[blockIdx.x];
+    pdl_trigger();
+    const int2 blk = blocks[blockIdx.x + pdl_wait()];
     if (threadIdx.x == 0) sf = b.frames[blk.x];
     block_sync();
     const BatchFrame &f = sf;
     const uint64_t nz = (uint64_t)f.g.w * f.g.h;
     const uint64_t ncells = f.g.image ? nz + f.g.h : nz;
-    const uint64_t end = min(ncells, (uint64_t)blk.y + kBatchResolveChunk);   // chunks start on runs
+    const uint64_t end = min(ncells, (uint64_t)blk.y + b.resolve_chunk);   // chunks start on runs
     if (!(f.g.w & 1)) {
         // an even-width frame by pairs of cells (resolve_even), four per thread at a time
         const uint64_t pend = (end + 1) / 2;
@@ -367,7 +473,7 @@ __global__ void __launch_bounds__(256, 4) batch_resolve_kernel(BatchDev b, const
         return;
     }
     const int lane = threadIdx.x & 31;
-    for (uint32_t i = threadIdx.x; i < kBatchResolveChunk / kBatchRun; i += blockDim.x) {
+    for (uint32_t i = threadIdx.x; i < b.resolve_chunk / kBatchRun; i += blockDim.x) {
         const uint64_t p = (uint64_t)blk.y / kBatchRun + i;
         resolve_run<kBatchRun>(f.g, f.fb, p, kBatchRun * p < end, lane, f.vec != 0);
     }
@@ -378,7 +484,9 @@ cudaError_t prepare_batch_kernels()
     const int bytes = (int)setup_smem_bytes(kMaxTrianglesPerBlock, true);
     cudaError_t e;
     if ((e = cudaFuncSetAttribute(batch_setup_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) ||
-        (e = cudaFuncSetAttribute(batch_setup_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
+        (e = cudaFuncSetAttribute(batch_setup_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) ||
+        (e = cudaFuncSetAttribute(batch_setup_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) ||
+        (e = cudaFuncSetAttribute(batch_setup_kernel<true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
         return e;
     return cudaFuncSetAttribute(batch_newline_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 128 * 1024);
@@ -406,6 +514,31 @@ cudaError_t launch_batch_setup(const BatchDev &b, const int2 *blocks, uint32_t n
         else batch_setup_kernel<false, false><<<grid, block, smem, s>>>(b, blocks);
     }
     return cudaGetLastError();
+}
+
+cudaError_t launch_batch_fold_setup(const BatchDev &b, const int2 *blocks, uint32_t nblocks, bool small,
+                                    cudaStream_t s)
+{
+    if (!nblocks) return cudaSuccess;
+    if (small) return launch_pdl(batch_fold_setup_kernel<4>, dim3(nblocks), dim3(128), kFoldSmemBytes, s, b, blocks);
+    if (!valid_triangles_per_block(b.tpb)) return cudaErrorInvalidValue;
+    const size_t smem = setup_smem_bytes(b.tpb, true);
+    const dim3 grid(nblocks), block(setup_block_threads(b.tpb));
+    if (b.tpb > kSetupChunk) batch_setup_kernel<true, true, true><<<grid, block, smem, s>>>(b, blocks);
+    else batch_setup_kernel<true, false, true><<<grid, block, smem, s>>>(b, blocks);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_batch_fold_large(const BatchDev &b, cudaStream_t s)
+{
+    return launch_pdl(batch_fold_large_kernel, dim3(4u * (unsigned)device_sm_count()), dim3(256), 0, s, b);
+}
+
+cudaError_t launch_batch_reset(const BatchReset &r, cudaStream_t s)
+{
+    const uint64_t most = std::max<uint64_t>(std::max<uint64_t>(r.nmats, r.ntiles), std::max<uint64_t>(r.nnl, r.n4));
+    const uint64_t blocks = std::min<uint64_t>((most + 255) / 256, 16ull * (uint64_t)device_sm_count());
+    return launch_pdl(batch_reset_kernel, dim3((unsigned)std::max<uint64_t>(blocks, 1)), dim3(256), 0, s, r);
 }
 
 cudaError_t launch_batch_newline(const BatchDev &b, const int2 *blocks, uint32_t nblocks, int max_nl,
@@ -476,8 +609,7 @@ cudaError_t launch_batch_items(const BatchDev &b, cudaStream_t s)
 cudaError_t launch_batch_resolve(const BatchDev &b, const int2 *blocks, uint32_t nblocks, cudaStream_t s)
 {
     if (!nblocks) return cudaSuccess;
-    batch_resolve_kernel<<<nblocks, 256, 0, s>>>(b, blocks);
-    return cudaGetLastError();
+    return launch_pdl(batch_resolve_kernel, dim3(nblocks), dim3(256), 0, s, b, blocks);
 }
 
 }  // namespace sloth

@@ -32,10 +32,15 @@ struct sloth_batch {
     std::vector<sloth_frame_desc> frames;
     std::vector<const sloth_mesh *> meshes;   // per draw
     std::vector<float> transforms;            // 16 per draw
+    std::vector<uint32_t> draw_ntri;          // per draw: its mesh's triangles and span2
+    std::vector<float> draw_span2;
     int shape = 0;
     int direct_max = 0;                       // FrameGeom::direct_max of every frame
     bool persistent = true;                   // raster over the device queue (else one CTA per item)
     int tpb = kDefaultTrianglesPerBlock;      // triangles per setup block
+    bool small_fold = false;                  // few enough triangles for 32 a block
+    bool fold_ok = false;                     // the draws' estimates allow frames without tiles
+    bool folded = false;                      // the graph, and the last render, draw without tiles
 
     // layout (per shape)
     std::vector<BatchFrame> hframes;
@@ -77,8 +82,10 @@ struct sloth_batch {
     uint32_t *h_overflow = nullptr;           // pinned
     uint32_t *error = nullptr;                // device error word of the raster (sticky)
     uint32_t *h_error = nullptr;              // pinned
-    int2 *blk[4] = {nullptr, nullptr, nullptr, nullptr};   // vertex, triangle, newline, resolve
-    uint32_t nblk[4] = {0, 0, 0, 0};
+    // block tables: vertex, triangle, newline, resolve, small fold
+    int2 *blk[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    uint32_t nblk[5] = {0, 0, 0, 0, 0};
+    uint32_t resolve_chunk = kBatchResolveChunk;
 
     cudaGraphExec_t graph = nullptr;
     bool rendered = false;
@@ -113,6 +120,7 @@ struct MeshView {
     uint32_t nvert, ntri;
     int device;
     const uint32_t *order, *oidx;   // setup's order of an indexed mesh (MeshDev), or null
+    float span2;                    // sum of the triangles' longest edges squared (mesh_span2)
 };
 MeshView sloth_mesh_view(const sloth_mesh *m);
 }
@@ -178,6 +186,27 @@ void free_layout(sloth_batch *b)
     b->rendered = false;
 }
 
+// Whether a batch's frames can be drawn without tiles (fold.cuh): every draw within the
+// limits of a context's draw (draws_without_tiles) and every frame's estimate too.  Measured
+// with the GPU full (us a render, tiles / tiles with direct folds of 64 / fold): 64 frames of
+// 160x48 with 5k triangles 87 / 50 / 43; 64 of 640x360 with 5k 314 / 341 / 251, with 82k
+// 770 / 514 / 487, with an 8k soup of 1.2e7 samples a frame 486 / 526 / 470, of 4.1e7
+// 498 / 531 / 990.
+bool batch_folds(const sloth_batch *b)
+{
+    for (const sloth_frame_desc &fd : b->frames) {
+        float frame = 0.0f;
+        for (uint32_t k = 0; k < fd.ndraws; ++k) {
+            const uint32_t d = fd.first_draw + k, n = b->draw_ntri[d];
+            if (n == 0) continue;
+            if (n > kFoldMaxTriangles || !(b->draw_span2[d] > 0.0f)) return false;
+            frame += fold_estimate(b->draw_span2[d], n, b->h_mats[d], (int)fd.width, (int)fd.height);
+        }
+        if (!(frame <= kFoldMaxSamples)) return false;
+    }
+    return true;
+}
+
 void set_mats(sloth_batch *b)
 {
     for (size_t f = 0; f < b->frames.size(); ++f) {
@@ -187,6 +216,7 @@ void set_mats(sloth_batch *b)
             sloth_mat4_mul(fd.utransform, &b->transforms[16 * (size_t)d], b->h_mats[d].m);
         }
     }
+    b->fold_ok = batch_folds(b);
 }
 
 // Lay out every frame for tile shape `shape` and allocate the batch's buffers.
@@ -206,8 +236,16 @@ sloth_status build(sloth_batch *b, int shape)
     std::vector<BatchDraw> hd(nd);
     uint64_t keys = 0, nl = 0, rec = 0, vert = 0, cells = 0, zs = 0;
     uint32_t tiles = 0;
+    // a resolve block takes 8192 cells, or 2048 when those blocks would not fill the GPU
+    // twice over (24 frames of 160x48: 24 blocks, 27 us)
+    uint64_t all_cells = 0, all_tri = 0;
+    for (const sloth_frame_desc &fd : b->frames) all_cells += (uint64_t)fd.width * fd.height;
+    for (const sloth_mesh *m : b->meshes) all_tri += sloth_mesh_view(m).ntri;
+    b->resolve_chunk = all_cells / kBatchResolveChunk < 8ull * (uint64_t)device_sm_count() ? kBatchResolveSmall
+                                                                                           : kBatchResolveChunk;
+    b->small_fold = all_tri <= kBatchSmallFold;
     b->max_nl = 1;
-    std::vector<int2> bv, bt, bn, br;
+    std::vector<int2> bv, bt, bn, br, bs;
     for (uint32_t f = 0; f < nf; ++f) {
         const sloth_frame_desc &fd = b->frames[f];
         FrameGeom g{};
@@ -260,6 +298,8 @@ sloth_status build(sloth_batch *b, int shape)
             bd.vert_off = (uint32_t)vert;
             for (uint32_t q = 0; q < (mv.nvert + 3) / 4; q += 256) bv.push_back(make_int2((int)d, (int)q));
             for (uint32_t t = 0; t < mv.ntri; t += (uint32_t)b->tpb) bt.push_back(make_int2((int)d, (int)t));
+            if (b->small_fold)
+                for (uint32_t t = 0; t < mv.ntri; t += kFoldBlockTris) bs.push_back(make_int2((int)d, (int)t));
             if (g.image)
                 for (uint32_t t = 0; t < mv.ntri; t += kBatchNewlineChunk) bn.push_back(make_int2((int)d, (int)t));
             local += mv.ntri;
@@ -267,7 +307,7 @@ sloth_status build(sloth_batch *b, int shape)
         }
         rec += local;
         const uint64_t nc = g.image ? nz + g.h : nz;
-        for (uint64_t c = 0; c < nc; c += kBatchResolveChunk) br.push_back(make_int2((int)f, (int)c));
+        for (uint64_t c = 0; c < nc; c += b->resolve_chunk) br.push_back(make_int2((int)f, (int)c));
     }
     if (rec > 0x7fffffffull) return sloth_ctx_fail(b->ctx, SLOTH_ERR_LIMIT, "batch has more than 2^31 triangles");
     tile_off[nf] = tiles;
@@ -325,8 +365,8 @@ sloth_status build(sloth_batch *b, int shape)
     BCU(b, cudaMemcpy(b->d_frames, b->hframes.data(), nf * sizeof(BatchFrame), cudaMemcpyHostToDevice));
     BCU(b, cudaMemcpy(b->d_draws, hd.data(), nd * sizeof(BatchDraw), cudaMemcpyHostToDevice));
     BCU(b, cudaMemcpy(b->frame_tile_off, tile_off.data(), (nf + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    std::vector<int2> *tabs[4] = {&bv, &bt, &bn, &br};
-    for (int i = 0; i < 4; ++i) {
+    std::vector<int2> *tabs[5] = {&bv, &bt, &bn, &br, &bs};
+    for (int i = 0; i < 5; ++i) {
         b->nblk[i] = (uint32_t)tabs[i]->size();
         BCU(b, balloc(&b->blk[i], tabs[i]->size()));
         if (!tabs[i]->empty())
@@ -356,32 +396,81 @@ BatchDev dev_view(sloth_batch *b)
     d.depth_cull = sloth_ctx_depth_cull(b->ctx);
     d.tpb = b->tpb;
     d.direct_max = b->direct_max;
+    d.fold = b->folded ? 1 : 0;
+    d.resolve_chunk = b->resolve_chunk;
     return d;
 }
 
-// Stage 1: reset, matrices, vertices (once shading wants them), setup, newline, large
-// counts, scan.
+// The resets of a render, in one launch (the keys' runs past the first in one each).
+cudaError_t enqueue_reset(sloth_batch *b, cudaStream_t s)
+{
+    cudaError_t e;
+    // small triangles (all triangles without tiles) fold into the global keys during setup:
+    // every tile's keys start empty and current (kBatchGen), otherwise no tile is current
+    const bool keys = b->folded || b->direct_max > 0;
+    BatchReset r{};
+    r.tile_count = b->bb.tile_count;
+    r.tile_cursor = b->bb.tile_cursor;
+    r.tile_gen = b->tile_gen;
+    r.ntiles = b->total_tiles;
+    r.gen = keys ? kBatchGen : 0u;
+    r.nltree = b->nltree;
+    r.nnl = (uint32_t)b->total_nl;
+    r.large_count = b->bb.large_count;
+    r.fill_count = b->fill_count;
+    r.overflow = b->overflow;
+    r.fragments = b->fragments;
+    r.mats = reinterpret_cast<float4 *>(b->d_mats);
+    r.mats_host = reinterpret_cast<const float4 *>(b->h_mats);
+    r.nmats = (uint32_t)b->meshes.size() * (uint32_t)(sizeof(Mat4) / sizeof(float4));
+    r.half_shift = 63u;
+    if (keys && !b->key_runs.empty()) {
+        const auto &kr = b->key_runs[0];
+        r.keys = reinterpret_cast<uint4 *>(b->keys + kr.off);
+        r.n4 = kr.even ? kr.n / 4 : kr.n / 2;
+        if (kr.even) {
+            r.half_shift = 0;   // log2(tw / 4), as in launch_clear_keys
+            while ((4u << r.half_shift) < (uint32_t)kTileShapes[b->shape][0]) ++r.half_shift;
+        }
+    }
+    if ((e = launch_batch_reset(r, s))) return e;
+    for (size_t i = 1; keys && i < b->key_runs.size(); ++i) {
+        const auto &kr = b->key_runs[i];
+        if ((e = launch_clear_keys(b->keys + kr.off, kr.n, kTileShapes[b->shape][0], kr.even, s))) return e;
+    }
+    return cudaSuccess;
+}
+
+// A render without tiles: reset, vertices (once shading wants them, beside the setup),
+// setup and fold, queued triangles, resolve.
+cudaError_t enqueue_folded(sloth_batch *b, const BatchDev &d, cudaStream_t s)
+{
+    cudaError_t e;
+    if ((e = enqueue_reset(b, s))) return e;
+    const bool side = b->want_tv || !b->small_fold;   // work beside the fold
+    if (b->want_tv) {
+        if ((e = cudaEventRecord(b->ev_setup, s))) return e;
+        if ((e = cudaStreamWaitEvent(b->nl_s, b->ev_setup, 0))) return e;
+        if ((e = launch_batch_vertex(d, b->blk[0], b->nblk[0], b->nl_s))) return e;
+    }
+    const int table = b->small_fold ? 4 : 1;
+    if ((e = launch_batch_fold_setup(d, b->blk[table], b->nblk[table], b->small_fold, s))) return e;
+    if (!b->small_fold) {   // the small fold reduces the newline rows itself
+        if ((e = cudaEventRecord(b->ev_fill, s))) return e;
+        if ((e = cudaStreamWaitEvent(b->nl_s, b->ev_fill, 0))) return e;
+        if ((e = launch_batch_newline(d, b->blk[2], b->nblk[2], b->max_nl, b->nl_s))) return e;
+    }
+    if (side && (e = cudaEventRecord(b->ev_nl, b->nl_s))) return e;
+    if ((e = launch_batch_fold_large(d, s))) return e;
+    if (side && (e = cudaStreamWaitEvent(s, b->ev_nl, 0))) return e;
+    return launch_batch_resolve(d, b->blk[3], b->nblk[3], s);
+}
+
+// Stage 1: reset, vertices (once shading wants them), setup, newline, large counts, scan.
 cudaError_t enqueue_front(sloth_batch *b, const BatchDev &d, cudaStream_t s)
 {
     cudaError_t e;
-    if ((e = cudaMemsetAsync(b->bb.tile_count, 0, (size_t)b->total_tiles * 4, s))) return e;
-    if ((e = cudaMemsetAsync(b->bb.tile_cursor, 0, (size_t)b->total_tiles * 4, s))) return e;
-    if (b->direct_max > 0) {
-        // small triangles fold into the global keys during setup: every tile's keys start
-        // empty and current (kBatchGen is 0x01 in every byte)
-        for (const auto &kr : b->key_runs)
-            if ((e = launch_clear_keys(b->keys + kr.off, kr.n, kTileShapes[b->shape][0], kr.even, s))) return e;
-        if ((e = cudaMemsetAsync(b->tile_gen, 0x01, (size_t)b->total_tiles * 4, s))) return e;
-    } else {
-        if ((e = cudaMemsetAsync(b->tile_gen, 0, (size_t)b->total_tiles * 4, s))) return e;
-    }
-    if ((e = cudaMemsetAsync(b->nltree, 0xff, (size_t)b->total_nl * 4, s))) return e;
-    if ((e = cudaMemsetAsync(b->bb.large_count, 0, 8, s))) return e;
-    if ((e = cudaMemsetAsync(b->fill_count, 0, 4, s))) return e;
-    if ((e = cudaMemsetAsync(b->fragments, 0, 8, s))) return e;
-    if ((e = cudaMemsetAsync(b->overflow, 0, 4, s))) return e;
-    if ((e = cudaMemcpyAsync(b->d_mats, b->h_mats, b->meshes.size() * sizeof(Mat4), cudaMemcpyHostToDevice, s)))
-        return e;
+    if ((e = enqueue_reset(b, s))) return e;
     if (b->want_tv && (e = launch_batch_vertex(d, b->blk[0], b->nblk[0], s))) return e;
     if ((e = launch_batch_setup(d, b->blk[1], b->nblk[1], s))) return e;
     if ((e = cudaEventRecord(b->ev_setup, s))) return e;
@@ -414,6 +503,11 @@ sloth_status render_planned(sloth_batch *b)
 {
     cudaStream_t s = b->stream;
     BatchDev d = dev_view(b);
+    if (b->folded) {   // no entries to size
+        BCU(b, enqueue_folded(b, d, s));
+        b->rendered = true;
+        return SLOTH_OK;
+    }
     BCU(b, enqueue_front(b, d, s));
     BCU(b, cudaMemcpyAsync(b->h_total, b->bb.tile_offset + b->total_tiles, 4, cudaMemcpyDeviceToHost, s));
     BCU(b, cudaStreamSynchronize(s));
@@ -443,8 +537,8 @@ sloth_status capture(sloth_batch *b)
     const BatchDev d = dev_view(b);
     cudaGraph_t g = nullptr;
     BCU(b, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = enqueue_front(b, d, s);
-    if (e == cudaSuccess) e = enqueue_back(b, d, s);
+    cudaError_t e = b->folded ? enqueue_folded(b, d, s) : enqueue_front(b, d, s);
+    if (e == cudaSuccess && !b->folded) e = enqueue_back(b, d, s);
     cudaError_t e2 = cudaStreamEndCapture(s, &g);
     if (e != cudaSuccess || e2 != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -577,7 +671,10 @@ sloth_status sloth_batch_create(sloth_ctx *ctx, const sloth_frame_desc *frames, 
     b->stream = sloth_ctx_stream(ctx);
     b->frames.assign(frames, frames + nframes);
     for (uint32_t d = 0; d < ndraws; ++d) {
+        const MeshView mv = sloth_mesh_view(draws[d].mesh);
         b->meshes.push_back(draws[d].mesh);
+        b->draw_ntri.push_back(mv.ntri);
+        b->draw_span2.push_back(mv.span2);
         b->transforms.insert(b->transforms.end(), draws[d].transform, draws[d].transform + 16);
     }
     if (cudaMallocHost(&b->h_mats, (ndraws ? ndraws : 1) * sizeof(Mat4)) != cudaSuccess ||
@@ -632,7 +729,13 @@ sloth_status sloth_batch_render(sloth_batch *b)
     if (!b || !b->ctx) return SLOTH_ERR_INVALID_ARGUMENT;
     BCU(b, cudaSetDevice(b->device));
     b->vis_valid = false;
-    if (!b->rendered || !b->bb.entries) return render_planned(b);
+    const bool fold = b->fold_ok && sloth_ctx_depth_cull(b->ctx);
+    if (fold != b->folded) {
+        b->folded = fold;
+        if (b->graph) cudaGraphExecDestroy(b->graph);
+        b->graph = nullptr;
+    }
+    if (!b->rendered || (!b->folded && !b->bb.entries)) return render_planned(b);
     if (!b->graph && b->stream != nullptr) {
         const sloth_status st = capture(b);
         if (st != SLOTH_OK) return st;

@@ -53,7 +53,27 @@ struct BatchDev {
     int depth_cull;
     int tpb;                   // triangles per setup block (the triangle block table's step)
     int direct_max;            // the frames' FrameGeom::direct_max (the same for every frame)
+    int fold;                  // every frame is drawn without tiles (fold.cuh): the queued
+                               // triangles are in bb.large_queue and large_frame
+    uint32_t resolve_chunk;    // cells per resolve block (the resolve table's step)
 };
+
+// What a render empties before it starts, in one launch.
+struct BatchReset {
+    uint32_t *tile_count, *tile_cursor, *tile_gen;
+    uint32_t ntiles, gen;      // the generation every tile gets
+    int32_t *nltree;
+    uint32_t nnl;
+    uint32_t *large_count, *fill_count, *overflow;
+    unsigned long long *fragments;
+    float4 *mats;              // device matrices, and the pinned ones they are copied from
+    const float4 *mats_host;
+    uint32_t nmats;            // in float4
+    uint4 *keys;               // keys to empty: n4 16-byte stores, in the even half of each
+    uint64_t n4;               // tile row (2^half_shift stores) or, half_shift 63, all in a row
+    uint32_t half_shift;
+};
+cudaError_t launch_batch_reset(const BatchReset &r, cudaStream_t s);
 
 // Block tables: one int2 (item, start) per block, built on the host.
 cudaError_t launch_batch_vertex(const BatchDev &b, const int2 *blocks, uint32_t nblocks, cudaStream_t s);
@@ -64,10 +84,18 @@ cudaError_t launch_batch_bin_large(const BatchDev &b, bool fill, cudaStream_t s)
 cudaError_t launch_batch_fill(const BatchDev &b, cudaStream_t s);
 cudaError_t launch_batch_items(const BatchDev &b, cudaStream_t s);
 cudaError_t launch_batch_raster(const BatchDev &b, int tw, int th, bool persistent, cudaStream_t s);
+// frames without tiles: setup and fold (blocks: a kFoldBlockTris table when small, else the
+// setup table), then the queued triangles
+cudaError_t launch_batch_fold_setup(const BatchDev &b, const int2 *blocks, uint32_t nblocks, bool small,
+                                    cudaStream_t s);
+cudaError_t launch_batch_fold_large(const BatchDev &b, cudaStream_t s);
 cudaError_t launch_batch_resolve(const BatchDev &b, const int2 *blocks, uint32_t nblocks, cudaStream_t s);
 cudaError_t prepare_batch_kernels();
 
 constexpr uint32_t kBatchNewlineChunk = 8192;   // triangles per newline block
 constexpr uint32_t kBatchResolveChunk = 8192;   // cells per resolve block (four rounds of its threads)
+constexpr uint32_t kBatchResolveSmall = 2048;   // the same (one round) for batches of few blocks
+constexpr uint32_t kFoldBlockTris = 32;         // triangles per block of a small fold's table
+constexpr uint32_t kBatchSmallFold = 1u << 18;  // triangles up to which a fold uses that table
 
 }  // namespace sloth

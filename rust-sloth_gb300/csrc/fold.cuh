@@ -71,6 +71,22 @@ __device__ __forceinline__ int fold_queue_slot(const FoldQueue &q, bool mid, boo
     return -1;
 }
 
+// How a triangle that build_record kept is walked: by its block (mine), by one warp (mid) or
+// by many (large).  A triangle the direct walk does not size (no edge of dy > 0,
+// non-finite, or more than 2^31 samples) is left to the row walk.
+struct FoldClass {
+    bool mine, mid, large;
+};
+__device__ __forceinline__ FoldClass fold_class(const TriRecord &r, const DirectWalk &dw)
+{
+    const uint64_t walked = (uint64_t)(r.xe + 1 - r.x0) * (uint32_t)(r.y1 - r.y0);
+    FoldClass c;
+    c.mine = dw.direct && walked <= kFoldBlockSamples;
+    c.mid = !c.mine && walked <= kFoldWarpSamples;
+    c.large = !c.mine && !c.mid;
+    return c;
+}
+
 // Newline rows [y0, y1) of draw index v into the frame's tree (nltree_update with
 // reductions, which return nothing to wait for).
 __device__ __forceinline__ void nltree_reduce(int32_t *tree, int n, int y0, int y1, int32_t v)
@@ -99,7 +115,7 @@ __device__ __forceinline__ void fold_triangles(const MeshDev &mesh, const Mat4 &
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (wid == 0) {
         const uint32_t p = p0 + lane;
-        bool mine = false, mid = false, large = false;
+        FoldClass c{false, false, false};
         uint32_t gtri = 0;
         int n = 0;
         DirectWalk dw{false, 0, 0u};
@@ -118,18 +134,13 @@ __device__ __forceinline__ void fold_triangles(const MeshDev &mesh, const Mat4 &
             if (keep) {
                 r = build_record(p1, p2, p3, rgb, g.w, g.h, INT_MAX, &dw);
                 if (r.x0 < r.xe) {
-                    // a triangle the direct walk does not size (none of dy > 0, non-finite, or
-                    // more than 2^31 samples) is left to the row walk
-                    const uint64_t walked = (uint64_t)(r.xe + 1 - r.x0) * (uint32_t)(r.y1 - r.y0);
-                    mine = dw.direct && walked <= kFoldBlockSamples;
-                    mid = !mine && walked <= kFoldWarpSamples;
-                    large = !mine && !mid;
+                    c = fold_class(r, dw);
                     store_record(fb.records + gtri, r, 1u, true);
                 }
             }
         }
-        if (mine) n = direct_stage(true, r, gtri, dw.xend, dw.exit_mask, 0u);
-        const int q = fold_queue_slot(queue, mid, large);
+        if (c.mine) n = direct_stage(true, r, gtri, dw.xend, dw.exit_mask, 0u);
+        const int q = fold_queue_slot(queue, c.mid, c.large);
         if (q >= 0) {
             queue.tri[q] = gtri;
             if (queue.frame) queue.frame[q] = frame;

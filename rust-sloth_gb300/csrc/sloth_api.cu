@@ -365,10 +365,11 @@ struct MeshView {
     uint32_t nvert, ntri;
     int device;
     const uint32_t *order, *oidx;   // setup's order of an indexed mesh (MeshDev), or null
+    float span2;                    // sum of the triangles' longest edges squared (mesh_span2)
 };
 MeshView sloth_mesh_view(const sloth_mesh *m)
 {
-    return MeshView{m->x, m->y, m->z, m->idx, m->rgb, m->nvert, m->ntri, m->device, m->order, m->oidx};
+    return MeshView{m->x, m->y, m->z, m->idx, m->rgb, m->nvert, m->ntri, m->device, m->order, m->oidx, m->span2};
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1011,16 +1012,10 @@ static sloth_status poll_entry_max(sloth_ctx *ctx)
 // (positions may have been updated since), and the tiles bound what a wrong one costs.
 // With culling off a caller counts or compares the tile raster's fragments, and the wait
 // test needs its tile loads: both keep it.
-constexpr uint32_t kFoldMaxTriangles = 131072;
-constexpr float kFoldMaxSamples = 16777216.0f;
 static bool draws_without_tiles(const sloth_ctx *ctx, const sloth_mesh *mesh, const Mat4 &M)
 {
     if (!ctx->depth_cull || ctx->fb.wait_test || mesh->ntri > kFoldMaxTriangles || !(mesh->span2 > 0.0f)) return false;
-    const float *m = M.m;
-    const float sx = std::sqrt(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
-    const float sy = std::sqrt(m[4] * m[4] + m[5] * m[5] + m[6] * m[6]);
-    const float cells = (float)ctx->g.w * (float)ctx->g.h;
-    return std::fmin(mesh->span2 * sx * sy, (float)mesh->ntri * cells) <= kFoldMaxSamples;   // false for NaN
+    return fold_estimate(mesh->span2, mesh->ntri, M, ctx->g.w, ctx->g.h) <= kFoldMaxSamples;   // false for NaN
 }
 
 // One draw without tiles: every tile's keys made current first (once a frame).

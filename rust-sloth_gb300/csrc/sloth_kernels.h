@@ -4,6 +4,7 @@
 // context's stream.  Each launcher enqueues one kernel and returns the launch status.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -190,6 +191,20 @@ cudaError_t launch_bin_fill(uint32_t tri_base, const FrameGeom &g, const FrameBu
                             cudaStream_t s);
 cudaError_t launch_bin_fill_large(uint32_t tri_base, const FrameGeom &g, const FrameBuffers &fb,
                                   const BinBuffers &bb, cudaStream_t s);
+
+// Estimated samples of a draw: the sum of its triangles' longest edges squared (span2) times
+// the scale of the matrix's x and y rows, at most every cell for every triangle.  Where the
+// lines lie is with the dispatch (draws_without_tiles, batch_folds).
+constexpr uint32_t kFoldMaxTriangles = 131072;
+constexpr float kFoldMaxSamples = 16777216.0f;
+inline float fold_estimate(float span2, uint32_t ntri, const Mat4 &M, int w, int h)
+{
+    const float *m = M.m;
+    const float sx = std::sqrt(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
+    const float sy = std::sqrt(m[4] * m[4] + m[5] * m[5] + m[6] * m[6]);
+    const float est = span2 * sx * sy, most = (float)ntri * (float)w * (float)h;
+    return est > most ? most : est;   // NaN stays NaN
+}
 
 // Drawing without tiles (fold.cuh).  launch_fold_begin: the keys of tiles that are not
 // current (all: of every tile) emptied and the tiles made current; with frame, the resets

@@ -1,0 +1,74 @@
+"""The batch tests with depth culling off, which keeps a batch's tile raster (batches of few
+samples otherwise go without tiles), and a batch that changes from one to the other."""
+import numpy as np
+import pytest
+
+import sloth_gpu as S
+import workloads as W
+from oracle import oracle as O
+from gpu_helpers import assert_same, oracle_render
+from test_gpu_batch import (check_frames, dev_mesh, mixed_frames,                          # noqa: F401
+                            test_batch_dense_frames_split_tiles, test_batch_entry_overflow_replans,
+                            test_batch_exact_across_setting_changes, test_batch_matches_oracle_and_replays)
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = S.Context(0)
+    c.set_depth_cull(False)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("big", [False, True])
+def test_batch_changes_between_fold_and_tiles(big):
+    """A batch rendered without tiles, then with (culling off, or transforms whose estimate
+    is past the fold's), then without again: planned and replayed, every frame exact."""
+    with S.Context(0) as c:
+        m = W.soup(9000, seed=6, n_large=20)
+        dm = dev_mesh(c, m)
+        R = O.euler_rotation(*W.cli_rotation(yaw=0.8))
+        frames = []
+        for w, h, image in ((160, 48, True), (161, 47, False), (320, 180, True)):
+            U = O.viewport_transform(w, h, O.scene_extent([m["bbox_max"]]))
+            frames.append({"w": w, "h": h, "image": image, "U": U, "draws": [(dm, R), (dm, R)]})
+        b = S.Batch(c, frames)
+        # 60 times the size: most triangles cover the frame, the estimate is far past the limit
+        far = O.mat4_mul(R, np.diag([60.0, 60.0, 60.0, 1.0]).astype(np.float32))
+        for step, tiles in enumerate((False, True, False)):
+            Rk = far if tiles and big else R
+            if big:
+                b.set_transforms(np.stack([Rk] * 6))
+            else:
+                c.set_depth_cull(not tiles)
+            for rep in range(3):
+                b.render()
+                for i, f in enumerate(frames):
+                    ref = oracle_render([m, m], Rk, f["w"], f["h"], f["image"], U=f["U"])
+                    assert_same((*b.read(i), None), ref, f"step {step} render {rep} frame {i}")
+        b.close()
+
+
+@pytest.mark.parametrize("tpb", [128, 4096])
+def test_batch_fold_of_many_triangles(tpb):
+    """More than 2^18 triangles: the fold goes through the batch's setup kernel, with the
+    newline rows beside it, in chunks of one and of several per block."""
+    with S.Context(0) as c:
+        a, s = W.displaced_icosphere(5, seed=2), W.soup(3000, seed=7, n_large=6, sigma=0.05)
+        da, ds = dev_mesh(c, a), dev_mesh(c, s)
+        frames, refs = [], []
+        for k in range(14):
+            w, h, image = ((160, 48, True), (97, 61, False))[k % 2]
+            U = O.viewport_transform(w, h, O.scene_extent([a["bbox_max"], s["bbox_max"]]))
+            R = O.euler_rotation(*W.cli_rotation(pitch=0.5 * k))
+            frames.append({"w": w, "h": h, "image": image, "U": U, "draws": [(da, R), (ds, R)]})
+            refs.append(oracle_render([a, s], R, w, h, image, U=U))
+        b = S.Batch(c, frames)
+        b.set_triangles_per_block(tpb)
+        for rep in range(2):
+            b.render()
+            for i, ref in enumerate(refs):
+                assert_same((*b.read(i), None), ref, f"tpb {tpb} render {rep} frame {i}")
+        b.close()
