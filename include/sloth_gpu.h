@@ -279,7 +279,9 @@ void sloth_batch_destroy(sloth_batch *batch);
 /* Replace every draw's transform (16 floats per draw); waits for the previous render. */
 sloth_status sloth_batch_set_transforms(sloth_batch *batch, const float *transforms);
 /* Render every frame (asynchronous on the context's stream).  The first render sizes the
- * tile-entry buffer (one host synchronisation); later renders replay a CUDA graph. */
+ * tile-entry buffer (one host synchronisation); later renders replay a CUDA graph.  A render
+ * that outgrows the buffer is rasterized by a slower exact fallback on the device, and a
+ * later render or read sizes the buffer again. */
 sloth_status sloth_batch_render(sloth_batch *batch);
 /* Copy one frame's buffers to host memory (any may be NULL); blocks.  If the last render
  * outgrew the tile-entry buffer, it is re-planned and re-rendered first. */

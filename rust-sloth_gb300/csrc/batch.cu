@@ -370,7 +370,8 @@ __device__ __forceinline__ uint32_t frame_of_tile(const BatchDev &b, uint32_t ti
 }
 
 // One thread per global tile: the tile's raster items (tile, slice); a tile rasterized in
-// slices gets its keys cleared and its generation set first (bin_items_kernel, per frame).
+// slices gets its keys cleared and its generation set first (bin_items_kernel, per frame),
+// and so does every tile when the entries outgrew their buffer (batch_overflow_fold).
 __global__ void __launch_bounds__(256) batch_items_kernel(BatchDev b)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -379,10 +380,10 @@ __global__ void __launch_bounds__(256) batch_items_kernel(BatchDev b)
     const uint32_t nt = b.total_tiles;
     const SplitParams sp{b.bb.slice_offset[nt + 1], b.bb.slice_offset[nt + 2]};
     const uint32_t cnt = b.bb.tile_count[t], ns = tile_slices(cnt, sp);
-    const bool split = cnt > sp.threshold;
+    const bool split = cnt > sp.threshold, outgrew = b.bb.tile_offset[nt] > b.bb.capacity;
     const uint32_t off = item_offset(b.bb.slice_offset, nt, t, cnt, sp.threshold);
     for (uint32_t k = 0; k < ns && off + k < b.bb.item_capacity; ++k) b.bb.items[off + k] = make_uint2(t, k);
-    if (split) {
+    if (split || outgrew) {
         const BatchFrame &f = b.frames[frame_of_tile(b, t)];
         const uint32_t lt = t - f.tile_off;
         if (f.fb.tile_gen[lt] != f.fb.gen) {
@@ -412,6 +413,31 @@ __device__ __forceinline__ bool batch_raster_item(TileSmem<TW, TH> &S, const Bat
                                b.bb.entries + b.bb.tile_offset[it.x] + first, b.depth_cull, phase, split);
 }
 
+// A render whose entries outgrew their buffer (its fill wrote what fitted) is rasterized
+// without tiles: every binned triangle is in the fill list or the large queue, and the
+// warps of the grid fold their samples straight into the keys, which batch_items_kernel has
+// made current.  The frames are exact, so nothing has to wait for the count; the host grows
+// the buffer before a later render.  Not inlined: the raster keeps its registers.
+__device__ __noinline__ void batch_overflow_fold(const BatchDev &b)
+{
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    uint32_t frags = 0;
+    const uint32_t n = *b.fill_count;
+    for (uint32_t i = warp; i < n; i += nwarps) {
+        const uint4 e = b.fill_list[i];
+        const BatchFrame &f = b.frames[e.x];
+        frags += fold_queued<32, 1>(e.y, 0u, 1u, true, f.g, f.fb);
+    }
+    constexpr uint32_t kParts = 64;
+    const uint32_t front = b.bb.large_count[0], all = front + b.bb.large_count[1];
+    for (uint32_t i = warp; i < all * kParts; i += nwarps) {
+        const uint32_t k = i / kParts, q = k < front ? k : b.bb.large_cap - 1u - (k - front);
+        const BatchFrame &f = b.frames[b.large_frame[q]];
+        frags += fold_queued<kFoldRows, 1>(b.bb.large_queue[q], i % kParts, kParts, true, f.g, f.fb);
+    }
+    add_frags_warp(frags, b.frames[0].fb.fragments);
+}
+
 // Raster over every frame's tiles in one launch.  Persistent form (the default): a grid of
 // SMs x resident CTAs, each CTA taking the next item of the device-side (frame, tile)
 // queue -- the item list, split tiles' slices first -- from a counter (b.queue, zeroed by
@@ -424,14 +450,18 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterMinBlocks) batch_raster
     __shared__ TileSmem<TW, TH> S;
     __shared__ uint32_t s_item;
     if (b.bb.tile_offset[b.total_tiles] > b.bb.capacity) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) *b.overflow = 1;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            *b.overflow = 1;
+            b.status[0] = 1;
+        }
+        batch_overflow_fold(b);
         return;
     }
     const uint32_t nitems = min(b.bb.slice_offset[b.total_tiles], b.bb.item_capacity);
     if (!kPersistent && blockIdx.x >= nitems) return;
     uint32_t phase = 0;
     if (!kPersistent) {
-        batch_raster_item<TW, TH>(S, b, blockIdx.x, phase);
+        if (!batch_raster_item<TW, TH>(S, b, blockIdx.x, phase) && threadIdx.x == 0) b.status[1] = 1;
         return;
     }
     for (;;) {
@@ -439,7 +469,10 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterMinBlocks) batch_raster
         block_sync();
         const uint32_t i = s_item;   // thread 0 writes the next claim only after raster_tile's last barrier
         if (i >= nitems) break;
-        if (!batch_raster_item<TW, TH>(S, b, i, phase)) break;
+        if (!batch_raster_item<TW, TH>(S, b, i, phase)) {
+            if (threadIdx.x == 0) b.status[1] = 1;
+            break;
+        }
     }
 }
 

@@ -7,7 +7,8 @@
 // pass of each kernel and one persistent raster pass over a device-side (frame, tile)
 // queue.  After the first render (which sizes the tile-entry buffer on the host) the
 // whole sequence is captured in a CUDA graph and replayed.  If a later render's entries
-// outgrow the buffer, the raster reports it and the next read re-plans and re-renders.
+// outgrow the buffer, the raster folds its triangles without tiles and reports it, and the
+// next read or render sizes the buffer again.
 #include <cstring>
 #include <string>
 #include <vector>
@@ -82,6 +83,7 @@ struct sloth_batch {
     uint32_t *h_overflow = nullptr;           // pinned
     uint32_t *error = nullptr;                // device error word of the raster (sticky)
     uint32_t *h_error = nullptr;              // pinned
+    uint32_t *status = nullptr;               // pinned, written by the raster (BatchDev::status)
     // block tables: vertex, triangle, newline, resolve, small fold
     int2 *blk[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     uint32_t nblk[5] = {0, 0, 0, 0, 0};
@@ -390,6 +392,7 @@ BatchDev dev_view(sloth_batch *b)
     d.bb.capacity = (uint32_t)(b->entries_cap > 0xffffffffu ? 0xffffffffu : b->entries_cap);
     d.large_frame = b->large_frame;
     d.overflow = b->overflow;
+    d.status = b->status;
     d.queue = b->queue;
     d.fill_list = b->fill_list;
     d.fill_count = b->fill_count;
@@ -503,6 +506,7 @@ sloth_status render_planned(sloth_batch *b)
 {
     cudaStream_t s = b->stream;
     BatchDev d = dev_view(b);
+    b->status[0] = 0;
     if (b->folded) {   // no entries to size
         BCU(b, enqueue_folded(b, d, s));
         b->rendered = true;
@@ -586,9 +590,11 @@ sloth_status diff_prepare(sloth_batch *b, const float *vertex_rgb, const float *
             BCU(b, cudaMemcpy(b->diff_blk, t.data(), t.size() * sizeof(int2), cudaMemcpyHostToDevice));
         b->ndiff_blk = (uint32_t)t.size();
     }
-    // the keys of the last render must be complete (re-render if its entries overflowed)
-    sloth_status st = settle(b);
-    if (st != SLOTH_OK) return st;
+    // The last render's keys are complete on the stream whether or not its entries fitted
+    // (batch_overflow_fold), so nothing is waited for: with a wait here and one in the
+    // backward call a fit of 64 views at 256x256 took 529 us a step, without 436.
+    if (*(volatile uint32_t *)&b->status[1])
+        return sloth_ctx_fail(b->ctx, SLOTH_ERR_DEVICE_FAULT, "a raster block gave up waiting for its tile copy");
     if (!b->want_tv) {
         // the first shading of this batch: transform the vertices the last render drew, and
         // let every later render do it too (the graph is captured again)
@@ -622,6 +628,7 @@ void sloth_batch_detach(sloth_batch *b)
     if (b->h_total) cudaFreeHost(b->h_total);
     if (b->h_overflow) cudaFreeHost(b->h_overflow);
     if (b->h_error) cudaFreeHost(b->h_error);
+    if (b->status) cudaFreeHost(b->status);
     bfree(b->error);
     for (cudaEvent_t *ev : {&b->ev_setup, &b->ev_nl, &b->ev_fill, &b->ev_aux})
         if (*ev) {
@@ -634,7 +641,7 @@ void sloth_batch_detach(sloth_batch *b)
             *st = nullptr;
         }
     b->h_mats = nullptr;
-    b->h_total = b->h_overflow = b->h_error = nullptr;
+    b->h_total = b->h_overflow = b->h_error = b->status = nullptr;
     b->ctx = nullptr;
     b->stream = nullptr;
     b->rendered = false;
@@ -679,7 +686,8 @@ sloth_status sloth_batch_create(sloth_ctx *ctx, const sloth_frame_desc *frames, 
     }
     if (cudaMallocHost(&b->h_mats, (ndraws ? ndraws : 1) * sizeof(Mat4)) != cudaSuccess ||
         cudaMallocHost(&b->h_total, 4) != cudaSuccess || cudaMallocHost(&b->h_overflow, 4) != cudaSuccess ||
-        cudaMallocHost(&b->h_error, 4) != cudaSuccess || cudaMalloc(&b->error, 4) != cudaSuccess ||
+        cudaMallocHost(&b->h_error, 4) != cudaSuccess || cudaMallocHost(&b->status, 8) != cudaSuccess ||
+        cudaMalloc(&b->error, 4) != cudaSuccess ||
         cudaMemset(b->error, 0, 4) != cudaSuccess ||
         cudaStreamCreateWithFlags(&b->nl_s, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&b->aux_s, cudaStreamNonBlocking) != cudaSuccess ||
@@ -692,6 +700,7 @@ sloth_status sloth_batch_create(sloth_ctx *ctx, const sloth_frame_desc *frames, 
         delete b;
         return sloth_ctx_fail(ctx, SLOTH_ERR_OUT_OF_MEMORY, "batch host buffers");
     }
+    b->status[0] = b->status[1] = 0;
     sloth_ctx_register_batch(ctx, b);
     b->direct_max = sloth_ctx_direct_samples(ctx);
     set_mats(b);
@@ -735,7 +744,10 @@ sloth_status sloth_batch_render(sloth_batch *b)
         if (b->graph) cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
     }
-    if (!b->rendered || (!b->folded && !b->bb.entries)) return render_planned(b);
+    // a render known to have outgrown its entries: the buffer grows before the next one
+    // (settle does the same for a caller that reads)
+    const bool grow = !b->folded && *(volatile uint32_t *)&b->status[0];
+    if (grow || !b->rendered || (!b->folded && !b->bb.entries)) return render_planned(b);
     if (!b->graph && b->stream != nullptr) {
         const sloth_status st = capture(b);
         if (st != SLOTH_OK) return st;

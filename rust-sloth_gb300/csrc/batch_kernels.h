@@ -45,6 +45,8 @@ struct BatchDev {
     BinBuffers bb;             // global tile arrays and entries
     uint32_t *large_frame;     // frame of each large-queue entry
     uint32_t *overflow;        // set when the entries outgrew their capacity
+    volatile uint32_t *status; // pinned host words: [0] a render's entries outgrew their capacity,
+                               // [1] a raster block gave up waiting for its keys
     uint32_t *queue;           // the persistent raster's next item (zeroed by the item kernel)
     uint4 *fill_list;          // (frame, frame-local draw index, slot in its first tile, 0) of
                                // every small binned triangle, appended by setup: the fill walks

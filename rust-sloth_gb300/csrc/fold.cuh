@@ -194,7 +194,7 @@ __device__ __forceinline__ void fold_row_span(float dx, float dy, float ax, floa
 // whose cell already holds a nearer key is dropped before the reduction: the plain load may
 // be older than the key in L2, and keys only fall, so it can only keep a sample that was not
 // needed.
-template <int kRows>
+template <int kRows, int kUnroll = kFoldUnroll>
 __device__ __forceinline__ uint32_t fold_queued(uint32_t gtri, uint32_t part, uint32_t parts, bool filter,
                                                 const FrameGeom &g, const FrameBuffers &fb)
 {
@@ -232,18 +232,18 @@ __device__ __forceinline__ uint32_t fold_queued(uint32_t gtri, uint32_t part, ui
             if (lane >= d) end += o;
         }
         const int total = __shfl_sync(0xffffffffu, end, kRows - 1), xoff = lo - (end - len);
-        for (int base = 0; base < total; base += 32 * kFoldUnroll) {
-            int row[kFoldUnroll];   // the rows whose spans end at or before the sample
+        for (int base = 0; base < total; base += 32 * kUnroll) {
+            int row[kUnroll];   // the rows whose spans end at or before the sample
 #pragma unroll
-            for (int u = 0; u < kFoldUnroll; ++u) row[u] = 0;
+            for (int u = 0; u < kUnroll; ++u) row[u] = 0;
 #pragma unroll
             for (int step = kRows / 2; step > 0; step >>= 1)
 #pragma unroll
-                for (int u = 0; u < kFoldUnroll; ++u)
+                for (int u = 0; u < kUnroll; ++u)
                     if (__shfl_sync(0xffffffffu, end, row[u] + step - 1) <= base + 32 * u + lane) row[u] += step;
-            unsigned long long *kp[kFoldUnroll], key[kFoldUnroll];
+            unsigned long long *kp[kUnroll], key[kUnroll];
 #pragma unroll
-            for (int u = 0; u < kFoldUnroll; ++u) {
+            for (int u = 0; u < kUnroll; ++u) {
                 const int k = base + 32 * u + lane, y = ya + row[u];
                 const int x = k + __shfl_sync(0xffffffffu, xoff, row[u]);
                 key[u] = kEmptyKey;
@@ -261,15 +261,15 @@ __device__ __forceinline__ uint32_t fold_queued(uint32_t gtri, uint32_t part, ui
                 }
             }
             if (filter) {
-                unsigned long long cur[kFoldUnroll];
+                unsigned long long cur[kUnroll];
 #pragma unroll
-                for (int u = 0; u < kFoldUnroll; ++u) cur[u] = key[u] != kEmptyKey ? *kp[u] : 0ull;
+                for (int u = 0; u < kUnroll; ++u) cur[u] = key[u] != kEmptyKey ? *kp[u] : 0ull;
 #pragma unroll
-                for (int u = 0; u < kFoldUnroll; ++u)
+                for (int u = 0; u < kUnroll; ++u)
                     if (key[u] >= cur[u]) key[u] = kEmptyKey;
             }
 #pragma unroll
-            for (int u = 0; u < kFoldUnroll; ++u)
+            for (int u = 0; u < kUnroll; ++u)
                 if (key[u] != kEmptyKey) red_min_u64(kp[u], key[u]);
         }
     }

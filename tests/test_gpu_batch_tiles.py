@@ -72,3 +72,41 @@ def test_batch_fold_of_many_triangles(tpb):
             for i, ref in enumerate(refs):
                 assert_same((*b.read(i), None), ref, f"tpb {tpb} render {rep} frame {i}")
         b.close()
+
+
+@pytest.mark.parametrize("direct,persistent", [(0, True), (16, False)])
+def test_batch_overflow_is_exact_on_the_device(ctx, direct, persistent):
+    """A graph replay whose entries outgrow the buffer: the frames in device memory are exact
+    without a read that re-plans, at odd and even widths, and so are the next renders', one
+    of which grows the buffer."""
+    torch = pytest.importorskip("torch")
+
+    class Dev:
+        def __init__(self, ptr, n):
+            self.__cuda_array_interface__ = {"shape": (n,), "typestr": "<i4", "data": (ptr, False), "version": 3}
+
+    m = W.soup(3000, seed=41, n_large=10)
+    dm = dev_mesh(ctx, m)
+    small = O.mat4_mul(O.euler_rotation(*W.cli_rotation()), np.diag([0.05, 0.05, 0.05, 1.0]).astype(np.float32))
+    frames = []
+    for w, h, image in ((640, 360, True), (321, 181, False)):
+        frames.append({"w": w, "h": h, "image": image, "U": O.viewport_transform(w, h, 1.0), "draws": [(dm, small)]})
+    b = S.Batch(ctx, frames)
+    b.set_direct_samples(direct)
+    b.set_persistent(persistent)
+    b.render()
+    b.render()                      # graph captured with the small entry buffer
+    R = O.euler_rotation(*W.cli_rotation(yaw=0.3))
+    b.set_transforms(np.stack([R] * 2))
+    for rep in range(3):
+        b.render()
+        torch.cuda.synchronize()
+        for i, f in enumerate(frames):
+            ref = oracle_render([m], R, f["w"], f["h"], f["image"], U=f["U"])
+            c, z = S.C.c_void_p(), S.C.c_void_p()
+            assert b.lib.sloth_batch_frame_buffers(b.h, i, S.C.byref(c), S.C.byref(z)) == S.OK
+            cells = torch.as_tensor(Dev(c.value, ref.cells.size), device="cuda").cpu().numpy()
+            zz = torch.as_tensor(Dev(z.value, ref.z.size), device="cuda").cpu().numpy()
+            assert np.array_equal(cells, ref.cells.view(np.int32)), f"render {rep} frame {i}"
+            assert np.array_equal(zz, ref.z.view(np.int32)), f"render {rep} frame {i}"
+    b.close()
