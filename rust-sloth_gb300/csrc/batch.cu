@@ -21,42 +21,10 @@ __device__ __forceinline__ Viewport vp_batch(const FrameGeom &g)
     return Viewport{g.w, g.h, g.image, g.tw, g.th, g.ntx, g.nty, g.pitch};
 }
 
-// blocks[i] = (draw, first vertex quad): four vertices per thread, float4 SoA loads.
-__global__ void __launch_bounds__(256) batch_vertex_kernel(BatchDev b, const int2 *__restrict__ blocks)
-{
-    const int2 blk = blocks[blockIdx.x];
-    const BatchDraw &d = b.draws[blk.x];
-    const Mat4 M = b.mats[blk.x];
-    const uint32_t nv = d.mesh.nvert;
-    const uint32_t q = (uint32_t)blk.y + threadIdx.x;
-    const uint32_t i0 = q * 4;
-    if (i0 >= nv) return;
-    float xs[4], ys[4], zs[4];
-    if (i0 + 4 <= nv) {
-        const float4 X = __ldg(reinterpret_cast<const float4 *>(d.mesh.x) + q);
-        const float4 Y = __ldg(reinterpret_cast<const float4 *>(d.mesh.y) + q);
-        const float4 Z = __ldg(reinterpret_cast<const float4 *>(d.mesh.z) + q);
-        xs[0] = X.x; xs[1] = X.y; xs[2] = X.z; xs[3] = X.w;
-        ys[0] = Y.x; ys[1] = Y.y; ys[2] = Y.z; ys[3] = Y.w;
-        zs[0] = Z.x; zs[1] = Z.y; zs[2] = Z.z; zs[3] = Z.w;
-    } else {
-        for (int k = 0; k < 4; ++k) {
-            const uint32_t i = i0 + k < nv ? i0 + k : nv - 1;
-            xs[k] = d.mesh.x[i]; ys[k] = d.mesh.y[i]; zs[k] = d.mesh.z[i];
-        }
-    }
-    float4 *tv = b.tv + d.vert_off;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        if (i0 + k < nv)
-            tv[i0 + k] = make_float4(row_dot(&M.m[0], xs[k], ys[k], zs[k]), row_dot(&M.m[4], xs[k], ys[k], zs[k]),
-                                     row_dot(&M.m[8], xs[k], ys[k], zs[k]), 0.0f);
-}
-
 // The three vertices of triangle t of draw d, at position p of setup's order of the mesh,
 // transformed by the draw's matrix M in place (the vertex kernel's operations): a mesh
 // shared by many views stays in L2, and no transformed-vertex buffer is written and read
-// back for the render.
+// back.
 __device__ __forceinline__ void batch_triangle_vertices(const BatchDraw &d, const Mat4 &M, uint32_t p, uint32_t t,
                                                         float4 &p1, float4 &p2, float4 &p3)
 {
@@ -523,13 +491,6 @@ cudaError_t prepare_batch_kernels()
         return e;
     return cudaFuncSetAttribute(batch_newline_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 128 * 1024);
-}
-
-cudaError_t launch_batch_vertex(const BatchDev &b, const int2 *blocks, uint32_t nblocks, cudaStream_t s)
-{
-    if (!nblocks) return cudaSuccess;
-    batch_vertex_kernel<<<nblocks, 256, 0, s>>>(b, blocks);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_batch_setup(const BatchDev &b, const int2 *blocks, uint32_t nblocks, cudaStream_t s)

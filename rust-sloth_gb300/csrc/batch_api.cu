@@ -26,6 +26,9 @@ using namespace sloth;
 // with the byte 0x01 (every tile current), so the value has 0x01 in every byte.
 constexpr uint32_t kBatchGen = 0x01010101u;
 
+// Block tables: setup, newline, resolve, small fold.
+enum { kTabSetup, kTabNewline, kTabResolve, kTabFold, kTables };
+
 struct sloth_batch {
     sloth_ctx *ctx = nullptr;
     int device = 0;
@@ -47,7 +50,7 @@ struct sloth_batch {
     std::vector<BatchFrame> hframes;
     std::vector<uint64_t> cell_off, z_off;    // per frame
     uint32_t total_tiles = 0;
-    uint64_t total_cells = 0, total_z = 0, total_keys = 0, total_nl = 0, total_rec = 0, total_vert = 0;
+    uint64_t total_cells = 0, total_z = 0, total_keys = 0, total_nl = 0, total_rec = 0;
     // runs of consecutive frames' keys with the same width parity: (first key, keys, even width)
     struct KeyRun {
         uint64_t off, n;
@@ -61,7 +64,6 @@ struct sloth_batch {
     BatchDraw *d_draws = nullptr;
     Mat4 *d_mats = nullptr;
     Mat4 *h_mats = nullptr;                   // pinned
-    float4 *tv = nullptr;                     // transformed vertices: written for shading only (want_tv)
     TriRecord *records = nullptr;
     uint32_t *rows = nullptr;                 // packed sample rows per record (setup -> newline)
     uint64_t *keys = nullptr;
@@ -84,9 +86,8 @@ struct sloth_batch {
     uint32_t *error = nullptr;                // device error word of the raster (sticky)
     uint32_t *h_error = nullptr;              // pinned
     uint32_t *status = nullptr;               // pinned, written by the raster (BatchDev::status)
-    // block tables: vertex, triangle, newline, resolve, small fold
-    int2 *blk[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    uint32_t nblk[5] = {0, 0, 0, 0, 0};
+    int2 *blk[kTables] = {nullptr, nullptr, nullptr, nullptr};   // block tables (kTab*)
+    uint32_t nblk[kTables] = {0, 0, 0, 0};
     uint32_t resolve_chunk = kBatchResolveChunk;
 
     cudaGraphExec_t graph = nullptr;
@@ -101,7 +102,6 @@ struct sloth_batch {
     uint32_t ndiff_blk = 0;
     uint2 *vis = nullptr;                     // stored visibility, one per depth cell
     bool vis_valid = false;                   // vis holds the last render's visibility
-    bool want_tv = false;                     // shading has been used: renders fill tv
 
     FlushScratch flush;
 };
@@ -158,7 +158,6 @@ void free_layout(sloth_batch *b)
     bfree(b->d_frames);
     bfree(b->d_draws);
     bfree(b->d_mats);
-    bfree(b->tv);
     bfree(b->records);
     bfree(b->rows);
     bfree(b->keys);
@@ -236,7 +235,7 @@ sloth_status build(sloth_batch *b, int shape)
     std::vector<uint64_t> key_off(nf), nl_off(nf), rec_off(nf);
     std::vector<uint32_t> tile_off(nf + 1, 0);
     std::vector<BatchDraw> hd(nd);
-    uint64_t keys = 0, nl = 0, rec = 0, vert = 0, cells = 0, zs = 0;
+    uint64_t keys = 0, nl = 0, rec = 0, cells = 0, zs = 0;
     uint32_t tiles = 0;
     // a resolve block takes 8192 cells, or 2048 when those blocks would not fill the GPU
     // twice over (24 frames of 160x48: 24 blocks, 27 us)
@@ -247,7 +246,7 @@ sloth_status build(sloth_batch *b, int shape)
                                                                                            : kBatchResolveChunk;
     b->small_fold = all_tri <= kBatchSmallFold;
     b->max_nl = 1;
-    std::vector<int2> bv, bt, bn, br, bs;
+    std::vector<int2> bt, bn, br, bs;
     for (uint32_t f = 0; f < nf; ++f) {
         const sloth_frame_desc &fd = b->frames[f];
         FrameGeom g{};
@@ -297,15 +296,12 @@ sloth_status build(sloth_batch *b, int shape)
             bd.frame = f;
             bd.rec_off = (uint32_t)(rec + local);
             bd.local_base = local;
-            bd.vert_off = (uint32_t)vert;
-            for (uint32_t q = 0; q < (mv.nvert + 3) / 4; q += 256) bv.push_back(make_int2((int)d, (int)q));
             for (uint32_t t = 0; t < mv.ntri; t += (uint32_t)b->tpb) bt.push_back(make_int2((int)d, (int)t));
             if (b->small_fold)
                 for (uint32_t t = 0; t < mv.ntri; t += kFoldBlockTris) bs.push_back(make_int2((int)d, (int)t));
             if (g.image)
                 for (uint32_t t = 0; t < mv.ntri; t += kBatchNewlineChunk) bn.push_back(make_int2((int)d, (int)t));
             local += mv.ntri;
-            vert += mv.nvert;
         }
         rec += local;
         const uint64_t nc = g.image ? nz + g.h : nz;
@@ -321,9 +317,7 @@ sloth_status build(sloth_batch *b, int shape)
     b->total_keys = keys;
     b->total_nl = nl;
     b->total_rec = rec;
-    b->total_vert = vert;
 
-    BCU(b, balloc(&b->tv, vert));
     BCU(b, balloc(&b->records, rec));
     BCU(b, balloc(&b->rows, rec));
     BCU(b, balloc(&b->keys, keys));
@@ -367,8 +361,8 @@ sloth_status build(sloth_batch *b, int shape)
     BCU(b, cudaMemcpy(b->d_frames, b->hframes.data(), nf * sizeof(BatchFrame), cudaMemcpyHostToDevice));
     BCU(b, cudaMemcpy(b->d_draws, hd.data(), nd * sizeof(BatchDraw), cudaMemcpyHostToDevice));
     BCU(b, cudaMemcpy(b->frame_tile_off, tile_off.data(), (nf + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    std::vector<int2> *tabs[5] = {&bv, &bt, &bn, &br, &bs};
-    for (int i = 0; i < 5; ++i) {
+    std::vector<int2> *tabs[kTables] = {&bt, &bn, &br, &bs};
+    for (int i = 0; i < kTables; ++i) {
         b->nblk[i] = (uint32_t)tabs[i]->size();
         BCU(b, balloc(&b->blk[i], tabs[i]->size()));
         if (!tabs[i]->empty())
@@ -383,7 +377,6 @@ BatchDev dev_view(sloth_batch *b)
     d.frames = b->d_frames;
     d.draws = b->d_draws;
     d.mats = b->d_mats;
-    d.tv = b->tv;
     d.nframes = (uint32_t)b->frames.size();
     d.ndraws = (uint32_t)b->meshes.size();
     d.total_tiles = b->total_tiles;
@@ -444,41 +437,34 @@ cudaError_t enqueue_reset(sloth_batch *b, cudaStream_t s)
     return cudaSuccess;
 }
 
-// A render without tiles: reset, vertices (once shading wants them, beside the setup),
-// setup and fold, queued triangles, resolve.
+// A render without tiles: reset, setup and fold, queued triangles, resolve.
 cudaError_t enqueue_folded(sloth_batch *b, const BatchDev &d, cudaStream_t s)
 {
     cudaError_t e;
     if ((e = enqueue_reset(b, s))) return e;
-    const bool side = b->want_tv || !b->small_fold;   // work beside the fold
-    if (b->want_tv) {
-        if ((e = cudaEventRecord(b->ev_setup, s))) return e;
-        if ((e = cudaStreamWaitEvent(b->nl_s, b->ev_setup, 0))) return e;
-        if ((e = launch_batch_vertex(d, b->blk[0], b->nblk[0], b->nl_s))) return e;
-    }
-    const int table = b->small_fold ? 4 : 1;
+    const bool side = !b->small_fold;   // the newline fold beside the rest
+    const int table = b->small_fold ? kTabFold : kTabSetup;
     if ((e = launch_batch_fold_setup(d, b->blk[table], b->nblk[table], b->small_fold, s))) return e;
-    if (!b->small_fold) {   // the small fold reduces the newline rows itself
+    if (side) {   // the small fold reduces the newline rows itself
         if ((e = cudaEventRecord(b->ev_fill, s))) return e;
         if ((e = cudaStreamWaitEvent(b->nl_s, b->ev_fill, 0))) return e;
-        if ((e = launch_batch_newline(d, b->blk[2], b->nblk[2], b->max_nl, b->nl_s))) return e;
+        if ((e = launch_batch_newline(d, b->blk[kTabNewline], b->nblk[kTabNewline], b->max_nl, b->nl_s))) return e;
     }
     if (side && (e = cudaEventRecord(b->ev_nl, b->nl_s))) return e;
     if ((e = launch_batch_fold_large(d, s))) return e;
     if (side && (e = cudaStreamWaitEvent(s, b->ev_nl, 0))) return e;
-    return launch_batch_resolve(d, b->blk[3], b->nblk[3], s);
+    return launch_batch_resolve(d, b->blk[kTabResolve], b->nblk[kTabResolve], s);
 }
 
-// Stage 1: reset, vertices (once shading wants them), setup, newline, large counts, scan.
+// Stage 1: reset, setup, newline, large counts, scan.
 cudaError_t enqueue_front(sloth_batch *b, const BatchDev &d, cudaStream_t s)
 {
     cudaError_t e;
     if ((e = enqueue_reset(b, s))) return e;
-    if (b->want_tv && (e = launch_batch_vertex(d, b->blk[0], b->nblk[0], s))) return e;
-    if ((e = launch_batch_setup(d, b->blk[1], b->nblk[1], s))) return e;
+    if ((e = launch_batch_setup(d, b->blk[kTabSetup], b->nblk[kTabSetup], s))) return e;
     if ((e = cudaEventRecord(b->ev_setup, s))) return e;
     if ((e = cudaStreamWaitEvent(b->nl_s, b->ev_setup, 0))) return e;
-    if ((e = launch_batch_newline(d, b->blk[2], b->nblk[2], b->max_nl, b->nl_s))) return e;
+    if ((e = launch_batch_newline(d, b->blk[kTabNewline], b->nblk[kTabNewline], b->max_nl, b->nl_s))) return e;
     if ((e = cudaEventRecord(b->ev_nl, b->nl_s))) return e;
     if ((e = launch_batch_bin_large(d, false, s))) return e;
     return launch_bin_scan(b->total_tiles, d.bb, s);
@@ -498,7 +484,7 @@ cudaError_t enqueue_back(sloth_batch *b, const BatchDev &d, cudaStream_t s)
     const int tw = kTileShapes[b->shape][0], th = kTileShapes[b->shape][1];
     if ((e = launch_batch_raster(d, tw, th, b->persistent, s))) return e;
     if ((e = cudaStreamWaitEvent(s, b->ev_nl, 0))) return e;   // the newline tree is complete
-    return launch_batch_resolve(d, b->blk[3], b->nblk[3], s);
+    return launch_batch_resolve(d, b->blk[kTabResolve], b->nblk[kTabResolve], s);
 }
 
 // Render without the graph: stage 1, size the entries from the scan total, stage 2.
@@ -595,16 +581,6 @@ sloth_status diff_prepare(sloth_batch *b, const float *vertex_rgb, const float *
     // backward call a fit of 64 views at 256x256 took 529 us a step, without 436.
     if (*(volatile uint32_t *)&b->status[1])
         return sloth_ctx_fail(b->ctx, SLOTH_ERR_DEVICE_FAULT, "a raster block gave up waiting for its tile copy");
-    if (!b->want_tv) {
-        // the first shading of this batch: transform the vertices the last render drew, and
-        // let every later render do it too (the graph is captured again)
-        BCU(b, launch_batch_vertex(dev_view(b), b->blk[0], b->nblk[0], b->stream));
-        b->want_tv = true;
-        if (b->graph) {
-            cudaGraphExecDestroy(b->graph);
-            b->graph = nullptr;
-        }
-    }
     return SLOTH_OK;
 }
 
@@ -840,10 +816,10 @@ sloth_status sloth_batch_set_triangles_per_block(sloth_batch *b, int tpb)
             const uint32_t ntri = sloth_mesh_view(b->meshes[d]).ntri;
             for (uint32_t t = 0; t < ntri; t += (uint32_t)tpb) bt.push_back(make_int2((int)d, (int)t));
         }
-    bfree(b->blk[1]);
-    b->nblk[1] = (uint32_t)bt.size();
-    BCU(b, balloc(&b->blk[1], bt.size()));
-    if (!bt.empty()) BCU(b, cudaMemcpy(b->blk[1], bt.data(), bt.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    bfree(b->blk[kTabSetup]);
+    b->nblk[kTabSetup] = (uint32_t)bt.size();
+    BCU(b, balloc(&b->blk[kTabSetup], bt.size()));
+    if (!bt.empty()) BCU(b, cudaMemcpy(b->blk[kTabSetup], bt.data(), bt.size() * sizeof(int2), cudaMemcpyHostToDevice));
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;

@@ -31,14 +31,12 @@ struct BatchDraw {
     uint32_t frame;
     uint32_t rec_off;          // global record of the draw's first triangle
     uint32_t local_base;       // frame-local draw index of the draw's first triangle
-    uint32_t vert_off;         // first transformed vertex of the draw
 };
 
 struct BatchDev {
     const BatchFrame *frames;
     const BatchDraw *draws;
     const Mat4 *mats;          // per draw: utransform * transform
-    float4 *tv;                // transformed vertices of every draw
     uint32_t nframes, ndraws;
     uint32_t total_tiles;
     const uint32_t *frame_tile_off;   // nframes + 1 (for tile -> frame lookups)
@@ -78,7 +76,6 @@ struct BatchReset {
 cudaError_t launch_batch_reset(const BatchReset &r, cudaStream_t s);
 
 // Block tables: one int2 (item, start) per block, built on the host.
-cudaError_t launch_batch_vertex(const BatchDev &b, const int2 *blocks, uint32_t nblocks, cudaStream_t s);
 cudaError_t launch_batch_setup(const BatchDev &b, const int2 *blocks, uint32_t nblocks, cudaStream_t s);
 cudaError_t launch_batch_newline(const BatchDev &b, const int2 *blocks, uint32_t nblocks, int max_nl,
                                  cudaStream_t s);

@@ -10,8 +10,8 @@ namespace sloth {
 
 constexpr uint32_t kDiffChunk = 2048;   // depth cells (or samples) per block
 
-// blocks[i] = (frame, first depth cell), chunks of kDiffChunk over w*h per frame; the
-// same table walks the w*h samples (x in [0,w), y in [0,h)) of the backward pass.
+// blocks[i] = (frame, first depth cell), chunks of kDiffChunk (even) over w*h per frame, for
+// both passes.
 cudaError_t launch_batch_shade(const BatchDev &b, const int2 *blocks, uint32_t nblocks, const float *vrgb,
                                const float *light, float *rgb, uint2 *vis, cudaStream_t s);
 cudaError_t launch_batch_shade_backward(const BatchDev &b, const int2 *blocks, uint32_t nblocks, const float *vrgb,
