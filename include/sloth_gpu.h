@@ -234,6 +234,9 @@ void sloth_mesh_destroy(sloth_mesh *mesh);
  * the copy direction).  The buffers must stay valid until the next synchronising call. */
 sloth_status sloth_mesh_update(sloth_mesh *mesh, const float *x, const float *y, const float *z,
                                const uint8_t *rgb);
+/* sloth_mesh_update from device memory in one kernel: positions as x, y, z triples (3*nvert
+ * floats) and face colours (3*ntri bytes). */
+sloth_status sloth_mesh_update_interleaved(sloth_mesh *mesh, const float *xyz, const uint8_t *rgb);
 sloth_status sloth_mesh_info(const sloth_mesh *mesh, uint32_t *ntri, float bbox_max[3]);
 
 /* ---- the hot path ----------------------------------------------------------------- */

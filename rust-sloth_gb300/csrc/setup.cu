@@ -5,6 +5,7 @@
 // recomputes utransform*transform per triangle and normal() per covered sample; both
 // are the same value every time, so they are formed once (matrix on the host, normal
 // here) with the same operation order (record.cuh).
+#include <algorithm>
 #include <atomic>
 
 #include "bin_common.cuh"
@@ -312,6 +313,36 @@ cudaError_t launch_vertex_transform(const MeshDev &mesh, const Mat4 &M, float4 *
     if (mesh.nvert == 0) return cudaSuccess;
     const uint32_t quads = (mesh.nvert + 3) / 4;
     vertex_transform_kernel<<<(quads + 255) / 256, 256, 0, s>>>(mesh, M, tv);
+    return cudaGetLastError();
+}
+
+// A mesh's arrays from interleaved positions and packed colours: each element once, so bound
+// by its launch at the sizes meshes are refitted at (three strided copies and four memcpys
+// before).  The colours go by words where both ends allow it.
+__global__ void __launch_bounds__(256)
+mesh_split_kernel(const float *__restrict__ xyz, const uint8_t *__restrict__ rgb, float *x, float *y, float *z,
+                  uint8_t *rgb_out, uint32_t nvert, uint64_t nbytes, int words)
+{
+    const uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = i0; i < nvert; i += step) {
+        x[i] = xyz[3 * i];
+        y[i] = xyz[3 * i + 1];
+        z[i] = xyz[3 * i + 2];
+    }
+    const uint64_t nw = words ? nbytes / 4 : 0;
+    for (uint64_t i = i0; i < nw; i += step)
+        reinterpret_cast<uint32_t *>(rgb_out)[i] = reinterpret_cast<const uint32_t *>(rgb)[i];
+    for (uint64_t i = 4 * nw + i0; i < nbytes; i += step) rgb_out[i] = rgb[i];
+}
+
+cudaError_t launch_mesh_split(const float *xyz, const uint8_t *rgb, float *x, float *y, float *z, uint8_t *rgb_out,
+                              uint32_t nvert, uint32_t ntri, cudaStream_t s)
+{
+    const uint64_t n = std::max<uint64_t>(nvert, ntri);
+    if (n == 0) return cudaSuccess;
+    const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, 8ull * (uint64_t)device_sm_count());
+    mesh_split_kernel<<<(unsigned)blocks, 256, 0, s>>>(xyz, rgb, x, y, z, rgb_out, nvert, 3ull * ntri,
+                                                       (reinterpret_cast<uintptr_t>(rgb) & 3u) == 0);
     return cudaGetLastError();
 }
 

@@ -970,6 +970,16 @@ sloth_status sloth_mesh_update(sloth_mesh *m, const float *x, const float *y, co
     return SLOTH_OK;
 }
 
+sloth_status sloth_mesh_update_interleaved(sloth_mesh *m, const float *xyz, const uint8_t *rgb)
+{
+    if (!m || !m->ctx) return SLOTH_ERR_INVALID_ARGUMENT;
+    sloth_ctx *ctx = m->ctx;
+    if ((m->nvert && !xyz) || (m->ntri && !rgb)) return fail(ctx, SLOTH_ERR_INVALID_ARGUMENT, "xyz or rgb is NULL");
+    CU(ctx, cudaSetDevice(m->device));
+    CU(ctx, launch_mesh_split(xyz, rgb, m->x, m->y, m->z, m->rgb, m->nvert, m->ntri, ctx->stream));
+    return SLOTH_OK;
+}
+
 sloth_status sloth_mesh_info(const sloth_mesh *m, uint32_t *ntri, float bbox_max[3])
 {
     if (!m) return SLOTH_ERR_INVALID_ARGUMENT;

@@ -167,6 +167,10 @@ cudaError_t launch_clear_keys(uint64_t *keys, uint64_t ncells, int tw, bool even
 cudaError_t launch_frame_reset(const FrameBuffers &fb, const BinBuffers &bb, uint32_t nl_nodes, uint32_t ntiles,
                                bool frame, bool draw, bool tiles_current, cudaStream_t s);
 
+// positions split from x, y, z triples and face colours copied into a mesh's arrays.
+cudaError_t launch_mesh_split(const float *xyz, const uint8_t *rgb, float *x, float *y, float *z, uint8_t *rgb_out,
+                              uint32_t nvert, uint32_t ntri, cudaStream_t s);
+
 // vertex transform: tv[i] = (M*v_i).xyz (nalgebra order), float4 per vertex.
 cudaError_t launch_vertex_transform(const MeshDev &mesh, const Mat4 &M, float4 *tv,
                                     cudaStream_t s);

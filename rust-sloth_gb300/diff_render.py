@@ -48,30 +48,40 @@ class ShadedViews:
         self._keep = None
 
     def _check_stream(self):
-        if torch.cuda.current_stream(self.device).cuda_stream != self.stream.cuda_stream:
+        if torch.cuda.current_stream(self.ctx.device).cuda_stream != self.stream.cuda_stream:
             raise RuntimeError("ShadedViews used outside its stream")
 
     def render(self, pos: torch.Tensor):
         """Upload (nvert, 3) positions and render every view."""
         self._check_stream()
+        self._render(pos)
+
+    def _render(self, pos: torch.Tensor):
         p = pos.detach().to(torch.float32)
-        x, y, z = p[:, 0].contiguous(), p[:, 1].contiguous(), p[:, 2].contiguous()
-        self._keep = (x, y, z)          # the copies read them asynchronously
-        self.mesh.update_device(x.data_ptr(), y.data_ptr(), z.data_ptr(), self.face_rgb.data_ptr())
+        if p.device == self.device and p.shape == (self.nvert, 3):
+            self._keep = p = p.contiguous()     # the kernel reads it asynchronously
+            self.mesh.update_interleaved(p.data_ptr(), self.face_rgb.data_ptr())
+        else:                                   # host positions, or more rows or columns
+            x, y, z = p[:, 0].contiguous(), p[:, 1].contiguous(), p[:, 2].contiguous()
+            self._keep = (x, y, z)              # the copies read them asynchronously
+            self.mesh.update_device(x.data_ptr(), y.data_ptr(), z.data_ptr(), self.face_rgb.data_ptr())
         self.batch.render()
 
     def shade(self, vrgb: torch.Tensor, light: torch.Tensor) -> torch.Tensor:
         """(ncells, 3) f32 image of the last render."""
         self._check_stream()
+        return self._shade(vrgb, light)
+
+    def _shade(self, vrgb: torch.Tensor, light: torch.Tensor) -> torch.Tensor:
         out = torch.empty(self.ncells, 3, dtype=torch.float32, device=self.device)
         self.batch.shade(vrgb.data_ptr(), light.data_ptr(), out.data_ptr(), self.store_visibility)
         return out
 
     def shade_backward(self, vrgb, light, grad_rgb):
         self._check_stream()
-        gpos = torch.zeros(self.nvert, 3, dtype=torch.float32, device=self.device)
-        gcol = torch.zeros(self.nvert, 3, dtype=torch.float32, device=self.device)
-        gl = torch.zeros(3, dtype=torch.float32, device=self.device)
+        # one buffer, cleared at once
+        buf = torch.zeros(2 * self.nvert + 1, 3, dtype=torch.float32, device=self.device)
+        gpos, gcol, gl = buf[:self.nvert], buf[self.nvert:2 * self.nvert], buf[2 * self.nvert]
         self.batch.shade_backward(vrgb.data_ptr(), light.data_ptr(), grad_rgb.data_ptr(), gpos.data_ptr(),
                                   gcol.data_ptr(), gl.data_ptr())
         return gpos, gcol, gl
@@ -90,8 +100,9 @@ class _ShadeFn(torch.autograd.Function):
     def forward(ctx, pos, vrgb, light, views: ShadedViews):
         vrgb_c = vrgb.detach().contiguous().to(torch.float32)
         light_c = light.detach().contiguous().to(torch.float32)
-        views.render(pos)
-        rgb = views.shade(vrgb_c, light_c)
+        views._check_stream()
+        views._render(pos)
+        rgb = views._shade(vrgb_c, light_c)
         ctx.views = views
         ctx.save_for_backward(vrgb_c, light_c)
         return rgb
