@@ -764,8 +764,8 @@ sloth_status sloth_batch_flush(sloth_batch *b, uint32_t frame, int format, char 
     sloth_status st = settle(b);
     if (st != SLOTH_OK) return st;
     const uint64_t nc = b->cell_off[frame + 1] - b->cell_off[frame];
-    BCU(b, flush_run(b->flush, b->cells + b->cell_off[frame], nc, b->frames[frame].image ? 1 : 0, format, b->stream,
-                     bytes));
+    BCU(b, flush_run(b->flush, b->cells + b->cell_off[frame], nc, b->frames[frame].image ? 1 : 0, format,
+                     out != nullptr, b->stream, bytes));
     if (!out) return SLOTH_OK;
     if (capacity < *bytes) return sloth_ctx_fail(b->ctx, SLOTH_ERR_LIMIT, "flush output buffer too small");
     BCU(b, cudaMemcpyAsync(out, b->flush.out, *bytes, cudaMemcpyDeviceToHost, b->stream));

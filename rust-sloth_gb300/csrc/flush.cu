@@ -14,7 +14,7 @@
 //
 // Three launches: per-chunk byte counts, one block scanning the chunk counts, and the
 // formatter, which builds each chunk's text in shared memory and writes it out in one
-// contiguous run.
+// contiguous run.  A call that only asks for the size stops after the scan.
 #include <cstdint>
 
 #include "flush_kernels.h"
@@ -38,65 +38,85 @@ __device__ __forceinline__ uint32_t cell_bytes(uint32_t cell, int format)
     return format == kFlushAnsi ? 31u + d : 29u + d;
 }
 
-__device__ __forceinline__ uint32_t put_str(char *o, const char *s)
-{
-    uint32_t n = 0;
-    while (s[n]) {
-        o[n] = s[n];
-        ++n;
+// Appends bytes to a run of shared text, a word at a time: the bytes collect in a 64-bit
+// register and leave as whole words, so a cell costs about ten stores instead of forty.
+// The first and last words of a thread's run are shared with its neighbours' and are
+// written by bytes.
+struct Emit {
+    char *text;
+    uint32_t pos;     // byte position of the collected bytes' word (a multiple of 4)
+    uint32_t fill;    // bytes in the register, those before the run's start included
+    uint32_t skip;    // bytes of the first word that belong to the run before
+    uint64_t acc;
+
+    __device__ __forceinline__ Emit(char *t, uint32_t off) : text(t), pos(off & ~3u), fill(off & 3u), skip(off & 3u), acc(0) {}
+    // n bytes (1..4) from the low end of w; the bytes above them are zero
+    __device__ __forceinline__ void put(uint32_t w, uint32_t n)
+    {
+        acc |= (uint64_t)w << (8 * fill);
+        fill += n;
+        if (fill >= 4) {
+            if (skip) {
+                for (uint32_t k = skip; k < 4; ++k) text[pos + k] = (char)(acc >> (8 * k));
+                skip = 0;
+            } else {
+                *reinterpret_cast<uint32_t *>(text + pos) = (uint32_t)acc;
+            }
+            acc >>= 32;
+            pos += 4;
+            fill -= 4;
+        }
     }
-    return n;
+    __device__ __forceinline__ void end()
+    {
+        for (uint32_t k = skip; k < fill; ++k) text[pos + k] = (char)(acc >> (8 * k));
+    }
+    // a decimal number (0..255) and the character after it
+    __device__ __forceinline__ void number(uint32_t v, uint32_t after)
+    {
+        const uint32_t h = v / 100, t = v / 10 - 10 * h, u = v - 10 * (v / 10);
+        const uint32_t n = ndigits(v);
+        const uint32_t d = n == 3 ? (h | t << 8 | u << 16) + 0x303030u : n == 2 ? (t | u << 8) + 0x3030u : u + 0x30u;
+        put(d | after << (8 * n), n + 1);
+    }
+};
+
+__host__ __device__ constexpr uint32_t word4(const char *s)
+{
+    return (uint32_t)(uint8_t)s[0] | (uint32_t)(uint8_t)s[1] << 8 | (uint32_t)(uint8_t)s[2] << 16 |
+           (uint32_t)(uint8_t)s[3] << 24;
+}
+__host__ __device__ constexpr uint32_t word3(const char *s)
+{
+    return (uint32_t)(uint8_t)s[0] | (uint32_t)(uint8_t)s[1] << 8 | (uint32_t)(uint8_t)s[2] << 16;
 }
 
-__device__ __forceinline__ uint32_t put_u8(char *o, uint32_t v)
+__device__ __forceinline__ void put_cell(Emit &o, uint32_t cell, int format)
 {
-    if (v >= 100) {
-        o[0] = (char)('0' + v / 100);
-        o[1] = (char)('0' + (v / 10) % 10);
-        o[2] = (char)('0' + v % 10);
-        return 3;
-    }
-    if (v >= 10) {
-        o[0] = (char)('0' + v / 10);
-        o[1] = (char)('0' + v % 10);
-        return 2;
-    }
-    o[0] = (char)('0' + v);
-    return 1;
-}
-
-__device__ __forceinline__ uint32_t put_cell(char *o, uint32_t cell, int format)
-{
-    const char ch = (char)(cell & 255u);
+    const uint32_t ch = cell & 255u;
     if (format == kFlushPlain) {
-        o[0] = ch;
-        return 1;
+        o.put(ch, 1);
+        return;
     }
     const uint32_t r = (cell >> 8) & 255u, g = (cell >> 16) & 255u, b = cell >> 24;
-    uint32_t n = 0;
     if (format == kFlushAnsi) {
-        n += put_str(o + n, "\x1b[48;2;25;25;25m\x1b[38;2;");
-        n += put_u8(o + n, r);
-        o[n++] = ';';
-        n += put_u8(o + n, g);
-        o[n++] = ';';
-        n += put_u8(o + n, b);
-        o[n++] = 'm';
-        o[n++] = ch;
-        n += put_str(o + n, "\x1b[0m");
+        constexpr uint32_t w0 = word4("\x1b[48"), w1 = word4(";2;2"), w2 = word4("5;25"), w3 = word4(";25m"),
+                           w4 = word4("\x1b[38"), w5 = word3(";2;"), w6 = word3("\x1b[0");
+        o.put(w0, 4); o.put(w1, 4); o.put(w2, 4); o.put(w3, 4); o.put(w4, 4); o.put(w5, 3);
+        o.number(r, ';');
+        o.number(g, ';');
+        o.number(b, 'm');
+        o.put(ch | w6 << 8, 4);
+        o.put('m', 1);
     } else {
-        n += put_str(o + n, "<span style=\"color:rgb(");
-        n += put_u8(o + n, r);
-        o[n++] = ',';
-        n += put_u8(o + n, g);
-        o[n++] = ',';
-        n += put_u8(o + n, b);
-        o[n++] = ')';
-        o[n++] = '"';
-        o[n++] = '>';
-        o[n++] = ch;
+        constexpr uint32_t w0 = word4("<spa"), w1 = word4("n st"), w2 = word4("yle="), w3 = word4("\"col"),
+                           w4 = word4("or:r"), w5 = word3("gb(");
+        o.put(w0, 4); o.put(w1, 4); o.put(w2, 4); o.put(w3, 4); o.put(w4, 4); o.put(w5, 3);
+        o.number(r, ',');
+        o.number(g, ',');
+        o.number(b, ')');
+        o.put((uint32_t)'"' | (uint32_t)'>' << 8 | ch << 16, 3);
     }
-    return n;
 }
 
 // Block-wide exclusive scan of one value per thread; returns the prefix, *total the sum.
@@ -182,13 +202,17 @@ flush_scan_kernel(uint64_t *__restrict__ chunk_bytes, uint32_t nchunks, uint32_t
     if (threadIdx.x == 0) *size = carry + suffix;
 }
 
-// Each block formats its chunk into shared memory, then copies it out.
+// Each block formats its chunk into shared memory, then copies it out: the text starts at
+// the place in shared memory that its destination has in a 16-byte line, so that all but
+// the ends go out in 16-byte stores.  The ends of the whole text (a terminal's MoveTo, the
+// line feed of the plain form) are the first and last blocks'.  230k cells of HTML took
+// 39 us with byte stores, in shared memory and out of it, and 13 us as here.
 __global__ void __launch_bounds__(kFlushThreads)
 flush_write_kernel(const uint32_t *__restrict__ cells, uint64_t ncells, int format,
-                   const uint64_t *__restrict__ chunk_off, char *__restrict__ out)
+                   const uint64_t *__restrict__ chunk_off, char *__restrict__ out, int image, int suffix)
 {
     __shared__ uint32_t ws[32];
-    __shared__ char text[kFlushChunk * kMaxCellBytes];
+    __shared__ __align__(16) char text[kFlushChunk * kMaxCellBytes + 16];
     const uint64_t c0 = (uint64_t)blockIdx.x * kFlushChunk + (uint64_t)threadIdx.x * kFlushCellsPerThread;
     uint32_t cv[kFlushCellsPerThread];
     uint32_t n = 0;
@@ -198,27 +222,33 @@ flush_write_kernel(const uint32_t *__restrict__ cells, uint64_t ncells, int form
         if (c0 + k < ncells) n += cell_bytes(cv[k], format);
     }
     uint32_t total;
-    uint32_t off = block_exclusive_scan(n, ws, &total);
+    const uint32_t off = block_exclusive_scan(n, ws, &total);
+    char *dst = out + chunk_off[blockIdx.x];
+    const uint32_t lead = (uint32_t)reinterpret_cast<uintptr_t>(dst) & 15u;
+    Emit o(text, lead + off);
 #pragma unroll
     for (int k = 0; k < kFlushCellsPerThread; ++k)
-        if (c0 + k < ncells) off += put_cell(text + off, cv[k], format);
+        if (c0 + k < ncells) put_cell(o, cv[k], format);
+    o.end();
     block_sync();
-    char *dst = out + chunk_off[blockIdx.x];
-    for (uint32_t i = threadIdx.x; i < total; i += blockDim.x) dst[i] = text[i];
-}
-
-__global__ void flush_ends_kernel(char *__restrict__ out, const uint64_t *__restrict__ size, int image, int suffix)
-{
-    if (threadIdx.x != 0) return;
-    if (!image) {
-        out[0] = '\x1b';
-        out[1] = '[';
-        out[2] = '1';
-        out[3] = ';';
-        out[4] = '1';
-        out[5] = 'H';
+    // bytes [lead, lead + total) of text: line i of 16 bytes starts at dst - lead + 16*i
+    char *line0 = dst - lead;
+    const uint32_t last = lead + total;
+    for (uint32_t i = threadIdx.x; 16 * i < last; i += blockDim.x) {
+        const uint32_t b0 = 16 * i;
+        if (b0 >= lead && b0 + 16 <= last) {
+            reinterpret_cast<uint4 *>(line0)[i] = reinterpret_cast<const uint4 *>(text)[i];
+        } else {
+            for (uint32_t k = max(b0, lead); k < min(b0 + 16, last); ++k) line0[k] = text[k];
+        }
     }
-    if (suffix) out[*size - 1] = '\n';
+    if (threadIdx.x == 0) {
+        if (blockIdx.x == 0 && !image) {
+            const char move[6] = {'\x1b', '[', '1', ';', '1', 'H'};
+            for (int k = 0; k < 6; ++k) out[k] = move[k];
+        }
+        if (blockIdx.x == gridDim.x - 1 && suffix) dst[total] = '\n';
+    }
 }
 
 }  // namespace
@@ -241,12 +271,12 @@ cudaError_t launch_flush(const uint32_t *cells, uint64_t ncells, int image, int 
     const uint32_t suffix = format == kFlushPlain ? 1u : 0u;
     if (nch) flush_count_kernel<<<nch, kFlushThreads, 0, s>>>(cells, ncells, format, chunk_bytes);
     flush_scan_kernel<<<1, 1024, 0, s>>>(chunk_bytes, nch, prefix, suffix, size);
-    if (nch) flush_write_kernel<<<nch, kFlushThreads, 0, s>>>(cells, ncells, format, chunk_bytes, out);
-    flush_ends_kernel<<<1, 32, 0, s>>>(out, size, image, (int)suffix);
+    if (nch && out)
+        flush_write_kernel<<<nch, kFlushThreads, 0, s>>>(cells, ncells, format, chunk_bytes, out, image, (int)suffix);
     return cudaGetLastError();
 }
 
-cudaError_t flush_run(FlushScratch &f, const uint32_t *cells, uint64_t ncells, int image, int format,
+cudaError_t flush_run(FlushScratch &f, const uint32_t *cells, uint64_t ncells, int image, int format, bool text,
                       cudaStream_t s, uint64_t *bytes)
 {
     cudaError_t e;
@@ -270,7 +300,8 @@ cudaError_t flush_run(FlushScratch &f, const uint32_t *cells, uint64_t ncells, i
         if ((e = cudaMalloc(&f.out, need)) != cudaSuccess) return e;
         f.out_cap = need;
     }
-    if ((e = launch_flush(cells, ncells, image, format, f.chunks, f.size_d, f.out, s)) != cudaSuccess) return e;
+    if ((e = launch_flush(cells, ncells, image, format, f.chunks, f.size_d, text ? f.out : nullptr, s)) != cudaSuccess)
+        return e;
     if ((e = cudaMemcpyAsync(f.size_h, f.size_d, sizeof(uint64_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
         return e;
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;

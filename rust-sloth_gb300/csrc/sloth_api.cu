@@ -654,7 +654,7 @@ sloth_status sloth_ctx_read(sloth_ctx *ctx, uint32_t *cells, float *z, int32_t *
     return report_device_error(ctx);
 }
 
-static sloth_status ctx_flush(sloth_ctx *ctx, int format, uint64_t *bytes)
+static sloth_status ctx_flush(sloth_ctx *ctx, int format, bool text, uint64_t *bytes)
 {
     if (format < SLOTH_FLUSH_PLAIN || format > SLOTH_FLUSH_HTML)
         return fail(ctx, SLOTH_ERR_INVALID_ARGUMENT, "unknown flush format %d", format);
@@ -665,7 +665,7 @@ static sloth_status ctx_flush(sloth_ctx *ctx, int format, uint64_t *bytes)
     const uint64_t ncells = ctx->g.image ? nz + ctx->g.h : nz;
     if ((st = queue_error_copy(ctx)) != SLOTH_OK) return st;
     CU(ctx, timed(ctx, "flush", [&] {
-        return flush_run(ctx->flush, ctx->fb.cells_out, ncells, ctx->g.image, format, ctx->stream, bytes);
+        return flush_run(ctx->flush, ctx->fb.cells_out, ncells, ctx->g.image, format, text, ctx->stream, bytes);
     }));
     return report_device_error(ctx);
 }
@@ -674,7 +674,7 @@ sloth_status sloth_ctx_flush(sloth_ctx *ctx, int format, char *out, uint64_t cap
 {
     if (!ctx) return SLOTH_ERR_INVALID_ARGUMENT;
     if (!bytes) return fail(ctx, SLOTH_ERR_INVALID_ARGUMENT, "bytes is NULL");
-    sloth_status st = ctx_flush(ctx, format, bytes);
+    sloth_status st = ctx_flush(ctx, format, out != nullptr, bytes);
     if (st != SLOTH_OK || !out) return st;
     if (capacity < *bytes) return fail(ctx, SLOTH_ERR_LIMIT, "flush needs %llu bytes", (unsigned long long)*bytes);
     CU(ctx, cudaMemcpyAsync(out, ctx->flush.out, *bytes, cudaMemcpyDeviceToHost, ctx->stream));
@@ -686,7 +686,7 @@ sloth_status sloth_ctx_flush_device(sloth_ctx *ctx, int format, const char **dev
 {
     if (!ctx) return SLOTH_ERR_INVALID_ARGUMENT;
     if (!bytes || !device_bytes) return fail(ctx, SLOTH_ERR_INVALID_ARGUMENT, "bytes/device_bytes is NULL");
-    sloth_status st = ctx_flush(ctx, format, bytes);
+    sloth_status st = ctx_flush(ctx, format, true, bytes);
     if (st != SLOTH_OK) return st;
     *device_bytes = ctx->flush.out;
     return SLOTH_OK;
