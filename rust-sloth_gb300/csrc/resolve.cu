@@ -1,5 +1,7 @@
 // resolve.cu -- depth keys -> depth buffer, frame cells and winners (one frame).
 // The per-cell rule is in resolve_common.cuh.
+#include <algorithm>
+
 #include "launch.cuh"
 #include "resolve_common.cuh"
 
@@ -41,6 +43,32 @@ cudaError_t launch_resolve(const FrameGeom &g, const FrameBuffers &fb, cudaStrea
     const int vec = ((reinterpret_cast<uintptr_t>(fb.cells_out) | reinterpret_cast<uintptr_t>(fb.z_out) |
                       reinterpret_cast<uintptr_t>(fb.winner_out)) & (4u * kRun - 1u)) == 0;
     return launch_pdl(resolve_kernel, dim3((unsigned)blocks), dim3(256), 0, s, g, fb, vec);
+}
+
+// A small frame's buffers and the error word into one page-locked buffer, by words of 16
+// bytes (the sources start allocations, the parts of the destination 16-byte lines; a part's
+// last line is copied by words).  Three or four copies of a few kilobytes cost the host and
+// the copy engine about 10 us each; this is one launch behind the resolve.
+__global__ void __launch_bounds__(256) readback_kernel(ReadBack r)
+{
+    pdl_trigger();
+    const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x + pdl_wait(), step = gridDim.x * blockDim.x;
+    if (i0 == 0) *r.error_out = *r.error;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (!r.n[k]) continue;
+        const uint32_t n = r.n[k];
+        for (uint32_t i = i0; i < n / 4; i += step)
+            reinterpret_cast<uint4 *>(r.out[k])[i] = reinterpret_cast<const uint4 *>(r.in[k])[i];
+        if (i0 < (n & 3u)) r.out[k][(n & ~3u) + i0] = r.in[k][(n & ~3u) + i0];
+    }
+}
+
+cudaError_t launch_readback(const ReadBack &r, cudaStream_t s)
+{
+    const uint32_t most = (std::max(r.n[0], std::max(r.n[1], r.n[2])) + 3) / 4;
+    const uint32_t blocks = std::max(1u, std::min((most + 255) / 256, (uint32_t)device_sm_count()));
+    return launch_pdl(readback_kernel, dim3(blocks), dim3(256), 0, s, r);
 }
 
 }  // namespace sloth

@@ -84,6 +84,7 @@ struct sloth_ctx {
     bool max_pending = false;      // a copy of d_max is on its way
     unsigned long long *h_frags = nullptr;   // pinned
     uint32_t *h_error = nullptr;   // pinned copy of fb.error
+    uint32_t *h_stage = nullptr;   // pinned: a small frame's buffers on their way to the caller
     uint32_t tri_base = 0;
     bool dirty = true;
     bool reset_pending = false;    // a clear's resets, folded into the next launch that needs them
@@ -554,6 +555,7 @@ void sloth_ctx_destroy(sloth_ctx *ctx)
     if (ctx->aux_ev) cudaEventDestroy(ctx->aux_ev);
     if (ctx->h_frags) cudaFreeHost(ctx->h_frags);
     if (ctx->h_error) cudaFreeHost(ctx->h_error);
+    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     dfree(ctx->fb.error);
     if (ctx->h_max) cudaFreeHost(ctx->h_max);
     dfree(ctx->d_max);
@@ -633,6 +635,41 @@ sloth_status sloth_ctx_sizes(const sloth_ctx *ctx, uint64_t *frame_cells, uint64
     return SLOTH_OK;
 }
 
+// Frames of at most kStageCells cells are read through page-locked memory (readback_kernel):
+// 160x48 with all three buffers 71 us a frame with a copy each, 43 so; larger ones keep
+// the copy engine, whose copies need no second pass over the bytes on the host.
+constexpr size_t kStageCells = 32768;
+static bool stage_memory(sloth_ctx *ctx)
+{
+    if (cudaMallocHost(&ctx->h_stage, (3 * (kStageCells + 4) + 4) * sizeof(uint32_t)) == cudaSuccess) return true;
+    cudaGetLastError();
+    ctx->h_stage = nullptr;
+    return false;
+}
+
+static sloth_status read_staged(sloth_ctx *ctx, uint32_t *cells, float *z, int32_t *winner, uint32_t ncells,
+                                uint32_t nz)
+{
+    ReadBack r{};
+    r.error = ctx->fb.error;
+    r.error_out = ctx->h_stage;
+    const void *in[3] = {ctx->fb.cells_out, ctx->fb.z_out, ctx->fb.winner_out};
+    void *to[3] = {cells, z, winner};
+    uint32_t at = 4;
+    for (int k = 0; k < 3; ++k) {
+        r.in[k] = static_cast<const uint32_t *>(in[k]);
+        r.out[k] = ctx->h_stage + at;
+        r.n[k] = !to[k] ? 0u : k == 0 ? ncells : nz;
+        at += (r.n[k] + 3u) & ~3u;
+    }
+    CU(ctx, timed(ctx, "readback", [&] { return launch_readback(r, ctx->stream); }));
+    CU(ctx, cudaStreamSynchronize(ctx->stream));
+    for (int k = 0; k < 3; ++k)
+        if (r.n[k]) memcpy(to[k], r.out[k], r.n[k] * sizeof(uint32_t));
+    *ctx->h_error = ctx->h_stage[0];
+    return report_device_error(ctx);
+}
+
 sloth_status sloth_ctx_read(sloth_ctx *ctx, uint32_t *cells, float *z, int32_t *winner)
 {
     if (!ctx) return SLOTH_ERR_INVALID_ARGUMENT;
@@ -641,6 +678,8 @@ sloth_status sloth_ctx_read(sloth_ctx *ctx, uint32_t *cells, float *z, int32_t *
     if (st != SLOTH_OK) return st;
     const size_t nz = (size_t)ctx->g.w * ctx->g.h;
     const size_t ncells = ctx->g.image ? nz + ctx->g.h : nz;
+    if (ncells <= kStageCells && (ctx->h_stage || stage_memory(ctx)))
+        return read_staged(ctx, cells, z, winner, (uint32_t)ncells, (uint32_t)nz);
     if (cells)
         CU(ctx, cudaMemcpyAsync(cells, ctx->fb.cells_out, ncells * sizeof(uint32_t),
                                 cudaMemcpyDeviceToHost, ctx->stream));

@@ -235,6 +235,17 @@ cudaError_t launch_raster(const FrameGeom &g, const FrameBuffers &fb, const BinB
 // resolve: keys -> z, frame cells, winners.
 cudaError_t launch_resolve(const FrameGeom &g, const FrameBuffers &fb, cudaStream_t s);
 
+// Copies of up to three device buffers (cells, depth, winners; n words each, 0: none) and the
+// error word into page-locked host memory.
+struct ReadBack {
+    const uint32_t *in[3];
+    uint32_t *out[3];
+    uint32_t n[3];
+    const uint32_t *error;
+    uint32_t *error_out;
+};
+cudaError_t launch_readback(const ReadBack &r, cudaStream_t s);
+
 constexpr int kTileW = 64;   // default tile: cells (even)
 constexpr int kTileH = 32;   // rows
 
