@@ -43,6 +43,7 @@ struct TileSmem {
     uint32_t next, zmax_u, zmax_w;
     uint32_t rmu[32], rmw[32];          // the same bounds per row of the tile
     uint32_t frags[kRasterThreads / 32];
+    int spans[kRasterThreads / 32][32]; // per warp: the rows of its walk (raster_part)
 };
 
 // ---- bulk copies of the key tile (cp.async.bulk, completion on an mbarrier) ----
@@ -109,17 +110,25 @@ __device__ __forceinline__ void fence_proxy_async_smem()
 constexpr uint32_t kWaitPolls = 1u << 22;   // polls of a bulk-copy barrier before giving up
 constexpr uint32_t kTestWaitPolls = 1u << 10;   // the same under the wait test hook
 
+// Index of sample (x, y)'s key in the tile at (R0, C0), less y*TW + x: the key of column 2x
+// of row y (unwrapped), or of column 2x - w of row y+1 (wrapped; odd columns, of an odd
+// width, are the second half of the row).
+template <int TW, int kNotWrapped>
+__device__ __forceinline__ int key_base(int R0, int C0, int w)
+{
+    return kNotWrapped ? -R0 * TW - (C0 >> 1)
+                       : (1 - R0) * TW + ((w & 1) ? TW / 2 : 0) - ((w + C0 + 1) >> 1);
+}
+
 // One sample of the reference's loop body: edge test, depth, key folded into the tile.
 // With a depth bound zb of the triangle in this tile (0: none), a cell already nearer
 // than zb is passed over before the edge test: no depth of the triangle can beat it.
 template <int TW, int kNotWrapped>
-__device__ __forceinline__ void fold_sample(const TriRecord &r, uint32_t gtri, int x, int y, int R0, int C0,
-                                            int w, unsigned long long *skeys, uint32_t &frags, uint32_t zb,
+__device__ __forceinline__ void fold_sample(const TriRecord &r, uint32_t gtri, int x, int y, int kbase,
+                                            unsigned long long *skeys, uint32_t &frags, uint32_t zb,
                                             const EdgeRows *rows = nullptr)
 {
-    const int row = kNotWrapped ? (y - R0) : (y + 1 - R0);
-    const int col = kNotWrapped ? (2 * x - C0) : (2 * x - w - C0);
-    unsigned long long *p = &skeys[row * TW + key_col(col, TW)];
+    unsigned long long *p = &skeys[kbase + y * TW + x];
     if (zb > *(volatile const uint32_t *)(reinterpret_cast<const uint32_t *>(p) + 1)) return;
     // with the row's edge terms given (a walk along one row), only the column terms remain
     const EdgeVals e = rows ? eval_edges_row(r, *rows, (float)x) : eval_edges(r, (float)x, (float)y);
@@ -166,18 +175,19 @@ constexpr int kSpanMinSamples = 128;
 // kFlagFiniteXY: lane i bounds row c.ya + i to the columns that can pass all three edges
 // (at most 32 rows: a part lies in one tile) -- none when the row's depth bound (rowmax,
 // indexed by tile row) is below the entry's depth bound zb -- and the warp walks the
-// concatenated spans
-// 32 samples at a time, each lane finding its row by a binary search over the spans'
-// running ends.  Otherwise the rectangle, row-major, 32 samples at a time.  Every walked
-// sample gets the exact test.
+// concatenated spans 32 samples at a time.  A step's rows are found from the bits of the
+// spans that start in it: the rows that are not empty leave their number and column offset
+// in the warp's spans array in order, and a lane's row is the one the starts up to its
+// sample count to (a binary search over the spans' ends by shuffles took twice the
+// instructions, and the raster is bound by their issue).  Otherwise the rectangle,
+// row-major, 32 samples at a time.  Every walked sample gets the exact test.
 template <int TW, int kNotWrapped>
-__device__ __forceinline__ void raster_part(const TriRecord &r, uint32_t gtri, Rect c, int R0,
+__device__ __forceinline__ void raster_part(const TriRecord &r, uint32_t gtri, const Rect &c, int R0,
                                             int C0, int w, unsigned long long *skeys, int lane,
-                                            uint32_t &frags, const uint32_t *rowmax, uint32_t zb)
+                                            uint32_t &frags, const uint32_t *rowmax, uint32_t zb, int *spans)
 {
-    if (c.empty()) return;
     const bool finite = (r.flags & kFlagFiniteXY) != 0;
-    if (finite && !rect_may_cover(r, c)) return;
+    const int kbase = key_base<TW, kNotWrapped>(R0, C0, w);
     const int bw = c.xb - c.xa;
     const int area = bw * (c.yb - c.ya);
     if (finite && area > kSpanMinSamples) {
@@ -197,16 +207,22 @@ __device__ __forceinline__ void raster_part(const TriRecord &r, uint32_t gtri, R
             if (lane >= d) end += o;
         }
         const int total = __shfl_sync(0xffffffffu, end, 31);
-        const int xoff = lo - (end - len);   // column of span sample k of this row: k + xoff
+        const int start = end - len;
+        const unsigned some = __ballot_sync(0xffffffffu, len > 0);
+        __syncwarp();   // the lanes have read the spans of the warp's last walk
+        // (column of span sample k of this row less k, row of the part)
+        if (len > 0) spans[__popc(some & ((1u << lane) - 1u))] = (lo - start) * 32 + lane;
+        __syncwarp();
+        int rank = -1;   // rows that start before this step, less one
+        const int y0 = c.ya;
         for (int base = 0; base < total; base += 32) {
+            const unsigned at = (unsigned)(start - base);
+            const unsigned starts = __reduce_or_sync(0xffffffffu, len > 0 && at < 32u ? 1u << at : 0u);
             const int k = base + lane;
-            // the row of sample k: the number of rows whose spans end at or before k
-            int row = 0;
-#pragma unroll
-            for (int step = 16; step > 0; step >>= 1)
-                if (__shfl_sync(0xffffffffu, end, row + step - 1) <= k) row += step;
-            const int x = k + __shfl_sync(0xffffffffu, xoff, row);
-            if (k < total) fold_sample<TW, kNotWrapped>(r, gtri, x, c.ya + row, R0, C0, w, skeys, frags, zb);
+            const int sp = spans[rank + __popc(starts & (0xffffffffu >> (31 - lane)))];
+            rank += __popc(starts);
+            const int x = k + (sp >> 5);
+            if (k < total) fold_sample<TW, kNotWrapped>(r, gtri, x, y0 + (sp & 31), kbase, skeys, frags, zb);
         }
         return;
     }
@@ -216,7 +232,7 @@ __device__ __forceinline__ void raster_part(const TriRecord &r, uint32_t gtri, R
     const int q = (int)(32.5f * rbw), rem = 32 - q * bw;
     int dy = (int)(((float)lane + 0.5f) * rbw), dx = lane - dy * bw;
     for (int k = lane; k < area; k += 32) {
-        fold_sample<TW, kNotWrapped>(r, gtri, c.xa + dx, c.ya + dy, R0, C0, w, skeys, frags, zb);
+        fold_sample<TW, kNotWrapped>(r, gtri, c.xa + dx, c.ya + dy, kbase, skeys, frags, zb);
         dx += rem;
         dy += q;
         if (dx >= bw) {
@@ -250,10 +266,11 @@ template <int TW, int kNotWrapped>
 __device__ __forceinline__ void raster_serial(const TriRecord &r, uint32_t gtri, const Rect &c, int R0, int C0,
                                               int w, unsigned long long *skeys, uint32_t &frags, uint32_t zb)
 {
+    const int kbase = key_base<TW, kNotWrapped>(R0, C0, w);
     for (int y = c.ya; y < c.yb; ++y) {
         const EdgeRows rows = edge_rows(r, (float)y);
         for (int x = c.xa; x < c.xb; ++x)
-            fold_sample<TW, kNotWrapped>(r, gtri, x, y, R0, C0, w, skeys, frags, zb, &rows);
+            fold_sample<TW, kNotWrapped>(r, gtri, x, y, kbase, skeys, frags, zb, &rows);
     }
 }
 
@@ -510,22 +527,27 @@ __device__ __forceinline__ bool raster_tile(TileSmem<TW, TH> &S, const FrameGeom
                 if ((uint32_t)(ent >> 32) > (((uint32_t)ent & 0x80000000u) ? max(zu, zw) : zu)) live = false;
             }
             const uint32_t gtri = (uint32_t)ent & 0x7fffffffu;
+            // An entry without wrapped samples in this tile has unwrapped ones, whose exact
+            // corner test listed it (tile_hit): they need neither the test again nor the
+            // wrapped part's clipping.
+            const bool wraps = ((uint32_t)ent & 0x80000000u) != 0;
             // the sample range (x0, xe, y0, y1) alone sizes the tile's part of the triangle
             int area = 0;
             if (live) {
                 const int4 xr = __ldg(reinterpret_cast<const int4 *>(fb.records + gtri) + 4);
                 const Rect U = unwrapped_part(vp, xr.x, xr.y, xr.z, xr.w);
-                const Rect W = wrapped_part(vp, xr.x, xr.y, xr.z, xr.w);
                 if (!U.empty()) area += rect_area(clip_unwrapped(vp, U, tr, tc));
-                if (!W.empty()) area += rect_area(clip_wrapped(vp, W, tr, tc));
+                if (wraps) area += rect_area(clip_wrapped(vp, wrapped_part(vp, xr.x, xr.y, xr.z, xr.w), tr, tc));
             }
             const int small = __popc(__ballot_sync(0xffffffffu, live && area <= kSerialWideSamples));
             const bool serial = live && area <= (small >= 16 ? kSerialWideSamples : kSerialMaxSamples);
             if (serial) {
                 const TriRecord r = load_record(fb.records, gtri);
                 const uint32_t zb = depth_cull ? (uint32_t)(ent >> 32) : 0u;
-                raster_serial<TW, 1>(r, gtri, tile_part<1>(r, vp, tr, tc), R0, C0, g.w, S.keys, frags, zb);
-                raster_serial<TW, 0>(r, gtri, tile_part<0>(r, vp, tr, tc), R0, C0, g.w, S.keys, frags, zb);
+                const Rect cu = wraps ? tile_part<1>(r, vp, tr, tc)
+                                      : clip_unwrapped(vp, unwrapped_part(vp, r.x0, r.xe, r.y0, r.y1), tr, tc);
+                raster_serial<TW, 1>(r, gtri, cu, R0, C0, g.w, S.keys, frags, zb);
+                if (wraps) raster_serial<TW, 0>(r, gtri, tile_part<0>(r, vp, tr, tc), R0, C0, g.w, S.keys, frags, zb);
             }
             unsigned coop = __ballot_sync(0xffffffffu, live && !serial);
             while (coop) {
@@ -546,17 +568,19 @@ __device__ __forceinline__ bool raster_tile(TileSmem<TW, TH> &S, const FrameGeom
                 }
                 const int src = __ffs(coop) - 1;
                 coop &= coop - 1;
-                const uint32_t gt = __shfl_sync(0xffffffffu, gtri, src);
+                const uint32_t lo = __shfl_sync(0xffffffffu, (uint32_t)ent, src), gt = lo & 0x7fffffffu;
                 const uint32_t zb = depth_cull ? __shfl_sync(0xffffffffu, (uint32_t)(ent >> 32), src) : 0u;
                 const TriRecord r = load_record(fb.records, gt);
-                const Rect U = unwrapped_part(vp, r.x0, r.xe, r.y0, r.y1);
-                if (!U.empty())
-                    raster_part<TW, 1>(r, gt, clip_unwrapped(vp, U, tr, tc), R0, C0, g.w, S.keys, lane, frags,
-                                       S.rmu, zb);
-                const Rect W = wrapped_part(vp, r.x0, r.xe, r.y0, r.y1);
-                if (!W.empty())
-                    raster_part<TW, 0>(r, gt, clip_wrapped(vp, W, tr, tc), R0, C0, g.w, S.keys, lane, frags,
-                                       S.rmw, zb);
+                if (!(lo & 0x80000000u)) {
+                    const Rect c = clip_unwrapped(vp, unwrapped_part(vp, r.x0, r.xe, r.y0, r.y1), tr, tc);
+                    raster_part<TW, 1>(r, gt, c, R0, C0, g.w, S.keys, lane, frags, S.rmu, zb, S.spans[wid]);
+                } else {
+                    const Rect cu = tile_part<1>(r, vp, tr, tc), cw = tile_part<0>(r, vp, tr, tc);
+                    if (!cu.empty())
+                        raster_part<TW, 1>(r, gt, cu, R0, C0, g.w, S.keys, lane, frags, S.rmu, zb, S.spans[wid]);
+                    if (!cw.empty())
+                        raster_part<TW, 0>(r, gt, cw, R0, C0, g.w, S.keys, lane, frags, S.rmw, zb, S.spans[wid]);
+                }
             }
         }
         block_sync();
