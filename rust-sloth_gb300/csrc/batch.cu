@@ -445,37 +445,44 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterMinBlocks) batch_raster
 }
 
 // blocks[i] = (frame, first cell): runs of kBatchRun frame cells per lane (resolve_run),
-// written with one store per buffer when the frame's outputs are aligned.  Four resident
-// blocks per SM (64 registers, no spills): the winners' record loads are latency-bound, and
-// the fourth block's loads in flight took config 3 from 3.33 to 3.22 ms.
+// written with one store per buffer when the frame's outputs are aligned.  Eight resident
+// blocks per SM (32 registers): the winners' record loads are latency-bound, and the warps
+// that wait on them at once count more than the loads each has in flight (uneven batch:
+// four blocks with four pairs of cells a thread 297 us, eight blocks with two 229).
 constexpr int kBatchRun = 2;
 static_assert(kFoldBlockTris == kFoldTris, "the host's table steps by the block's triangles");
 static_assert(kBatchResolveChunk % (kBatchRun * 256) == 0 && kBatchResolveSmall % (kBatchRun * 256) == 0,
               "whole runs, the same trip count in every warp");
 
-__global__ void __launch_bounds__(256, 4) batch_resolve_kernel(BatchDev b, const int2 *__restrict__ blocks)
+constexpr int kBatchPairs = 2;   // pairs of cells per thread of an even-width frame
+
+// kOdd: the batch has frames of odd width.
+template <bool kOdd>
+__global__ void __launch_bounds__(256, 8) batch_resolve_kernel(BatchDev b, const int2 *__restrict__ blocks)
 {
-    // the frame's descriptor in shared memory: read there, its fields are not reloaded
-    // from global memory after each of the block's output stores
+    // the frame's descriptor in shared memory, a word a thread: read there, its fields are
+    // not reloaded from global memory after each of the block's output stores
     __shared__ BatchFrame sf;
+    constexpr uint32_t kWords = sizeof(BatchFrame) / 4;
+    static_assert(sizeof(BatchFrame) % 4 == 0 && kWords <= 256, "a word a thread");
     pdl_trigger();
     const int2 blk = blocks[blockIdx.x + pdl_wait()];
-    if (threadIdx.x == 0) sf = b.frames[blk.x];
+    if (threadIdx.x < kWords)
+        reinterpret_cast<uint32_t *>(&sf)[threadIdx.x] =
+            reinterpret_cast<const uint32_t *>(b.frames + blk.x)[threadIdx.x];
     block_sync();
     const BatchFrame &f = sf;
-    const uint64_t nz = (uint64_t)f.g.w * f.g.h;
-    const uint64_t ncells = f.g.image ? nz + f.g.h : nz;
-    const uint64_t end = min(ncells, (uint64_t)blk.y + b.resolve_chunk);   // chunks start on runs
-    if (!(f.g.w & 1)) {
-        // an even-width frame by pairs of cells (resolve_even), four per thread at a time
-        const uint64_t pend = (end + 1) / 2;
-        for (uint64_t p0 = (uint64_t)blk.y / 2; p0 < pend; p0 += 4 * blockDim.x)
-            resolve_even<4>(f.g, f.fb, p0 + threadIdx.x, blockDim.x, pend, f.vec != 0);
+    const uint32_t ncells = frame_cells(f.g), first = (uint32_t)blk.y;
+    const uint32_t end = min(ncells - first, b.resolve_chunk) + first;   // chunks start on runs
+    if (!kOdd || !(f.g.w & 1)) {
+        const uint32_t pend = end / 2 + (end & 1u);
+        for (uint32_t p0 = first / 2; p0 < pend; p0 += kBatchPairs * blockDim.x)
+            resolve_even<kBatchPairs>(f.g, f.fb, p0 + threadIdx.x, blockDim.x, pend, f.vec != 0);
         return;
     }
     const int lane = threadIdx.x & 31;
     for (uint32_t i = threadIdx.x; i < b.resolve_chunk / kBatchRun; i += blockDim.x) {
-        const uint64_t p = (uint64_t)blk.y / kBatchRun + i;
+        const uint32_t p = first / kBatchRun + i;
         resolve_run<kBatchRun>(f.g, f.fb, p, kBatchRun * p < end, lane, f.vec != 0);
     }
 }
@@ -600,10 +607,10 @@ cudaError_t launch_batch_items(const BatchDev &b, cudaStream_t s)
     return cudaGetLastError();
 }
 
-cudaError_t launch_batch_resolve(const BatchDev &b, const int2 *blocks, uint32_t nblocks, cudaStream_t s)
+cudaError_t launch_batch_resolve(const BatchDev &b, const int2 *blocks, uint32_t nblocks, bool odd, cudaStream_t s)
 {
     if (!nblocks) return cudaSuccess;
-    return launch_pdl(batch_resolve_kernel, dim3(nblocks), dim3(256), 0, s, b, blocks);
+    return launch_pdl(odd ? batch_resolve_kernel<true> : batch_resolve_kernel<false>, dim3(nblocks), dim3(256), 0, s, b, blocks);
 }
 
 }  // namespace sloth

@@ -89,6 +89,7 @@ struct sloth_batch {
     int2 *blk[kTables] = {nullptr, nullptr, nullptr, nullptr};   // block tables (kTab*)
     uint32_t nblk[kTables] = {0, 0, 0, 0};
     uint32_t resolve_chunk = kBatchResolveChunk;
+    bool any_odd = false;                     // some frame has an odd width
 
     cudaGraphExec_t graph = nullptr;
     bool rendered = false;
@@ -240,7 +241,11 @@ sloth_status build(sloth_batch *b, int shape)
     // a resolve block takes 8192 cells, or 2048 when those blocks would not fill the GPU
     // twice over (24 frames of 160x48: 24 blocks, 27 us)
     uint64_t all_cells = 0, all_tri = 0;
-    for (const sloth_frame_desc &fd : b->frames) all_cells += (uint64_t)fd.width * fd.height;
+    b->any_odd = false;
+    for (const sloth_frame_desc &fd : b->frames) {
+        all_cells += (uint64_t)fd.width * fd.height;
+        b->any_odd = b->any_odd || (fd.width & 1u);
+    }
     for (const sloth_mesh *m : b->meshes) all_tri += sloth_mesh_view(m).ntri;
     b->resolve_chunk = all_cells / kBatchResolveChunk < 8ull * (uint64_t)device_sm_count() ? kBatchResolveSmall
                                                                                            : kBatchResolveChunk;
@@ -453,7 +458,7 @@ cudaError_t enqueue_folded(sloth_batch *b, const BatchDev &d, cudaStream_t s)
     if (side && (e = cudaEventRecord(b->ev_nl, b->nl_s))) return e;
     if ((e = launch_batch_fold_large(d, s))) return e;
     if (side && (e = cudaStreamWaitEvent(s, b->ev_nl, 0))) return e;
-    return launch_batch_resolve(d, b->blk[kTabResolve], b->nblk[kTabResolve], s);
+    return launch_batch_resolve(d, b->blk[kTabResolve], b->nblk[kTabResolve], b->any_odd, s);
 }
 
 // Stage 1: reset, setup, newline, large counts, scan.
@@ -484,7 +489,7 @@ cudaError_t enqueue_back(sloth_batch *b, const BatchDev &d, cudaStream_t s)
     const int tw = kTileShapes[b->shape][0], th = kTileShapes[b->shape][1];
     if ((e = launch_batch_raster(d, tw, th, b->persistent, s))) return e;
     if ((e = cudaStreamWaitEvent(s, b->ev_nl, 0))) return e;   // the newline tree is complete
-    return launch_batch_resolve(d, b->blk[kTabResolve], b->nblk[kTabResolve], s);
+    return launch_batch_resolve(d, b->blk[kTabResolve], b->nblk[kTabResolve], b->any_odd, s);
 }
 
 // Render without the graph: stage 1, size the entries from the scan total, stage 2.

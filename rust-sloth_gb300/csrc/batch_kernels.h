@@ -88,7 +88,8 @@ cudaError_t launch_batch_raster(const BatchDev &b, int tw, int th, bool persiste
 cudaError_t launch_batch_fold_setup(const BatchDev &b, const int2 *blocks, uint32_t nblocks, bool small,
                                     cudaStream_t s);
 cudaError_t launch_batch_fold_large(const BatchDev &b, cudaStream_t s);
-cudaError_t launch_batch_resolve(const BatchDev &b, const int2 *blocks, uint32_t nblocks, cudaStream_t s);
+// odd: some frame has an odd width
+cudaError_t launch_batch_resolve(const BatchDev &b, const int2 *blocks, uint32_t nblocks, bool odd, cudaStream_t s);
 cudaError_t prepare_batch_kernels();
 
 constexpr uint32_t kBatchNewlineChunk = 8192;   // triangles per newline block

@@ -9,25 +9,28 @@ namespace sloth {
 
 // Runs of kRun frame cells; each warp takes 32 consecutive runs (resolve_run).  An
 // even-width frame goes by pairs of cells instead, kEvenPairs per thread (resolve_even).
+// The winner's key and record are two dependent loads from L2 or memory, so what counts is
+// the warps that wait on them at once: eight blocks an SM with one pair a thread (32
+// registers) take 34 us for 3840x2160 over a million triangles, four blocks with four pairs
+// 47; an odd 1921x1079 takes 18 at eight blocks, 24 at four.
 constexpr int kRun = 2;
-constexpr int kEvenPairs = 4;
+constexpr int kEvenPairs = 1;
 
-__global__ void __launch_bounds__(256, 4) resolve_kernel(FrameGeom g, FrameBuffers fb, int vec)
+template <bool kEven>
+__global__ void __launch_bounds__(256, 8) resolve_kernel(FrameGeom g, FrameBuffers fb, int vec)
 {
     pdl_trigger();
-    const uint32_t tid = threadIdx.x + pdl_wait();
-    const uint64_t nz = (uint64_t)g.w * g.h;
-    const uint64_t ncells = g.image ? nz + g.h : nz;
-    if (!(g.w & 1)) {
-        const uint64_t npairs = (ncells + 1) / 2, span = (uint64_t)blockDim.x * kEvenPairs;
-        for (uint64_t base = blockIdx.x * span; base < npairs; base += (uint64_t)gridDim.x * span)
-            resolve_even<kEvenPairs>(g, fb, base + tid, blockDim.x, npairs, vec != 0);
+    const uint32_t tid = threadIdx.x + pdl_wait(), ncells = frame_cells(g);
+    if (kEven) {
+        const uint32_t npairs = ncells / 2 + (ncells & 1u), span = blockDim.x * kEvenPairs;
+        for (uint64_t base = (uint64_t)blockIdx.x * span; base < npairs; base += (uint64_t)gridDim.x * span)
+            resolve_even<kEvenPairs>(g, fb, (uint32_t)base + tid, blockDim.x, npairs, vec != 0);
         return;
     }
-    const uint64_t nruns = (ncells + kRun - 1) / kRun;
+    const uint32_t nruns = ncells / kRun + (ncells % kRun != 0);
     const int lane = threadIdx.x & 31;
-    for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x; base < nruns; base += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t p = base + tid;
+    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < nruns; base += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t p = (uint32_t)base + tid;
         resolve_run<kRun>(g, fb, p, p < nruns, lane, vec != 0);
     }
 }
@@ -38,11 +41,12 @@ cudaError_t launch_resolve(const FrameGeom &g, const FrameBuffers &fb, cudaStrea
     if (ncells == 0) return cudaSuccess;
     const uint64_t per_block = 256ull * kRun * ((g.w & 1) ? 1 : kEvenPairs);   // cells
     uint64_t blocks = (ncells + per_block - 1) / per_block;
-    const uint64_t cap = 32ull * (uint64_t)device_sm_count();   // four resident CTAs per SM (64 registers), eight waves
+    const uint64_t cap = 64ull * (uint64_t)device_sm_count();   // eight resident CTAs per SM, eight waves
     if (blocks > cap) blocks = cap;
     const int vec = ((reinterpret_cast<uintptr_t>(fb.cells_out) | reinterpret_cast<uintptr_t>(fb.z_out) |
                       reinterpret_cast<uintptr_t>(fb.winner_out)) & (4u * kRun - 1u)) == 0;
-    return launch_pdl(resolve_kernel, dim3((unsigned)blocks), dim3(256), 0, s, g, fb, vec);
+    return launch_pdl((g.w & 1) ? resolve_kernel<false> : resolve_kernel<true>, dim3((unsigned)blocks), dim3(256), 0, s, g,
+                      fb, vec);
 }
 
 // A small frame's buffers and the error word into one page-locked buffer, by words of 16

@@ -91,65 +91,27 @@ __device__ __forceinline__ Cand decode(const FrameGeom &g, const FrameBuffers &f
     return decode_rows(g, fb, key, r, cc, __ldg(p), __ldg(p + 1), z_out);
 }
 
-// Resolve frame cell c (and depth cell c when c < w*h) of one frame.
-__device__ __forceinline__ void resolve_cell(const FrameGeom &g, const FrameBuffers &fb, uint64_t c)
+// Cell counts of a frame and cell indices are 32-bit: 65535 x 65535 cells and their 65535
+// newline cells are fewer than 2^32.
+__device__ __forceinline__ uint32_t depth_cells(const FrameGeom &g) { return (uint32_t)g.w * (uint32_t)g.h; }
+__device__ __forceinline__ uint32_t frame_cells(const FrameGeom &g)
 {
-    const uint64_t nz = (uint64_t)g.w * g.h;
-    if (c >= nz) {
-        fb.cells_out[c] = (uint32_t)' ';
-        return;
-    }
-    const int r = (int)(c / g.w), cc = (int)(c - (uint64_t)r * g.w);
-    bool have = false;
-    Cand best{0, 0, 0, (uint32_t)' '};
-    const uint64_t kc = key_at(g, fb, r, cc);
-    if (kc != kEmptyKey) {
-        float z;
-        best = decode(g, fb, kc, r, cc, &z);
-        have = true;
-        fb.z_out[c] = z;
-        fb.winner_out[c] = (int32_t)best.tri;
-    } else {
-        fb.z_out[c] = kFltMax;
-        fb.winner_out[c] = -1;
-    }
-    if (c > 0) {
-        const int pr = cc > 0 ? r : r - 1, pc = cc > 0 ? cc - 1 : g.w - 1;
-        const uint64_t kp = key_at(g, fb, pr, pc);
-        if (kp != kEmptyKey) {
-            const Cand b = decode(g, fb, kp, pr, pc, nullptr);
-            if (!have || later(b, best)) best = b;
-            have = true;
-        }
-        if (g.image && (c - 1) % g.w == 0) {
-            const uint64_t yn = (c - 1) / g.w;
-            if (yn < (uint64_t)g.h) {
-                const int32_t t = nltree_query(fb.nltree, g.nl_size, (int)yn);
-                if (t >= 0) {
-                    const Cand n{(uint32_t)t, (int32_t)yn, INT_MAX, (uint32_t)'\n'};
-                    if (!have || later(n, best)) best = n;
-                    have = true;
-                }
-            }
-        }
-    }
-    fb.cells_out[c] = best.cell;
+    return depth_cells(g) + (g.image ? (uint32_t)g.h : 0u);
 }
 
 // The newline candidate of frame cell c (r, cc its row and column when c < w*h), if the
 // frame is in image mode and c = y*w+1 for a row y some triangle spans.
-__device__ __forceinline__ bool newline_at(const FrameGeom &g, const FrameBuffers &fb, uint64_t c, uint64_t nz, int r,
+__device__ __forceinline__ bool newline_at(const FrameGeom &g, const FrameBuffers &fb, uint32_t c, uint32_t nz, int r,
                                           int cc, Cand &out)
 {
     if (!g.image || c == 0) return false;
-    uint64_t yn;
+    uint32_t yn;
     if (c < nz && g.w > 1) {
         if (cc != 1) return false;
-        yn = (uint64_t)r;
+        yn = (uint32_t)r;
     } else {
-        if ((c - 1) % (uint64_t)g.w != 0) return false;
-        yn = (c - 1) / (uint64_t)g.w;
-        if (yn >= (uint64_t)g.h) return false;
+        yn = (c - 1) / (uint32_t)g.w;
+        if (c - 1 != yn * (uint32_t)g.w || yn >= (uint32_t)g.h) return false;
     }
     const int32_t t = nltree_query(fb.nltree, g.nl_size, (int)yn);
     if (t < 0) return false;
@@ -163,124 +125,21 @@ __device__ __forceinline__ Cand shfl_up_cand(const Cand &c)
                 __shfl_up_sync(0xffffffffu, c.x, 1), __shfl_up_sync(0xffffffffu, c.cell, 1)};
 }
 
-// Resolve frame cells c0 = 2p and c0+1, and depth cells c0 and c0+1, of one frame (the
-// rule of resolve_cell).  Called by all 32 lanes of a warp with consecutive p in lane
-// order; lanes with valid false (past the end) write nothing.  Depth cell c0-1's winner
-// is the previous lane's second depth cell (lane 0 decodes it itself), so a pair costs
-// two key reads and two record decodes.
-__device__ __forceinline__ void resolve_pair(const FrameGeom &g, const FrameBuffers &fb, uint64_t p, bool valid,
-                                             int lane)
-{
-    const uint64_t nz = (uint64_t)g.w * g.h;
-    const uint64_t ncells = g.image ? nz + g.h : nz;
-    const uint64_t c0 = 2 * p;
-    int r0 = 0, cc0 = 0;
-    if (valid && c0 < nz) {
-        if (nz <= 0xffffffffull) {
-            r0 = (int)((uint32_t)c0 / (uint32_t)g.w);
-        } else {
-            r0 = (int)(c0 / (uint64_t)g.w);
-        }
-        cc0 = (int)(c0 - (uint64_t)r0 * g.w);
-    }
-    int r1 = r0, cc1 = cc0 + 1;
-    if (cc1 == g.w) {
-        ++r1;
-        cc1 = 0;
-    }
-    Cand k0{0, 0, 0, (uint32_t)' '}, k1{0, 0, 0, (uint32_t)' '};
-    bool h0 = false, h1 = false;
-    float z0 = kFltMax, z1 = kFltMax;
-    if (valid && c0 < nz) {
-        const uint64_t k = key_at(g, fb, r0, cc0);
-        if (k != kEmptyKey) {
-            k0 = decode(g, fb, k, r0, cc0, &z0);
-            h0 = true;
-        }
-    }
-    if (valid && c0 + 1 < nz) {
-        const uint64_t k = key_at(g, fb, r1, cc1);
-        if (k != kEmptyKey) {
-            k1 = decode(g, fb, k, r1, cc1, &z1);
-            h1 = true;
-        }
-    }
-    // depth cell c0-1
-    Cand km = shfl_up_cand(k1);
-    bool hm = __shfl_up_sync(0xffffffffu, (int)h1, 1) != 0;
-    if (lane == 0) {
-        hm = false;
-        if (valid && c0 >= 1 && c0 - 1 < nz) {
-            int rm, cm;
-            if (c0 < nz) {
-                rm = cc0 > 0 ? r0 : r0 - 1;
-                cm = cc0 > 0 ? cc0 - 1 : g.w - 1;
-            } else {
-                rm = g.h - 1;
-                cm = g.w - 1;
-            }
-            const uint64_t k = key_at(g, fb, rm, cm);
-            if (k != kEmptyKey) {
-                km = decode(g, fb, k, rm, cm, nullptr);
-                hm = true;
-            }
-        }
-    }
-    if (!valid) return;
-    // frame cell c0: depth cells c0 and c0-1, newline; frame cell c0+1: c0+1 and c0
-    if (c0 < ncells) {
-        bool have = h0;
-        Cand best = k0;
-        if (hm && (!have || later(km, best))) {
-            best = km;
-            have = true;
-        }
-        Cand n;
-        if (newline_at(g, fb, c0, nz, r0, cc0, n) && (!have || later(n, best))) best = n;
-        fb.cells_out[c0] = best.cell;
-    }
-    if (c0 + 1 < ncells) {
-        bool have = h1;
-        Cand best = k1;
-        if (h0 && (!have || later(k0, best))) {
-            best = k0;
-            have = true;
-        }
-        Cand n;
-        if (newline_at(g, fb, c0 + 1, nz, r1, cc1, n) && (!have || later(n, best))) best = n;
-        fb.cells_out[c0 + 1] = best.cell;
-    }
-    if (c0 < nz) {
-        fb.z_out[c0] = z0;
-        fb.winner_out[c0] = h0 ? (int32_t)k0.tri : -1;
-    }
-    if (c0 + 1 < nz) {
-        fb.z_out[c0 + 1] = z1;
-        fb.winner_out[c0 + 1] = h1 ? (int32_t)k1.tri : -1;
-    }
-}
-
 // Resolve frame cells c0 = K*p .. c0+K-1 and the depth cells among them, of one frame
-// (the rule of resolve_cell).  Called by all 32 lanes of a warp with consecutive p in
+// (the rule above).  Called by all 32 lanes of a warp with consecutive p in
 // lane order; lanes with valid false (past the end) write nothing.  Depth cell c0-1's
 // winner is the previous lane's last depth cell (lane 0 decodes it itself).  With vec the
 // outputs are 4K-byte aligned and a lane's K cells go out in one store per buffer.
 template <int K>
-__device__ __forceinline__ void resolve_run(const FrameGeom &g, const FrameBuffers &fb, uint64_t p, bool valid,
+__device__ __forceinline__ void resolve_run(const FrameGeom &g, const FrameBuffers &fb, uint32_t p, bool valid,
                                             int lane, bool vec)
 {
     static_assert(K == 2 || K == 4, "one 8- or 16-byte store per lane and buffer");
-    const uint64_t nz = (uint64_t)g.w * g.h;
-    const uint64_t ncells = g.image ? nz + g.h : nz;
-    const uint64_t c0 = K * p;
+    const uint32_t nz = depth_cells(g), ncells = frame_cells(g), c0 = K * p;
     int r0 = 0, cc0 = 0;
     if (valid && c0 < nz) {
-        if (nz <= 0xffffffffull) {
-            r0 = (int)((uint32_t)c0 / (uint32_t)g.w);
-        } else {
-            r0 = (int)(c0 / (uint64_t)g.w);
-        }
-        cc0 = (int)(c0 - (uint64_t)r0 * g.w);
+        r0 = (int)(c0 / (uint32_t)g.w);
+        cc0 = (int)(c0 - (uint32_t)r0 * (uint32_t)g.w);
     }
     int rj[K], cj[K];
     uint64_t key[K];
@@ -326,7 +185,7 @@ __device__ __forceinline__ void resolve_run(const FrameGeom &g, const FrameBuffe
     uint32_t out[K];
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-        const uint64_t c = c0 + j;
+        const uint32_t c = c0 + j;
         bool have = hc[j];
         Cand best = kc[j];
         const Cand &prev = j == 0 ? km : kc[j - 1];
@@ -374,27 +233,26 @@ __device__ __forceinline__ void resolve_run(const FrameGeom &g, const FrameBuffe
 // only even depth columns there (y*w + 2x is even), so depth cell c0+1 never has a winner:
 // frame cell c0 takes the winner of depth cell c0 (its left neighbour c0-1 is odd and the
 // newline cells y*w+1 are odd), and frame cell c0+1 the later of that winner and, when c0
-// starts a row, the row's newline (the rule of resolve_cell).  A thread resolves the J
+// starts a row, the row's newline.  A thread resolves the J
 // pairs p0 + j*stride below pend, issuing every key load first, then every winner's record
 // loads, then the arithmetic and stores: J independent chains in flight instead of one.
 // With vec the outputs are 8-byte aligned and a pair goes out in one store per buffer.
 template <int J>
-__device__ __forceinline__ void resolve_even(const FrameGeom &g, const FrameBuffers &fb, uint64_t p0, uint32_t stride,
-                                             uint64_t pend, bool vec)
+__device__ __forceinline__ void resolve_even(const FrameGeom &g, const FrameBuffers &fb, uint32_t p0, uint32_t stride,
+                                             uint32_t pend, bool vec)
 {
-    const uint64_t nz = (uint64_t)g.w * g.h;
-    const uint64_t ncells = g.image ? nz + g.h : nz;
+    const uint32_t nz = depth_cells(g), ncells = frame_cells(g);
     uint64_t key[J];
     int rr[J], cc[J];
 #pragma unroll
     for (int j = 0; j < J; ++j) {
-        const uint64_t c0 = 2 * (p0 + (uint64_t)j * stride);
+        const uint32_t p = p0 + j * stride, c0 = 2 * p;
         key[j] = kEmptyKey;
         rr[j] = 0;
         cc[j] = 0;
-        if (c0 < nz) {
-            rr[j] = nz <= 0xffffffffull ? (int)((uint32_t)c0 / (uint32_t)g.w) : (int)(c0 / (uint64_t)g.w);
-            cc[j] = (int)(c0 - (uint64_t)rr[j] * g.w);
+        if (p < pend && c0 < nz) {
+            rr[j] = (int)(c0 / (uint32_t)g.w);
+            cc[j] = (int)(c0 - (uint32_t)rr[j] * (uint32_t)g.w);
             key[j] = key_at(g, fb, rr[j], cc[j]);
         }
     }
@@ -410,9 +268,9 @@ __device__ __forceinline__ void resolve_even(const FrameGeom &g, const FrameBuff
     }
 #pragma unroll
     for (int j = 0; j < J; ++j) {
-        const uint64_t p = p0 + (uint64_t)j * stride;
+        const uint32_t p = p0 + j * stride;
         if (p >= pend) continue;
-        const uint64_t c0 = 2 * p;
+        const uint32_t c0 = 2 * p;
         const bool have = key[j] != kEmptyKey;
         float z = kFltMax;
         Cand best{0, 0, 0, (uint32_t)' '};
