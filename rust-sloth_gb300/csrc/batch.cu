@@ -58,16 +58,20 @@ __device__ __forceinline__ void batch_setup_triangle(const BatchDev &b, const Ba
         large = sp.large;
     }
     const bool binned = live && !large && !direct && sp.ntiles != 0;
+    uint32_t hits;
     const uint32_t slot1 = count_small_tiles_warp(binned, r, vp, sp, b.bb.tile_count + f.tile_off,
-                                                  b.bb.tile_cursor + f.tile_off);
+                                                  b.bb.tile_cursor + f.tile_off, hits);
     // the fill's work list: one atomic per warp
     const unsigned bm = __ballot_sync(0xffffffffu, binned);
     if (bm) {
         const int lane = threadIdx.x & 31;
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(b.fill_count, (uint32_t)__popc(bm));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (binned) b.fill_list[base + __popc(bm & ((1u << lane) - 1u))] = make_uint4(d.frame, d.local_base + t, slot1, 0u);
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(b.fill_count, (uint32_t)__popc(bm));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(bm & ((1u << lane) - 1u));
+        if (binned) {
+            b.bb.fill_list[at] = fill_entry(r, sp, d.local_base + t, slot1, f.tile_off, vp.ntx, d.frame);
+            b.bb.fill_meta[at] = fill_meta(sp, hits, vp.ntx);
+        }
     }
     if (__any_sync(0xffffffffu, large)) {
         const int q = large_slot(large, sp.ntiles, b.bb.large_count, b.bb.large_cap);
@@ -308,20 +312,18 @@ __global__ void __launch_bounds__(256) batch_bin_large_kernel(BatchDev b)
 __global__ void __launch_bounds__(kSetupThreads, kFillMinBlocks) batch_fill_kernel(BatchDev b)
 {
     const uint32_t n = *b.fill_count;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        const bool live = i < n;
-        const uint4 e = live ? b.fill_list[i] : make_uint4(0u, 0u, 0u, 0u);
-        const BatchFrame &f = b.frames[e.x];
-        const Viewport vp = vp_batch(f.g);
-        TriRecord r;
-        TileSpan sp{};
-        if (live) {
-            r = load_record(f.fb.records, e.y);
-            sp = tile_span(vp, r);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint4 e = b.bb.fill_list[i];
+        const uint32_t meta = b.bb.fill_meta[i];
+        if (!(meta & kFillReread)) {
+            fill_listed(e, meta, b.bb.tile_offset, b.bb.tile_cursor, b.bb.entries, b.bb.capacity);
+        } else {
+            const BatchFrame &f = b.frames[e.z];
+            const Viewport vp = vp_batch(f.g);
+            const TriRecord r = load_record(f.fb.records, e.x);
+            fill_small(r, e.x, vp, tile_span(vp, r), b.bb.tile_offset, b.bb.tile_cursor, b.bb.entries, b.bb.capacity,
+                       e.y, f.tile_off);
         }
-        fill_small_warp(live, r, e.y, vp, sp, b.bb.tile_offset, b.bb.tile_cursor, b.bb.entries, b.bb.capacity, e.z,
-                        f.tile_off);
     }
 }
 
@@ -392,9 +394,9 @@ __device__ __noinline__ void batch_overflow_fold(const BatchDev &b)
     uint32_t frags = 0;
     const uint32_t n = *b.fill_count;
     for (uint32_t i = warp; i < n; i += nwarps) {
-        const uint4 e = b.fill_list[i];
-        const BatchFrame &f = b.frames[e.x];
-        frags += fold_queued<32, 1>(e.y, 0u, 1u, true, f.g, f.fb);
+        const uint4 e = b.bb.fill_list[i];
+        const BatchFrame &f = b.frames[(b.bb.fill_meta[i] & kFillReread) ? e.z : frame_of_tile(b, e.w)];
+        frags += fold_queued<32, 1>(e.x, 0u, 1u, true, f.g, f.fb);
     }
     constexpr uint32_t kParts = 64;
     const uint32_t front = b.bb.large_count[0], all = front + b.bb.large_count[1];

@@ -79,8 +79,7 @@ struct sloth_batch {
     uint32_t *large_frame = nullptr;
     uint32_t *overflow = nullptr;
     uint32_t *queue = nullptr;                // the persistent raster's item counter
-    uint4 *fill_list = nullptr;               // the fill's work list (one entry per record at most)
-    uint32_t *fill_count = nullptr;
+    uint32_t *fill_count = nullptr;           // entries of bb.fill_list
     uint32_t *h_total = nullptr;              // pinned
     uint32_t *h_overflow = nullptr;           // pinned
     uint32_t *error = nullptr;                // device error word of the raster (sticky)
@@ -181,7 +180,7 @@ void free_layout(sloth_batch *b)
     b->bb.item_capacity = 0;
     bfree(b->overflow);
     bfree(b->queue);
-    bfree(b->fill_list);
+    bfree(b->bb.fill_list);
     bfree(b->fill_count);
     for (auto &p : b->blk) bfree(p);
     b->entries_cap = 0;
@@ -343,7 +342,8 @@ sloth_status build(sloth_batch *b, int shape)
     BCU(b, balloc(&b->bb.slice_offset, tiles + kSliceExtra));
     BCU(b, balloc(&b->overflow, 1));
     BCU(b, balloc(&b->queue, 1));
-    BCU(b, balloc(&b->fill_list, rec));
+    BCU(b, balloc(&b->bb.fill_list, fill_words16(rec)));
+    b->bb.fill_meta = reinterpret_cast<uint32_t *>(b->bb.fill_list + rec);
     BCU(b, balloc(&b->fill_count, 1));
     BCU(b, balloc(&b->d_mats, nd));
     for (uint32_t f = 0; f < nf; ++f) {
@@ -392,7 +392,6 @@ BatchDev dev_view(sloth_batch *b)
     d.overflow = b->overflow;
     d.status = b->status;
     d.queue = b->queue;
-    d.fill_list = b->fill_list;
     d.fill_count = b->fill_count;
     d.depth_cull = sloth_ctx_depth_cull(b->ctx);
     d.tpb = b->tpb;

@@ -46,10 +46,7 @@ struct BatchDev {
     volatile uint32_t *status; // pinned host words: [0] a render's entries outgrew their capacity,
                                // [1] a raster block gave up waiting for its keys
     uint32_t *queue;           // the persistent raster's next item (zeroed by the item kernel)
-    uint4 *fill_list;          // (frame, frame-local draw index, slot in its first tile, 0) of
-                               // every small binned triangle, appended by setup: the fill walks
-                               // only these
-    uint32_t *fill_count;      // entries of fill_list (zeroed at the start of a render)
+    uint32_t *fill_count;      // entries of bb.fill_list (zeroed at the start of a render)
     int depth_cull;
     int tpb;                   // triangles per setup block (the triangle block table's step)
     int direct_max;            // the frames' FrameGeom::direct_max (the same for every frame)

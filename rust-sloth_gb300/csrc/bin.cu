@@ -5,7 +5,7 @@
 // cells it can write: count (setup kernel for small triangles, one warp per large
 // triangle here), exclusive scan over tiles, then fill (bin_common.cuh).
 #include "bin_common.cuh"
-#include "direct.cuh"
+#include "record.cuh"
 #include "sloth_kernels.h"
 
 namespace sloth {
@@ -250,24 +250,21 @@ bin_items_kernel(uint32_t n, FrameGeom g, FrameBuffers fb, BinBuffers bb)
 }
 
 // The small binned triangles setup listed, 256 per block and round (grid-stride): their
-// tile entries.  Only their records are read.
+// tile entries.
 __global__ void __launch_bounds__(kSetupThreads, kFillMinBlocks)
-bin_fill_kernel(uint32_t tri_base, FrameGeom g, FrameBuffers fb, BinBuffers bb)
+bin_fill_kernel(FrameGeom g, FrameBuffers fb, BinBuffers bb)
 {
     const uint32_t n = bb.large_count[2];
-    const Viewport vp = vp_of(g);
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        const bool live = i < n;
-        const uint2 e = live ? bb.fill_list[i] : make_uint2(0u, 0u);
-        const uint32_t gtri = tri_base + e.x;
-        TriRecord r;
-        TileSpan sp{};
-        if (live) {
-            r = load_record(fb.records, gtri);
-            sp = tile_span(vp, r);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint4 e = bb.fill_list[i];
+        const uint32_t meta = bb.fill_meta[i];
+        if (!(meta & kFillReread)) {
+            fill_listed(e, meta, bb.tile_offset, bb.tile_cursor, bb.entries, bb.capacity);
+        } else {
+            const Viewport vp = vp_of(g);
+            const TriRecord r = load_record(fb.records, e.x);
+            fill_small(r, e.x, vp, tile_span(vp, r), bb.tile_offset, bb.tile_cursor, bb.entries, bb.capacity, e.y, 0u);
         }
-        fill_small_warp(live, r, gtri, vp, sp, bb.tile_offset, bb.tile_cursor, bb.entries, bb.capacity, e.y);
     }
 }
 
@@ -297,10 +294,9 @@ cudaError_t launch_bin_items(uint32_t ntiles, const FrameGeom &g, const FrameBuf
     return cudaGetLastError();
 }
 
-cudaError_t launch_bin_fill(uint32_t tri_base, const FrameGeom &g, const FrameBuffers &fb, const BinBuffers &bb,
-                            cudaStream_t s)
+cudaError_t launch_bin_fill(const FrameGeom &g, const FrameBuffers &fb, const BinBuffers &bb, cudaStream_t s)
 {
-    bin_fill_kernel<<<kFillMinBlocks * 2 * device_sm_count(), kSetupThreads, 0, s>>>(tri_base, g, fb, bb);
+    bin_fill_kernel<<<kFillMinBlocks * 2 * device_sm_count(), kSetupThreads, 0, s>>>(g, fb, bb);
     return cudaGetLastError();
 }
 

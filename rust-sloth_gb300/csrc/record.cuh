@@ -329,26 +329,54 @@ __device__ __forceinline__ float4 transform_vertex(const MeshDev &mesh, const Ma
     return make_float4(row_dot(&M.m[0], x, y, z), row_dot(&M.m[4], x, y, z), row_dot(&M.m[8], x, y, z), 0.0f);
 }
 
+// What setup leaves for the fill of a small binned triangle (at most 16 tiles): its draw
+// index, its slot in its first tile, the ordered depth bound of its entries and the first
+// tile of its rectangle, and in meta the rectangle's tiles it hits (bit i: tile i, row-major),
+// the rectangle's width and the tile grid's.  The fill then reads no record and tests no
+// tile again.  A triangle with wrapped samples keeps kFillReread instead, with its frame in
+// place of the bound: its entries need their wrapped parts, from the record.
+constexpr uint32_t kFillReread = 0x80000000u;
+static_assert(kSmallMaxTilesDev == 16, "one bit per tile of the rectangle");
+
+__device__ __forceinline__ uint32_t fill_meta(const TileSpan &sp, uint32_t hits, int ntx)
+{
+    if (!sp.W.empty()) return kFillReread;
+    return hits | (uint32_t)(sp.TU.xb - sp.TU.xa - 1) << 16 | (uint32_t)(ntx - 1) << 20;   // ntx <= 2048
+}
+
+__device__ __forceinline__ uint4 fill_entry(const TriRecord &r, const TileSpan &sp, uint32_t gtri, uint32_t slot1,
+                                            uint32_t tile_base, int ntx, uint32_t frame)
+{
+    return make_uint4(gtri, slot1, sp.W.empty() ? ordered_z(r.zlo) : frame,
+                      tile_base + (uint32_t)(sp.TU.ya * ntx + sp.TU.xa));
+}
+
 // Counts the small triangle's tiles (bin count pass) and returns the triangle's slot among
 // the entries of its first tile.  A triangle's first tile (the first tile_hit in the loop
-// order below, which fill_small_warp repeats) is counted in tile_count with one atomic per
+// order below, which the fill repeats) is counted in tile_count with one atomic per
 // distinct tile of the warp, whose returned value gives each lane its slot; its other
 // tiles are counted in tile_extra without a slot (the fill takes theirs from the tile's
-// cursor).  Called by all 32 lanes (lanes with active false count nothing and get 0).
+// cursor).  Called by all 32 lanes (lanes with active false count nothing and get 0).  hits
+// gets the tiles of the unwrapped rectangle that are hit (fill_meta).
 __device__ __forceinline__ uint32_t count_small_tiles_warp(bool active, const TriRecord &r, const Viewport &vp,
                                                            const TileSpan &sp, uint32_t *tile_count,
-                                                           uint32_t *tile_extra)
+                                                           uint32_t *tile_extra, uint32_t &hits)
 {
     uint32_t first = 0xffffffffu;
+    hits = 0;
     if (active) {
         auto hit = [&](int tr, int tc) {
             const uint32_t tile = tr * vp.ntx + tc;
             if (first == 0xffffffffu) first = tile;
             else atomicAdd(&tile_extra[tile], 1u);
         };
+        uint32_t bit = 1u;
         for (int tr = sp.TU.ya; tr < sp.TU.yb; ++tr)
-            for (int tc = sp.TU.xa; tc < sp.TU.xb; ++tc)
-                if (tile_hit(r, vp, sp.U, sp.W, tr, tc)) hit(tr, tc);
+            for (int tc = sp.TU.xa; tc < sp.TU.xb; ++tc, bit <<= 1)
+                if (tile_hit(r, vp, sp.U, sp.W, tr, tc)) {
+                    hits |= bit;
+                    hit(tr, tc);
+                }
         for (int tr = sp.TW.ya; tr < sp.TW.yb; ++tr)
             for (int tc = sp.TW.xa; tc < sp.TW.xb; ++tc) {
                 if (in_rect(sp.TU, tr, tc)) continue;

@@ -93,15 +93,17 @@ __device__ __forceinline__ void setup_triangle(uint32_t tri_base, const FrameGeo
     // binning: count tiles of small triangles here and list them for the fill, queue the
     // rest for warps
     const bool binned = live && !large && !direct && sp.ntiles != 0;
-    const uint32_t slot1 = count_small_tiles_warp(binned, r, vp, sp, bb.tile_count, bb.tile_cursor);
-    if (bb.fill_list) {
-        const unsigned bm = __ballot_sync(0xffffffffu, binned);
-        if (bm) {
-            const int lane = threadIdx.x & 31;
-            uint32_t first = 0;
-            if (lane == 0) first = atomicAdd(&bb.large_count[2], (uint32_t)__popc(bm));
-            first = __shfl_sync(0xffffffffu, first, 0);
-            if (binned) bb.fill_list[first + __popc(bm & ((1u << lane) - 1u))] = make_uint2(t, slot1);
+    uint32_t hits;
+    const uint32_t slot1 = count_small_tiles_warp(binned, r, vp, sp, bb.tile_count, bb.tile_cursor, hits);
+    const unsigned bm = __ballot_sync(0xffffffffu, binned);
+    if (bm) {
+        const int lane = threadIdx.x & 31;
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&bb.large_count[2], (uint32_t)__popc(bm));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(bm & ((1u << lane) - 1u));
+        if (binned) {
+            bb.fill_list[at] = fill_entry(r, sp, tri_base + t, slot1, 0u, vp.ntx, 0u);
+            bb.fill_meta[at] = fill_meta(sp, hits, vp.ntx);
         }
     }
     // warp-ballot compaction of the large-triangle queue

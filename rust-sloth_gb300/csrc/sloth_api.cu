@@ -1121,7 +1121,9 @@ sloth_status sloth_draw_mesh(sloth_ctx *ctx, const sloth_mesh *mesh, const float
     if ((st = ensure_records(ctx, (size_t)ctx->tri_base + mesh->ntri)) != SLOTH_OK) return st;
     if (mesh->idx && (st = ensure_scratch(ctx, &ctx->tv, &ctx->tv_cap, mesh->nvert)) != SLOTH_OK) return st;
     if ((st = ensure_scratch(ctx, &ctx->bb.large_queue, &ctx->large_cap, mesh->ntri)) != SLOTH_OK) return st;
-    if ((st = ensure_scratch(ctx, &ctx->bb.fill_list, &ctx->fill_cap, mesh->ntri)) != SLOTH_OK) return st;
+    // the fill list, and after its ntri entries their 4-byte metas
+    if ((st = ensure_scratch(ctx, &ctx->bb.fill_list, &ctx->fill_cap, fill_words16(mesh->ntri))) != SLOTH_OK) return st;
+    ctx->bb.fill_meta = reinterpret_cast<uint32_t *>(ctx->bb.fill_list + mesh->ntri);
     if (!ctx->bb.large_count) CU(ctx, dalloc(&ctx->bb.large_count, 3));
     ctx->bb.large_cap = mesh->ntri;
 
@@ -1161,7 +1163,7 @@ sloth_status sloth_draw_mesh(sloth_ctx *ctx, const sloth_mesh *mesh, const float
                       ctx->aux));
         CU(ctx, cudaEventRecord(ctx->aux_ev, ctx->aux));
         CU(ctx, timed(ctx, "bin_fill", [&] {
-               return launch_bin_fill(ctx->tri_base, g, ctx->fb, ctx->bb, s);
+               return launch_bin_fill(g, ctx->fb, ctx->bb, s);
            }));
         CU(ctx, cudaStreamWaitEvent(s, ctx->aux_ev, 0));
         size_t icap = ctx->bb.item_capacity;

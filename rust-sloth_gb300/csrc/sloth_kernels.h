@@ -55,9 +55,8 @@ struct BinBuffers {
     uint32_t *large_count;   // 3: big triangles queued, other large triangles queued, and
                              // (contexts) small binned triangles listed in fill_list
     uint32_t large_cap;
-    uint2 *fill_list;        // large_cap: (draw-local index, slot in its first tile) of the
-                             // small binned triangles (setup appends, the fill walks them);
-                             // null: none kept
+    uint4 *fill_list;        // large_cap: the small binned triangles (setup appends, the fill
+    uint32_t *fill_meta;     // walks them; fill_entry and fill_meta in record.cuh)
     uint32_t *slice_offset;  // ntiles + kSliceExtra: per tile the first raster item of its
                              // slices within its class (item_offset); [ntiles] = items,
                              // [ntiles+1] = split threshold, [ntiles+2] = slice size,
@@ -68,6 +67,9 @@ struct BinBuffers {
     uint32_t item_capacity;
     uint32_t *max_total;     // optional: the scan folds each draw's entry total in (atomicMax)
 };
+
+// 16-byte words of a fill list of n entries and their metas behind it.
+inline size_t fill_words16(size_t n) { return n + (n + 3) / 4; }
 
 // A tile holding many more entries than the launch's mean is rasterized in slices by
 // separate CTAs, which fold their keys into the tile's with a 64-bit global atomicMin (the
@@ -191,8 +193,7 @@ cudaError_t launch_bin_scan(uint32_t ntiles, const BinBuffers &bb, cudaStream_t 
 cudaError_t launch_bin_items(uint32_t ntiles, const FrameGeom &g, const FrameBuffers &fb, const BinBuffers &bb,
                              cudaStream_t s);
 // small binned triangles' tile entries: the ones setup listed in bb.fill_list
-cudaError_t launch_bin_fill(uint32_t tri_base, const FrameGeom &g, const FrameBuffers &fb, const BinBuffers &bb,
-                            cudaStream_t s);
+cudaError_t launch_bin_fill(const FrameGeom &g, const FrameBuffers &fb, const BinBuffers &bb, cudaStream_t s);
 cudaError_t launch_bin_fill_large(uint32_t tri_base, const FrameGeom &g, const FrameBuffers &fb,
                                   const BinBuffers &bb, cudaStream_t s);
 
