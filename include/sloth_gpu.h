@@ -93,10 +93,10 @@ sloth_status sloth_spatial_order(const float *x, const float *y, const float *z,
 /* ---- context (src/context.rs:12-49) ------------------------------------------------- */
 
 /* Create a context on CUDA device `device`.  `stream` is a cudaStream_t to order all
- * work on, or NULL for a library-owned stream: a draw forks two kernels onto the
- * context's own helper streams (the newline fold, the large-triangle fill) and joins
- * them back into `stream` before the draw's raster, the resolve, the next draw and
- * sloth_ctx_synchronize, so results read from `stream` are complete.  The context starts
+ * work on, or NULL for a library-owned stream: a large draw in image mode forks one kernel
+ * onto the context's own helper stream (the newline fold) and joins it back into `stream`
+ * before the resolve, the next draw and sloth_ctx_synchronize, so results read from
+ * `stream` are complete.  The context starts
  * blank like Context::blank(image=false) (src/context.rs:22-34): 0x0 viewport, identity
  * utransform.  Contexts are independent: different host threads may drive different
  * contexts at once. */
@@ -393,8 +393,9 @@ sloth_status sloth_render_noalloc(const float *x, const float *y, const float *z
 
 /* Enable (1) / disable (0) CUDA-event timing of each kernel the context launches.
  * sloth_ctx_kernel_time() then reports the summed device time (ms) and launch count
- * of kernel `name` ("setup", "bin_count_large", "bin_scan", "bin_fill", "bin_fill_large",
- * "bin_items", "raster", "resolve") since timing was enabled; blocks until the events complete. */
+ * of kernel `name` ("reset", "vertex", "setup", "bin_count_large", "bin_scan", "newline",
+ * "bin_fill", "raster", "fold", "fold_large", "resolve", "readback"; a draw launches those of
+ * its path) since timing was enabled; blocks until the events complete. */
 sloth_status sloth_ctx_set_timing(sloth_ctx *ctx, int enable);
 sloth_status sloth_ctx_kernel_time(sloth_ctx *ctx, const char *name, double *ms, uint64_t *launches);
 /* Number of kernels launched by this context since creation. */

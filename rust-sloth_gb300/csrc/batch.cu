@@ -10,6 +10,7 @@
 #include "direct.cuh"
 #include "fold.cuh"
 #include "launch.cuh"
+#include "newline.cuh"
 #include "raster_common.cuh"
 #include "record.cuh"
 #include "resolve_common.cuh"
@@ -54,7 +55,7 @@ __device__ __forceinline__ void batch_setup_triangle(const BatchDev &b, const Ba
         if (!direct) sp = tile_span(vp, r);   // a direct triangle is not binned
         // a triangle with nothing to rasterize is never read back here (the fill walks the
         // fill list, the newline the packed rows): its record is not written
-        if (direct || sp.ntiles != 0) store_record(f.fb.records + d.local_base + t, r, sp.ntiles, direct);
+        if (direct || sp.ntiles != 0) store_record(f.fb.records + d.local_base + t, r, direct);
         large = sp.large;
     }
     const bool binned = live && !large && !direct && sp.ntiles != 0;
@@ -102,7 +103,7 @@ __device__ __forceinline__ void batch_fold_triangle(const BatchDev &b, const Bat
         r = build_record(p1, p2, p3, rgb, f.g.w, f.g.h, INT_MAX, &dw);
         if (r.x0 < r.xe) {
             c = fold_class(r, dw);
-            store_record(f.fb.records + d.local_base + t, r, 1u, true);
+            store_record(f.fb.records + d.local_base + t, r, true);
         }
     }
     const FoldQueue queue{b.bb.large_queue, b.large_frame, b.bb.large_count, b.bb.large_cap};
@@ -199,8 +200,7 @@ __global__ void __launch_bounds__(32 * kWarps) batch_fold_setup_kernel(BatchDev 
     __shared__ BatchDraw sd;
     __shared__ BatchFrame sf;
     __shared__ Mat4 sm;
-    pdl_trigger();
-    const uint32_t zero = pdl_wait();
+    const uint32_t zero = pdl_begin();
     const int2 blk = blocks[blockIdx.x + zero];
     if (threadIdx.x < 16) sm.m[threadIdx.x] = b.mats[blk.x].m[threadIdx.x];
     if (threadIdx.x == 0) {
@@ -212,12 +212,30 @@ __global__ void __launch_bounds__(32 * kWarps) batch_fold_setup_kernel(BatchDev 
     fold_triangles<kWarps>(sd.mesh, sm, (uint32_t)blk.y, sd.local_base, sf.g, sf.fb, queue, sd.frame);
 }
 
-// The queued triangles of every frame (fold_large_kernel).
-__global__ void __launch_bounds__(256) batch_fold_large_kernel(BatchDev b)
+// newline_block of a chunk of a draw.
+template <bool kShared>
+__device__ __forceinline__ void batch_newline_block(const BatchDev &b, int2 blk, int32_t *stree)
 {
-    pdl_trigger();
-    const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x + pdl_wait()) >> 5;
-    const uint32_t large = b.bb.large_count[0], mid = b.bb.large_count[1], nwarps = (gridDim.x * blockDim.x) >> 5;
+    const BatchDraw &d = b.draws[blk.x];
+    const BatchFrame &f = b.frames[d.frame];
+    const uint32_t lo = (uint32_t)blk.y, hi = min(d.mesh.ntri, lo + kNewlineChunk);
+    newline_block<kShared>(stree, f.g.nl_size, lo, hi, d.mesh.order, f.fb.rows + d.local_base, d.local_base,
+                           f.fb.nltree);
+}
+
+// The queued triangles of every frame (fold_large_kernel), after nnl blocks of newline chunks.
+__global__ void __launch_bounds__(256) batch_fold_large_kernel(BatchDev b, const int2 *__restrict__ nl, uint32_t nnl)
+{
+    extern __shared__ int32_t stree[];
+    uint32_t blk = blockIdx.x;
+    if (blk < nnl) {
+        batch_newline_block<true>(b, nl[blk], stree);
+        return;
+    }
+    blk -= nnl;
+    const uint32_t first = (blk * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t large = b.bb.large_count[0], mid = b.bb.large_count[1],
+                   nwarps = ((gridDim.x - nnl) * blockDim.x) >> 5;
     const uint32_t parts = fold_parts(large), cut = large * parts, items = cut + mid;
     const bool filter = large + mid > kFoldFilterMin;
     unsigned long long *counter = b.frames[0].fb.fragments;   // the batch's one counter
@@ -239,10 +257,9 @@ __global__ void __launch_bounds__(256) batch_fold_large_kernel(BatchDev b)
 __global__ void __launch_bounds__(256) batch_reset_kernel(BatchReset r)
 {
     const uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
-    pdl_trigger();
     const uint64_t mask = r.half_shift < 63u ? (1ull << r.half_shift) - 1ull : ~0ull;
     const uint4 empty = make_uint4(~0u, ~0u, ~0u, ~0u);
-    for (uint64_t i = i0 + pdl_wait(); i < r.nmats; i += step) r.mats[i] = r.mats_host[i];
+    for (uint64_t i = i0; i < r.nmats; i += step) r.mats[i] = r.mats_host[i];
     if (i0 == 0) {
         r.large_count[0] = r.large_count[1] = 0u;
         *r.fill_count = 0u;
@@ -258,43 +275,19 @@ __global__ void __launch_bounds__(256) batch_reset_kernel(BatchReset r)
         r.keys[r.half_shift < 63u ? ((v >> r.half_shift) << (r.half_shift + 1)) | (v & mask) : v] = empty;
 }
 
-// blocks[i] = (draw, first triangle of a chunk): newline segment tree of the draw's frame.
+// blocks[i] = (draw, first triangle of a chunk): the newline rows in a launch of their own.
 template <bool kShared>
 __global__ void __launch_bounds__(1024) batch_newline_kernel(BatchDev b, const int2 *__restrict__ blocks)
 {
     extern __shared__ int32_t stree[];
-    const int2 blk = blocks[blockIdx.x];
-    const BatchDraw &d = b.draws[blk.x];
-    const BatchFrame &f = b.frames[d.frame];
-    if (!f.g.image) return;
-    const int n = f.g.nl_size;
-    int32_t *tree = kShared ? stree : f.fb.nltree;
-    if (kShared) {
-        for (int i = threadIdx.x; i < 2 * n; i += blockDim.x) stree[i] = -1;
-        block_sync();
-    }
-    const uint32_t lo = (uint32_t)blk.y, hi = min(d.mesh.ntri, lo + kBatchNewlineChunk);
-    for (uint32_t p = lo + threadIdx.x; p < hi; p += blockDim.x) {
-        const int32_t v = (int32_t)(d.local_base + mesh_triangle(d.mesh, p));
-        const uint32_t yr = __ldg(f.fb.rows + d.local_base + p);
-        nltree_update(tree, n, (int)(yr & 0xffffu), (int)(yr >> 16), v, kShared);
-    }
-    if (kShared) {
-        block_sync();
-        for (int i = threadIdx.x; i < 2 * n; i += blockDim.x) {
-            const int32_t v = stree[i];
-            if (v >= 0 && *(volatile int32_t *)&f.fb.nltree[i] < v) atomicMax(&f.fb.nltree[i], v);
-        }
-    }
+    batch_newline_block<kShared>(b, blocks[blockIdx.x], stree);
 }
 
-// One warp per queued large triangle, any frame.
+// One warp per part of a queued large triangle, any frame: warp `warp` of nwarps.
 template <bool kFill>
-__global__ void __launch_bounds__(256) batch_bin_large_kernel(BatchDev b)
+__device__ __forceinline__ void batch_large_items(const BatchDev &b, uint32_t warp, uint32_t nwarps)
 {
     const int lane = threadIdx.x & 31;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t items = large_items(b.bb.large_count);
     for (uint32_t it = warp; it < items; it += nwarps) {
         uint32_t q, part, nparts;
@@ -306,25 +299,10 @@ __global__ void __launch_bounds__(256) batch_bin_large_kernel(BatchDev b)
     }
 }
 
-// The small binned triangles setup listed, 256 per block and round (grid-stride): their
-// tile entries.  A warp's lanes may hold triangles of different frames; their tiles are
-// global tile indices.
-__global__ void __launch_bounds__(kSetupThreads, kFillMinBlocks) batch_fill_kernel(BatchDev b)
+__global__ void __launch_bounds__(256) batch_count_large_kernel(BatchDev b)
 {
-    const uint32_t n = *b.fill_count;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint4 e = b.bb.fill_list[i];
-        const uint32_t meta = b.bb.fill_meta[i];
-        if (!(meta & kFillReread)) {
-            fill_listed(e, meta, b.bb.tile_offset, b.bb.tile_cursor, b.bb.entries, b.bb.capacity);
-        } else {
-            const BatchFrame &f = b.frames[e.z];
-            const Viewport vp = vp_batch(f.g);
-            const TriRecord r = load_record(f.fb.records, e.x);
-            fill_small(r, e.x, vp, tile_span(vp, r), b.bb.tile_offset, b.bb.tile_cursor, b.bb.entries, b.bb.capacity,
-                       e.y, f.tile_off);
-        }
-    }
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    batch_large_items<false>(b, warp, (gridDim.x * blockDim.x) >> 5);
 }
 
 __device__ __forceinline__ uint32_t frame_of_tile(const BatchDev &b, uint32_t tile)
@@ -339,14 +317,11 @@ __device__ __forceinline__ uint32_t frame_of_tile(const BatchDev &b, uint32_t ti
     return lo;
 }
 
-// One thread per global tile: the tile's raster items (tile, slice); a tile rasterized in
-// slices gets its keys cleared and its generation set first (bin_items_kernel, per frame),
+// Global tile t: the tile's raster items (tile, slice); a tile rasterized in
+// slices gets its keys cleared and its generation set first (bin_tile_items, per frame),
 // and so does every tile when the entries outgrew their buffer (batch_overflow_fold).
-__global__ void __launch_bounds__(256) batch_items_kernel(BatchDev b)
+__device__ __forceinline__ void batch_tile_items(const BatchDev &b, uint32_t t)
 {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t == 0) *b.queue = 0u;   // the persistent raster's item counter
-    if (t >= b.total_tiles) return;
     const uint32_t nt = b.total_tiles;
     const SplitParams sp{b.bb.slice_offset[nt + 1], b.bb.slice_offset[nt + 2]};
     const uint32_t cnt = b.bb.tile_count[t], ns = tile_slices(cnt, sp);
@@ -367,8 +342,53 @@ __global__ void __launch_bounds__(256) batch_items_kernel(BatchDev b)
     }
 }
 
+// A fill's blocks, part after part (bin_fill_kernel): newline chunks, large triangles, tiles'
+// raster items, the rest the small triangles setup listed.  A warp's lanes may hold triangles
+// of different frames; their tiles are global tile indices.
+struct BatchFillParts {
+    uint32_t newline, large, items;
+};
+
+__global__ void __launch_bounds__(kSetupThreads, kFillMinBlocks)
+batch_fill_kernel(BatchDev b, const int2 *__restrict__ nl, BatchFillParts parts)
+{
+    extern __shared__ int32_t stree[];
+    uint32_t blk = blockIdx.x;
+    if (blk < parts.newline) {
+        batch_newline_block<true>(b, nl[blk], stree);
+        return;
+    }
+    blk -= parts.newline;
+    if (blk < parts.large) {
+        batch_large_items<true>(b, (blk * blockDim.x + threadIdx.x) >> 5, (parts.large * blockDim.x) >> 5);
+        return;
+    }
+    blk -= parts.large;
+    if (blk < parts.items) {
+        const uint32_t t = blk * blockDim.x + threadIdx.x;
+        if (t == 0) *b.queue = 0u;   // the persistent raster's item counter
+        if (t < b.total_tiles) batch_tile_items(b, t);
+        return;
+    }
+    blk -= parts.items;
+    const uint32_t n = *b.fill_count, step = (gridDim.x - parts.newline - parts.large - parts.items) * blockDim.x;
+    for (uint32_t i = blk * blockDim.x + threadIdx.x; i < n; i += step) {
+        const uint4 e = b.bb.fill_list[i];
+        const uint32_t meta = b.bb.fill_meta[i];
+        if (!(meta & kFillReread)) {
+            fill_listed(e, meta, b.bb.tile_offset, b.bb.tile_cursor, b.bb.entries, b.bb.capacity);
+        } else {
+            const BatchFrame &f = b.frames[e.z];
+            const Viewport vp = vp_batch(f.g);
+            const TriRecord r = load_record(f.fb.records, e.x);
+            fill_small(r, e.x, vp, tile_span(vp, r), b.bb.tile_offset, b.bb.tile_cursor, b.bb.entries, b.bb.capacity,
+                       e.y, f.tile_off);
+        }
+    }
+}
+
 // Raster item i (a tile, or a slice of a split tile, of any frame) of the item list built by
-// batch_items_kernel; false when its key load gave up (raster_tile).
+// the fill; false when its key load gave up (raster_tile).
 template <int TW, int TH>
 __device__ __forceinline__ bool batch_raster_item(TileSmem<TW, TH> &S, const BatchDev &b, uint32_t i, uint32_t &phase)
 {
@@ -385,7 +405,7 @@ __device__ __forceinline__ bool batch_raster_item(TileSmem<TW, TH> &S, const Bat
 
 // A render whose entries outgrew their buffer (its fill wrote what fitted) is rasterized
 // without tiles: every binned triangle is in the fill list or the large queue, and the
-// warps of the grid fold their samples straight into the keys, which batch_items_kernel has
+// warps of the grid fold their samples straight into the keys, which the fill has
 // made current.  The frames are exact, so nothing has to wait for the count; the host grows
 // the buffer before a later render.  Not inlined: the raster keeps its registers.
 __device__ __noinline__ void batch_overflow_fold(const BatchDev &b)
@@ -411,7 +431,7 @@ __device__ __noinline__ void batch_overflow_fold(const BatchDev &b)
 // Raster over every frame's tiles in one launch.  Persistent form (the default): a grid of
 // SMs x resident CTAs, each CTA taking the next item of the device-side (frame, tile)
 // queue -- the item list, split tiles' slices first -- from a counter (b.queue, zeroed by
-// batch_items_kernel) until the queue is empty.  The item is claimed by thread 0 and read
+// the fill) until the queue is empty.  The item is claimed by thread 0 and read
 // by every thread after a barrier, so the whole CTA leaves the loop together.  The other
 // form launches one CTA per item and leaves the balancing to the hardware block scheduler.
 template <int TW, int TH, bool kPersistent>
@@ -419,8 +439,9 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterMinBlocks) batch_raster
 {
     __shared__ TileSmem<TW, TH> S;
     __shared__ uint32_t s_item;
+    const uint32_t blk = blockIdx.x;
     if (b.bb.tile_offset[b.total_tiles] > b.bb.capacity) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (blk == 0 && threadIdx.x == 0) {
             *b.overflow = 1;
             b.status[0] = 1;
         }
@@ -428,10 +449,10 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterMinBlocks) batch_raster
         return;
     }
     const uint32_t nitems = min(b.bb.slice_offset[b.total_tiles], b.bb.item_capacity);
-    if (!kPersistent && blockIdx.x >= nitems) return;
+    if (!kPersistent && blk >= nitems) return;
     uint32_t phase = 0;
     if (!kPersistent) {
-        if (!batch_raster_item<TW, TH>(S, b, blockIdx.x, phase) && threadIdx.x == 0) b.status[1] = 1;
+        if (!batch_raster_item<TW, TH>(S, b, blk, phase) && threadIdx.x == 0) b.status[1] = 1;
         return;
     }
     for (;;) {
@@ -452,6 +473,7 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterMinBlocks) batch_raster
 // that wait on them at once count more than the loads each has in flight (uneven batch:
 // four blocks with four pairs of cells a thread 297 us, eight blocks with two 229).
 constexpr int kBatchRun = 2;
+static_assert(kBatchNewlineChunk == kNewlineChunk, "the host's table steps by the block's chunk");
 static_assert(kFoldBlockTris == kFoldTris, "the host's table steps by the block's triangles");
 static_assert(kBatchResolveChunk % (kBatchRun * 256) == 0 && kBatchResolveSmall % (kBatchRun * 256) == 0,
               "whole runs, the same trip count in every warp");
@@ -467,8 +489,7 @@ __global__ void __launch_bounds__(256, 8) batch_resolve_kernel(BatchDev b, const
     __shared__ BatchFrame sf;
     constexpr uint32_t kWords = sizeof(BatchFrame) / 4;
     static_assert(sizeof(BatchFrame) % 4 == 0 && kWords <= 256, "a word a thread");
-    pdl_trigger();
-    const int2 blk = blocks[blockIdx.x + pdl_wait()];
+    const int2 blk = blocks[blockIdx.x];
     if (threadIdx.x < kWords)
         reinterpret_cast<uint32_t *>(&sf)[threadIdx.x] =
             reinterpret_cast<const uint32_t *>(b.frames + blk.x)[threadIdx.x];
@@ -499,7 +520,7 @@ cudaError_t prepare_batch_kernels()
         (e = cudaFuncSetAttribute(batch_setup_kernel<true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
         return e;
     return cudaFuncSetAttribute(batch_newline_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                128 * 1024);
+                                (int)kNewlineSharedBytes);
 }
 
 cudaError_t launch_batch_setup(const BatchDev &b, const int2 *blocks, uint32_t nblocks, cudaStream_t s)
@@ -507,16 +528,10 @@ cudaError_t launch_batch_setup(const BatchDev &b, const int2 *blocks, uint32_t n
     if (!nblocks) return cudaSuccess;
     if (!valid_triangles_per_block(b.tpb)) return cudaErrorInvalidValue;
     const size_t smem = setup_smem_bytes(b.tpb, b.direct_max > 0);   // prepare_batch_kernels: above 48 KB
-    const dim3 grid(nblocks), block(setup_block_threads(b.tpb));
     const bool chunks = b.tpb > kSetupChunk;
-    if (b.direct_max > 0) {
-        if (chunks) batch_setup_kernel<true, true><<<grid, block, smem, s>>>(b, blocks);
-        else batch_setup_kernel<true, false><<<grid, block, smem, s>>>(b, blocks);
-    } else {
-        if (chunks) batch_setup_kernel<false, true><<<grid, block, smem, s>>>(b, blocks);
-        else batch_setup_kernel<false, false><<<grid, block, smem, s>>>(b, blocks);
-    }
-    return cudaGetLastError();
+    return launch(b.direct_max > 0 ? (chunks ? batch_setup_kernel<true, true> : batch_setup_kernel<true, false>)
+                                       : (chunks ? batch_setup_kernel<false, true> : batch_setup_kernel<false, false>),
+                      dim3(nblocks), dim3(setup_block_threads(b.tpb)), smem, s, b, blocks);
 }
 
 cudaError_t launch_batch_fold_setup(const BatchDev &b, const int2 *blocks, uint32_t nblocks, bool small,
@@ -526,46 +541,50 @@ cudaError_t launch_batch_fold_setup(const BatchDev &b, const int2 *blocks, uint3
     if (small) return launch_pdl(batch_fold_setup_kernel<4>, dim3(nblocks), dim3(128), kFoldSmemBytes, s, b, blocks);
     if (!valid_triangles_per_block(b.tpb)) return cudaErrorInvalidValue;
     const size_t smem = setup_smem_bytes(b.tpb, true);
-    const dim3 grid(nblocks), block(setup_block_threads(b.tpb));
-    if (b.tpb > kSetupChunk) batch_setup_kernel<true, true, true><<<grid, block, smem, s>>>(b, blocks);
-    else batch_setup_kernel<true, false, true><<<grid, block, smem, s>>>(b, blocks);
-    return cudaGetLastError();
+    return launch(b.tpb > kSetupChunk ? batch_setup_kernel<true, true, true> : batch_setup_kernel<true, false, true>,
+                      dim3(nblocks), dim3(setup_block_threads(b.tpb)), smem, s, b, blocks);
 }
 
-cudaError_t launch_batch_fold_large(const BatchDev &b, cudaStream_t s)
+bool batch_newline_part(uint32_t nblocks, int max_nl)
 {
-    return launch_pdl(batch_fold_large_kernel, dim3(4u * (unsigned)device_sm_count()), dim3(256), 0, s, b);
+    return nblocks <= kNewlinePartTriangles / kNewlineChunk && newline_tree_bytes(max_nl) <= kNewlinePartBytes;
+}
+
+cudaError_t launch_batch_fold_large(const BatchDev &b, const int2 *newline, uint32_t nnewline, int max_nl, cudaStream_t s)
+{
+    return launch(batch_fold_large_kernel, dim3(nnewline + 4u * (unsigned)device_sm_count()), dim3(256),
+                      nnewline ? newline_tree_bytes(max_nl) : 0, s, b, newline, nnewline);
 }
 
 cudaError_t launch_batch_reset(const BatchReset &r, cudaStream_t s)
 {
     const uint64_t most = std::max<uint64_t>(std::max<uint64_t>(r.nmats, r.ntiles), std::max<uint64_t>(r.nnl, r.n4));
     const uint64_t blocks = std::min<uint64_t>((most + 255) / 256, 16ull * (uint64_t)device_sm_count());
-    return launch_pdl(batch_reset_kernel, dim3((unsigned)std::max<uint64_t>(blocks, 1)), dim3(256), 0, s, r);
+    return launch(batch_reset_kernel, dim3((unsigned)std::max<uint64_t>(blocks, 1)), dim3(256), 0, s, r);
 }
 
 cudaError_t launch_batch_newline(const BatchDev &b, const int2 *blocks, uint32_t nblocks, int max_nl,
                                  cudaStream_t s)
 {
     if (!nblocks) return cudaSuccess;
-    const size_t smem = 2 * (size_t)max_nl * sizeof(int32_t);
-    if (smem <= 128 * 1024) batch_newline_kernel<true><<<nblocks, 1024, smem, s>>>(b, blocks);
-    else batch_newline_kernel<false><<<nblocks, 1024, 0, s>>>(b, blocks);
-    return cudaGetLastError();
+    const size_t smem = newline_tree_bytes(max_nl);
+    if (smem <= kNewlineSharedBytes)
+        return launch(batch_newline_kernel<true>, dim3(nblocks), dim3(1024), smem, s, b, blocks);
+    return launch(batch_newline_kernel<false>, dim3(nblocks), dim3(1024), 0, s, b, blocks);
 }
 
-cudaError_t launch_batch_bin_large(const BatchDev &b, bool fill, cudaStream_t s)
+cudaError_t launch_batch_count_large(const BatchDev &b, cudaStream_t s)
 {
-    const int grid = 8 * device_sm_count();   // eight CTAs of 8 warps per SM; the warps stride over the items
-    if (fill) batch_bin_large_kernel<true><<<grid, 256, 0, s>>>(b);
-    else batch_bin_large_kernel<false><<<grid, 256, 0, s>>>(b);
-    return cudaGetLastError();
+    // eight CTAs of 8 warps per SM; the warps stride over the items
+    return launch(batch_count_large_kernel, dim3(8u * (unsigned)device_sm_count()), dim3(256), 0, s, b);
 }
 
-cudaError_t launch_batch_fill(const BatchDev &b, cudaStream_t s)
+cudaError_t launch_batch_fill(const BatchDev &b, const int2 *newline, uint32_t nnewline, int max_nl, cudaStream_t s)
 {
-    batch_fill_kernel<<<kFillMinBlocks * 2 * device_sm_count(), kSetupThreads, 0, s>>>(b);
-    return cudaGetLastError();
+    const uint32_t sms = (uint32_t)device_sm_count();
+    const BatchFillParts parts{nnewline, 4u * sms, (b.total_tiles + kSetupThreads - 1) / kSetupThreads};
+    return launch(batch_fill_kernel, dim3(parts.newline + parts.large + parts.items + 2u * kFillMinBlocks * sms),
+                      dim3(kSetupThreads), nnewline ? newline_tree_bytes(max_nl) : 0, s, b, newline, parts);
 }
 
 // Resident CTAs per SM of a raster kernel (looked up once per kernel and device).
@@ -591,28 +610,19 @@ cudaError_t launch_batch_raster(const BatchDev &b, int tw, int th, bool persiste
             if (dev >= 0 && dev < 64 && !per_sm[dev]) per_sm[dev] = resident_ctas(batch_raster_kernel<W_, H_, true>); \
             const uint32_t slots = (uint32_t)device_sm_count() * (dev >= 0 && dev < 64 ? per_sm[dev] : 1); \
             const uint32_t grid = slots < b.bb.item_capacity ? slots : b.bb.item_capacity;     \
-            batch_raster_kernel<W_, H_, true><<<grid, kRasterThreads, 0, s>>>(b);              \
-        } else {                                                                               \
-            batch_raster_kernel<W_, H_, false><<<b.bb.item_capacity, kRasterThreads, 0, s>>>(b); \
+            return launch(batch_raster_kernel<W_, H_, true>, dim3(grid), dim3(kRasterThreads), 0, s, b); \
         }                                                                                      \
-        return cudaGetLastError();                                                             \
+        return launch(batch_raster_kernel<W_, H_, false>, dim3(b.bb.item_capacity), dim3(kRasterThreads), 0, s, b); \
     }
     SLOTH_TILE_SHAPES(SLOTH_BATCH_RASTER_CASE)
 #undef SLOTH_BATCH_RASTER_CASE
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_batch_items(const BatchDev &b, cudaStream_t s)
-{
-    if (!b.total_tiles) return cudaSuccess;
-    batch_items_kernel<<<(b.total_tiles + 255) / 256, 256, 0, s>>>(b);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_batch_resolve(const BatchDev &b, const int2 *blocks, uint32_t nblocks, bool odd, cudaStream_t s)
 {
     if (!nblocks) return cudaSuccess;
-    return launch_pdl(odd ? batch_resolve_kernel<true> : batch_resolve_kernel<false>, dim3(nblocks), dim3(256), 0, s, b, blocks);
+    return launch(odd ? batch_resolve_kernel<true> : batch_resolve_kernel<false>, dim3(nblocks), dim3(256), 0, s, b, blocks);
 }
 
 }  // namespace sloth

@@ -92,10 +92,9 @@ struct sloth_batch {
 
     cudaGraphExec_t graph = nullptr;
     bool rendered = false;
-    // side branches of a render: the newline fold (beside the binning) and the
-    // large-triangle fill (beside the small one), forked from and joined into `stream`
-    cudaStream_t nl_s = nullptr, aux_s = nullptr;
-    cudaEvent_t ev_setup = nullptr, ev_nl = nullptr, ev_fill = nullptr, ev_aux = nullptr;
+    // a large batch's newline fold beside the rest: forked from and joined into `stream`
+    cudaStream_t nl_s = nullptr;
+    cudaEvent_t ev_setup = nullptr, ev_nl = nullptr;
 
     // differentiable shading
     int2 *diff_blk = nullptr;                 // (frame, first depth cell) per kDiffChunk
@@ -441,53 +440,55 @@ cudaError_t enqueue_reset(sloth_batch *b, cudaStream_t s)
     return cudaSuccess;
 }
 
+// The newline rows of the draws setup has taken, on the batch's own stream.
+cudaError_t fork_newline(sloth_batch *b, const BatchDev &d, cudaStream_t s)
+{
+    cudaError_t e;
+    if ((e = cudaEventRecord(b->ev_setup, s))) return e;
+    if ((e = cudaStreamWaitEvent(b->nl_s, b->ev_setup, 0))) return e;
+    if ((e = launch_batch_newline(d, b->blk[kTabNewline], b->nblk[kTabNewline], b->max_nl, b->nl_s))) return e;
+    return cudaEventRecord(b->ev_nl, b->nl_s);
+}
+
 // A render without tiles: reset, setup and fold, queued triangles, resolve.
 cudaError_t enqueue_folded(sloth_batch *b, const BatchDev &d, cudaStream_t s)
 {
     cudaError_t e;
     if ((e = enqueue_reset(b, s))) return e;
-    const bool side = !b->small_fold;   // the newline fold beside the rest
     const int table = b->small_fold ? kTabFold : kTabSetup;
     if ((e = launch_batch_fold_setup(d, b->blk[table], b->nblk[table], b->small_fold, s))) return e;
-    if (side) {   // the small fold reduces the newline rows itself
-        if ((e = cudaEventRecord(b->ev_fill, s))) return e;
-        if ((e = cudaStreamWaitEvent(b->nl_s, b->ev_fill, 0))) return e;
-        if ((e = launch_batch_newline(d, b->blk[kTabNewline], b->nblk[kTabNewline], b->max_nl, b->nl_s))) return e;
-    }
-    if (side && (e = cudaEventRecord(b->ev_nl, b->nl_s))) return e;
-    if ((e = launch_batch_fold_large(d, s))) return e;
-    if (side && (e = cudaStreamWaitEvent(s, b->ev_nl, 0))) return e;
+    // the small fold reduces the newline rows itself
+    const uint32_t nnl = b->small_fold ? 0u : b->nblk[kTabNewline];
+    const bool part = batch_newline_part(nnl, b->max_nl), fork = nnl && !part;
+    if (fork && (e = fork_newline(b, d, s))) return e;
+    if ((e = launch_batch_fold_large(d, b->blk[kTabNewline], part ? nnl : 0u, b->max_nl, s))) return e;
+    if (fork && (e = cudaStreamWaitEvent(s, b->ev_nl, 0))) return e;
     return launch_batch_resolve(d, b->blk[kTabResolve], b->nblk[kTabResolve], b->any_odd, s);
 }
 
-// Stage 1: reset, setup, newline, large counts, scan.
+// Stage 1: reset, setup (and the newline fold of a large batch beside the rest), large
+// counts, scan.
 cudaError_t enqueue_front(sloth_batch *b, const BatchDev &d, cudaStream_t s)
 {
     cudaError_t e;
     if ((e = enqueue_reset(b, s))) return e;
     if ((e = launch_batch_setup(d, b->blk[kTabSetup], b->nblk[kTabSetup], s))) return e;
-    if ((e = cudaEventRecord(b->ev_setup, s))) return e;
-    if ((e = cudaStreamWaitEvent(b->nl_s, b->ev_setup, 0))) return e;
-    if ((e = launch_batch_newline(d, b->blk[kTabNewline], b->nblk[kTabNewline], b->max_nl, b->nl_s))) return e;
-    if ((e = cudaEventRecord(b->ev_nl, b->nl_s))) return e;
-    if ((e = launch_batch_bin_large(d, false, s))) return e;
+    if (b->nblk[kTabNewline] && !batch_newline_part(b->nblk[kTabNewline], b->max_nl) && (e = fork_newline(b, d, s)))
+        return e;
+    if ((e = launch_batch_count_large(d, s))) return e;
     return launch_bin_scan(b->total_tiles, d.bb, s);
 }
 
-// Stage 2: fill, persistent raster, resolve.
+// Stage 2: fill (and newline rows), raster, resolve.
 cudaError_t enqueue_back(sloth_batch *b, const BatchDev &d, cudaStream_t s)
 {
     cudaError_t e;
-    if ((e = cudaEventRecord(b->ev_fill, s))) return e;
-    if ((e = cudaStreamWaitEvent(b->aux_s, b->ev_fill, 0))) return e;
-    if ((e = launch_batch_bin_large(d, true, b->aux_s))) return e;
-    if ((e = cudaEventRecord(b->ev_aux, b->aux_s))) return e;
-    if ((e = launch_batch_fill(d, s))) return e;
-    if ((e = cudaStreamWaitEvent(s, b->ev_aux, 0))) return e;
-    if ((e = launch_batch_items(d, s))) return e;
+    const uint32_t nnl = b->nblk[kTabNewline];
+    const bool part = batch_newline_part(nnl, b->max_nl);
+    if ((e = launch_batch_fill(d, b->blk[kTabNewline], part ? nnl : 0u, b->max_nl, s))) return e;
     const int tw = kTileShapes[b->shape][0], th = kTileShapes[b->shape][1];
     if ((e = launch_batch_raster(d, tw, th, b->persistent, s))) return e;
-    if ((e = cudaStreamWaitEvent(s, b->ev_nl, 0))) return e;   // the newline tree is complete
+    if (nnl && !part && (e = cudaStreamWaitEvent(s, b->ev_nl, 0))) return e;   // the newline tree is complete
     return launch_batch_resolve(d, b->blk[kTabResolve], b->nblk[kTabResolve], b->any_odd, s);
 }
 
@@ -599,7 +600,6 @@ void sloth_batch_detach(sloth_batch *b)
     cudaSetDevice(b->device);
     cudaStreamSynchronize(b->stream);
     if (b->nl_s) cudaStreamSynchronize(b->nl_s);
-    if (b->aux_s) cudaStreamSynchronize(b->aux_s);
     free_layout(b);
     bfree(b->diff_blk);
     bfree(b->vis);
@@ -610,16 +610,13 @@ void sloth_batch_detach(sloth_batch *b)
     if (b->h_error) cudaFreeHost(b->h_error);
     if (b->status) cudaFreeHost(b->status);
     bfree(b->error);
-    for (cudaEvent_t *ev : {&b->ev_setup, &b->ev_nl, &b->ev_fill, &b->ev_aux})
+    for (cudaEvent_t *ev : {&b->ev_setup, &b->ev_nl})
         if (*ev) {
             cudaEventDestroy(*ev);
             *ev = nullptr;
         }
-    for (cudaStream_t *st : {&b->nl_s, &b->aux_s})
-        if (*st) {
-            cudaStreamDestroy(*st);
-            *st = nullptr;
-        }
+    if (b->nl_s) cudaStreamDestroy(b->nl_s);
+    b->nl_s = nullptr;
     b->h_mats = nullptr;
     b->h_total = b->h_overflow = b->h_error = b->status = nullptr;
     b->ctx = nullptr;
@@ -670,11 +667,8 @@ sloth_status sloth_batch_create(sloth_ctx *ctx, const sloth_frame_desc *frames, 
         cudaMalloc(&b->error, 4) != cudaSuccess ||
         cudaMemset(b->error, 0, 4) != cudaSuccess ||
         cudaStreamCreateWithFlags(&b->nl_s, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&b->aux_s, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->ev_setup, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->ev_nl, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b->ev_fill, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b->ev_aux, cudaEventDisableTiming) != cudaSuccess ||
         prepare_batch_kernels() != cudaSuccess) {
         sloth_batch_detach(b);
         delete b;

@@ -45,7 +45,7 @@ struct BatchDev {
     uint32_t *overflow;        // set when the entries outgrew their capacity
     volatile uint32_t *status; // pinned host words: [0] a render's entries outgrew their capacity,
                                // [1] a raster block gave up waiting for its keys
-    uint32_t *queue;           // the persistent raster's next item (zeroed by the item kernel)
+    uint32_t *queue;           // the persistent raster's next item (zeroed by the fill)
     uint32_t *fill_count;      // entries of bb.fill_list (zeroed at the start of a render)
     int depth_cull;
     int tpb;                   // triangles per setup block (the triangle block table's step)
@@ -74,22 +74,27 @@ cudaError_t launch_batch_reset(const BatchReset &r, cudaStream_t s);
 
 // Block tables: one int2 (item, start) per block, built on the host.
 cudaError_t launch_batch_setup(const BatchDev &b, const int2 *blocks, uint32_t nblocks, cudaStream_t s);
+// whether the fill's and the fold's blocks take a newline table of nblocks blocks and trees
+// of max_nl leaves; launch_batch_newline when they do not
+bool batch_newline_part(uint32_t nblocks, int max_nl);
 cudaError_t launch_batch_newline(const BatchDev &b, const int2 *blocks, uint32_t nblocks, int max_nl,
                                  cudaStream_t s);
-cudaError_t launch_batch_bin_large(const BatchDev &b, bool fill, cudaStream_t s);
-cudaError_t launch_batch_fill(const BatchDev &b, cudaStream_t s);
-cudaError_t launch_batch_items(const BatchDev &b, cudaStream_t s);
+cudaError_t launch_batch_count_large(const BatchDev &b, cudaStream_t s);
+// the tile entries, the raster items and nnewline blocks of the newline table (0 unless
+// batch_newline_part)
+cudaError_t launch_batch_fill(const BatchDev &b, const int2 *newline, uint32_t nnewline, int max_nl, cudaStream_t s);
 cudaError_t launch_batch_raster(const BatchDev &b, int tw, int th, bool persistent, cudaStream_t s);
 // frames without tiles: setup and fold (blocks: a kFoldBlockTris table when small, else the
 // setup table), then the queued triangles
 cudaError_t launch_batch_fold_setup(const BatchDev &b, const int2 *blocks, uint32_t nblocks, bool small,
                                     cudaStream_t s);
-cudaError_t launch_batch_fold_large(const BatchDev &b, cudaStream_t s);
+cudaError_t launch_batch_fold_large(const BatchDev &b, const int2 *newline, uint32_t nnewline, int max_nl,
+                                    cudaStream_t s);
 // odd: some frame has an odd width
 cudaError_t launch_batch_resolve(const BatchDev &b, const int2 *blocks, uint32_t nblocks, bool odd, cudaStream_t s);
 cudaError_t prepare_batch_kernels();
 
-constexpr uint32_t kBatchNewlineChunk = 8192;   // triangles per newline block
+constexpr uint32_t kBatchNewlineChunk = 8192;   // triangles per newline block (kNewlineChunk)
 constexpr uint32_t kBatchResolveChunk = 8192;   // cells per resolve block (four rounds of its threads)
 constexpr uint32_t kBatchResolveSmall = 2048;   // the same (one round) for batches of few blocks
 constexpr uint32_t kFoldBlockTris = 32;         // triangles per block of a small fold's table

@@ -4,7 +4,11 @@
 // (src/rasterizer.rs:69-70).  Here each triangle is listed in the tiles whose depth
 // cells it can write: count (setup kernel for small triangles, one warp per large
 // triangle here), exclusive scan over tiles, then fill (bin_common.cuh).
+#include <algorithm>
+
 #include "bin_common.cuh"
+#include "launch.cuh"
+#include "newline.cuh"
 #include "record.cuh"
 #include "sloth_kernels.h"
 
@@ -15,14 +19,12 @@ __device__ __forceinline__ Viewport vp_of(const FrameGeom &g)
     return Viewport{g.w, g.h, g.image, g.tw, g.th, g.ntx, g.nty, g.pitch};
 }
 
-// Warps over the parts of the queued large triangles.
+// Warps over the parts of the queued large triangles: warp `warp` of nwarps.
 template <bool kFill>
-__global__ void __launch_bounds__(256)
-bin_large_kernel(uint32_t tri_base, FrameGeom g, FrameBuffers fb, BinBuffers bb)
+__device__ __forceinline__ void bin_large_items(uint32_t tri_base, const FrameGeom &g, const FrameBuffers &fb,
+                                                const BinBuffers &bb, uint32_t warp, uint32_t nwarps)
 {
     const int lane = threadIdx.x & 31;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t items = large_items(bb.large_count);
     const Viewport vp = vp_of(g);
     for (uint32_t it = warp; it < items; it += nwarps) {
@@ -32,6 +34,13 @@ bin_large_kernel(uint32_t tri_base, FrameGeom g, FrameBuffers fb, BinBuffers bb)
         bin_large_warp<kFill>(fb.records + gtri, gtri, vp, bb.tile_count, bb.tile_cursor, bb.entries,
                               bb.capacity, lane, part, nparts);
     }
+}
+
+__global__ void __launch_bounds__(256)
+bin_count_large_kernel(uint32_t tri_base, FrameGeom g, FrameBuffers fb, BinBuffers bb)
+{
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x + pdl_begin()) >> 5;
+    bin_large_items<false>(tri_base, g, fb, bb, warp, (gridDim.x * blockDim.x) >> 5);
 }
 
 __device__ __forceinline__ SplitParams split_params(const BinBuffers &bb, uint32_t n)
@@ -77,7 +86,7 @@ __global__ void __launch_bounds__(1024) bin_scan_kernel(uint32_t n, BinBuffers b
     __shared__ uint32_t carry[kV];
     __shared__ SplitParams sp_s;
     __shared__ uint32_t light_s;
-    const uint32_t tid = threadIdx.x;
+    const uint32_t tid = threadIdx.x + pdl_wait();   // its dependents would wait on the whole GPU meanwhile
     const int lane = tid & 31, wid = tid >> 5;
     // pass 1: entries and non-empty tiles, four consecutive tiles per thread and step as in
     // pass 2; the first step's counts stay in registers for pass 2
@@ -202,7 +211,6 @@ __global__ void __launch_bounds__(1024) bin_scan_kernel(uint32_t n, BinBuffers b
         block_sync();
     }
     if (tid == 0) {
-        if (bb.max_total) atomicMax(bb.max_total, carry[0]);
         bb.tile_offset[n] = carry[0];
         bb.slice_offset[n] = carry[1] + carry[2] + carry[3];
         bb.slice_offset[n + 1] = sp.threshold;
@@ -213,16 +221,14 @@ __global__ void __launch_bounds__(1024) bin_scan_kernel(uint32_t n, BinBuffers b
     }
 }
 
-// One thread per tile: the raster items (tile, slice) of the tile, and for a tile that is
+// Tile t: the raster items (tile, slice) of the tile, and for a tile that is
 // rasterized in slices, its keys cleared (unless they hold keys of earlier draws since
 // the clear) and its generation set before the slices fold into them.  When the draw's
 // entries outgrew the buffer (the raster folds its triangles without tiles), every tile
 // gets that treatment instead.
-__global__ void __launch_bounds__(256)
-bin_items_kernel(uint32_t n, FrameGeom g, FrameBuffers fb, BinBuffers bb)
+__device__ __forceinline__ void bin_tile_items(uint32_t t, uint32_t n, const FrameGeom &g, const FrameBuffers &fb,
+                                               const BinBuffers &bb)
 {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
     if (bb.tile_offset[n] > bb.capacity) {
         if (fb.tile_gen[t] != fb.gen) {
             const int tr = (int)t / g.ntx, tc = (int)t - tr * g.ntx;
@@ -249,13 +255,43 @@ bin_items_kernel(uint32_t n, FrameGeom g, FrameBuffers fb, BinBuffers bb)
     }
 }
 
-// The small binned triangles setup listed, 256 per block and round (grid-stride): their
-// tile entries.
+// A fill's blocks, part after part: newline chunks, large triangles, tiles' raster items,
+// the rest the small triangles.  The parts read what setup and the scan left and do not
+// touch each other, so they share one launch: as four launches on three streams, with the
+// events between them, they and the waits around them left the GPU idle for a tenth of a
+// frame of a million triangles.  The longest blocks start first.
+struct FillParts {
+    uint32_t newline, large, items;
+};
+
 __global__ void __launch_bounds__(kSetupThreads, kFillMinBlocks)
-bin_fill_kernel(FrameGeom g, FrameBuffers fb, BinBuffers bb)
+bin_fill_kernel(uint32_t ntri, const uint32_t *__restrict__ order, uint32_t tri_base, uint32_t ntiles, FrameGeom g,
+                FrameBuffers fb, BinBuffers bb, FillParts parts)
 {
-    const uint32_t n = bb.large_count[2];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    extern __shared__ int32_t stree[];
+    uint32_t blk = blockIdx.x + pdl_begin();
+    if (blk < parts.newline) {
+        const uint32_t lo = blk * kNewlineChunk;
+        newline_block<true>(stree, g.nl_size, lo, min(ntri, lo + kNewlineChunk), order, fb.rows + tri_base, tri_base,
+                            fb.nltree);
+        return;
+    }
+    blk -= parts.newline;
+    if (blk < parts.large) {
+        bin_large_items<true>(tri_base, g, fb, bb, (blk * blockDim.x + threadIdx.x) >> 5,
+                              (parts.large * blockDim.x) >> 5);
+        return;
+    }
+    blk -= parts.large;
+    if (blk < parts.items) {
+        const uint32_t t = blk * blockDim.x + threadIdx.x;
+        if (t < ntiles) bin_tile_items(t, ntiles, g, fb, bb);
+        return;
+    }
+    blk -= parts.items;
+    // the small triangles setup listed
+    const uint32_t n = bb.large_count[2], step = (gridDim.x - parts.newline - parts.large - parts.items) * blockDim.x;
+    for (uint32_t i = blk * blockDim.x + threadIdx.x; i < n; i += step) {
         const uint4 e = bb.fill_list[i];
         const uint32_t meta = bb.fill_meta[i];
         if (!(meta & kFillReread)) {
@@ -268,43 +304,36 @@ bin_fill_kernel(FrameGeom g, FrameBuffers fb, BinBuffers bb)
     }
 }
 
-static int large_grid()
-{
-    return 8 * device_sm_count();   // up to eight CTAs of 8 warps per SM; the warps stride over the items
-}
-
 cudaError_t launch_bin_count_large(uint32_t tri_base, const FrameGeom &g, const FrameBuffers &fb,
                                    const BinBuffers &bb, cudaStream_t s)
 {
-    bin_large_kernel<false><<<large_grid(), 256, 0, s>>>(tri_base, g, fb, bb);
-    return cudaGetLastError();
+    // up to eight CTAs of 8 warps per SM; the warps stride over the items
+    return launch_pdl(bin_count_large_kernel, dim3(8u * (unsigned)device_sm_count()), dim3(256), 0, s, tri_base, g, fb,
+                      bb);
 }
 
 cudaError_t launch_bin_scan(uint32_t ntiles, const BinBuffers &bb, cudaStream_t s)
 {
-    bin_scan_kernel<<<1, 1024, 0, s>>>(ntiles, bb);
-    return cudaGetLastError();
+    return launch_pdl(bin_scan_kernel, dim3(1), dim3(1024), 0, s, ntiles, bb);
 }
 
-cudaError_t launch_bin_items(uint32_t ntiles, const FrameGeom &g, const FrameBuffers &fb, const BinBuffers &bb,
-                             cudaStream_t s)
+bool newline_in_fill(uint32_t ntri, const FrameGeom &g)
 {
-    if (ntiles == 0) return cudaSuccess;
-    bin_items_kernel<<<(ntiles + 255) / 256, 256, 0, s>>>(ntiles, g, fb, bb);
-    return cudaGetLastError();
+    return g.image && ntri <= kNewlinePartTriangles && newline_tree_bytes(g.nl_size) <= kNewlinePartBytes;
 }
 
-cudaError_t launch_bin_fill(const FrameGeom &g, const FrameBuffers &fb, const BinBuffers &bb, cudaStream_t s)
+cudaError_t launch_bin_fill(uint32_t ntri, const uint32_t *order, uint32_t tri_base, uint32_t ntiles,
+                            const FrameGeom &g, const FrameBuffers &fb, const BinBuffers &bb, cudaStream_t s)
 {
-    bin_fill_kernel<<<kFillMinBlocks * 2 * device_sm_count(), kSetupThreads, 0, s>>>(g, fb, bb);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_bin_fill_large(uint32_t tri_base, const FrameGeom &g, const FrameBuffers &fb,
-                                  const BinBuffers &bb, cudaStream_t s)
-{
-    bin_large_kernel<true><<<large_grid(), 256, 0, s>>>(tri_base, g, fb, bb);
-    return cudaGetLastError();
+    const uint32_t sms = (uint32_t)device_sm_count();
+    FillParts parts{};
+    parts.newline = newline_in_fill(ntri, g) ? (ntri + kNewlineChunk - 1) / kNewlineChunk : 0u;
+    parts.large = 4u * sms;
+    parts.items = (ntiles + kSetupThreads - 1) / kSetupThreads;
+    const uint32_t small = std::min(2u * kFillMinBlocks * sms, (ntri + kSetupThreads - 1) / kSetupThreads);
+    const size_t smem = parts.newline ? newline_tree_bytes(g.nl_size) : 0;
+    return launch_pdl(bin_fill_kernel, dim3(parts.newline + parts.large + parts.items + std::max(small, 1u)),
+                      dim3(kSetupThreads), smem, s, ntri, order, tri_base, ntiles, g, fb, bb, parts);
 }
 
 }  // namespace sloth

@@ -12,8 +12,7 @@ namespace sloth {
 __global__ void __launch_bounds__(256)
 fold_begin_kernel(FrameGeom g, FrameBuffers fb, uint32_t nl_nodes, int frame, int all, uint32_t *queue_counts)
 {
-    pdl_trigger();
-    const uint32_t t = blockIdx.x + pdl_wait();
+    const uint32_t t = blockIdx.x + pdl_begin();
     if (frame)
         for (uint32_t i = t * blockDim.x + threadIdx.x; i < nl_nodes; i += gridDim.x * blockDim.x) fb.nltree[i] = -1;
     if (t == 0 && threadIdx.x == 0) {
@@ -41,8 +40,7 @@ template <int kWarps>
 __global__ void __launch_bounds__(32 * kWarps)
 fold_setup_kernel(MeshDev mesh, Mat4 M, uint32_t tri_base, FrameGeom g, FrameBuffers fb, FoldQueue queue)
 {
-    pdl_trigger();
-    fold_triangles<kWarps>(mesh, M, blockIdx.x * kFoldTris + pdl_wait(), tri_base, g, fb, queue, 0u);
+    fold_triangles<kWarps>(mesh, M, blockIdx.x * kFoldTris + pdl_begin(), tri_base, g, fb, queue, 0u);
 }
 
 // The queued triangles' items over the warps of the grid, the large ones' first.  next: the
@@ -51,8 +49,7 @@ fold_setup_kernel(MeshDev mesh, Mat4 M, uint32_t tri_base, FrameGeom g, FrameBuf
 __global__ void __launch_bounds__(256)
 fold_large_kernel(FrameGeom g, FrameBuffers fb, FoldQueue queue, uint32_t *next)
 {
-    pdl_trigger();
-    const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x + pdl_wait()) >> 5;
+    const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x + pdl_begin()) >> 5;
     if (blockIdx.x == 0 && threadIdx.x < 2) next[threadIdx.x] = 0u;
     const uint32_t large = queue.count[0], mid = queue.count[1], nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t parts = fold_parts(large), cut = large * parts, items = cut + mid;

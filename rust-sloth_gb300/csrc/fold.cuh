@@ -135,7 +135,7 @@ __device__ __forceinline__ void fold_triangles(const MeshDev &mesh, const Mat4 &
                 r = build_record(p1, p2, p3, rgb, g.w, g.h, INT_MAX, &dw);
                 if (r.x0 < r.xe) {
                     c = fold_class(r, dw);
-                    store_record(fb.records + gtri, r, 1u, true);
+                    store_record(fb.records + gtri, r, true);
                 }
             }
         }

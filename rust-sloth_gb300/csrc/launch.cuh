@@ -21,8 +21,26 @@ __device__ __forceinline__ uint32_t pdl_wait()
     return zero;
 }
 
-// Lets the dependents of this kernel be scheduled once every block has called it or left.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// pdl_wait, and then lets this kernel's dependents be scheduled (once every block has come
+// here or left).  Not before the wait: a chain of kernels would all become resident behind
+// the first, and take the SMs from work on other streams (the newline fold of the uneven
+// batch, launched so, ran after the fill instead of beside the scan: 1612 us a pass became 1716).
+__device__ __forceinline__ uint32_t pdl_begin()
+{
+    const uint32_t zero = pdl_wait();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    return zero;
+}
+
+// An ordinary launch with the same arguments: what the kernels of a captured graph use, where
+// the edges between dependents cost what they save (uneven batch 1583 us a pass with them,
+// 1561 without; 24 views of 160x48 38.4 and 36.0).
+template <class... K, class... A>
+cudaError_t launch(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
+{
+    kernel<<<grid, block, smem, s>>>(static_cast<K>(args)...);
+    return cudaGetLastError();
+}
 
 template <class... K, class... A>
 cudaError_t launch_pdl(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)

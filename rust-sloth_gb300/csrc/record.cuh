@@ -71,13 +71,10 @@ __device__ __forceinline__ int sat_hi(float f)
     return f > 0.0f ? (int)f : 0;
 }
 
-// Stores a record.  A triangle with no tile (culled, empty sample range) only ever has its
-// sample range read -- by a context's overflow fold and the no-allocation raster, which
-// stop there -- so only that row is written, with zeros in row 5 beside it (store_row4: a
-// whole 32-byte sector, which the memory writes back without reading it first).  A direct
-// triangle (direct.cuh) is never binned nor rasterized again: only the rows the resolve
-// (0-1, 5) and a context's overflow fold (4) read are written.
-__device__ __forceinline__ void store_record(TriRecord *dst, const TriRecord &r, uint32_t ntiles, bool direct = false)
+// Stores a record.  A direct triangle (direct.cuh) is never binned nor rasterized again: only
+// the rows the resolve and the shading (0-1, 5) and the walk of queued triangles (4) read
+// are written, row 4 beside row 5 as one whole 32-byte sector.
+__device__ __forceinline__ void store_record(TriRecord *dst, const TriRecord &r, bool direct = false)
 {
     const int4 *src = reinterpret_cast<const int4 *>(&r);
     int4 *d = reinterpret_cast<int4 *>(dst);
@@ -86,29 +83,16 @@ __device__ __forceinline__ void store_record(TriRecord *dst, const TriRecord &r,
         d[1] = src[1];
         d[4] = src[4];
         d[5] = src[5];
-    } else if (ntiles != 0) {
-        *dst = r;
     } else {
-        d[4] = make_int4(r.x0, r.xe, r.y0, r.y1);
-        d[5] = make_int4(0, 0, 0, 0);
+        *dst = r;
     }
-}
-
-// Record rows 4 (the sample range, row4) and 5 (zeros) of a triangle with nothing to
-// rasterize (store_record).
-__device__ __forceinline__ void store_row4(TriRecord *dst, int4 row4)
-{
-    int4 *d = reinterpret_cast<int4 *>(dst);
-    d[4] = row4;
-    d[5] = make_int4(0, 0, 0, 0);
 }
 
 // The first steps of build_record, for a setup kernel that sets triangles aside before the
 // rest of their setup: the sample range and the back-face proof over the untightened range
 // (the same operations as build_record).  Returns false for a triangle with an empty range
-// or proven to cover no sample, with `row4` its record row 4 (x0, xe, y0, y1) -- all that
-// is ever read of such a triangle; true when the triangle needs build_record.  Either way
-// row4.z and row4.w are the rows [y0, y1) the record will hold.
+// or proven to cover no sample; true when the triangle needs build_record.  Either way
+// row4.z and row4.w are the rows [y0, y1) the record would hold.
 __device__ __forceinline__ bool needs_setup(float4 p1, float4 p2, float4 p3, int w, int h, int4 &row4)
 {
     TriRecord r;   // the fields orient_bound reads

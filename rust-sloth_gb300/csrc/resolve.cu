@@ -19,8 +19,7 @@ constexpr int kEvenPairs = 1;
 template <bool kEven>
 __global__ void __launch_bounds__(256, 8) resolve_kernel(FrameGeom g, FrameBuffers fb, int vec)
 {
-    pdl_trigger();
-    const uint32_t tid = threadIdx.x + pdl_wait(), ncells = frame_cells(g);
+    const uint32_t tid = threadIdx.x + pdl_begin(), ncells = frame_cells(g);
     if (kEven) {
         const uint32_t npairs = ncells / 2 + (ncells & 1u), span = blockDim.x * kEvenPairs;
         for (uint64_t base = (uint64_t)blockIdx.x * span; base < npairs; base += (uint64_t)gridDim.x * span)
@@ -55,8 +54,7 @@ cudaError_t launch_resolve(const FrameGeom &g, const FrameBuffers &fb, cudaStrea
 // the copy engine about 10 us each; this is one launch behind the resolve.
 __global__ void __launch_bounds__(256) readback_kernel(ReadBack r)
 {
-    pdl_trigger();
-    const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x + pdl_wait(), step = gridDim.x * blockDim.x;
+    const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x + pdl_begin(), step = gridDim.x * blockDim.x;
     if (i0 == 0) *r.error_out = *r.error;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {

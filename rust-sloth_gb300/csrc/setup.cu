@@ -10,6 +10,8 @@
 
 #include "bin_common.cuh"
 #include "direct.cuh"
+#include "launch.cuh"
+#include "newline.cuh"
 #include "record.cuh"
 #include "sloth_kernels.h"
 
@@ -19,7 +21,7 @@ namespace sloth {
 __global__ void __launch_bounds__(256) vertex_transform_kernel(MeshDev mesh, Mat4 M, float4 *tv)
 {
     const uint32_t nv = mesh.nvert;
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;   // quad index
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x + pdl_begin();   // quad index
     const uint32_t i0 = q * 4;
     if (i0 >= nv) return;
     float xs[4], ys[4], zs[4];
@@ -87,7 +89,9 @@ __device__ __forceinline__ void setup_triangle(uint32_t tri_base, const FrameGeo
         r = build_record(p1, p2, p3, rgb, g.w, g.h, kDirect ? g.direct_max : 0, kDirect ? &dw : nullptr);
         direct = dw.direct;
         if (!direct) sp = tile_span(vp, r);   // a direct triangle is not binned
-        store_record(fb.records + tri_base + t, r, sp.ntiles, direct);
+        // a triangle with nothing to rasterize is never read back (the fill and the overflow
+        // fold walk the lists, the newline the packed rows): its record is not written
+        if (direct || sp.ntiles != 0) store_record(fb.records + tri_base + t, r, direct);
         large = sp.large;
     }
     // binning: count tiles of small triangles here and list them for the fill, queue the
@@ -122,7 +126,7 @@ __device__ __forceinline__ void setup_triangle(uint32_t tri_base, const FrameGeo
 
 // A block takes tpb triangles, in chunks of setup_chunk(tpb), each in two phases.  Phase 1:
 // every triangle gets its sample range and the back-face proof (needs_setup); those with
-// nothing to rasterize store their range row and are done, the others are queued in
+// nothing to rasterize are done, the others are queued in
 // shared memory with their vertices and colour.  Phase 2: the queued triangles, dense in
 // the lanes, get the rest of their setup (setup_triangle) without touching global memory
 // for their inputs again.  Back faces are about half of a closed mesh's triangles, and
@@ -140,7 +144,7 @@ setup_kernel(MeshDev mesh, const float4 *__restrict__ tv, Mat4 M, uint32_t tri_b
     const SetupStash st{cap};
     if (threadIdx.x == 0) sq_n = 0;
     block_sync();
-    const uint32_t t0 = blockIdx.x * (uint32_t)tpb, t_end = min(mesh.ntri, t0 + (uint32_t)tpb);
+    const uint32_t t0 = blockIdx.x * (uint32_t)tpb + pdl_begin(), t_end = min(mesh.ntri, t0 + (uint32_t)tpb);
     uint32_t base = 0;
     for (uint32_t c0 = t0; c0 < t_end; c0 += cap) {
         // two triangles per round, their vertex loads issued together (the trip count is
@@ -164,11 +168,9 @@ setup_kernel(MeshDev mesh, const float4 *__restrict__ tv, Mat4 M, uint32_t tri_b
             }
             int4 row4;
             const bool kt = lt && needs_setup(a1, a2, a3, g.w, g.h, row4);
-            if (lt && !kt) store_row4(fb.records + tri_base + tp, row4);
             if (lt) fb.rows[tri_base + p] = pack_rows(row4.z, row4.w);
             stash_push(st, &sq_n, base, kt, tp, a1, a2, a3, ca);
             const bool ku = lu && needs_setup(b1, b2, b3, g.w, g.h, row4);
-            if (lu && !ku) store_row4(fb.records + tri_base + tq, row4);
             if (lu) fb.rows[tri_base + q] = pack_rows(row4.z, row4.w);
             stash_push(st, &sq_n, base, ku, tq, b1, b2, b3, cb);
         }
@@ -188,58 +190,29 @@ setup_kernel(MeshDev mesh, const float4 *__restrict__ tv, Mat4 M, uint32_t tri_b
     }
 }
 
-// Newline sentinels (src/rasterizer.rs:89-91): in image mode every row y in [y0,y1) of
-// every triangle gets frame cell y*w+1 = '\n' after the row's samples.  The resolve needs,
-// per row, the last triangle in draw order that wrote it: the maximum draw index whose
-// [y0,y1) contains y.  Each triangle folds its interval into a max segment tree with
-// O(log h) node updates (canonical decomposition); a row's value is the maximum over its
-// leaf-to-root path.  Each block builds a tree for a chunk of triangles in shared memory,
-// then merges its non-empty nodes into the frame's tree.  The rows come from the packed
-// array setup wrote (4 bytes a triangle, read in setup's order: order maps a position to
-// its triangle), not from the records' row 4.
+// The newline rows of a draw (newline.cuh) in a launch of their own.
 template <bool kShared>
 __global__ void __launch_bounds__(1024)
-newline_kernel(uint32_t ntri, const uint32_t *__restrict__ order, uint32_t tri_base, uint32_t chunk, FrameGeom g,
-               FrameBuffers fb)
+newline_kernel(uint32_t ntri, const uint32_t *__restrict__ order, uint32_t tri_base, FrameGeom g, FrameBuffers fb)
 {
     extern __shared__ int32_t stree[];
-    const int n = g.nl_size;
-    int32_t *tree = kShared ? stree : fb.nltree;
-    if (kShared) {
-        for (int i = threadIdx.x; i < 2 * n; i += blockDim.x) stree[i] = -1;
-        block_sync();
-    }
-    const uint32_t lo = blockIdx.x * chunk, hi = min(ntri, lo + chunk);
-    for (uint32_t p = lo + threadIdx.x; p < hi; p += blockDim.x) {
-        const int32_t v = (int32_t)(tri_base + (order ? __ldg(order + p) : p));
-        const uint32_t yr = __ldg(fb.rows + tri_base + p);
-        nltree_update(tree, n, (int)(yr & 0xffffu), (int)(yr >> 16), v, kShared);
-    }
-    if (kShared) {
-        block_sync();
-        for (int i = threadIdx.x; i < 2 * n; i += blockDim.x) {
-            const int32_t v = stree[i];
-            if (v >= 0 && *(volatile int32_t *)&fb.nltree[i] < v) atomicMax(&fb.nltree[i], v);
-        }
-    }
+    const uint32_t lo = blockIdx.x * kNewlineChunk + pdl_begin(), hi = min(ntri, lo + kNewlineChunk);
+    newline_block<kShared>(stree, g.nl_size, lo, hi, order, fb.rows + tri_base, tri_base, fb.nltree);
 }
 
 cudaError_t launch_newline(uint32_t ntri, const uint32_t *order, uint32_t tri_base, const FrameGeom &g,
                            const FrameBuffers &fb, cudaStream_t s)
 {
     if (ntri == 0 || !g.image) return cudaSuccess;
-    const uint32_t chunk = 8192;
-    const uint32_t blocks = (ntri + chunk - 1) / chunk;
-    const size_t smem = 2 * (size_t)g.nl_size * sizeof(int32_t);
-    if (smem <= 128 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(newline_kernel<true>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
+    const uint32_t blocks = (ntri + kNewlineChunk - 1) / kNewlineChunk;
+    const size_t smem = newline_tree_bytes(g.nl_size);
+    if (smem <= kNewlineSharedBytes) {
+        cudaError_t e = cudaFuncSetAttribute(newline_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)kNewlineSharedBytes);
         if (e != cudaSuccess) return e;
-        newline_kernel<true><<<blocks, 1024, smem, s>>>(ntri, order, tri_base, chunk, g, fb);
-    } else {
-        newline_kernel<false><<<blocks, 1024, 0, s>>>(ntri, order, tri_base, chunk, g, fb);
+        return launch_pdl(newline_kernel<true>, dim3(blocks), dim3(1024), smem, s, ntri, order, tri_base, g, fb);
     }
-    return cudaGetLastError();
+    return launch_pdl(newline_kernel<false>, dim3(blocks), dim3(1024), 0, s, ntri, order, tri_base, g, fb);
 }
 
 // The resets of a frame (device error word, fragment counter, newline tree: frame) and of
@@ -248,7 +221,7 @@ __global__ void __launch_bounds__(256)
 frame_reset_kernel(FrameBuffers fb, BinBuffers bb, uint32_t nl_nodes, uint32_t ntiles, int frame, int draw,
                    int tiles_current)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x + pdl_begin();
     if (frame && i < nl_nodes) fb.nltree[i] = -1;
     if (draw && i < ntiles) bb.tile_count[i] = bb.tile_cursor[i] = 0u;
     if (tiles_current && i < ntiles) fb.tile_gen[i] = fb.gen;
@@ -265,9 +238,8 @@ cudaError_t launch_frame_reset(const FrameBuffers &fb, const BinBuffers &bb, uin
                                bool frame, bool draw, bool tiles_current, cudaStream_t s)
 {
     const uint32_t n = max(frame ? nl_nodes : 1u, (draw || tiles_current) ? ntiles : 1u);
-    frame_reset_kernel<<<(n + 255) / 256, 256, 0, s>>>(fb, bb, nl_nodes, ntiles, frame ? 1 : 0, draw ? 1 : 0,
-                                                       tiles_current ? 1 : 0);
-    return cudaGetLastError();
+    return launch_pdl(frame_reset_kernel, dim3((n + 255) / 256), dim3(256), 0, s, fb, bb, nl_nodes, ntiles,
+                      frame ? 1 : 0, draw ? 1 : 0, tiles_current ? 1 : 0);
 }
 
 // Keys the samples can write set to the empty key (all bytes 0xff) in a run of tile rows of
@@ -314,8 +286,7 @@ cudaError_t launch_vertex_transform(const MeshDev &mesh, const Mat4 &M, float4 *
 {
     if (mesh.nvert == 0) return cudaSuccess;
     const uint32_t quads = (mesh.nvert + 3) / 4;
-    vertex_transform_kernel<<<(quads + 255) / 256, 256, 0, s>>>(mesh, M, tv);
-    return cudaGetLastError();
+    return launch_pdl(vertex_transform_kernel, dim3((quads + 255) / 256), dim3(256), 0, s, mesh, M, tv);
 }
 
 // A mesh's arrays from interleaved positions and packed colours: each element once, so bound
@@ -374,14 +345,10 @@ cudaError_t launch_setup(const MeshDev &mesh, const float4 *tv, const Mat4 &M, u
     const size_t smem = setup_smem_bytes(tpb, g.direct_max > 0);   // prepare_setup_kernels: above 48 KB
     const dim3 grid(blocks), block(setup_block_threads(tpb));
     const bool chunks = tpb > kSetupChunk;
-    if (g.direct_max > 0) {
-        if (chunks) setup_kernel<true, true><<<grid, block, smem, s>>>(mesh, tv, M, tri_base, g, fb, bb, tpb);
-        else setup_kernel<true, false><<<grid, block, smem, s>>>(mesh, tv, M, tri_base, g, fb, bb, tpb);
-    } else {
-        if (chunks) setup_kernel<false, true><<<grid, block, smem, s>>>(mesh, tv, M, tri_base, g, fb, bb, tpb);
-        else setup_kernel<false, false><<<grid, block, smem, s>>>(mesh, tv, M, tri_base, g, fb, bb, tpb);
-    }
-    return cudaGetLastError();
+    void (*kernel)(MeshDev, const float4 *, Mat4, uint32_t, FrameGeom, FrameBuffers, BinBuffers, int) =
+        g.direct_max > 0 ? (chunks ? setup_kernel<true, true> : setup_kernel<true, false>)
+                         : (chunks ? setup_kernel<false, true> : setup_kernel<false, false>);
+    return launch_pdl(kernel, grid, block, smem, s, mesh, tv, M, tri_base, g, fb, bb, tpb);
 }
 
 }  // namespace sloth

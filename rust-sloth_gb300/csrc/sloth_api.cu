@@ -3,8 +3,8 @@
 // Host-side restatement of the reference's per-frame driver around the hot path:
 // Context::blank/update/clear (src/context.rs:22-45, 93-141), draw_mesh
 // (src/rasterizer.rs:39-46) and the buffer reads that Context::flush prints.  All device
-// memory is owned here; all work is ordered on the context's stream (two kernels of a
-// draw run on helper streams forked from it and joined back).  There is no CPU fallback:
+// memory is owned here; all work is ordered on the context's stream (a large draw's newline
+// fold runs on a helper stream forked from it and joined back).  There is no CPU fallback:
 // if CUDA or the kernels are unavailable every call fails with SLOTH_ERR_CUDA.
 //
 // Host float math below must be compiled with -ffp-contract=off (see build.py).
@@ -76,25 +76,17 @@ struct sloth_ctx {
     size_t fill_cap = 0;
     float4 *tv = nullptr;
     size_t tv_cap = 0;
-    uint32_t *h_total = nullptr;   // pinned
-    cudaEvent_t total_ev = nullptr;   // h_total has arrived
-    uint32_t *d_max = nullptr;     // largest entry total of any draw (the scan's atomicMax)
-    uint32_t *h_max = nullptr;     // pinned copy of d_max
-    cudaEvent_t max_ev = nullptr;  // h_max has arrived
-    bool max_pending = false;      // a copy of d_max is on its way
+    uint32_t *h_total = nullptr;   // pinned: the first draw's entries
+    cudaStream_t nl_stream = nullptr;   // a large draw's newline fold, beside its other kernels
+    cudaEvent_t setup_ev = nullptr, nl_ev = nullptr;
+    bool nl_pending = false;            // such a fold not yet joined into the ctx stream
+    uint32_t *h_outgrew = nullptr; // pinned: the entries of a draw that outgrew the buffer (the raster)
     unsigned long long *h_frags = nullptr;   // pinned
     uint32_t *h_error = nullptr;   // pinned copy of fb.error
     uint32_t *h_stage = nullptr;   // pinned: a small frame's buffers on their way to the caller
     uint32_t tri_base = 0;
     bool dirty = true;
     bool reset_pending = false;    // a clear's resets, folded into the next launch that needs them
-    cudaStream_t side = nullptr;   // the entry-count copy, off the draw's stream
-    cudaEvent_t scan_ev = nullptr;
-    cudaStream_t nl_stream = nullptr;   // the newline fold, beside the binning kernels
-    cudaStream_t aux = nullptr;         // the large-triangle fill, beside the small one
-    cudaEvent_t fill_ev = nullptr, aux_ev = nullptr;
-    cudaEvent_t setup_ev = nullptr, nl_ev = nullptr;
-    bool nl_pending = false;            // a newline fold not yet joined into the ctx stream
 
     // instrumentation and options
     int depth_cull = 1;
@@ -181,19 +173,16 @@ static cudaError_t timed(sloth_ctx *ctx, const char *name, F &&launch, cudaStrea
     return e;
 }
 
-// Waits for the context's helper streams (newline fold, entry-count copy) before device
-// memory they may read is released.
-static void quiesce_helpers(sloth_ctx *ctx)
+// Waits for a newline fold on its own stream before device memory it reads is released.
+static void quiesce_newline(sloth_ctx *ctx)
 {
-    if (ctx->nl_stream) cudaStreamSynchronize(ctx->nl_stream);
-    if (ctx->aux) cudaStreamSynchronize(ctx->aux);
-    if (ctx->side) cudaStreamSynchronize(ctx->side);
+    if (ctx->nl_pending) cudaStreamSynchronize(ctx->nl_stream);
     ctx->nl_pending = false;
 }
 
 static void free_frame(sloth_ctx *ctx)
 {
-    quiesce_helpers(ctx);
+    quiesce_newline(ctx);
     dfree(ctx->fb.keys);
     dfree(ctx->fb.tile_gen);
     dfree(ctx->fb.nltree);
@@ -259,7 +248,7 @@ static sloth_status ensure_records(sloth_ctx *ctx, size_t need)
         CU(ctx, cudaMemcpyAsync(n, ctx->fb.records, (size_t)ctx->tri_base * sizeof(TriRecord),
                                 cudaMemcpyDeviceToDevice, ctx->stream));
     CU(ctx, cudaStreamSynchronize(ctx->stream));
-    quiesce_helpers(ctx);
+    quiesce_newline(ctx);
     dfree(ctx->fb.records);
     dfree(ctx->fb.rows);
     ctx->fb.records = n;
@@ -275,7 +264,7 @@ static sloth_status ensure_scratch(sloth_ctx *ctx, T **p, size_t *cap, size_t ne
     size_t c = *cap ? *cap : 1024;
     while (c < need) c *= 2;
     CU(ctx, cudaStreamSynchronize(ctx->stream));
-    quiesce_helpers(ctx);
+    quiesce_newline(ctx);
     dfree(*p);
     CU(ctx, dalloc(p, c));
     *cap = c;
@@ -329,6 +318,24 @@ static sloth_status join_newline(sloth_ctx *ctx)
     if (!ctx->nl_pending) return SLOTH_OK;
     CU(ctx, cudaStreamWaitEvent(ctx->stream, ctx->nl_ev, 0));
     ctx->nl_pending = false;
+    return SLOTH_OK;
+}
+
+// The newline fold of a draw's triangles on its own stream, after everything queued so far.
+static sloth_status fork_newline(sloth_ctx *ctx, const MeshDev &md)
+{
+    if (!ctx->nl_stream) {
+        CU(ctx, cudaStreamCreateWithFlags(&ctx->nl_stream, cudaStreamNonBlocking));
+        CU(ctx, cudaEventCreateWithFlags(&ctx->setup_ev, cudaEventDisableTiming));
+        CU(ctx, cudaEventCreateWithFlags(&ctx->nl_ev, cudaEventDisableTiming));
+    }
+    CU(ctx, cudaEventRecord(ctx->setup_ev, ctx->stream));
+    CU(ctx, cudaStreamWaitEvent(ctx->nl_stream, ctx->setup_ev, 0));
+    CU(ctx, timed(ctx, "newline", [&] {
+           return launch_newline(md.ntri, md.order, ctx->tri_base, ctx->g, ctx->fb, ctx->nl_stream);
+       }, ctx->nl_stream));
+    CU(ctx, cudaEventRecord(ctx->nl_ev, ctx->nl_stream));
+    ctx->nl_pending = true;
     return SLOTH_OK;
 }
 
@@ -473,47 +480,24 @@ sloth_status sloth_ctx_create(sloth_ctx **out, int device, void *stream)
         ctx->own_stream = true;
     }
     if (cudaMallocHost(&ctx->h_total, sizeof(uint32_t)) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->total_ev, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->scan_ev, cudaEventDisableTiming) != cudaSuccess ||
         prepare_setup_kernels() != cudaSuccess ||
-        cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&ctx->nl_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->fill_ev, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->aux_ev, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->setup_ev, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->nl_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaMallocHost(&ctx->h_frags, sizeof(unsigned long long)) != cudaSuccess ||
         cudaMallocHost(&ctx->h_error, sizeof(uint32_t)) != cudaSuccess ||
         cudaMalloc(&ctx->fb.error, sizeof(uint32_t)) != cudaSuccess ||
         cudaMemset(ctx->fb.error, 0, sizeof(uint32_t)) != cudaSuccess ||
-        cudaMallocHost(&ctx->h_max, sizeof(uint32_t)) != cudaSuccess ||
-        cudaMalloc(&ctx->d_max, sizeof(uint32_t)) != cudaSuccess ||
-        cudaMemset(ctx->d_max, 0, sizeof(uint32_t)) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->max_ev, cudaEventDisableTiming) != cudaSuccess) {
+        cudaMallocHost(&ctx->h_outgrew, sizeof(uint32_t)) != cudaSuccess) {
         if (ctx->h_total) cudaFreeHost(ctx->h_total);
-        if (ctx->total_ev) cudaEventDestroy(ctx->total_ev);
-        if (ctx->scan_ev) cudaEventDestroy(ctx->scan_ev);
-        if (ctx->side) cudaStreamDestroy(ctx->side);
-        if (ctx->nl_stream) cudaStreamDestroy(ctx->nl_stream);
-        if (ctx->aux) cudaStreamDestroy(ctx->aux);
-        if (ctx->setup_ev) cudaEventDestroy(ctx->setup_ev);
-        if (ctx->nl_ev) cudaEventDestroy(ctx->nl_ev);
-        if (ctx->fill_ev) cudaEventDestroy(ctx->fill_ev);
-        if (ctx->aux_ev) cudaEventDestroy(ctx->aux_ev);
         if (ctx->h_frags) cudaFreeHost(ctx->h_frags);
         if (ctx->h_error) cudaFreeHost(ctx->h_error);
         if (ctx->fb.error) cudaFree(ctx->fb.error);
-        if (ctx->h_max) cudaFreeHost(ctx->h_max);
-        if (ctx->d_max) cudaFree(ctx->d_max);
-        if (ctx->max_ev) cudaEventDestroy(ctx->max_ev);
+        if (ctx->h_outgrew) cudaFreeHost(ctx->h_outgrew);
         if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
         delete ctx;
         return SLOTH_ERR_OUT_OF_MEMORY;
     }
     *ctx->h_error = 0;
-    *ctx->h_max = 0;
-    ctx->bb.max_total = ctx->d_max;
+    *ctx->h_outgrew = 0;
+    ctx->bb.outgrew = ctx->h_outgrew;
     *out = ctx;
     return SLOTH_OK;
 }
@@ -523,7 +507,7 @@ void sloth_ctx_destroy(sloth_ctx *ctx)
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
-    quiesce_helpers(ctx);
+    quiesce_newline(ctx);
     // batches lose their device memory and meshes their context; destroying either
     // afterwards only frees what is left
     for (sloth_batch *b : ctx->batches) sloth_batch_detach(b);
@@ -544,22 +528,14 @@ void sloth_ctx_destroy(sloth_ctx *ctx)
     dfree(ctx->bb.items);
     dfree(ctx->tv);
     if (ctx->h_total) cudaFreeHost(ctx->h_total);
-    if (ctx->total_ev) cudaEventDestroy(ctx->total_ev);
-    if (ctx->scan_ev) cudaEventDestroy(ctx->scan_ev);
-    if (ctx->side) cudaStreamDestroy(ctx->side);
     if (ctx->nl_stream) cudaStreamDestroy(ctx->nl_stream);
-    if (ctx->aux) cudaStreamDestroy(ctx->aux);
     if (ctx->setup_ev) cudaEventDestroy(ctx->setup_ev);
     if (ctx->nl_ev) cudaEventDestroy(ctx->nl_ev);
-    if (ctx->fill_ev) cudaEventDestroy(ctx->fill_ev);
-    if (ctx->aux_ev) cudaEventDestroy(ctx->aux_ev);
     if (ctx->h_frags) cudaFreeHost(ctx->h_frags);
     if (ctx->h_error) cudaFreeHost(ctx->h_error);
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     dfree(ctx->fb.error);
-    if (ctx->h_max) cudaFreeHost(ctx->h_max);
-    dfree(ctx->d_max);
-    if (ctx->max_ev) cudaEventDestroy(ctx->max_ev);
+    if (ctx->h_outgrew) cudaFreeHost(ctx->h_outgrew);
     flush_release(ctx->flush);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -1037,17 +1013,12 @@ sloth_status sloth_mesh_info(const sloth_mesh *m, uint32_t *ntri, float bbox_max
 // context's stream (it frees the old buffer); it happens rarely, as the buffer doubles.
 static sloth_status poll_entry_max(sloth_ctx *ctx)
 {
-    if (!ctx->max_pending) return SLOTH_OK;
-    const cudaError_t q = cudaEventQuery(ctx->max_ev);
-    if (q == cudaErrorNotReady) return SLOTH_OK;
-    ctx->max_pending = false;
-    CU(ctx, q);
-    if (ctx->bb.entries && *ctx->h_max > ctx->bb.capacity) {
-        size_t ecap = ctx->bb.capacity;
-        sloth_status st = ensure_scratch(ctx, &ctx->bb.entries, &ecap, *ctx->h_max);
-        if (st != SLOTH_OK) return st;
-        ctx->bb.capacity = (uint32_t)(ecap > 0xffffffffu ? 0xffffffffu : ecap);
-    }
+    const uint32_t most = *(volatile uint32_t *)ctx->h_outgrew;
+    if (!ctx->bb.entries || most <= ctx->bb.capacity) return SLOTH_OK;
+    size_t ecap = ctx->bb.capacity;
+    sloth_status st = ensure_scratch(ctx, &ctx->bb.entries, &ecap, most);
+    if (st != SLOTH_OK) return st;
+    ctx->bb.capacity = (uint32_t)(ecap > 0xffffffffu ? 0xffffffffu : ecap);
     return SLOTH_OK;
 }
 
@@ -1137,68 +1108,34 @@ sloth_status sloth_draw_mesh(sloth_ctx *ctx, const sloth_mesh *mesh, const float
     const float4 *tv = mesh->idx ? ctx->tv : nullptr;
     if (tv) CU(ctx, timed(ctx, "vertex", [&] { return launch_vertex_transform(md, M, ctx->tv, s); }));
     CU(ctx, timed(ctx, "setup", [&] { return launch_setup(md, tv, M, ctx->tri_base, g, ctx->fb, ctx->bb, s, ctx->tpb); }));
-    // the newline fold reads the records and feeds only the resolve: on its own stream,
-    // beside the binning kernels
-    CU(ctx, cudaEventRecord(ctx->setup_ev, s));
-    CU(ctx, cudaStreamWaitEvent(ctx->nl_stream, ctx->setup_ev, 0));
-    CU(ctx, timed(ctx, "newline", [&] { return launch_newline(mesh->ntri, mesh->order, ctx->tri_base, g, ctx->fb, ctx->nl_stream); },
-                  ctx->nl_stream));
-    CU(ctx, cudaEventRecord(ctx->nl_ev, ctx->nl_stream));
-    ctx->nl_pending = true;
+    if (g.image && !newline_in_fill(mesh->ntri, g) && (st = fork_newline(ctx, md)) != SLOTH_OK) return st;
     CU(ctx, timed(ctx, "bin_count_large",[&] { return launch_bin_count_large(ctx->tri_base, g, ctx->fb, ctx->bb, s); }));
     CU(ctx, timed(ctx, "bin_scan", [&] { return launch_bin_scan(ntiles, ctx->bb, s); }));
     // The entry count is known only on the device.  With an entry buffer from earlier draws
-    // the rest of the draw goes ahead with it and the host does not wait: the fill kernels
-    // write no slot past the capacity, and when the count is above it the raster launch
+    // the rest of the draw goes ahead with it and the host does not wait: the fill
+    // writes no slot past the capacity, and when the count is above it the raster launch
     // folds the draw's binned triangles straight into the keys instead of rasterizing tiles
-    // (the same keys).  The device's running maximum of the counts comes back on
-    // a side stream, and a later draw grows the buffer from it (poll_entry_max).  The first
-    // draw on a context, with no buffer yet, waits for its count and sizes the buffer.
-    auto rest = [&](size_t entries_bound) -> sloth_status {
-        // the small and the large fill take slots from the same cursors (atomics): they
-        // run side by side, the large one on the aux stream
-        CU(ctx, cudaEventRecord(ctx->fill_ev, s));
-        CU(ctx, cudaStreamWaitEvent(ctx->aux, ctx->fill_ev, 0));
-        CU(ctx, timed(ctx, "bin_fill_large", [&] { return launch_bin_fill_large(ctx->tri_base, g, ctx->fb, ctx->bb, ctx->aux); },
-                      ctx->aux));
-        CU(ctx, cudaEventRecord(ctx->aux_ev, ctx->aux));
-        CU(ctx, timed(ctx, "bin_fill", [&] {
-               return launch_bin_fill(g, ctx->fb, ctx->bb, s);
-           }));
-        CU(ctx, cudaStreamWaitEvent(s, ctx->aux_ev, 0));
-        size_t icap = ctx->bb.item_capacity;
-        sloth_status st2;
-        if ((st2 = ensure_scratch(ctx, &ctx->bb.items, &icap, raster_item_bound(ntiles, entries_bound))) != SLOTH_OK)
-            return st2;
-        ctx->bb.item_capacity = (uint32_t)icap;
-        CU(ctx, timed(ctx, "bin_items", [&] { return launch_bin_items(ntiles, g, ctx->fb, ctx->bb, s); }));
-        CU(ctx, timed(ctx, "raster", [&] {
-               return launch_raster(g, ctx->fb, ctx->bb, ctx->depth_cull, mesh->ntri, ctx->tri_base, s);
-           }));
-        return SLOTH_OK;
-    };
-    if (ctx->bb.entries && ctx->bb.capacity > 0) {
-        if ((st = rest(ctx->bb.capacity)) != SLOTH_OK) return st;
-        if (!ctx->max_pending) {
-            CU(ctx, cudaEventRecord(ctx->scan_ev, s));
-            CU(ctx, cudaStreamWaitEvent(ctx->side, ctx->scan_ev, 0));
-            CU(ctx, cudaMemcpyAsync(ctx->h_max, ctx->d_max, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->side));
-            CU(ctx, cudaEventRecord(ctx->max_ev, ctx->side));
-            ctx->max_pending = true;
-        }
-    } else {
-        CU(ctx, cudaEventRecord(ctx->scan_ev, s));
-        CU(ctx, cudaStreamWaitEvent(ctx->side, ctx->scan_ev, 0));
-        CU(ctx, cudaMemcpyAsync(ctx->h_total, ctx->bb.tile_offset + ntiles, sizeof(uint32_t),
-                                cudaMemcpyDeviceToHost, ctx->side));
-        CU(ctx, cudaEventRecord(ctx->total_ev, ctx->side));
-        CU(ctx, cudaEventSynchronize(ctx->total_ev));
-        const uint32_t total = *ctx->h_total;
+    // (the same keys) and reports the count in a pinned word, from which a later draw grows
+    // the buffer (poll_entry_max).  The first draw on a context, with no buffer yet, waits
+    // for its count and sizes the buffer.
+    size_t bound = ctx->bb.capacity;
+    if (!ctx->bb.entries || ctx->bb.capacity == 0) {
+        CU(ctx, cudaMemcpyAsync(ctx->h_total, ctx->bb.tile_offset + ntiles, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        CU(ctx, cudaStreamSynchronize(s));
+        bound = *ctx->h_total;
         size_t ecap = ctx->bb.capacity;
-        if ((st = ensure_scratch(ctx, &ctx->bb.entries, &ecap, total)) != SLOTH_OK) return st;
+        if ((st = ensure_scratch(ctx, &ctx->bb.entries, &ecap, bound)) != SLOTH_OK) return st;
         ctx->bb.capacity = (uint32_t)(ecap > 0xffffffffu ? 0xffffffffu : ecap);
-        if ((st = rest(total)) != SLOTH_OK) return st;
     }
+    size_t icap = ctx->bb.item_capacity;
+    if ((st = ensure_scratch(ctx, &ctx->bb.items, &icap, raster_item_bound(ntiles, bound))) != SLOTH_OK) return st;
+    ctx->bb.item_capacity = (uint32_t)icap;
+    CU(ctx, timed(ctx, "bin_fill", [&] {
+           return launch_bin_fill(mesh->ntri, mesh->order, ctx->tri_base, ntiles, g, ctx->fb, ctx->bb, s);
+       }));
+    CU(ctx, timed(ctx, "raster", [&] {
+           return launch_raster(g, ctx->fb, ctx->bb, ctx->depth_cull, ctx->tri_base, s);
+       }));
     ctx->tri_base += mesh->ntri;
     ctx->dirty = true;
     return SLOTH_OK;

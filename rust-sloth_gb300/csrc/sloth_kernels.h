@@ -65,7 +65,8 @@ struct BinBuffers {
                              // light threshold (entries)
     uint2 *items;            // item_capacity: (tile, slice) of each raster CTA
     uint32_t item_capacity;
-    uint32_t *max_total;     // optional: the scan folds each draw's entry total in (atomicMax)
+    volatile uint32_t *outgrew;   // contexts: a pinned host word, the entries of a draw that
+                             // outgrew the buffer
 };
 
 // 16-byte words of a fill list of n entries and their metas behind it.
@@ -183,19 +184,19 @@ cudaError_t launch_vertex_transform(const MeshDev &mesh, const Mat4 &M, float4 *
 cudaError_t launch_setup(const MeshDev &mesh, const float4 *tv, const Mat4 &M, uint32_t tri_base,
                          const FrameGeom &g, const FrameBuffers &fb, const BinBuffers &bb,
                          cudaStream_t s, int tpb = kDefaultTrianglesPerBlock);
-// newline sentinels (image mode): fold each triangle's row range into the segment tree.
-// The packed rows are in setup's order of the mesh: order is the mesh's MeshDev::order.
+// newline sentinels (image mode) of a draw whose fill does not take them (newline_in_fill):
+// each triangle's row range into the segment tree.  The packed rows are in setup's order of
+// the mesh: order is the mesh's MeshDev::order.
+bool newline_in_fill(uint32_t ntri, const FrameGeom &g);
 cudaError_t launch_newline(uint32_t ntri, const uint32_t *order, uint32_t tri_base, const FrameGeom &g,
                            const FrameBuffers &fb, cudaStream_t s);
 cudaError_t launch_bin_count_large(uint32_t tri_base, const FrameGeom &g, const FrameBuffers &fb,
                                    const BinBuffers &bb, cudaStream_t s);
 cudaError_t launch_bin_scan(uint32_t ntiles, const BinBuffers &bb, cudaStream_t s);
-cudaError_t launch_bin_items(uint32_t ntiles, const FrameGeom &g, const FrameBuffers &fb, const BinBuffers &bb,
-                             cudaStream_t s);
-// small binned triangles' tile entries: the ones setup listed in bb.fill_list
-cudaError_t launch_bin_fill(const FrameGeom &g, const FrameBuffers &fb, const BinBuffers &bb, cudaStream_t s);
-cudaError_t launch_bin_fill_large(uint32_t tri_base, const FrameGeom &g, const FrameBuffers &fb,
-                                  const BinBuffers &bb, cudaStream_t s);
+// the tile entries (small triangles from the fill list, large ones from their queue), the
+// raster items and, when newline_in_fill, the newline rows of the draw's ntri triangles
+cudaError_t launch_bin_fill(uint32_t ntri, const uint32_t *order, uint32_t tri_base, uint32_t ntiles,
+                            const FrameGeom &g, const FrameBuffers &fb, const BinBuffers &bb, cudaStream_t s);
 
 // Estimated samples of a draw: the sum of its triangles' longest edges squared (span2) times
 // the scale of the matrix's x and y rows, at most every cell for every triangle.  Where the
@@ -227,11 +228,11 @@ cudaError_t launch_fold_large(const FrameGeom &g, const FrameBuffers &fb, uint32
 
 // per-tile raster: 64-bit atomicMin of depth keys in shared memory, merged into keys.  A
 // draw whose tile entries outgrew the entry buffer (the scan total is above the capacity;
-// its fill wrote what fitted) is rasterized by the same launch without tiles: the item
-// kernel has made every tile's keys current, and one warp per binned triangle of the draw
-// (ntri triangles from tri_base) folds its covered samples straight into the global keys.
+// its fill wrote what fitted) is rasterized by the same launch without tiles: the fill has
+// made every tile's keys current, and the warps fold the covered samples of the listed and
+// queued triangles straight into the global keys.
 cudaError_t launch_raster(const FrameGeom &g, const FrameBuffers &fb, const BinBuffers &bb, int depth_cull,
-                          uint32_t ntri, uint32_t tri_base, cudaStream_t s);
+                          uint32_t tri_base, cudaStream_t s);
 
 // resolve: keys -> z, frame cells, winners.
 cudaError_t launch_resolve(const FrameGeom &g, const FrameBuffers &fb, cudaStream_t s);
