@@ -234,21 +234,10 @@ __global__ void __launch_bounds__(256) batch_fold_large_kernel(BatchDev b, const
     }
     blk -= nnl;
     const uint32_t first = (blk * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t large = b.bb.large_count[0], mid = b.bb.large_count[1],
-                   nwarps = ((gridDim.x - nnl) * blockDim.x) >> 5;
-    const uint32_t parts = fold_parts(large), cut = large * parts, items = cut + mid;
-    const bool filter = large + mid > kFoldFilterMin;
-    unsigned long long *counter = b.frames[0].fb.fragments;   // the batch's one counter
-    uint32_t frags = 0;
-    for (uint32_t it = first; it < items; it += nwarps) {
-        const uint32_t q = it < cut ? it / parts : b.bb.large_cap - 1u - (it - cut);
-        const BatchFrame &f = b.frames[b.large_frame[q]];
-        const FrameGeom g = f.g;
-        const FrameBuffers fb = f.fb;
-        frags += it < cut ? fold_queued<kFoldRows>(b.bb.large_queue[q], it % parts, parts, filter, g, fb)
-                          : fold_queued<32>(b.bb.large_queue[q], 0u, 1u, filter, g, fb);
-    }
-    add_frags_warp(frags, counter);
+    const FoldQueue queue{b.bb.large_queue, b.large_frame, b.bb.large_count, b.bb.large_cap};
+    const uint32_t frags = fold_queue_walk(queue, first, ((gridDim.x - nnl) * blockDim.x) >> 5,
+                                           [&](uint32_t q) -> const BatchFrame & { return b.frames[b.large_frame[q]]; });
+    add_frags_warp(frags, b.frames[0].fb.fragments);   // the batch's one counter
 }
 
 // Everything a render starts from: counters, tile counts and generations, the newline
@@ -534,11 +523,12 @@ cudaError_t launch_batch_setup(const BatchDev &b, const int2 *blocks, uint32_t n
                       dim3(nblocks), dim3(setup_block_threads(b.tpb)), smem, s, b, blocks);
 }
 
-cudaError_t launch_batch_fold_setup(const BatchDev &b, const int2 *blocks, uint32_t nblocks, bool small,
+cudaError_t launch_batch_fold_setup(const BatchDev &b, const int2 *blocks, uint32_t nblocks, int warps,
                                     cudaStream_t s)
 {
     if (!nblocks) return cudaSuccess;
-    if (small) return launch_pdl(batch_fold_setup_kernel<4>, dim3(nblocks), dim3(128), kFoldSmemBytes, s, b, blocks);
+    if (warps == 4) return launch_pdl(batch_fold_setup_kernel<4>, dim3(nblocks), dim3(128), kFoldSmemBytes, s, b, blocks);
+    if (warps == 1) return launch_pdl(batch_fold_setup_kernel<1>, dim3(nblocks), dim3(32), kFoldSmemBytes, s, b, blocks);
     if (!valid_triangles_per_block(b.tpb)) return cudaErrorInvalidValue;
     const size_t smem = setup_smem_bytes(b.tpb, true);
     return launch(b.tpb > kSetupChunk ? batch_setup_kernel<true, true, true> : batch_setup_kernel<true, false, true>,

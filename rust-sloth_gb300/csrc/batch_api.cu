@@ -29,6 +29,10 @@ constexpr uint32_t kBatchGen = 0x01010101u;
 // Block tables: setup, newline, resolve, small fold.
 enum { kTabSetup, kTabNewline, kTabResolve, kTabFold, kTables };
 
+// How a render draws without tiles: not at all, or with the setup of 32 triangles to a block
+// of four warps or of one, or with the batch's own setup kernel (b.tpb a block).
+enum class FoldForm { none, warps4, warps1, setup };
+
 struct sloth_batch {
     sloth_ctx *ctx = nullptr;
     int device = 0;
@@ -42,9 +46,8 @@ struct sloth_batch {
     int direct_max = 0;                       // FrameGeom::direct_max of every frame
     bool persistent = true;                   // raster over the device queue (else one CTA per item)
     int tpb = kDefaultTrianglesPerBlock;      // triangles per setup block
-    bool small_fold = false;                  // few enough triangles for 32 a block
-    bool fold_ok = false;                     // the draws' estimates allow frames without tiles
-    bool folded = false;                      // the graph, and the last render, draw without tiles
+    FoldForm fold = FoldForm::none;           // what the draws' estimates allow
+    FoldForm folded = FoldForm::none;         // how the graph, and the last render, draw
 
     // layout (per shape)
     std::vector<BatchFrame> hframes;
@@ -186,25 +189,37 @@ void free_layout(sloth_batch *b)
     b->rendered = false;
 }
 
-// Whether a batch's frames can be drawn without tiles (fold.cuh): every draw within the
-// limits of a context's draw (draws_without_tiles) and every frame's estimate too.  Measured
+// Whether and how a batch's frames can be drawn without tiles (fold.cuh): every draw within
+// the limits of a context's draw (draws_without_tiles) and every frame's estimate too.  Measured
 // with the GPU full (us a render, tiles / tiles with direct folds of 64 / fold): 64 frames of
 // 160x48 with 5k triangles 87 / 50 / 43; 64 of 640x360 with 5k 314 / 341 / 251, with 82k
 // 770 / 514 / 487, with an 8k soup of 1.2e7 samples a frame 486 / 526 / 470, of 4.1e7
 // 498 / 531 / 990.
-bool batch_folds(const sloth_batch *b)
+// The form: few triangles are spread over four warps for each 32.  From kFoldMany on the
+// GPU is full, and one warp walks what little 32 triangles of a few samples have (us, four
+// warps / one / setup kernel: 123k triangles of 3 samples in 24 frames 31 / 25 / 28, of 120
+// 82 / 107 / 107).  Above kFoldMany4, where four warps would only queue, triangles
+// with hardly a sample each (mostly back faces and misses) go to the setup kernel, which
+// closes up the lanes left (491k of 0.2: 82 / 58 / 41; of 30: 108 / 99 / 114).
+FoldForm batch_folds(const sloth_batch *b)
 {
+    double est = 0.0, tri = 0.0;
     for (const sloth_frame_desc &fd : b->frames) {
         float frame = 0.0f;
         for (uint32_t k = 0; k < fd.ndraws; ++k) {
             const uint32_t d = fd.first_draw + k, n = b->draw_ntri[d];
             if (n == 0) continue;
-            if (n > kFoldMaxTriangles || !(b->draw_span2[d] > 0.0f)) return false;
+            if (n > kFoldMaxTriangles || !(b->draw_span2[d] > 0.0f)) return FoldForm::none;
+            tri += n;
             frame += fold_estimate(b->draw_span2[d], n, b->h_mats[d], (int)fd.width, (int)fd.height);
         }
-        if (!(frame <= kFoldMaxSamples)) return false;
+        if (!(frame <= kFoldMaxSamples)) return FoldForm::none;
+        est += frame;
     }
-    return true;
+    const double each = tri > 0.0 ? est / tri : 0.0;
+    if (tri > kFoldTableTriangles) return FoldForm::setup;
+    if (tri > kFoldMany4) return each < 4.0 ? FoldForm::setup : FoldForm::warps1;
+    return tri >= kFoldMany && each <= 20.0 ? FoldForm::warps1 : FoldForm::warps4;
 }
 
 void set_mats(sloth_batch *b)
@@ -216,7 +231,7 @@ void set_mats(sloth_batch *b)
             sloth_mat4_mul(fd.utransform, &b->transforms[16 * (size_t)d], b->h_mats[d].m);
         }
     }
-    b->fold_ok = batch_folds(b);
+    b->fold = batch_folds(b);
 }
 
 // Lay out every frame for tile shape `shape` and allocate the batch's buffers.
@@ -247,7 +262,6 @@ sloth_status build(sloth_batch *b, int shape)
     for (const sloth_mesh *m : b->meshes) all_tri += sloth_mesh_view(m).ntri;
     b->resolve_chunk = all_cells / kBatchResolveChunk < 8ull * (uint64_t)device_sm_count() ? kBatchResolveSmall
                                                                                            : kBatchResolveChunk;
-    b->small_fold = all_tri <= kBatchSmallFold;
     b->max_nl = 1;
     std::vector<int2> bt, bn, br, bs;
     for (uint32_t f = 0; f < nf; ++f) {
@@ -300,7 +314,7 @@ sloth_status build(sloth_batch *b, int shape)
             bd.rec_off = (uint32_t)(rec + local);
             bd.local_base = local;
             for (uint32_t t = 0; t < mv.ntri; t += (uint32_t)b->tpb) bt.push_back(make_int2((int)d, (int)t));
-            if (b->small_fold)
+            if (all_tri <= kFoldTableTriangles)
                 for (uint32_t t = 0; t < mv.ntri; t += kFoldBlockTris) bs.push_back(make_int2((int)d, (int)t));
             if (g.image)
                 for (uint32_t t = 0; t < mv.ntri; t += kBatchNewlineChunk) bn.push_back(make_int2((int)d, (int)t));
@@ -395,7 +409,6 @@ BatchDev dev_view(sloth_batch *b)
     d.depth_cull = sloth_ctx_depth_cull(b->ctx);
     d.tpb = b->tpb;
     d.direct_max = b->direct_max;
-    d.fold = b->folded ? 1 : 0;
     d.resolve_chunk = b->resolve_chunk;
     return d;
 }
@@ -406,7 +419,7 @@ cudaError_t enqueue_reset(sloth_batch *b, cudaStream_t s)
     cudaError_t e;
     // small triangles (all triangles without tiles) fold into the global keys during setup:
     // every tile's keys start empty and current (kBatchGen), otherwise no tile is current
-    const bool keys = b->folded || b->direct_max > 0;
+    const bool keys = b->folded != FoldForm::none || b->direct_max > 0;
     BatchReset r{};
     r.tile_count = b->bb.tile_count;
     r.tile_cursor = b->bb.tile_cursor;
@@ -455,10 +468,13 @@ cudaError_t enqueue_folded(sloth_batch *b, const BatchDev &d, cudaStream_t s)
 {
     cudaError_t e;
     if ((e = enqueue_reset(b, s))) return e;
-    const int table = b->small_fold ? kTabFold : kTabSetup;
-    if ((e = launch_batch_fold_setup(d, b->blk[table], b->nblk[table], b->small_fold, s))) return e;
-    // the small fold reduces the newline rows itself
-    const uint32_t nnl = b->small_fold ? 0u : b->nblk[kTabNewline];
+    const bool own = b->folded == FoldForm::setup;
+    const int table = own ? kTabSetup : kTabFold;
+    if ((e = launch_batch_fold_setup(d, b->blk[table], b->nblk[table],
+                                     own ? 0 : b->folded == FoldForm::warps1 ? 1 : 4, s)))
+        return e;
+    // the blocks of 32 triangles reduce the newline rows themselves
+    const uint32_t nnl = own ? b->nblk[kTabNewline] : 0u;
     const bool part = batch_newline_part(nnl, b->max_nl), fork = nnl && !part;
     if (fork && (e = fork_newline(b, d, s))) return e;
     if ((e = launch_batch_fold_large(d, b->blk[kTabNewline], part ? nnl : 0u, b->max_nl, s))) return e;
@@ -498,7 +514,7 @@ sloth_status render_planned(sloth_batch *b)
     cudaStream_t s = b->stream;
     BatchDev d = dev_view(b);
     b->status[0] = 0;
-    if (b->folded) {   // no entries to size
+    if (b->folded != FoldForm::none) {   // no entries to size
         BCU(b, enqueue_folded(b, d, s));
         b->rendered = true;
         return SLOTH_OK;
@@ -532,8 +548,9 @@ sloth_status capture(sloth_batch *b)
     const BatchDev d = dev_view(b);
     cudaGraph_t g = nullptr;
     BCU(b, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = b->folded ? enqueue_folded(b, d, s) : enqueue_front(b, d, s);
-    if (e == cudaSuccess && !b->folded) e = enqueue_back(b, d, s);
+    const bool fold = b->folded != FoldForm::none;
+    cudaError_t e = fold ? enqueue_folded(b, d, s) : enqueue_front(b, d, s);
+    if (e == cudaSuccess && !fold) e = enqueue_back(b, d, s);
     cudaError_t e2 = cudaStreamEndCapture(s, &g);
     if (e != cudaSuccess || e2 != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -712,7 +729,7 @@ sloth_status sloth_batch_render(sloth_batch *b)
     if (!b || !b->ctx) return SLOTH_ERR_INVALID_ARGUMENT;
     BCU(b, cudaSetDevice(b->device));
     b->vis_valid = false;
-    const bool fold = b->fold_ok && sloth_ctx_depth_cull(b->ctx);
+    const FoldForm fold = sloth_ctx_depth_cull(b->ctx) ? b->fold : FoldForm::none;
     if (fold != b->folded) {
         b->folded = fold;
         if (b->graph) cudaGraphExecDestroy(b->graph);
@@ -720,8 +737,9 @@ sloth_status sloth_batch_render(sloth_batch *b)
     }
     // a render known to have outgrown its entries: the buffer grows before the next one
     // (settle does the same for a caller that reads)
-    const bool grow = !b->folded && *(volatile uint32_t *)&b->status[0];
-    if (grow || !b->rendered || (!b->folded && !b->bb.entries)) return render_planned(b);
+    const bool tiles = b->folded == FoldForm::none;
+    const bool grow = tiles && *(volatile uint32_t *)&b->status[0];
+    if (grow || !b->rendered || (tiles && !b->bb.entries)) return render_planned(b);
     if (!b->graph && b->stream != nullptr) {
         const sloth_status st = capture(b);
         if (st != SLOTH_OK) return st;

@@ -50,8 +50,6 @@ struct BatchDev {
     int depth_cull;
     int tpb;                   // triangles per setup block (the triangle block table's step)
     int direct_max;            // the frames' FrameGeom::direct_max (the same for every frame)
-    int fold;                  // every frame is drawn without tiles (fold.cuh): the queued
-                               // triangles are in bb.large_queue and large_frame
     uint32_t resolve_chunk;    // cells per resolve block (the resolve table's step)
 };
 
@@ -84,9 +82,10 @@ cudaError_t launch_batch_count_large(const BatchDev &b, cudaStream_t s);
 // batch_newline_part)
 cudaError_t launch_batch_fill(const BatchDev &b, const int2 *newline, uint32_t nnewline, int max_nl, cudaStream_t s);
 cudaError_t launch_batch_raster(const BatchDev &b, int tw, int th, bool persistent, cudaStream_t s);
-// frames without tiles: setup and fold (blocks: a kFoldBlockTris table when small, else the
-// setup table), then the queued triangles
-cudaError_t launch_batch_fold_setup(const BatchDev &b, const int2 *blocks, uint32_t nblocks, bool small,
+// frames without tiles: setup and fold (by blocks of `warps` warps, 4 or 1, over a
+// kFoldBlockTris table; 0: by the setup kernel over the setup table), which queues the larger
+// triangles in bb.large_queue and large_frame, then those
+cudaError_t launch_batch_fold_setup(const BatchDev &b, const int2 *blocks, uint32_t nblocks, int warps,
                                     cudaStream_t s);
 cudaError_t launch_batch_fold_large(const BatchDev &b, const int2 *newline, uint32_t nnewline, int max_nl,
                                     cudaStream_t s);
@@ -98,6 +97,10 @@ constexpr uint32_t kBatchNewlineChunk = 8192;   // triangles per newline block (
 constexpr uint32_t kBatchResolveChunk = 8192;   // cells per resolve block (four rounds of its threads)
 constexpr uint32_t kBatchResolveSmall = 2048;   // the same (one round) for batches of few blocks
 constexpr uint32_t kFoldBlockTris = 32;         // triangles per block of a small fold's table
-constexpr uint32_t kBatchSmallFold = 1u << 18;  // triangles up to which a fold uses that table
+// Triangles of a batch up to which it has that table, up to which its blocks may be of four
+// warps, and from which they may be of one (batch_folds)
+constexpr uint32_t kFoldTableTriangles = 1u << 20;
+constexpr uint32_t kFoldMany4 = 1u << 18;
+constexpr uint32_t kFoldMany = 1u << 16;
 
 }  // namespace sloth

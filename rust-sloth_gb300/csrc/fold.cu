@@ -46,19 +46,19 @@ fold_setup_kernel(MeshDev mesh, Mat4 M, uint32_t tri_base, FrameGeom g, FrameBuf
 // The queued triangles' items over the warps of the grid, the large ones' first.  next: the
 // counters the frame's next draw queues with, emptied here (the draw after that reuses
 // this one's).
+struct FoldFrame {
+    FrameGeom g;
+    FrameBuffers fb;
+};
+
 __global__ void __launch_bounds__(256)
-fold_large_kernel(FrameGeom g, FrameBuffers fb, FoldQueue queue, uint32_t *next)
+fold_large_kernel(const __grid_constant__ FoldFrame f, FoldQueue queue, uint32_t *next)
 {
     const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x + pdl_begin()) >> 5;
     if (blockIdx.x == 0 && threadIdx.x < 2) next[threadIdx.x] = 0u;
-    const uint32_t large = queue.count[0], mid = queue.count[1], nwarps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t parts = fold_parts(large), cut = large * parts, items = cut + mid;
-    const bool filter = large + mid > kFoldFilterMin;
-    uint32_t frags = 0;
-    for (uint32_t it = first; it < items; it += nwarps)
-        frags += it < cut ? fold_queued<kFoldRows>(queue.tri[it / parts], it % parts, parts, filter, g, fb)
-                          : fold_queued<32>(queue.tri[queue.cap - 1u - (it - cut)], 0u, 1u, filter, g, fb);
-    add_frags_warp(frags, fb.fragments);
+    const uint32_t frags = fold_queue_walk(queue, first, (gridDim.x * blockDim.x) >> 5,
+                                           [&](uint32_t) -> const FoldFrame & { return f; });
+    add_frags_warp(frags, f.fb.fragments);
 }
 
 cudaError_t launch_fold_begin(const FrameGeom &g, const FrameBuffers &fb, bool frame, bool all,
@@ -82,7 +82,7 @@ cudaError_t launch_fold_large(const FrameGeom &g, const FrameBuffers &fb, uint32
                               uint32_t *queue_counts, int parity, cudaStream_t s)
 {
     const FoldQueue q{queue, nullptr, queue_counts + 2 * parity, cap};
-    return launch_pdl(fold_large_kernel, dim3(4u * (unsigned)device_sm_count()), dim3(256), 0, s, g, fb, q,
+    return launch_pdl(fold_large_kernel, dim3(4u * (unsigned)device_sm_count()), dim3(256), 0, s, FoldFrame{g, fb}, q,
                       queue_counts + 2 * (parity ^ 1));
 }
 

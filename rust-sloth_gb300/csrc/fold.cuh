@@ -24,16 +24,18 @@ constexpr int kFoldTris = 32;
 // Triangles of more samples than this (rows times walked columns) are queued: the block
 // that set one up would walk it alone while the rest of the GPU is idle.
 constexpr uint32_t kFoldBlockSamples = 128;
-// Of the queued ones, those of at most kFoldWarpSamples samples are one warp item each, 32
-// rows at a time; larger ones are cut into `parts` items of every parts-th group of
-// kFoldRows rows: 64 items take a triangle of 512 rows in one group each, and an item past
-// the last row costs one cached load.  Thousands of them fill the grid at a quarter of that.
+// A queued triangle is cut into items of every parts-th group of kFoldRows rows: kFoldParts
+// items for the large ones (one group each up to 1024 rows), kFoldMidParts for those of at
+// most kFoldWarpSamples samples, or, when there are enough of them for a warp each, one item
+// of all their rows, 32 at a time.  Items are numbered part after part and a warp's lanes
+// look at 32 of them at once, so the items past a triangle's last row cost next to nothing.
 // A warp walks kFoldUnroll steps of 32 samples at once: the row searches, edge values and
 // key loads of a step are one chain, and the walk waits on its latency.
 constexpr uint32_t kFoldWarpSamples = 4096;
 constexpr int kFoldRows = 8;
+constexpr uint32_t kFoldParts = 128, kFoldMidParts = 8;
 constexpr int kFoldUnroll = 4;
-__device__ __forceinline__ uint32_t fold_parts(uint32_t large) { return large > 2048u ? 16u : 64u; }
+
 // With more queued triangles than this, cells that already hold a nearer key are left out
 // before the reduction (they may overdraw each other many times); with fewer, the load
 // would only lengthen each step.
@@ -271,6 +273,48 @@ __device__ __forceinline__ uint32_t fold_queued(uint32_t gtri, uint32_t part, ui
 #pragma unroll
             for (int u = 0; u < kUnroll; ++u)
                 if (key[u] != kEmptyKey) red_min_u64(kp[u], key[u]);
+        }
+    }
+    return frags;
+}
+
+// The queued triangles of one frame or many, over the warps of a grid (this is warp `warp` of
+// nwarps): frame_of(q) gives the frame of queue entry q as a pair of its geometry and buffers.
+template <class FrameOf>
+__device__ __forceinline__ uint32_t fold_queue_walk(const FoldQueue &queue, uint32_t warp, uint32_t nwarps,
+                                                    FrameOf frame_of)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t large = queue.count[0], mid = queue.count[1];
+    const bool whole = mid > nwarps / 2;   // a warp for each of the smaller ones
+    const uint32_t cut = large * kFoldParts, items = cut + mid * (whole ? 1u : kFoldMidParts);
+    const bool filter = large + mid > kFoldFilterMin;
+    uint32_t frags = 0;
+    for (uint32_t base = warp; base < items; base += 32u * nwarps) {
+        // lane l holds item base + l*nwarps: neighbouring items go to neighbouring warps
+        const uint32_t it = base + (uint32_t)lane * nwarps;
+        uint32_t q = 0, part = 0, tri = 0;
+        bool live = it < items && it >= base;
+        if (live) {
+            if (it < cut) {
+                part = it / large;
+                q = it - part * large;
+            } else {
+                part = (it - cut) / mid;
+                q = queue.cap - 1u - ((it - cut) - part * mid);
+            }
+            tri = queue.tri[q];
+            const int4 xr = *(reinterpret_cast<const int4 *>(frame_of(q).fb.records + tri) + 4);
+            live = xr.z + (int)part * kFoldRows < xr.w;
+        }
+        for (unsigned todo = __ballot_sync(0xffffffffu, live); todo; todo &= todo - 1u) {
+            const int src = __ffs(todo) - 1;
+            const uint32_t wq = __shfl_sync(0xffffffffu, q, src), wt = __shfl_sync(0xffffffffu, tri, src),
+                           wp = __shfl_sync(0xffffffffu, part, src), wi = __shfl_sync(0xffffffffu, it, src);
+            const auto &f = frame_of(wq);
+            if (wi < cut) frags += fold_queued<kFoldRows>(wt, wp, kFoldParts, filter, f.g, f.fb);
+            else if (!whole) frags += fold_queued<kFoldRows>(wt, wp, kFoldMidParts, filter, f.g, f.fb);
+            else frags += fold_queued<32>(wt, 0u, 1u, filter, f.g, f.fb);
         }
     }
     return frags;

@@ -53,7 +53,7 @@ def test_batch_changes_between_fold_and_tiles(big):
 
 @pytest.mark.parametrize("tpb", [128, 4096])
 def test_batch_fold_of_many_triangles(tpb):
-    """More than 2^18 triangles: the fold goes through the batch's setup kernel, with the
+    """More than 2^18 triangles of hardly a sample each: the fold goes through the batch's setup kernel, with the
     newline rows beside it, in chunks of one and of several per block."""
     with S.Context(0) as c:
         a, s = W.displaced_icosphere(5, seed=2), W.soup(3000, seed=7, n_large=6, sigma=0.05)
@@ -110,3 +110,27 @@ def test_batch_overflow_is_exact_on_the_device(ctx, direct, persistent):
             assert np.array_equal(cells, ref.cells.view(np.int32)), f"render {rep} frame {i}"
             assert np.array_equal(zz, ref.z.view(np.int32)), f"render {rep} frame {i}"
     b.close()
+
+
+def test_batch_fold_by_single_warps():
+    """71,680 triangles of about ten samples: the fold takes 32 triangles to a block of one
+    warp; then transforms a hundred times smaller, planned anew and replayed."""
+    with S.Context(0) as c:
+        a = W.displaced_icosphere(4, seed=2)
+        da = dev_mesh(c, a)
+        frames = []
+        for k in range(14):
+            w, h, image = ((320, 90, True), (161, 95, False))[k % 2]
+            frames.append({"w": w, "h": h, "image": image, "U": O.viewport_transform(w, h, O.scene_extent([a["bbox_max"]])),
+                           "draws": [(da, O.euler_rotation(*W.cli_rotation(pitch=0.5 * k)))]})
+        b = S.Batch(c, frames)
+        tiny = np.diag([0.01, 0.01, 0.01, 1.0]).astype(np.float32)
+        for scale in (None, tiny, None):
+            Rs = [f["draws"][0][1] if scale is None else O.mat4_mul(f["draws"][0][1], scale) for f in frames]
+            b.set_transforms(np.stack(Rs))
+            for rep in range(2):
+                b.render()
+                for i, f in enumerate(frames):
+                    ref = oracle_render([a], Rs[i], f["w"], f["h"], f["image"], U=f["U"])
+                    assert_same((*b.read(i), None), ref, f"render {rep} frame {i}")
+        b.close()
