@@ -156,24 +156,22 @@ __global__ void __launch_bounds__(kSetupThreads, kDirect ? kSetupMinBlocks : kFi
             const uint32_t q = p + blockDim.x;
             const bool lt = p < t_end, lu = q < c0 + cap && q < t_end;
             float4 a1, a2, a3, b1, b2, b3;
-            uint32_t ca = 0, cb = 0, tp = 0, tq = 0;
+            uint32_t tp = 0, tq = 0;
             if (lt) {
                 tp = mesh_triangle(d.mesh, p);
                 batch_triangle_vertices(d, sm, p, tp, a1, a2, a3);
-                ca = load_rgb(d.mesh.rgb, tp);
             }
             if (lu) {
                 tq = mesh_triangle(d.mesh, q);
                 batch_triangle_vertices(d, sm, q, tq, b1, b2, b3);
-                cb = load_rgb(d.mesh.rgb, tq);
             }
             int4 row4;
             const bool kt = lt && needs_setup(a1, a2, a3, f.g.w, f.g.h, row4);
             if (lt) f.fb.rows[d.local_base + p] = pack_rows(row4.z, row4.w);
-            stash_push(st, &sq_n, base, kt, tp, a1, a2, a3, ca);
+            stash_push(st, &sq_n, base, kt, tp, a1, a2, a3);
             const bool ku = lu && needs_setup(b1, b2, b3, f.g.w, f.g.h, row4);
             if (lu) f.fb.rows[d.local_base + q] = pack_rows(row4.z, row4.w);
-            stash_push(st, &sq_n, base, ku, tq, b1, b2, b3, cb);
+            stash_push(st, &sq_n, base, ku, tq, b1, b2, b3);
         }
         block_sync();
         const uint32_t total = sq_n, nq = total - base;
@@ -181,8 +179,11 @@ __global__ void __launch_bounds__(kSetupThreads, kDirect ? kSetupMinBlocks : kFi
             const uint32_t q = q0 + threadIdx.x;
             float4 p1, p2, p3;
             uint32_t rgb = 0, t = 0;
-            if (q < nq) t = st.get(q, p1, p2, p3, rgb);
-            const uint32_t stage = 11u * cap + (threadIdx.x >> 5) * (uint32_t)kDirectStageWords;
+            if (q < nq) {
+                t = st.get(q, p1, p2, p3);
+                rgb = load_rgb(d.mesh.rgb, t);
+            }
+            const uint32_t stage = 10u * cap + (threadIdx.x >> 5) * (uint32_t)kDirectStageWords;
             if constexpr (kFold) batch_fold_triangle(b, d, f, q < nq, t, p1, p2, p3, rgb, stage);
             else batch_setup_triangle<kDirect>(b, d, f, q < nq, t, p1, p2, p3, rgb, stage);
         }

@@ -72,6 +72,23 @@ __device__ __forceinline__ OrientBound orient_bound(const TriRecord &r)
     return ob;
 }
 
+// An upper bound of orient_bound(r).err from the triangle's bounding box: every |fl(p - a)| of
+// the three edges is at most the distance between the evaluation rectangle and the box's far
+// side, and so are the two of the orient (the box contains every vertex), so that each
+// product of the four determinants is bounded by an edge delta times one of two extents.
+__device__ __forceinline__ float loose_orient_err(const TriRecord &r, float mnx, float mxx, float mny, float mxy)
+{
+    const float kUp = 1.0f + 1.1920929e-07f;
+    const float xl = fminf((float)r.x0, mnx), xh = fmaxf((float)(r.xe - 1), mxx);
+    const float yl = fminf((float)r.y0, mny), yh = fmaxf((float)(r.y1 - 1), mxy);
+    const float ex = __fmul_ru(__fsub_ru(xh, xl), kUp), ey = __fmul_ru(__fsub_ru(yh, yl), kUp);
+    // edge 2's deltas count twice: once for its edge function, once for the orient
+    const float dx = __fadd_ru(__fadd_ru(fabsf(r.dx0), fabsf(r.dx1)), __fadd_ru(fabsf(r.dx2), fabsf(r.dx2)));
+    const float dy = __fadd_ru(__fadd_ru(fabsf(r.dy0), fabsf(r.dy1)), __fadd_ru(fabsf(r.dy2), fabsf(r.dy2)));
+    const float sum = __fadd_ru(__fmul_ru(dx, ey), __fmul_ru(dy, ex));
+    return __fadd_ru(__fmul_ru(kU8 * 1.00001f, sum), 8.0f * kTiny);
+}
+
 // True if no sample of the evaluation rectangle can have all three computed edge
 // functions >= 0.  For any point p the exact edge functions satisfy E0+E1+E2 = O (the
 // exact orient).  w_i >= 0 implies E_i >= -b_i, so coverage needs O >= -(b0+b1+b2), and

@@ -41,8 +41,9 @@ constexpr int kFoldUnroll = 4;
 // would only lengthen each step.
 constexpr uint32_t kFoldFilterMin = 512;
 
-// Dynamic shared memory of a fold block: one direct stage and the samples' running ends.
-constexpr size_t kFoldSmemBytes = (kDirectStageWords + 32) * 4;
+// Dynamic shared memory of a fold block: one direct stage and each lane's triangle's first
+// sample (-1: none), and the samples of all.
+constexpr size_t kFoldSmemBytes = (kDirectStageWords + 33) * 4;
 
 // Triangles too large for their block: draw index and frame (batches; null otherwise), the
 // large ones from the front of the cap entries, the others from the back; count[0] and
@@ -113,13 +114,12 @@ __device__ __forceinline__ void fold_triangles(const MeshDev &mesh, const Mat4 &
                                                const FrameGeom &g, const FrameBuffers &fb, const FoldQueue &queue,
                                                uint32_t frame)
 {
-    int *ends = reinterpret_cast<int *>(setup_smem + kDirectStageWords);
+    int *starts = reinterpret_cast<int *>(setup_smem + kDirectStageWords);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (wid == 0) {
         const uint32_t p = p0 + lane;
         FoldClass c{false, false, false};
         uint32_t gtri = 0;
-        int n = 0;
         DirectWalk dw{false, 0, 0u};
         TriRecord r;
         if (p < mesh.ntri) {
@@ -141,25 +141,21 @@ __device__ __forceinline__ void fold_triangles(const MeshDev &mesh, const Mat4 &
                 }
             }
         }
-        if (c.mine) n = direct_stage(true, r, gtri, dw.xend, dw.exit_mask, 0u);
         const int q = fold_queue_slot(queue, c.mid, c.large);
         if (q >= 0) {
             queue.tri[q] = gtri;
             if (queue.frame) queue.frame[q] = frame;
         }
-        int end = n;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int o = __shfl_up_sync(0xffffffffu, end, d);
-            if (lane >= d) end += o;
-        }
-        ends[lane] = end;
+        int start;
+        const int n = c.mine ? direct_columns(r, dw.xend, dw.exit_mask) * (r.y1 - r.y0) : 0;
+        const int all = direct_stage_warp(c.mine, n, r, gtri, dw.xend, dw.exit_mask, 0u, start);
+        starts[lane] = c.mine ? start : -1;
+        if (lane == 0) starts[32] = all;
     }
     if (kWarps > 1) block_sync();
     else __syncwarp();
-    const int end = ends[lane], prev = lane ? ends[lane - 1] : 0;
-    const int total = __shfl_sync(0xffffffffu, end, 31);
-    const uint32_t frags = direct_walk(end, prev, total, wid * 32, kWarps * 32, g.w, g.pitch, g.tw,
+    const int start = starts[lane];
+    const uint32_t frags = direct_walk(start >= 0, start, starts[32], wid * 32, kWarps * 32, g.w, g.pitch, g.tw,
                                        reinterpret_cast<unsigned long long *>(fb.keys), 0u);
     add_frags_warp(frags, fb.fragments);
 }

@@ -116,8 +116,10 @@ __device__ __forceinline__ bool needs_setup(float4 p1, float4 p2, float4 p3, int
                         fabsf(p2.y) < big && fabsf(p3.x) < big && fabsf(p3.y) < big;
     // the proof needs o < -err with err >= 0: a triangle whose computed orient o (the value
     // orient_bound computes first) is not negative is never proven empty, so the bound is
-    // worked out only for the others (back faces, mostly)
-    if (finite && edge_eval(r.dx2, r.dy2, r.v1x, r.v1y, r.v3x, r.v3y) < 0.0f && provably_empty(orient_bound(r))) {
+    // worked out only for the others (back faces, mostly), and the full one only for those
+    // that a looser one in a third of the operations does not prove
+    const float o = edge_eval(r.dx2, r.dy2, r.v1x, r.v1y, r.v3x, r.v3y);
+    if (finite && o < 0.0f && (o < -loose_orient_err(r, mnx, mxx, mny, mxy) || provably_empty(orient_bound(r)))) {
         row4 = make_int4(r.x0, r.x0, r.y0, r.y1);
         return false;
     }
@@ -137,31 +139,30 @@ __device__ __forceinline__ uint32_t load_rgb(const uint8_t *rgb, uint32_t t)
 }
 
 // The queue between a setup block's two phases, in dynamic shared memory
-// (setup_smem_bytes): per slot the triangle index, its packed colour and its three
-// transformed vertices, as 11 arrays of cap words so that consecutive slots fall in
-// different banks.  Phase 2 reads a queued triangle from here, not from global memory.
+// (setup_smem_bytes): per slot the triangle index and its three
+// transformed vertices, as 10 arrays of cap words so that consecutive slots fall in
+// different banks.  Phase 2 reads a queued triangle from here; its colour, which only the
+// record's store waits for, it loads itself (half the triangles never need theirs).
 // setup_smem (direct.cuh) is indexed itself, which keeps the accesses 32-bit shared ones.
 
 struct SetupStash {
     uint32_t cap;
 
-    __device__ __forceinline__ void put(uint32_t s, uint32_t t, float4 p1, float4 p2, float4 p3, uint32_t c) const
+    __device__ __forceinline__ void put(uint32_t s, uint32_t t, float4 p1, float4 p2, float4 p3) const
     {
         setup_smem[s] = t;
-        setup_smem[cap + s] = c;
         const float v[9] = {p1.x, p1.y, p1.z, p2.x, p2.y, p2.z, p3.x, p3.y, p3.z};
 #pragma unroll
-        for (int k = 0; k < 9; ++k) setup_smem[(2 + k) * cap + s] = __float_as_uint(v[k]);
+        for (int k = 0; k < 9; ++k) setup_smem[(1 + k) * cap + s] = __float_as_uint(v[k]);
     }
-    __device__ __forceinline__ uint32_t get(uint32_t s, float4 &p1, float4 &p2, float4 &p3, uint32_t &c) const
+    __device__ __forceinline__ uint32_t get(uint32_t s, float4 &p1, float4 &p2, float4 &p3) const
     {
         float v[9];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) v[k] = __uint_as_float(setup_smem[(2 + k) * cap + s]);
+        for (int k = 0; k < 9; ++k) v[k] = __uint_as_float(setup_smem[(1 + k) * cap + s]);
         p1 = make_float4(v[0], v[1], v[2], 0.0f);
         p2 = make_float4(v[3], v[4], v[5], 0.0f);
         p3 = make_float4(v[6], v[7], v[8], 0.0f);
-        c = setup_smem[cap + s];
         return setup_smem[s];
     }
 };
@@ -170,7 +171,7 @@ struct SetupStash {
 // lanes).  count is the block's running total of queued triangles and base its value when
 // the chunk began, so the chunk's slots are 0, 1, ... in the stash.
 __device__ __forceinline__ void stash_push(const SetupStash &st, uint32_t *count, uint32_t base, bool keep, uint32_t t,
-                                           float4 p1, float4 p2, float4 p3, uint32_t c)
+                                           float4 p1, float4 p2, float4 p3)
 {
     const unsigned m = __ballot_sync(0xffffffffu, keep);
     if (!m) return;
@@ -178,7 +179,7 @@ __device__ __forceinline__ void stash_push(const SetupStash &st, uint32_t *count
     uint32_t first = 0;
     if (lane == 0) first = atomicAdd(count, (uint32_t)__popc(m));
     first = __shfl_sync(0xffffffffu, first, 0) - base;
-    if (keep) st.put(first + __popc(m & ((1u << lane) - 1u)), t, p1, p2, p3, c);
+    if (keep) st.put(first + __popc(m & ((1u << lane) - 1u)), t, p1, p2, p3);
 }
 
 // How the setup thread rasterizes a direct triangle (direct.cuh): its samples lie in rows

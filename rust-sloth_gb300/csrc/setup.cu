@@ -127,9 +127,9 @@ __device__ __forceinline__ void setup_triangle(uint32_t tri_base, const FrameGeo
 // A block takes tpb triangles, in chunks of setup_chunk(tpb), each in two phases.  Phase 1:
 // every triangle gets its sample range and the back-face proof (needs_setup); those with
 // nothing to rasterize are done, the others are queued in
-// shared memory with their vertices and colour.  Phase 2: the queued triangles, dense in
-// the lanes, get the rest of their setup (setup_triangle) without touching global memory
-// for their inputs again.  Back faces are about half of a closed mesh's triangles, and
+// shared memory with their vertices.  Phase 2: the queued triangles, dense in
+// the lanes, get the rest of their setup (setup_triangle), loading only their colour again
+// from global memory.  Back faces are about half of a closed mesh's triangles, and
 // mixed through every warp: without the queue half the lanes of a warp would idle through
 // the front faces' work.  kDirect: compiled with the direct path (g.direct_max > 0), which
 // needs more registers.  kChunks: compiled for more than one chunk per block (tpb above
@@ -155,24 +155,22 @@ setup_kernel(MeshDev mesh, const float4 *__restrict__ tv, Mat4 M, uint32_t tri_b
             const uint32_t q = p + blockDim.x;
             const bool lt = p < t_end, lu = q < c0 + cap && q < t_end;
             float4 a1, a2, a3, b1, b2, b3;
-            uint32_t ca = 0, cb = 0, tp = 0, tq = 0;
+            uint32_t tp = 0, tq = 0;
             if (lt) {
                 tp = mesh_triangle(mesh, p);
                 triangle_vertices(mesh, tv, M, p, tp, a1, a2, a3);
-                ca = load_rgb(mesh.rgb, tp);
             }
             if (lu) {
                 tq = mesh_triangle(mesh, q);
                 triangle_vertices(mesh, tv, M, q, tq, b1, b2, b3);
-                cb = load_rgb(mesh.rgb, tq);
             }
             int4 row4;
             const bool kt = lt && needs_setup(a1, a2, a3, g.w, g.h, row4);
             if (lt) fb.rows[tri_base + p] = pack_rows(row4.z, row4.w);
-            stash_push(st, &sq_n, base, kt, tp, a1, a2, a3, ca);
+            stash_push(st, &sq_n, base, kt, tp, a1, a2, a3);
             const bool ku = lu && needs_setup(b1, b2, b3, g.w, g.h, row4);
             if (lu) fb.rows[tri_base + q] = pack_rows(row4.z, row4.w);
-            stash_push(st, &sq_n, base, ku, tq, b1, b2, b3, cb);
+            stash_push(st, &sq_n, base, ku, tq, b1, b2, b3);
         }
         block_sync();
         const uint32_t total = sq_n, nq = total - base;
@@ -180,9 +178,12 @@ setup_kernel(MeshDev mesh, const float4 *__restrict__ tv, Mat4 M, uint32_t tri_b
             const uint32_t q = q0 + threadIdx.x;
             float4 p1, p2, p3;
             uint32_t rgb = 0, t = 0;
-            if (q < nq) t = st.get(q, p1, p2, p3, rgb);
+            if (q < nq) {
+                t = st.get(q, p1, p2, p3);
+                rgb = load_rgb(mesh.rgb, t);
+            }
             setup_triangle<kDirect>(tri_base, g, fb, bb, q < nq, t, p1, p2, p3, rgb,
-                                    11u * cap + (threadIdx.x >> 5) * (uint32_t)kDirectStageWords);
+                                    10u * cap + (threadIdx.x >> 5) * (uint32_t)kDirectStageWords);
         }
         if (!kChunks) break;
         base = total;

@@ -143,14 +143,14 @@ inline bool valid_triangles_per_block(long long v) { return v == 128 || v == 256
 __host__ __device__ inline int setup_block_threads(int tpb) { return tpb < kSetupThreads ? tpb : kSetupThreads; }
 // A setup block takes its triangles in chunks of at most kSetupChunk.  Phase 1 of a chunk
 // queues, in shared memory, the triangles that need the rest of their setup together with
-// their transformed vertices and colour (record.cuh: SetupStash, 44 bytes a triangle).
+// their transformed vertices (record.cuh: SetupStash, 40 bytes a triangle).
 constexpr int kSetupChunk = 1024;
 __host__ __device__ inline int setup_chunk(int tpb) { return tpb < kSetupChunk ? tpb : kSetupChunk; }
 // Dynamic shared memory of a setup block: the stash, and with the direct path one stage of
-// 23 x 32 words per warp (direct.cuh) after it.
+// 16 x 32 words per warp (direct.cuh) after it.
 __host__ __device__ inline size_t setup_smem_bytes(int tpb, bool direct = false)
 {
-    return 44u * (size_t)setup_chunk(tpb) + (direct ? (size_t)(setup_block_threads(tpb) / 32) * 23u * 32u * 4u : 0u);
+    return 40u * (size_t)setup_chunk(tpb) + (direct ? (size_t)(setup_block_threads(tpb) / 32) * 16u * 32u * 4u : 0u);
 }
 // Sets the shared-memory limit of the setup kernels with the direct path (above the 48 KB
 // default), once per device; call before the first launch and outside stream capture.
