@@ -331,6 +331,25 @@ __device__ __forceinline__ void nltree_update(int32_t *tree, int n, int y0, int 
     }
 }
 
+// The newline rows [y0, y1) of a warp's 32 triangles (empty for lanes without one; called by
+// all lanes), row by row: triangles next to each other span the same few rows, and when that
+// is at most 32 in all, true, with `last` the largest draw index of row lo + lane (-1: none).
+// False when they span more.
+__device__ __forceinline__ bool warp_row_last(int y0, int y1, int32_t v, int &lo, int32_t &last)
+{
+    const bool some = y0 < y1;
+    lo = (int)__reduce_min_sync(0xffffffffu, some ? (unsigned)y0 : 0x7fffffffu);
+    const int hi = (int)__reduce_max_sync(0xffffffffu, some ? (unsigned)y1 : 0u);
+    last = -1;
+    if (hi - lo > 32) return false;   // hi < lo: no rows at all
+    const int lane = threadIdx.x & 31;
+    for (int y = lo; y < hi; ++y) {
+        const int32_t m = __reduce_max_sync(0xffffffffu, some && y >= y0 && y < y1 ? v : -1);
+        if (lane == y - lo) last = m;
+    }
+    return true;
+}
+
 // The last newline writer of row y: the maximum over the leaf-to-root path (-1: none).
 __device__ __forceinline__ int32_t nltree_query(const int32_t *tree, int n, int y)
 {
