@@ -95,6 +95,7 @@ struct sloth_ctx {
     int tpb = kDefaultTrianglesPerBlock;   // SLOTH_OPTION_TRIANGLES_PER_BLOCK
     bool keys_current = false;     // every tile's keys cleared for the current generation
     uint32_t *fold_counts = nullptr;   // queue counters of the draws without tiles (launch_fold_setup)
+    bool fold_begun = false;           // they were emptied in this frame
     int fold_parity = 0;               // the counter the frame's next such draw uses
     bool timing = false;
     std::map<std::string, KernelClock> clocks;
@@ -599,6 +600,7 @@ sloth_status sloth_ctx_clear(sloth_ctx *ctx)
     ctx->dirty = true;
     ctx->g.direct_max = ctx->direct_max;
     ctx->keys_current = false;
+    ctx->fold_begun = false;
     return SLOTH_OK;
 }
 
@@ -1038,13 +1040,14 @@ static bool draws_without_tiles(const sloth_ctx *ctx, const sloth_mesh *mesh, co
     return fold_estimate(mesh->span2, mesh->ntri, M, ctx->g.w, ctx->g.h) <= kFoldMaxSamples;   // false for NaN
 }
 
-// One draw without tiles: every tile's keys made current first (once a frame).
+// One draw without tiles: every tile's keys made current and the queue counters emptied first
+// (once a frame, also where a binned draw of direct samples has made the keys current).
 static sloth_status draw_folded(sloth_ctx *ctx, const sloth_mesh *mesh, const Mat4 &M)
 {
     sloth_status st;
     cudaStream_t s = ctx->stream;
     if (!ctx->fold_counts) CU(ctx, dalloc(&ctx->fold_counts, 4));
-    if (ctx->reset_pending || !ctx->keys_current) {
+    if (ctx->reset_pending || !ctx->keys_current || !ctx->fold_begun) {
         if ((st = join_newline(ctx)) != SLOTH_OK) return st;   // the last frame's fold into the tree
         const bool frame = ctx->reset_pending;
         CU(ctx, timed(ctx, "reset", [&] {
@@ -1052,6 +1055,7 @@ static sloth_status draw_folded(sloth_ctx *ctx, const sloth_mesh *mesh, const Ma
            }));
         ctx->reset_pending = false;
         ctx->keys_current = true;
+        ctx->fold_begun = true;
         ctx->fold_parity = 0;
     }
     const MeshDev md{mesh->x, mesh->y, mesh->z, mesh->idx, mesh->rgb, mesh->nvert, mesh->ntri, mesh->order, mesh->oidx};

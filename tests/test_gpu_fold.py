@@ -107,3 +107,25 @@ def test_context_fold_queue_classes(side):
             ctx.draw_mesh(dm, eye)
             check([a.view(np.int32) if a.dtype == np.float32 else a for a in ctx.read()],
                   oracle_render([m], eye, w, h, image, U=eye), f"side {side} {w}x{h}")
+
+
+@pytest.mark.parametrize("direct", [4, 16, 64])
+def test_context_fold_after_direct_draw(direct):
+    """A fresh context whose first draw is binned with direct samples on: that draw makes the
+    tiles' keys current, and the folds after it still start from empty queue counters."""
+    w, h = 161, 47
+    big, ico = W.soup(6000, seed=4, n_large=400, sigma=0.8), W.displaced_icosphere(2, seed=5)
+    R = O.euler_rotation(*W.cli_rotation(yaw=0.6, pitch=0.2))
+    U = O.viewport_transform(w, h, O.scene_extent([big["bbox_max"], ico["bbox_max"]]))
+    with S.Context(0) as c:
+        dev = {id(m): S.Mesh(c, m["x"], m["y"], m["z"], m["rgb"], m["idx"], m["bbox_max"]) for m in (ico, big)}
+        c.set_direct_samples(direct)
+        c.set_viewport(w, h, False)
+        c.set_utransform(U)
+        for k, order in enumerate(((big, ico, ico, big), (ico, big, ico), (big, ico))):
+            Rs = [R * np.float32(40.0) if m is big else R for m in order]
+            c.clear()
+            for m, Rm in zip(order, Rs):
+                c.draw_mesh(dev[id(m)], Rm)
+            check([a.view(np.int32) if a.dtype == np.float32 else a for a in c.read()],
+                  oracle_render(list(order), Rs, w, h, False, U=U), f"frame {k}")
