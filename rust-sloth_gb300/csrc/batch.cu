@@ -219,7 +219,7 @@ __device__ __forceinline__ void batch_newline_block(const BatchDev &b, int2 blk,
 {
     const BatchDraw &d = b.draws[blk.x];
     const BatchFrame &f = b.frames[d.frame];
-    const uint32_t lo = (uint32_t)blk.y, hi = min(d.mesh.ntri, lo + kNewlineChunk);
+    const uint32_t lo = (uint32_t)blk.y, hi = min(d.mesh.ntri, lo + b.newline_chunk);
     newline_block<kShared>(stree, f.g.nl_size, lo, hi, d.mesh.order, f.fb.rows + d.local_base, d.local_base,
                            f.fb.nltree);
 }
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterMinBlocks) batch_raster
 // that wait on them at once count more than the loads each has in flight (uneven batch:
 // four blocks with four pairs of cells a thread 297 us, eight blocks with two 229).
 constexpr int kBatchRun = 2;
-static_assert(kBatchNewlineChunk == kNewlineChunk, "the host's table steps by the block's chunk");
+static_assert(kBatchNewlineChunk == kNewlineChunk && kBatchNewlineFillChunk == kNewlineFillChunk, "the same chunks");
 static_assert(kFoldBlockTris == kFoldTris, "the host's table steps by the block's triangles");
 static_assert(kBatchResolveChunk % (kBatchRun * 256) == 0 && kBatchResolveSmall % (kBatchRun * 256) == 0,
               "whole runs, the same trip count in every warp");
@@ -536,9 +536,9 @@ cudaError_t launch_batch_fold_setup(const BatchDev &b, const int2 *blocks, uint3
                       dim3(nblocks), dim3(setup_block_threads(b.tpb)), smem, s, b, blocks);
 }
 
-bool batch_newline_part(uint32_t nblocks, int max_nl)
+bool batch_newline_part(uint64_t ntri, int max_nl)
 {
-    return nblocks <= kNewlinePartTriangles / kNewlineChunk && newline_tree_bytes(max_nl) <= kNewlinePartBytes;
+    return ntri <= kNewlinePartTriangles && newline_tree_bytes(max_nl) <= kNewlinePartBytes;
 }
 
 cudaError_t launch_batch_fold_large(const BatchDev &b, const int2 *newline, uint32_t nnewline, int max_nl, cudaStream_t s)

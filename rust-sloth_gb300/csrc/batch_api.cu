@@ -61,6 +61,7 @@ struct sloth_batch {
     };
     std::vector<KeyRun> key_runs;
     int max_nl = 1;
+    bool nl_part = false;                     // the fill's blocks take the newline table (batch_newline_part)
 
     // device memory
     BatchFrame *d_frames = nullptr;
@@ -263,6 +264,10 @@ sloth_status build(sloth_batch *b, int shape)
     b->resolve_chunk = all_cells / kBatchResolveChunk < 8ull * (uint64_t)device_sm_count() ? kBatchResolveSmall
                                                                                            : kBatchResolveChunk;
     b->max_nl = 1;
+    for (const sloth_frame_desc &fd : b->frames)
+        while (b->max_nl < (int)fd.height) b->max_nl <<= 1;
+    b->nl_part = batch_newline_part(all_tri, b->max_nl);
+    const uint32_t nl_chunk = b->nl_part ? kBatchNewlineFillChunk : kBatchNewlineChunk;
     std::vector<int2> bt, bn, br, bs;
     for (uint32_t f = 0; f < nf; ++f) {
         const sloth_frame_desc &fd = b->frames[f];
@@ -278,7 +283,6 @@ sloth_status build(sloth_batch *b, int shape)
         g.nl_size = 1;
         while (g.nl_size < g.h) g.nl_size <<= 1;
         g.direct_max = b->direct_max;
-        b->max_nl = g.nl_size > b->max_nl ? g.nl_size : b->max_nl;
         BatchFrame &bf = b->hframes[f];
         bf.g = g;
         bf.tile_off = tiles;
@@ -317,7 +321,7 @@ sloth_status build(sloth_batch *b, int shape)
             if (all_tri <= kFoldTableTriangles)
                 for (uint32_t t = 0; t < mv.ntri; t += kFoldBlockTris) bs.push_back(make_int2((int)d, (int)t));
             if (g.image)
-                for (uint32_t t = 0; t < mv.ntri; t += kBatchNewlineChunk) bn.push_back(make_int2((int)d, (int)t));
+                for (uint32_t t = 0; t < mv.ntri; t += nl_chunk) bn.push_back(make_int2((int)d, (int)t));
             local += mv.ntri;
         }
         rec += local;
@@ -410,6 +414,7 @@ BatchDev dev_view(sloth_batch *b)
     d.tpb = b->tpb;
     d.direct_max = b->direct_max;
     d.resolve_chunk = b->resolve_chunk;
+    d.newline_chunk = b->nl_part ? kBatchNewlineFillChunk : kBatchNewlineChunk;
     return d;
 }
 
@@ -475,9 +480,9 @@ cudaError_t enqueue_folded(sloth_batch *b, const BatchDev &d, cudaStream_t s)
         return e;
     // the blocks of 32 triangles reduce the newline rows themselves
     const uint32_t nnl = own ? b->nblk[kTabNewline] : 0u;
-    const bool part = batch_newline_part(nnl, b->max_nl), fork = nnl && !part;
+    const bool fork = nnl && !b->nl_part;
     if (fork && (e = fork_newline(b, d, s))) return e;
-    if ((e = launch_batch_fold_large(d, b->blk[kTabNewline], part ? nnl : 0u, b->max_nl, s))) return e;
+    if ((e = launch_batch_fold_large(d, b->blk[kTabNewline], fork ? 0u : nnl, b->max_nl, s))) return e;
     if (fork && (e = cudaStreamWaitEvent(s, b->ev_nl, 0))) return e;
     return launch_batch_resolve(d, b->blk[kTabResolve], b->nblk[kTabResolve], b->any_odd, s);
 }
@@ -489,8 +494,7 @@ cudaError_t enqueue_front(sloth_batch *b, const BatchDev &d, cudaStream_t s)
     cudaError_t e;
     if ((e = enqueue_reset(b, s))) return e;
     if ((e = launch_batch_setup(d, b->blk[kTabSetup], b->nblk[kTabSetup], s))) return e;
-    if (b->nblk[kTabNewline] && !batch_newline_part(b->nblk[kTabNewline], b->max_nl) && (e = fork_newline(b, d, s)))
-        return e;
+    if (b->nblk[kTabNewline] && !b->nl_part && (e = fork_newline(b, d, s))) return e;
     if ((e = launch_batch_count_large(d, s))) return e;
     return launch_bin_scan(b->total_tiles, d.bb, s);
 }
@@ -500,11 +504,10 @@ cudaError_t enqueue_back(sloth_batch *b, const BatchDev &d, cudaStream_t s)
 {
     cudaError_t e;
     const uint32_t nnl = b->nblk[kTabNewline];
-    const bool part = batch_newline_part(nnl, b->max_nl);
-    if ((e = launch_batch_fill(d, b->blk[kTabNewline], part ? nnl : 0u, b->max_nl, s))) return e;
+    if ((e = launch_batch_fill(d, b->blk[kTabNewline], b->nl_part ? nnl : 0u, b->max_nl, s))) return e;
     const int tw = kTileShapes[b->shape][0], th = kTileShapes[b->shape][1];
     if ((e = launch_batch_raster(d, tw, th, b->persistent, s))) return e;
-    if (nnl && !part && (e = cudaStreamWaitEvent(s, b->ev_nl, 0))) return e;   // the newline tree is complete
+    if (nnl && !b->nl_part && (e = cudaStreamWaitEvent(s, b->ev_nl, 0))) return e;   // the newline tree is complete
     return launch_batch_resolve(d, b->blk[kTabResolve], b->nblk[kTabResolve], b->any_odd, s);
 }
 

@@ -51,6 +51,7 @@ struct BatchDev {
     int tpb;                   // triangles per setup block (the triangle block table's step)
     int direct_max;            // the frames' FrameGeom::direct_max (the same for every frame)
     uint32_t resolve_chunk;    // cells per resolve block (the resolve table's step)
+    uint32_t newline_chunk;    // triangles per newline block (the newline table's step)
 };
 
 // What a render empties before it starts, in one launch.
@@ -72,9 +73,9 @@ cudaError_t launch_batch_reset(const BatchReset &r, cudaStream_t s);
 
 // Block tables: one int2 (item, start) per block, built on the host.
 cudaError_t launch_batch_setup(const BatchDev &b, const int2 *blocks, uint32_t nblocks, cudaStream_t s);
-// whether the fill's and the fold's blocks take a newline table of nblocks blocks and trees
-// of max_nl leaves; launch_batch_newline when they do not
-bool batch_newline_part(uint32_t nblocks, int max_nl);
+// whether the fill's and the fold's blocks take the newline table (by kBatchNewlineFillChunk)
+// of ntri triangles and trees of max_nl leaves; launch_batch_newline when they do not
+bool batch_newline_part(uint64_t ntri, int max_nl);
 cudaError_t launch_batch_newline(const BatchDev &b, const int2 *blocks, uint32_t nblocks, int max_nl,
                                  cudaStream_t s);
 cudaError_t launch_batch_count_large(const BatchDev &b, cudaStream_t s);
@@ -94,6 +95,7 @@ cudaError_t launch_batch_resolve(const BatchDev &b, const int2 *blocks, uint32_t
 cudaError_t prepare_batch_kernels();
 
 constexpr uint32_t kBatchNewlineChunk = 8192;   // triangles per newline block (kNewlineChunk)
+constexpr uint32_t kBatchNewlineFillChunk = 1024;   // the same as a part of the fill (kNewlineFillChunk)
 constexpr uint32_t kBatchResolveChunk = 8192;   // cells per resolve block (four rounds of its threads)
 constexpr uint32_t kBatchResolveSmall = 2048;   // the same (one round) for batches of few blocks
 constexpr uint32_t kFoldBlockTris = 32;         // triangles per block of a small fold's table

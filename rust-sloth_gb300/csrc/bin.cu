@@ -271,8 +271,8 @@ bin_fill_kernel(uint32_t ntri, const uint32_t *__restrict__ order, uint32_t tri_
     extern __shared__ int32_t stree[];
     uint32_t blk = blockIdx.x + pdl_begin();
     if (blk < parts.newline) {
-        const uint32_t lo = blk * kNewlineChunk;
-        newline_block<true>(stree, g.nl_size, lo, min(ntri, lo + kNewlineChunk), order, fb.rows + tri_base, tri_base,
+        const uint32_t lo = blk * kNewlineFillChunk;
+        newline_block<true>(stree, g.nl_size, lo, min(ntri, lo + kNewlineFillChunk), order, fb.rows + tri_base, tri_base,
                             fb.nltree);
         return;
     }
@@ -327,7 +327,7 @@ cudaError_t launch_bin_fill(uint32_t ntri, const uint32_t *order, uint32_t tri_b
 {
     const uint32_t sms = (uint32_t)device_sm_count();
     FillParts parts{};
-    parts.newline = newline_in_fill(ntri, g) ? (ntri + kNewlineChunk - 1) / kNewlineChunk : 0u;
+    parts.newline = newline_in_fill(ntri, g) ? (ntri + kNewlineFillChunk - 1) / kNewlineFillChunk : 0u;
     parts.large = 4u * sms;
     parts.items = (ntiles + kSetupThreads - 1) / kSetupThreads;
     const uint32_t small = std::min(2u * kFillMinBlocks * sms, (ntri + kSetupThreads - 1) / kSetupThreads);

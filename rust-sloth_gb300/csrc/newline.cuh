@@ -10,15 +10,20 @@
 
 namespace sloth {
 
-// Triangles per block.  A block builds a tree of its chunk in shared memory (2n nodes) and
+// Triangles per block of the newline kernel.  A block builds a tree of its chunk in shared memory (2n nodes) and
 // merges the nodes it touched into the frame's tree.
 constexpr uint32_t kNewlineChunk = 8192;
+// The same for a newline part of a fill or fold, whose blocks have a quarter of the threads:
+// the part must not outlast the rest of its launch, and in blocks of 8192 it did (us a frame of
+// a soup, 8192 / 2048 / 1024 / 512 a block: 8k triangles at 3840x1426 152 / 112 / 107 / 102,
+// 96k there 204 / 163 / 156 / 153, 96k at 1280x720 148 / 118 / 112 / 112).
+constexpr uint32_t kNewlineFillChunk = 1024;
 // The largest tree, in bytes, that a fill or fold kernel takes into its own blocks as one of
 // its parts: every block of the launch holds that much shared memory, and at 32 KB (frames
 // of up to 4096 rows) six still fit an SM.  Taller frames launch the newline kernel, and so
 // do more triangles than kNewlinePartTriangles: beside the rest on a stream of its own it
 // fills the raster's gaps too (a million triangles: 17 us as a part of the fill, none
-// there), which for a few blocks is not worth the fork and the join.
+// there), which for fewer is not worth the fork and the join.
 constexpr size_t kNewlinePartBytes = 32 * 1024;
 constexpr uint32_t kNewlinePartTriangles = 1u << 17;
 // The largest tree the newline kernel holds in shared memory; above it the frame's tree is
