@@ -148,8 +148,8 @@ sloth_status sloth_ctx_synchronize(sloth_ctx *ctx);
 sloth_status sloth_ctx_device_buffers(sloth_ctx *ctx, const uint32_t **cells, const float **z);
 
 /* Covered samples (all three edge functions >= 0, src/rasterizer.rs:75) since the last
- * clear, counted by the raster kernels over the triangles they evaluated: every covered
- * sample when SLOTH_OPTION_DEPTH_CULL is 0.  Blocks until pending work completes. */
+ * clear, counted by the raster kernels over what depth culling left (triangles, or samples
+ * where a draw goes without tiles): every covered sample when SLOTH_OPTION_DEPTH_CULL is 0.  Blocks until pending work completes. */
 sloth_status sloth_ctx_fragments(sloth_ctx *ctx, uint64_t *fragments);
 
 /* The bytes Context::flush(color, webify) prints for the frame (src/context.rs:50-92),

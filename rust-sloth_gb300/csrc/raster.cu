@@ -18,12 +18,12 @@ __device__ __noinline__ void overflow_fold(uint32_t tri_base, const FrameGeom &g
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     uint32_t frags = 0;
     const uint32_t n = bb.large_count[2];
-    for (uint32_t i = warp; i < n; i += nwarps) frags += fold_queued<32, 1>(bb.fill_list[i].x, 0u, 1u, true, g, fb);
+    for (uint32_t i = warp; i < n; i += nwarps) frags += fold_queued<32, false, 1>(bb.fill_list[i].x, 0u, 1u, true, g, fb);
     constexpr uint32_t kParts = 64;
     const uint32_t front = bb.large_count[0], all = front + bb.large_count[1];
     for (uint32_t i = warp; i < all * kParts; i += nwarps) {
         const uint32_t k = i / kParts, q = k < front ? k : bb.large_cap - 1u - (k - front);
-        frags += fold_queued<kFoldRows, 1>(tri_base + bb.large_queue[q], i % kParts, kParts, true, g, fb);
+        frags += fold_queued<kFoldRows, false, 1>(tri_base + bb.large_queue[q], i % kParts, kParts, true, g, fb);
     }
     add_frags_warp(frags, fb.fragments);
 }

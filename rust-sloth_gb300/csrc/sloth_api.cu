@@ -1024,20 +1024,26 @@ static sloth_status poll_entry_max(sloth_ctx *ctx)
     return SLOTH_OK;
 }
 
-// Whether a draw goes without tiles (fold.cuh).  The samples it will walk are estimated
+// Whether a draw goes without tiles (fold.cuh).  The samples it will walk (est) are estimated
 // from the mesh's edges as it was made and the matrix's scale; a mesh of no extent says
-// nothing.  Up to kFoldMaxSamples the tile raster's launches cost more than its culling
-// saves (us a frame, tiles / fold: 960 triangles at 160x48, 3e4 samples, 68 / 14; 82k at
-// 640x360, 8e5, 84 / 28; 5k at 1920x1080, 7e6, 78 / 32; 8k with 16 large ones at 1920x1080,
-// 1.5e7, 88 / 75; 8k at 1920x1080, 1e8, 111 / 127; at 640x360 the fold stays ahead up to
-// 1.5e8).  Above kFoldMaxTriangles the estimate is not trusted with the whole draw
+// nothing.  The fold takes about 14 us + 0.3 us per million samples; the tile raster 40 us of
+// launches, 0.2 us more per thousand triangles than the fold, and, as its lists grow with
+// them, 0.12 us per sample a cell gets (deep), but next to nothing per sample, which it
+// culls.  Hence the line; us a frame on both sides of it, tiles / fold: 500 triangles at
+// 1921x1079, est 4e5, 44 / 26; 8k at 1921x1079, 1.4e7, 68 / 55; 82k at 640x360, 8e5, 59 / 16;
+// 96k at 640x360, 1.2e8, deep 510, 285 / 110; 20k at 3840x2160, 2.9e7, 118 / 73; 64k at
+// 3840x1426, 1e8, 121 / 97 (tiles kept); 8k at 1921x1079, 1.2e8, 82 / 91; 32k at 1921x1079,
+// 4.1e8, 94 / 170.
+// Above kFoldMaxTriangles the estimate is not trusted with the whole draw
 // (positions may have been updated since), and the tiles bound what a wrong one costs.
 // With culling off a caller counts or compares the tile raster's fragments, and the wait
 // test needs its tile loads: both keep it.
 static bool draws_without_tiles(const sloth_ctx *ctx, const sloth_mesh *mesh, const Mat4 &M)
 {
     if (!ctx->depth_cull || ctx->fb.wait_test || mesh->ntri > kFoldMaxTriangles || !(mesh->span2 > 0.0f)) return false;
-    return fold_estimate(mesh->span2, mesh->ntri, M, ctx->g.w, ctx->g.h) <= kFoldMaxSamples;   // false for NaN
+    const float est = fold_estimate(mesh->span2, mesh->ntri, M, ctx->g.w, ctx->g.h);
+    const float deep = std::fmin(est / ((float)ctx->g.w * (float)ctx->g.h), 2000.0f);
+    return est <= 3e7f + 400.0f * (float)mesh->ntri + 2e5f * deep;   // false for NaN
 }
 
 // One draw without tiles: every tile's keys made current and the queue counters emptied first

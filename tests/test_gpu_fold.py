@@ -62,8 +62,8 @@ def test_noalloc_hostile(seed, w, h, image):
 @pytest.mark.parametrize("w,h,image", [(160, 48, True), (161, 47, False)])
 def test_context_mixes_fold_and_tiles(w, h, image):
     """Draws of one frame with and without tiles, in both orders, over frames and a resize:
-    each keeps the keys of the ones before it.  A draw goes without tiles by its estimated
-    samples, so the big soup (its triangles cover the frame) takes the tiles."""
+    each keeps the keys of the ones before it.  The big soup (its triangles cover the frame) is
+    drawn with culling off, which keeps the tiles whatever its size."""
     small, ico = W.soup(100, seed=3, sigma=0.05), W.displaced_icosphere(2, seed=5)
     big = W.soup(6000, seed=4, n_large=400, sigma=0.8)
     R = O.euler_rotation(*W.cli_rotation(yaw=0.6, pitch=0.2))
@@ -78,6 +78,7 @@ def test_context_mixes_fold_and_tiles(w, h, image):
             c.set_utransform(U)
             c.clear()
             for m, Rm in zip(order, Rs):
+                c.set_depth_cull(m is not big)
                 c.draw_mesh(dev[id(m)], Rm)
             check([a.view(np.int32) if a.dtype == np.float32 else a for a in c.read()],
                   oracle_render(list(order), Rs, ww, hh, image, U=U), f"mix {k} {ww}x{hh}")
@@ -112,7 +113,8 @@ def test_context_fold_queue_classes(side):
 @pytest.mark.parametrize("direct", [4, 16, 64])
 def test_context_fold_after_direct_draw(direct):
     """A fresh context whose first draw is binned with direct samples on: that draw makes the
-    tiles' keys current, and the folds after it still start from empty queue counters."""
+    tiles' keys current, and the folds after it still start from empty queue counters.  (With
+    culling off a draw keeps the tiles whatever its size.)"""
     w, h = 161, 47
     big, ico = W.soup(6000, seed=4, n_large=400, sigma=0.8), W.displaced_icosphere(2, seed=5)
     R = O.euler_rotation(*W.cli_rotation(yaw=0.6, pitch=0.2))
@@ -126,6 +128,7 @@ def test_context_fold_after_direct_draw(direct):
             Rs = [R * np.float32(40.0) if m is big else R for m in order]
             c.clear()
             for m, Rm in zip(order, Rs):
+                c.set_depth_cull(m is not big)
                 c.draw_mesh(dev[id(m)], Rm)
             check([a.view(np.int32) if a.dtype == np.float32 else a for a in c.read()],
                   oracle_render(list(order), Rs, w, h, False, U=U), f"frame {k}")
