@@ -17,7 +17,7 @@
 //   (free)    kMaxTri x 4 B           unused, as are the tile counts below: the header states
 //                                     the array's size
 //   keys      kMaxCells x 8 B         depth keys (tiles padded to 64x32 cells)
-//   queue     kMaxTri x 4 B + 16 B    triangles too large for their block, and their counters
+//   queue     kMaxTri x 4 B + 24 B    triangles too large for their block, and their counters
 //   tile_gen  kMaxTiles x 4 B         tile generations (cleared every call)
 //   nltree    2*kMaxNl x 4 B          newline segment tree (cleared every call)
 //   frags     8 B                     fragment counter (cleared every call)
@@ -42,7 +42,7 @@ constexpr size_t kOffOffset = align256(kOffCount + (size_t)kMaxTiles * 4);
 constexpr size_t kOffCursor = align256(kOffOffset + ((size_t)kMaxTiles + 1) * 4);
 constexpr size_t kOffQueue = align256(kOffCursor + (size_t)kMaxTiles * 4);
 constexpr size_t kOffQCount = align256(kOffQueue + (size_t)kMaxTri * 4);
-constexpr size_t kOffGen = align256(kOffQCount + 16);
+constexpr size_t kOffGen = align256(kOffQCount + 2 * kFoldSlots * 4);
 constexpr size_t kOffNl = align256(kOffGen + (size_t)kMaxTiles * 4);
 constexpr size_t kOffFrags = align256(kOffNl + 2 * (size_t)kMaxNl * 4);
 constexpr size_t kScratchBytes = align256(kOffFrags + 8);
@@ -123,8 +123,8 @@ extern "C" sloth_status sloth_render_noalloc(const float *x, const float *y, con
     Mat4 M;
     for (int i = 0; i < 16; ++i) M.m[i] = m[i];
     const MeshDev md{x, y, z, nullptr, rgb, 3 * ntri, ntri};
-    if (ntri && (launch_fold_setup(md, M, 0, g, fb, queue, kMaxTri, queue_counts, 0, s) != cudaSuccess ||
-                 launch_fold_large(g, fb, queue, kMaxTri, queue_counts, 0, s) != cudaSuccess))
+    if (ntri && (launch_fold_setup(md, M, 0, g, fb, queue, 2 * kMaxTri, queue_counts, 0, false, s) != cudaSuccess ||
+                 launch_fold_large(g, fb, queue, 2 * kMaxTri, queue_counts, 0, s) != cudaSuccess))
         return SLOTH_ERR_CUDA;
     if (launch_resolve(g, fb, s) != cudaSuccess) return SLOTH_ERR_CUDA;
     return SLOTH_OK;

@@ -51,6 +51,7 @@ struct sloth_mesh {
     uint32_t nvert = 0, ntri = 0;
     float bbox_max[3] = {0, 0, 0};
     uint32_t *order = nullptr, *oidx = nullptr;   // setup's order of an indexed mesh (spatial_order)
+    bool updated = false;   // positions may change on the stream (sloth_mesh_update*)
     float span2 = 0.0f;   // sum over the triangles of their longest edge squared, when made (mesh_span2)
 };
 
@@ -96,7 +97,8 @@ struct sloth_ctx {
     bool keys_current = false;     // every tile's keys cleared for the current generation
     uint32_t *fold_counts = nullptr;   // queue counters of the draws without tiles (launch_fold_setup)
     bool fold_begun = false;           // they were emptied in this frame
-    int fold_parity = 0;               // the counter the frame's next such draw uses
+    uint32_t fold_draws = 0;           // such draws of the frame so far
+    uint64_t fold_last = ~0ull;        // `launches` after the last one's, in its frame
     bool timing = false;
     std::map<std::string, KernelClock> clocks;
     uint64_t launches = 0;
@@ -601,6 +603,7 @@ sloth_status sloth_ctx_clear(sloth_ctx *ctx)
     ctx->g.direct_max = ctx->direct_max;
     ctx->keys_current = false;
     ctx->fold_begun = false;
+    ctx->fold_last = ~0ull;
     return SLOTH_OK;
 }
 
@@ -977,6 +980,7 @@ sloth_status sloth_mesh_update(sloth_mesh *m, const float *x, const float *y, co
     if (m->nvert && (!x || !y || !z)) return fail(ctx, SLOTH_ERR_INVALID_ARGUMENT, "vertex arrays are NULL");
     if (m->ntri && !rgb) return fail(ctx, SLOTH_ERR_INVALID_ARGUMENT, "rgb is NULL");
     CU(ctx, cudaSetDevice(m->device));
+    m->updated = true;
     const size_t nb = (size_t)m->nvert * sizeof(float);
     if (m->nvert) {
         CU(ctx, cudaMemcpyAsync(m->x, x, nb, cudaMemcpyDefault, ctx->stream));
@@ -993,6 +997,7 @@ sloth_status sloth_mesh_update_interleaved(sloth_mesh *m, const float *xyz, cons
     sloth_ctx *ctx = m->ctx;
     if ((m->nvert && !xyz) || (m->ntri && !rgb)) return fail(ctx, SLOTH_ERR_INVALID_ARGUMENT, "xyz or rgb is NULL");
     CU(ctx, cudaSetDevice(m->device));
+    m->updated = true;
     CU(ctx, launch_mesh_split(xyz, rgb, m->x, m->y, m->z, m->rgb, m->nvert, m->ntri, ctx->stream));
     return SLOTH_OK;
 }
@@ -1052,7 +1057,7 @@ static sloth_status draw_folded(sloth_ctx *ctx, const sloth_mesh *mesh, const Ma
 {
     sloth_status st;
     cudaStream_t s = ctx->stream;
-    if (!ctx->fold_counts) CU(ctx, dalloc(&ctx->fold_counts, 4));
+    if (!ctx->fold_counts) CU(ctx, dalloc(&ctx->fold_counts, 2 * kFoldSlots));
     if (ctx->reset_pending || !ctx->keys_current || !ctx->fold_begun) {
         if ((st = join_newline(ctx)) != SLOTH_OK) return st;   // the last frame's fold into the tree
         const bool frame = ctx->reset_pending;
@@ -1062,19 +1067,21 @@ static sloth_status draw_folded(sloth_ctx *ctx, const sloth_mesh *mesh, const Ma
         ctx->reset_pending = false;
         ctx->keys_current = true;
         ctx->fold_begun = true;
-        ctx->fold_parity = 0;
+        ctx->fold_draws = 0;
     }
     const MeshDev md{mesh->x, mesh->y, mesh->z, mesh->idx, mesh->rgb, mesh->nvert, mesh->ntri, mesh->order, mesh->oidx};
-    const int parity = ctx->fold_parity;
-    const uint32_t cap = (uint32_t)std::min<size_t>(ctx->large_cap, 0x7fffffffu);
+    const uint32_t draw = ctx->fold_draws, cap = (uint32_t)std::min<size_t>(ctx->large_cap, 0x7fffffffu);
+    // nothing of this context since the last such draw, and no kernel that writes the mesh
+    const bool beside = ctx->launches == ctx->fold_last && !mesh->updated && !ctx->timing;
     CU(ctx, timed(ctx, "fold", [&] {
-           return launch_fold_setup(md, M, ctx->tri_base, ctx->g, ctx->fb, ctx->bb.large_queue, cap, ctx->fold_counts, parity,
-                                    s);
+           return launch_fold_setup(md, M, ctx->tri_base, ctx->g, ctx->fb, ctx->bb.large_queue, cap, ctx->fold_counts, draw,
+                                    beside, s);
        }));
     CU(ctx, timed(ctx, "fold_large", [&] {
-           return launch_fold_large(ctx->g, ctx->fb, ctx->bb.large_queue, cap, ctx->fold_counts, parity, s);
+           return launch_fold_large(ctx->g, ctx->fb, ctx->bb.large_queue, cap, ctx->fold_counts, draw, s);
        }));
-    ctx->fold_parity ^= 1;
+    ctx->fold_draws++;
+    ctx->fold_last = ctx->launches;
     ctx->tri_base += mesh->ntri;
     ctx->dirty = true;
     return SLOTH_OK;
@@ -1095,7 +1102,8 @@ sloth_status sloth_draw_mesh(sloth_ctx *ctx, const sloth_mesh *mesh, const float
     sloth_mat4_mul(ctx->U, transform, M.m);
     if (draws_without_tiles(ctx, mesh, M)) {
         if ((st = ensure_records(ctx, (size_t)ctx->tri_base + mesh->ntri)) != SLOTH_OK) return st;
-        if ((st = ensure_scratch(ctx, &ctx->bb.large_queue, &ctx->large_cap, mesh->ntri)) != SLOTH_OK) return st;
+        if ((st = ensure_scratch(ctx, &ctx->bb.large_queue, &ctx->large_cap, 2 * (size_t)mesh->ntri)) != SLOTH_OK)
+            return st;
         return draw_folded(ctx, mesh, M);
     }
     if ((st = poll_entry_max(ctx)) != SLOTH_OK) return st;

@@ -215,16 +215,18 @@ inline float fold_estimate(float span2, uint32_t ntri, const Mat4 &M, int w, int
 // Drawing without tiles (fold.cuh).  launch_fold_begin: the keys of tiles that are not
 // current (all: of every tile) emptied and the tiles made current; with frame, the resets
 // of a clear.  launch_fold_setup: one draw's setup and the folds of its small triangles;
-// launch_fold_large: the walk of the triangles it queued.  queue holds cap >= mesh.ntri
-// entries and queue_counts two pairs of counters, used in turn by a frame's draws (parity 0,
-// 1, 0, ...).
+// launch_fold_large: the walk of the triangles it queued.  queue holds cap >= 2 * mesh.ntri
+// entries, half of them for every other draw of a frame (draw 0, 1, 2, ...), and queue_counts
+// kFoldSlots pairs of counters, used in turn; beside: the setup need not wait for the walk
+// launched just before it (fold_setup_kernel).
+constexpr uint32_t kFoldSlots = 3;
 cudaError_t launch_fold_begin(const FrameGeom &g, const FrameBuffers &fb, bool frame, bool all,
                               uint32_t *queue_counts, cudaStream_t s);
 cudaError_t launch_fold_setup(const MeshDev &mesh, const Mat4 &M, uint32_t tri_base, const FrameGeom &g,
                               const FrameBuffers &fb, uint32_t *queue, uint32_t cap, uint32_t *queue_counts,
-                              int parity, cudaStream_t s);
+                              uint32_t draw, bool beside, cudaStream_t s);
 cudaError_t launch_fold_large(const FrameGeom &g, const FrameBuffers &fb, uint32_t *queue, uint32_t cap,
-                              uint32_t *queue_counts, int parity, cudaStream_t s);
+                              uint32_t *queue_counts, uint32_t draw, cudaStream_t s);
 
 // per-tile raster: 64-bit atomicMin of depth keys in shared memory, merged into keys.  A
 // draw whose tile entries outgrew the entry buffer (the scan total is above the capacity;

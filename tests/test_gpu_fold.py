@@ -132,3 +132,40 @@ def test_context_fold_after_direct_draw(direct):
                 c.draw_mesh(dev[id(m)], Rm)
             check([a.view(np.int32) if a.dtype == np.float32 else a for a in c.read()],
                   oracle_render(list(order), Rs, w, h, False, U=U), f"frame {k}")
+
+
+def moved(m):
+    return dict(m, x=(m["x"] * np.float32(0.8) + np.float32(0.1)).astype(np.float32))
+
+
+@pytest.mark.parametrize("w,h,image", [(320, 200, True), (161, 95, False)])
+def test_context_fold_draws_in_a_row(w, h, image):
+    """Many folded draws in one frame: each one's setup runs beside the walk of the queue
+    before, in three sets of counters and two halves of a queue that grows on the way; a mesh
+    updated between its draws, and two contexts that draw in turn on one stream."""
+    ms = [W.soup(40 + 90 * k * k, seed=k, n_large=3 * k, sigma=0.01 + 0.05 * (k % 3)) for k in range(7)]
+    ms += [W.displaced_icosphere(3, seed=9)]
+    R = O.euler_rotation(*W.cli_rotation(yaw=0.6, pitch=0.2))
+    U = O.viewport_transform(w, h, O.scene_extent([m["bbox_max"] for m in ms]))
+    stream = torch.cuda.Stream()
+    with S.Context(0, stream=stream.cuda_stream) as a, S.Context(0, stream=stream.cuda_stream) as b:
+        dev = [S.Mesh(a, m["x"], m["y"], m["z"], m["rgb"], m["idx"], m["bbox_max"]) for m in ms]
+        for c in (a, b):
+            c.set_viewport(w, h, image)
+            c.set_utransform(U)
+        for frame in range(3):
+            drawn = {a: [], b: []}
+            a.clear()
+            b.clear()
+            for k in range(2 * len(ms)):
+                i = (5 * k + frame) % len(ms)
+                for c in (a, b) if k % 3 == 0 else (a,):
+                    c.draw_mesh(dev[i], R)
+                    drawn[c].append(ms[i])
+                if k == 9:
+                    i = (5 * (k + 1) + frame) % len(ms)
+                    ms[i] = moved(ms[i])
+                    dev[i].update(ms[i]["x"], ms[i]["y"], ms[i]["z"], ms[i]["rgb"])
+            for c in (a, b):
+                check([v.view(np.int32) if v.dtype == np.float32 else v for v in c.read()],
+                      oracle_render(drawn[c], R, w, h, image, U=U), f"frame {frame} {w}x{h}")
