@@ -413,7 +413,7 @@ __device__ __noinline__ void batch_overflow_fold(const BatchDev &b)
     for (uint32_t i = warp; i < all * kParts; i += nwarps) {
         const uint32_t k = i / kParts, q = k < front ? k : b.bb.large_cap - 1u - (k - front);
         const BatchFrame &f = b.frames[b.large_frame[q]];
-        frags += fold_queued<kFoldRows, false, 1>(b.bb.large_queue[q], i % kParts, kParts, true, f.g, f.fb);
+        frags += fold_queued<8, false, 1>(b.bb.large_queue[q], i % kParts, kParts, true, f.g, f.fb);
     }
     add_frags_warp(frags, b.frames[0].fb.fragments);
 }

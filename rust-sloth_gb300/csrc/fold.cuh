@@ -6,7 +6,7 @@
 // launches that each wait for the one before.  A draw of a few thousand triangles over few
 // samples is all launches.  Here it takes two: fold_triangles sets up 32 triangles per
 // block and walks their samples (direct.cuh) with every warp of the block, and queues the
-// triangles of more than kFoldQueueSamples samples; fold_large_part walks those with the
+// triangles of more than kFoldBlockSamples samples; fold_queue_walk walks those with the
 // warps of the whole GPU.  The minimum of a cell's keys does not depend on the order of
 // the folds, so the frame is the tile raster's bit for bit.  The newline rows go straight
 // into the frame's segment tree, whose nodes are maxima.
@@ -24,16 +24,20 @@ constexpr int kFoldTris = 32;
 // Triangles of more samples than this (rows times walked columns) are queued: the block
 // that set one up would walk it alone while the rest of the GPU is idle.
 constexpr uint32_t kFoldBlockSamples = 128;
-// A queued triangle is cut into items of every parts-th group of kFoldRows rows: kFoldParts
-// items for the large ones (one group each up to 1024 rows), kFoldMidParts for those of at
-// most kFoldWarpSamples samples, or, when there are enough of them for a warp each, one item
+// A queued triangle is cut into items of every parts-th group of rows: kFoldParts groups of
+// kFoldRows for the large ones (one group each up to 1024 rows), kFoldMidParts of kFoldMidRows
+// for those of at most kFoldWarpSamples samples, or, when there is one for every warp, one item
 // of all their rows, 32 at a time.  Items are numbered part after part and a warp's lanes
 // look at 32 of them at once, so the items past a triangle's last row cost next to nothing.
+// The walk is as long as its longest item, so a large one's groups are small, where the others'
+// would only be more items (rows of a group, large / other: 8 / 8, 4 / 4, 2 / 4, 2 / 8; us a
+// frame of 16 models at 1280x720 205, 182, 171, 163; of 10 of 5k at 1149x567 180, 180, 181,
+// 159; of 20k triangles at 640x360 27.8, 24.9, 23.5, 23.3).
 // A warp walks kFoldUnroll steps of 32 samples at once: the row searches, edge values and
 // key loads of a step are one chain, and the walk waits on its latency.
 constexpr uint32_t kFoldWarpSamples = 4096;
-constexpr int kFoldRows = 8;
-constexpr uint32_t kFoldParts = 128, kFoldMidParts = 8;
+constexpr int kFoldRows = 2, kFoldMidRows = 8;
+constexpr uint32_t kFoldParts = 512, kFoldMidParts = 8;
 constexpr int kFoldUnroll = 4;
 
 // With more queued triangles than this, cells that already hold a nearer key are left out
@@ -302,7 +306,7 @@ __device__ __forceinline__ uint32_t fold_queue_walk(const FoldQueue &queue, uint
 {
     const int lane = threadIdx.x & 31;
     const uint32_t large = queue.count[0], mid = queue.count[1];
-    const bool whole = mid > nwarps / 2;   // a warp for each of the smaller ones
+    const bool whole = mid > nwarps;   // a warp for each of the smaller ones
     const uint32_t cut = large * kFoldParts, items = cut + mid * (whole ? 1u : kFoldMidParts);
     const bool filter = large + mid > kFoldFilterMin;
     uint32_t frags = 0;
@@ -321,7 +325,7 @@ __device__ __forceinline__ uint32_t fold_queue_walk(const FoldQueue &queue, uint
             }
             tri = queue.tri[q];
             const int4 xr = *(reinterpret_cast<const int4 *>(frame_of(q).fb.records + tri) + 4);
-            live = xr.z + (int)part * kFoldRows < xr.w;
+            live = xr.z + (int)part * (it < cut ? kFoldRows : kFoldMidRows) < xr.w;
         }
         for (unsigned todo = __ballot_sync(0xffffffffu, live); todo; todo &= todo - 1u) {
             const int src = __ffs(todo) - 1;
@@ -329,7 +333,7 @@ __device__ __forceinline__ uint32_t fold_queue_walk(const FoldQueue &queue, uint
                            wp = __shfl_sync(0xffffffffu, part, src), wi = __shfl_sync(0xffffffffu, it, src);
             const auto &f = frame_of(wq);
             if (wi < cut) frags += fold_queued<kFoldRows>(wt, wp, kFoldParts, filter, f.g, f.fb);
-            else if (!whole) frags += fold_queued<kFoldRows>(wt, wp, kFoldMidParts, filter, f.g, f.fb);
+            else if (!whole) frags += fold_queued<kFoldMidRows>(wt, wp, kFoldMidParts, filter, f.g, f.fb);
             else frags += fold_queued<32>(wt, 0u, 1u, filter, f.g, f.fb);
         }
     }

@@ -23,7 +23,7 @@ __device__ __noinline__ void overflow_fold(uint32_t tri_base, const FrameGeom &g
     const uint32_t front = bb.large_count[0], all = front + bb.large_count[1];
     for (uint32_t i = warp; i < all * kParts; i += nwarps) {
         const uint32_t k = i / kParts, q = k < front ? k : bb.large_cap - 1u - (k - front);
-        frags += fold_queued<kFoldRows, false, 1>(tri_base + bb.large_queue[q], i % kParts, kParts, true, g, fb);
+        frags += fold_queued<8, false, 1>(tri_base + bb.large_queue[q], i % kParts, kParts, true, g, fb);
     }
     add_frags_warp(frags, fb.fragments);
 }
