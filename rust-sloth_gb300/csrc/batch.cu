@@ -313,23 +313,20 @@ __device__ __forceinline__ uint32_t frame_of_tile(const BatchDev &b, uint32_t ti
 __device__ __forceinline__ void batch_tile_items(const BatchDev &b, uint32_t t)
 {
     const uint32_t nt = b.total_tiles;
+    const bool live = t < nt, outgrew = b.bb.tile_offset[nt] > b.bb.capacity;
     const SplitParams sp{b.bb.slice_offset[nt + 1], b.bb.slice_offset[nt + 2]};
-    const uint32_t cnt = b.bb.tile_count[t], ns = tile_slices(cnt, sp);
-    const bool split = cnt > sp.threshold, outgrew = b.bb.tile_offset[nt] > b.bb.capacity;
-    const uint32_t off = item_offset(b.bb.slice_offset, nt, t, cnt, sp.threshold);
-    for (uint32_t k = 0; k < ns && off + k < b.bb.item_capacity; ++k) b.bb.items[off + k] = make_uint2(t, k);
-    if (split || outgrew) {
-        const BatchFrame &f = b.frames[frame_of_tile(b, t)];
-        const uint32_t lt = t - f.tile_off;
-        if (f.fb.tile_gen[lt] != f.fb.gen) {
-            const int tr = (int)lt / f.g.ntx, tc = (int)lt - tr * f.g.ntx;
-            unsigned long long *k0 = reinterpret_cast<unsigned long long *>(f.fb.keys) +
-                                     (size_t)tr * f.g.th * f.g.pitch + (size_t)tc * f.g.tw;
-            for (int r = 0; r < f.g.th; ++r)
-                for (int c = 0; c < live_keys_per_row(f.g.w, f.g.tw); ++c) k0[(size_t)r * f.g.pitch + c] = kEmptyKey;
-            f.fb.tile_gen[lt] = f.fb.gen;
-        }
+    const uint32_t cnt = live ? b.bb.tile_count[t] : 0u;
+    if (live) {
+        const uint32_t ns = tile_slices(cnt, sp), off = item_offset(b.bb.slice_offset, nt, t, cnt, sp.threshold);
+        for (uint32_t k = 0; k < ns && off + k < b.bb.item_capacity; ++k) b.bb.items[off + k] = make_uint2(t, k);
     }
+    bool empty = live && (cnt > sp.threshold || outgrew);
+    const BatchFrame &f = b.frames[empty ? frame_of_tile(b, t) : 0u];
+    const uint32_t lt = t - f.tile_off;
+    empty = empty && f.fb.tile_gen[lt] != f.fb.gen;
+    const int tr = (int)lt / f.g.ntx, tc = (int)lt - tr * f.g.ntx;
+    empty_tiles_warp(empty, f.fb.keys + (size_t)tr * f.g.th * f.g.pitch + (size_t)tc * f.g.tw, f.g);
+    if (empty) f.fb.tile_gen[lt] = f.fb.gen;
 }
 
 // A fill's blocks, part after part (bin_fill_kernel): newline chunks, large triangles, tiles'
@@ -357,7 +354,7 @@ batch_fill_kernel(BatchDev b, const int2 *__restrict__ nl, BatchFillParts parts)
     if (blk < parts.items) {
         const uint32_t t = blk * blockDim.x + threadIdx.x;
         if (t == 0) *b.queue = 0u;   // the persistent raster's item counter
-        if (t < b.total_tiles) batch_tile_items(b, t);
+        batch_tile_items(b, t);
         return;
     }
     blk -= parts.items;

@@ -229,30 +229,17 @@ __global__ void __launch_bounds__(1024) bin_scan_kernel(uint32_t n, BinBuffers b
 __device__ __forceinline__ void bin_tile_items(uint32_t t, uint32_t n, const FrameGeom &g, const FrameBuffers &fb,
                                                const BinBuffers &bb)
 {
-    if (bb.tile_offset[n] > bb.capacity) {
-        if (fb.tile_gen[t] != fb.gen) {
-            const int tr = (int)t / g.ntx, tc = (int)t - tr * g.ntx;
-            unsigned long long *k0 = reinterpret_cast<unsigned long long *>(fb.keys) +
-                                     (size_t)tr * g.th * g.pitch + (size_t)tc * g.tw;
-            for (int r = 0; r < g.th; ++r)
-                for (int c = 0; c < live_keys_per_row(g.w, g.tw); ++c) k0[(size_t)r * g.pitch + c] = kEmptyKey;
-            fb.tile_gen[t] = fb.gen;
-        }
-        return;
-    }
+    const bool live = t < n, outgrew = bb.tile_offset[n] > bb.capacity;
     const SplitParams sp = split_params(bb, n);
-    const uint32_t cnt = bb.tile_count[t], ns = tile_slices(cnt, sp);
-    const bool split = cnt > sp.threshold;
-    const uint32_t off = item_offset(bb.slice_offset, n, t, cnt, sp.threshold);
-    for (uint32_t k = 0; k < ns && off + k < bb.item_capacity; ++k) bb.items[off + k] = make_uint2(t, k);
-    if (split && fb.tile_gen[t] != fb.gen) {
-        const int tr = (int)t / g.ntx, tc = (int)t - tr * g.ntx;
-        unsigned long long *k0 = reinterpret_cast<unsigned long long *>(fb.keys) + (size_t)tr * g.th * g.pitch +
-                                 (size_t)tc * g.tw;
-        for (int r = 0; r < g.th; ++r)
-            for (int c = 0; c < live_keys_per_row(g.w, g.tw); ++c) k0[(size_t)r * g.pitch + c] = kEmptyKey;
-        fb.tile_gen[t] = fb.gen;
+    const uint32_t cnt = live ? bb.tile_count[t] : 0u;
+    if (live && !outgrew) {
+        const uint32_t ns = tile_slices(cnt, sp), off = item_offset(bb.slice_offset, n, t, cnt, sp.threshold);
+        for (uint32_t k = 0; k < ns && off + k < bb.item_capacity; ++k) bb.items[off + k] = make_uint2(t, k);
     }
+    const bool empty = live && (outgrew || cnt > sp.threshold) && fb.tile_gen[t] != fb.gen;
+    const int tr = (int)t / g.ntx, tc = (int)t - tr * g.ntx;
+    empty_tiles_warp(empty, fb.keys + (size_t)tr * g.th * g.pitch + (size_t)tc * g.tw, g);
+    if (empty) fb.tile_gen[t] = fb.gen;
 }
 
 // A fill's blocks, part after part: newline chunks, large triangles, tiles' raster items,
@@ -284,8 +271,7 @@ bin_fill_kernel(uint32_t ntri, const uint32_t *__restrict__ order, uint32_t tri_
     }
     blk -= parts.large;
     if (blk < parts.items) {
-        const uint32_t t = blk * blockDim.x + threadIdx.x;
-        if (t < ntiles) bin_tile_items(t, ntiles, g, fb, bb);
+        bin_tile_items(blk * blockDim.x + threadIdx.x, ntiles, g, fb, bb);
         return;
     }
     blk -= parts.items;
