@@ -1038,16 +1038,26 @@ static sloth_status poll_entry_max(sloth_ctx *ctx)
 // 1921x1079, est 4e5, 44 / 26; 8k at 1921x1079, 1.4e7, 68 / 55; 82k at 640x360, 8e5, 59 / 16;
 // 96k at 640x360, 1.2e8, deep 510, 285 / 110; 20k at 3840x2160, 2.9e7, 118 / 73; 64k at
 // 3840x1426, 1e8, 121 / 97 (tiles kept); 8k at 1921x1079, 1.2e8, 82 / 91; 32k at 1921x1079,
-// 4.1e8, 94 / 170.
-// Above kFoldMaxTriangles the estimate is not trusted with the whole draw
-// (positions may have been updated since), and the tiles bound what a wrong one costs.
+// 4.1e8, 94 / 170; 262k at 525x371, 3.8e7, 325 / 52; 200k at 1921x1079, 3.7e8, 139 / 190;
+// 500k at 1280x720, 1.6e8, 243 / 222; 1M there, 8.5e8, 466 / 596.  Above kFoldMaxTriangles
+// only for positions as they were made: the estimate of updated ones may be wrong, and the
+// tiles bound what that costs.  There the cells must not be too few for the triangles either,
+// whose reductions then queue at the same keys (200k at 160x48, 26 a cell, 62 / 55; 262k
+// there, 34, 56 / 70; 1M, 87 / 244); with direct samples on, the tile raster's setup folds the
+// small ones itself (500k fine ones at 1280x720 69 / 89); and the newline rows of a soup in no
+// order queue at the frame's tree (340k at 825x301 with direct samples 177 / 228).
 // With culling off a caller counts or compares the tile raster's fragments, and the wait
 // test needs its tile loads: both keep it.
 static bool draws_without_tiles(const sloth_ctx *ctx, const sloth_mesh *mesh, const Mat4 &M)
 {
-    if (!ctx->depth_cull || ctx->fb.wait_test || mesh->ntri > kFoldMaxTriangles || !(mesh->span2 > 0.0f)) return false;
+    if (!ctx->depth_cull || ctx->fb.wait_test || !(mesh->span2 > 0.0f)) return false;
+    const float cells = (float)ctx->g.w * (float)ctx->g.h;
+    if (mesh->ntri > kFoldMaxTriangles &&
+        (mesh->updated || mesh->ntri > kFoldMaxTrianglesMade || (float)mesh->ntri > 26.0f * cells ||
+         ctx->g.direct_max > 0 || (ctx->g.image && !mesh->order)))
+        return false;
     const float est = fold_estimate(mesh->span2, mesh->ntri, M, ctx->g.w, ctx->g.h);
-    const float deep = std::fmin(est / ((float)ctx->g.w * (float)ctx->g.h), 2000.0f);
+    const float deep = std::fmin(est / cells, 2000.0f);
     return est <= 3e7f + 400.0f * (float)mesh->ntri + 2e5f * deep;   // false for NaN
 }
 

@@ -202,6 +202,7 @@ cudaError_t launch_bin_fill(uint32_t ntri, const uint32_t *order, uint32_t tri_b
 // the scale of the matrix's x and y rows, at most every cell for every triangle.  Where the
 // lines lie is with the dispatch (draws_without_tiles, batch_folds).
 constexpr uint32_t kFoldMaxTriangles = 131072;
+constexpr uint32_t kFoldMaxTrianglesMade = 1u << 20;   // a context's mesh with the positions it was made with
 constexpr float kFoldMaxSamples = 16777216.0f;   // a batch's frame
 inline float fold_estimate(float span2, uint32_t ntri, const Mat4 &M, int w, int h)
 {

@@ -169,3 +169,23 @@ def test_context_fold_draws_in_a_row(w, h, image):
             for c in (a, b):
                 check([v.view(np.int32) if v.dtype == np.float32 else v for v in c.read()],
                       oracle_render(drawn[c], R, w, h, image, U=U), f"frame {frame} {w}x{h}")
+
+
+def test_context_fold_many_triangles():
+    """More triangles than an updated mesh folds: the mesh as it was made folds, the same mesh
+    after an update takes the tiles, and both frames are the oracle's."""
+    m = W.soup(131100, seed=11, n_large=3, sigma=0.01)
+    R = O.euler_rotation(*W.cli_rotation(yaw=0.6, pitch=0.2))
+    with S.Context(0) as c:
+        dm = S.Mesh(c, m["x"], m["y"], m["z"], m["rgb"], m["idx"], m["bbox_max"])
+        c.set_viewport(181, 90, False)
+        U = O.viewport_transform(181, 90, O.scene_extent([m["bbox_max"]]))
+        c.set_utransform(U)
+        for step in range(2):
+            if step:
+                m = moved(m)
+                dm.update(m["x"], m["y"], m["z"], m["rgb"])
+            c.clear()
+            c.draw_mesh(dm, R)
+            check([v.view(np.int32) if v.dtype == np.float32 else v for v in c.read()],
+                  oracle_render([m], R, 181, 90, False, U=U), f"step {step}")
