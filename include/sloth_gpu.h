@@ -189,7 +189,8 @@ sloth_status sloth_ctx_flush_device(sloth_ctx *ctx, int format, const char **dev
  *   its right edge) holds at most this many samples are rasterized by the setup kernel
  *   straight into the global depth keys (a 64-bit atomicMin per covered sample) instead of
  *   being binned into tiles; 0 (the default) bins every triangle.  0..SLOTH_MAX_DIRECT_SAMPLES;
- *   takes effect at the next sloth_ctx_clear.  Results are identical either way. */
+ *   takes effect at the next sloth_ctx_clear.  Results are identical either way.  A draw of few
+ *   samples goes without tiles altogether, whatever this says (depth culling on). */
 #define SLOTH_OPTION_DIRECT_SAMPLES 4
 #define SLOTH_MAX_DIRECT_SAMPLES 256
 /* SLOTH_OPTION_TRIANGLES_PER_BLOCK: triangles per block of the setup kernel, 128, 256 (the
