@@ -137,25 +137,33 @@ __global__ void __launch_bounds__(1024) bin_scan_kernel(uint32_t n, BinBuffers b
     block_sync();
     const SplitParams sp = sp_s;
     const uint32_t light = light_s;
-    // pass 2: the scans
+    // pass 2: the scans; the next step's counts are on their way while this one's are summed.
+    // One block's chain of loads, sums and stores: with those loads after the barriers, sums
+    // picked by an index (an array in local memory) and 4-byte stores, the scan of the uneven
+    // batch's 25k tiles took 40 us, so 20; 2k tiles 9.0 and 6.1.
+    uint32_t n1[4], n2[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        n1[k] = c1_0[k];
+        n2[k] = c2_0[k];
+    }
     for (uint32_t base = 0; base < n; base += 4 * 1024) {
         const uint32_t i0 = base + 4 * tid;
-        uint32_t c[4], c1[4], c2[4], cls[4], loc[kV] = {0, 0, 0, 0};
-        if (base == 0) {
+        uint32_t c[4], c1[4], c2[4], cls[4], ns[4], loc[kV] = {0, 0, 0, 0};
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                c1[k] = c1_0[k];
-                c2[k] = c2_0[k];
-            }
-        } else {
-            load_counts4(bb, n, i0, c1, c2);
+        for (int k = 0; k < 4; ++k) {
+            c1[k] = n1[k];
+            c2[k] = n2[k];
         }
+        if (base + 4 * 1024 < n) load_counts4(bb, n, i0 + 4 * 1024, n1, n2);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             c[k] = c1[k] + c2[k];
             cls[k] = c[k] > sp.threshold ? 1u : (c[k] < light ? 3u : 2u);
             loc[0] += c[k];
-            loc[cls[k]] += tile_slices(c[k], sp);
+            ns[k] = tile_slices(c[k], sp);
+#pragma unroll
+            for (uint32_t q = 1; q < kV; ++q) loc[q] += cls[k] == q ? ns[k] : 0u;
         }
         uint32_t v[kV];
 #pragma unroll
@@ -191,18 +199,32 @@ __global__ void __launch_bounds__(1024) bin_scan_kernel(uint32_t n, BinBuffers b
         uint32_t p[kV];
 #pragma unroll
         for (int q = 0; q < kV; ++q) p[q] = carry[q] + v[q] - loc[q] + (wid > 0 ? ws[q][wid - 1] : 0u);
+        // the first-tile entries take [offset, offset + c1) by their counted slots, the others
+        // the slots after them from the cursor
+        uint32_t off[4], cur[4], so[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            if (i0 + k < n) {
-                // the first-tile entries take [offset, offset + c1) by their counted slots,
-                // the others the slots after them from the cursor
-                bb.tile_offset[i0 + k] = p[0];
-                bb.tile_cursor[i0 + k] = p[0] + c1[k];
-                bb.tile_count[i0 + k] = c[k];
-                bb.slice_offset[i0 + k] = p[cls[k]];
-            }
+            off[k] = p[0];
+            cur[k] = p[0] + c1[k];
+            so[k] = cls[k] == 1u ? p[1] : cls[k] == 2u ? p[2] : p[3];
             p[0] += c[k];
-            p[cls[k]] += tile_slices(c[k], sp);
+#pragma unroll
+            for (uint32_t q = 1; q < kV; ++q) p[q] += cls[k] == q ? ns[k] : 0u;
+        }
+        if (i0 + 4 <= n) {
+            *reinterpret_cast<uint4 *>(bb.tile_offset + i0) = make_uint4(off[0], off[1], off[2], off[3]);
+            *reinterpret_cast<uint4 *>(bb.tile_cursor + i0) = make_uint4(cur[0], cur[1], cur[2], cur[3]);
+            *reinterpret_cast<uint4 *>(bb.tile_count + i0) = make_uint4(c[0], c[1], c[2], c[3]);
+            *reinterpret_cast<uint4 *>(bb.slice_offset + i0) = make_uint4(so[0], so[1], so[2], so[3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (i0 + k < n) {
+                    bb.tile_offset[i0 + k] = off[k];
+                    bb.tile_cursor[i0 + k] = cur[k];
+                    bb.tile_count[i0 + k] = c[k];
+                    bb.slice_offset[i0 + k] = so[k];
+                }
         }
         block_sync();                    // every thread has read the carries
         if (tid == blockDim.x - 1)
