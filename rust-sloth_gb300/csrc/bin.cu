@@ -138,9 +138,9 @@ __global__ void __launch_bounds__(1024) bin_scan_kernel(uint32_t n, BinBuffers b
     const SplitParams sp = sp_s;
     const uint32_t light = light_s;
     // pass 2: the scans; the next step's counts are on their way while this one's are summed.
-    // One block's chain of loads, sums and stores: with those loads after the barriers, sums
-    // picked by an index (an array in local memory) and 4-byte stores, the scan of the uneven
-    // batch's 25k tiles took 40 us, so 20; 2k tiles 9.0 and 6.1.
+    // One block's chain of loads, sums and stores: with those loads after the barriers and
+    // 4-byte stores, the scan of the uneven batch's 25k tiles took 40 us, so 20; 2k tiles 9.0
+    // and 6.1.
     uint32_t n1[4], n2[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
