@@ -405,12 +405,12 @@ __device__ __noinline__ void batch_overflow_fold(const BatchDev &b)
         const BatchFrame &f = b.frames[(b.bb.fill_meta[i] & kFillReread) ? e.z : frame_of_tile(b, e.w)];
         frags += fold_queued<32, false, 1>(e.x, 0u, 1u, true, f.g, f.fb);
     }
-    constexpr uint32_t kParts = 64;
-    const uint32_t front = b.bb.large_count[0], all = front + b.bb.large_count[1];
-    for (uint32_t i = warp; i < all * kParts; i += nwarps) {
-        const uint32_t k = i / kParts, q = k < front ? k : b.bb.large_cap - 1u - (k - front);
+    const OverflowItems items(b.bb.large_count[0], b.bb.large_count[1], b.bb.large_cap);
+    for (uint64_t i = warp; i < items.all; i += nwarps) {
+        uint32_t part;
+        const uint32_t q = items.entry(i, part);
         const BatchFrame &f = b.frames[b.large_frame[q]];
-        frags += fold_queued<8, false, 1>(b.bb.large_queue[q], i % kParts, kParts, true, f.g, f.fb);
+        frags += fold_queued<8, false, 1>(b.bb.large_queue[q], part, kOverflowParts, true, f.g, f.fb);
     }
     add_frags_warp(frags, b.frames[0].fb.fragments);
 }

@@ -14,6 +14,7 @@
 // Every tile's keys must be current (cleared or written since the clear) before the folds.
 #pragma once
 
+#include "fold_items.h"
 #include "raster_common.cuh"
 #include "record.cuh"
 
@@ -37,7 +38,6 @@ constexpr uint32_t kFoldBlockSamples = 128;
 // key loads of a step are one chain, and the walk waits on its latency.
 constexpr uint32_t kFoldWarpSamples = 4096;
 constexpr int kFoldRows = 2, kFoldMidRows = 8;
-constexpr uint32_t kFoldParts = 512, kFoldMidParts = 8;
 constexpr int kFoldUnroll = 4;
 
 // With more queued triangles than this, cells that already hold a nearer key are left out
@@ -307,32 +307,28 @@ __device__ __forceinline__ uint32_t fold_queue_walk(const FoldQueue &queue, uint
     const int lane = threadIdx.x & 31;
     const uint32_t large = queue.count[0], mid = queue.count[1];
     const bool whole = mid > nwarps;   // a warp for each of the smaller ones
-    const uint32_t cut = large * kFoldParts, items = cut + mid * (whole ? 1u : kFoldMidParts);
+    const FoldItems items(large, mid, queue.cap, whole);
     const bool filter = large + mid > kFoldFilterMin;
     uint32_t frags = 0;
-    for (uint32_t base = warp; base < items; base += 32u * nwarps) {
+    for (uint64_t base = warp; base < items.all; base += 32ull * nwarps) {
         // lane l holds item base + l*nwarps: neighbouring items go to neighbouring warps
-        const uint32_t it = base + (uint32_t)lane * nwarps;
+        const uint64_t it = base + (uint64_t)lane * nwarps;
         uint32_t q = 0, part = 0, tri = 0;
-        bool live = it < items && it >= base;
+        bool live = it < items.all;
+        const bool is_large = it < items.cut;
         if (live) {
-            if (it < cut) {
-                part = it / large;
-                q = it - part * large;
-            } else {
-                part = (it - cut) / mid;
-                q = queue.cap - 1u - ((it - cut) - part * mid);
-            }
+            q = items.entry(it, part);
             tri = queue.tri[q];
             const int4 xr = *(reinterpret_cast<const int4 *>(frame_of(q).fb.records + tri) + 4);
-            live = xr.z + (int)part * (it < cut ? kFoldRows : kFoldMidRows) < xr.w;
+            live = xr.z + (int)part * (is_large ? kFoldRows : kFoldMidRows) < xr.w;
         }
+        const unsigned larges = __ballot_sync(0xffffffffu, is_large);
         for (unsigned todo = __ballot_sync(0xffffffffu, live); todo; todo &= todo - 1u) {
             const int src = __ffs(todo) - 1;
             const uint32_t wq = __shfl_sync(0xffffffffu, q, src), wt = __shfl_sync(0xffffffffu, tri, src),
-                           wp = __shfl_sync(0xffffffffu, part, src), wi = __shfl_sync(0xffffffffu, it, src);
+                           wp = __shfl_sync(0xffffffffu, part, src);
             const auto &f = frame_of(wq);
-            if (wi < cut) frags += fold_queued<kFoldRows>(wt, wp, kFoldParts, filter, f.g, f.fb);
+            if (larges >> src & 1u) frags += fold_queued<kFoldRows>(wt, wp, kFoldParts, filter, f.g, f.fb);
             else if (!whole) frags += fold_queued<kFoldMidRows>(wt, wp, kFoldMidParts, filter, f.g, f.fb);
             else frags += fold_queued<32>(wt, 0u, 1u, filter, f.g, f.fb);
         }

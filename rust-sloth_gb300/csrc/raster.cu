@@ -19,11 +19,11 @@ __device__ __noinline__ void overflow_fold(uint32_t tri_base, const FrameGeom &g
     uint32_t frags = 0;
     const uint32_t n = bb.large_count[2];
     for (uint32_t i = warp; i < n; i += nwarps) frags += fold_queued<32, false, 1>(bb.fill_list[i].x, 0u, 1u, true, g, fb);
-    constexpr uint32_t kParts = 64;
-    const uint32_t front = bb.large_count[0], all = front + bb.large_count[1];
-    for (uint32_t i = warp; i < all * kParts; i += nwarps) {
-        const uint32_t k = i / kParts, q = k < front ? k : bb.large_cap - 1u - (k - front);
-        frags += fold_queued<8, false, 1>(tri_base + bb.large_queue[q], i % kParts, kParts, true, g, fb);
+    const OverflowItems items(bb.large_count[0], bb.large_count[1], bb.large_cap);
+    for (uint64_t i = warp; i < items.all; i += nwarps) {
+        uint32_t part;
+        const uint32_t q = items.entry(i, part);
+        frags += fold_queued<8, false, 1>(tri_base + bb.large_queue[q], part, kOverflowParts, true, g, fb);
     }
     add_frags_warp(frags, fb.fragments);
 }
