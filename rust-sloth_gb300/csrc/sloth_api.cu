@@ -274,11 +274,23 @@ static sloth_status ensure_scratch(sloth_ctx *ctx, T **p, size_t *cap, size_t ne
     return SLOTH_OK;
 }
 
+// The ctx stream waits for the last newline fold (before a resolve or the next draw).
+static sloth_status join_newline(sloth_ctx *ctx)
+{
+    if (!ctx->nl_pending) return SLOTH_OK;
+    CU(ctx, cudaStreamWaitEvent(ctx->stream, ctx->nl_ev, 0));
+    ctx->nl_pending = false;
+    return SLOTH_OK;
+}
+
 // A clear's resets (error word, fragments, newline tree) wait for the next launch that
-// reads them; a draw adds its own (tile counts, large-queue counters) to the same launch.
+// reads them; a draw adds its own (tile counts, large-queue counters) to the same launch.  The
+// last frame's newline fold writes the tree they empty: whoever empties it waits for that fold.
 static sloth_status apply_resets(sloth_ctx *ctx, bool draw)
 {
     if (!ctx->reset_pending && !draw) return SLOTH_OK;
+    sloth_status st = join_newline(ctx);
+    if (st != SLOTH_OK) return st;
     const bool frame = ctx->reset_pending;
     // a draw that folds small triangles straight into the global keys needs every tile's
     // keys valid for this generation: cleared once per frame, the tiles made current
@@ -312,15 +324,6 @@ static sloth_status report_device_error(sloth_ctx *ctx)
     if (*ctx->h_error)
         return fail(ctx, SLOTH_ERR_DEVICE_FAULT, "a raster block gave up waiting for its tile copy (code %u)",
                     *ctx->h_error);
-    return SLOTH_OK;
-}
-
-// The ctx stream waits for the last newline fold (before a resolve or the next draw).
-static sloth_status join_newline(sloth_ctx *ctx)
-{
-    if (!ctx->nl_pending) return SLOTH_OK;
-    CU(ctx, cudaStreamWaitEvent(ctx->stream, ctx->nl_ev, 0));
-    ctx->nl_pending = false;
     return SLOTH_OK;
 }
 
@@ -1130,8 +1133,7 @@ sloth_status sloth_draw_mesh(sloth_ctx *ctx, const sloth_mesh *mesh, const float
     const FrameGeom &g = ctx->g;
     const uint32_t ntiles = (uint32_t)(g.ntx * g.nty);
     cudaStream_t s = ctx->stream;
-    if ((st = join_newline(ctx)) != SLOTH_OK) return st;
-    if ((st = apply_resets(ctx, true)) != SLOTH_OK) return st;
+    if ((st = apply_resets(ctx, true)) != SLOTH_OK) return st;   // and the last draw's newline fold joined
     // indexed meshes share vertices: transformed once by the vertex kernel; soups in setup
     const float4 *tv = mesh->idx ? ctx->tv : nullptr;
     if (tv) CU(ctx, timed(ctx, "vertex", [&] { return launch_vertex_transform(md, M, ctx->tv, s); }));
