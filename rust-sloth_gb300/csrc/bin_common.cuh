@@ -81,7 +81,7 @@ __device__ __forceinline__ void bin_large_warp(const TriRecord *rec, uint32_t gt
                                                uint64_t *entries, uint32_t capacity, int lane, uint32_t part,
                                                uint32_t nparts)
 {
-    const int4 xr = __ldg(reinterpret_cast<const int4 *>(rec) + 4);
+    const int4 xr = *(reinterpret_cast<const int4 *>(rec) + 4);   // the kernel before wrote it
     const TileSpan sp = tile_span_of(vp, xr.x, xr.y, xr.z, xr.w);
     const int nu = (sp.TU.xb - sp.TU.xa) * (sp.TU.yb - sp.TU.ya);
     const int nw = (sp.TW.xb - sp.TW.xa) * (sp.TW.yb - sp.TW.ya);

@@ -11,9 +11,15 @@ namespace sloth {
 
 // Waits for the kernels this one depends on (returns at once after an ordinary launch).
 // Every kernel launched with launch_pdl calls it before its first access to global memory,
-// so that "the kernel before" always covers everything before that one too.  The zero it
-// returns is added to the indices of the loads that follow: read-only loads (__ldg) are not
-// ordered by the memory clobber, and this makes their addresses depend on the wait.
+// so that "the kernel before" always covers everything before that one too.
+//
+// Read-only loads (__ldg, const __restrict__) are for what nobody writes while the kernel
+// lives, and it lives from before the wait: a mesh, and what kernels before the one just
+// before it wrote (that one waited for them before it let this one start).  What the kernel
+// just before writes -- keys and tile generations for the resolve, transformed vertices for
+// setup, sample ranges for the large counts, entries for the raster -- is read by plain loads.
+// The zero it returns is added to the indices of the loads that follow: read-only loads are
+// not ordered by the memory clobber, and this makes their addresses depend on the wait.
 __device__ __forceinline__ uint32_t pdl_wait()
 {
     uint32_t zero;

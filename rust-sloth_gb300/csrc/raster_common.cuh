@@ -365,7 +365,7 @@ __device__ __forceinline__ void refresh_bounds(TileSmem<TW, TH> &S, int R0, int 
 // bit 0 the parity of the phase the next load completes.
 template <int TW, int TH>
 __device__ __forceinline__ bool raster_tile(TileSmem<TW, TH> &S, const FrameGeom &g, const FrameBuffers &fb,
-                                            int tile, uint32_t cnt, const uint64_t *__restrict__ entries,
+                                            int tile, uint32_t cnt, const uint64_t *entries,
                                             int depth_cull, uint32_t &phase, bool split = false)
 {
     static_assert(TH <= 32, "a tile part has at most 32 rows: one lane per row in raster_part");

@@ -59,13 +59,13 @@ __device__ __forceinline__ Viewport to_vp(const FrameGeom &g)
 // The three transformed vertices of triangle t, at position p of setup's order.  tv null
 // (soups): the thread transforms them itself, which saves the vertex kernel and its round
 // trip through memory.
-__device__ __forceinline__ void triangle_vertices(const MeshDev &mesh, const float4 *__restrict__ tv, const Mat4 &M,
+__device__ __forceinline__ void triangle_vertices(const MeshDev &mesh, const float4 *tv, const Mat4 &M,
                                                   uint32_t p, uint32_t t, float4 &p1, float4 &p2, float4 &p3)
 {
     uint32_t i1, i2, i3;
     mesh_corners(mesh, p, t, i1, i2, i3);
     if (tv) {
-        p1 = __ldg(tv + i1); p2 = __ldg(tv + i2); p3 = __ldg(tv + i3);
+        p1 = tv[i1]; p2 = tv[i2]; p3 = tv[i3];   // the vertex kernel just before wrote them
     } else {
         p1 = transform_vertex(mesh, M, i1); p2 = transform_vertex(mesh, M, i2); p3 = transform_vertex(mesh, M, i3);
     }
@@ -136,7 +136,7 @@ __device__ __forceinline__ void setup_triangle(uint32_t tri_base, const FrameGeo
 // kSetupChunk); the one-chunk form keeps fewer values live through phase 2.
 template <bool kDirect, bool kChunks>
 __global__ void __launch_bounds__(kSetupThreads, kDirect ? kSetupMinBlocks : kFillMinBlocks)
-setup_kernel(MeshDev mesh, const float4 *__restrict__ tv, Mat4 M, uint32_t tri_base, FrameGeom g,
+setup_kernel(MeshDev mesh, const float4 *tv, Mat4 M, uint32_t tri_base, FrameGeom g,
              FrameBuffers fb, BinBuffers bb, int tpb)
 {
     __shared__ uint32_t sq_n;
