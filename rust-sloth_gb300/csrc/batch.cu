@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(256) batch_fold_large_kernel(BatchDev b, const
     blk -= nnl;
     const uint32_t first = (blk * blockDim.x + threadIdx.x) >> 5;
     const FoldQueue queue{b.bb.large_queue, b.large_frame, b.bb.large_count, b.bb.large_cap};
-    const uint32_t frags = fold_queue_walk(queue, first, ((gridDim.x - nnl) * blockDim.x) >> 5,
+    const uint32_t frags = fold_queue_walk<uint64_t>(queue, first, ((gridDim.x - nnl) * blockDim.x) >> 5,
                                            [&](uint32_t q) -> const BatchFrame & { return b.frames[b.large_frame[q]]; });
     add_frags_warp(frags, b.frames[0].fb.fragments);   // the batch's one counter
 }

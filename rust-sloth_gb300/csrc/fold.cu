@@ -60,12 +60,17 @@ struct FoldFrame {
     FrameBuffers fb;
 };
 
+// 2^22 warps' worth of items above those of the most triangles a draw folds
+static_assert((uint64_t)kFoldMaxTrianglesMade * kFoldParts + (32ull << 22) < (1ull << 32) &&
+                  kFoldMaxTrianglesMade >= kFoldMaxTriangles && kFoldParts >= kFoldMidParts,
+              "32-bit items");
+
 __global__ void __launch_bounds__(256)
 fold_large_kernel(const __grid_constant__ FoldFrame f, FoldQueue queue, uint32_t *next)
 {
     const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x + pdl_begin()) >> 5;
     if (blockIdx.x == 0 && threadIdx.x < 2) next[threadIdx.x] = 0u;
-    const uint32_t frags = fold_queue_walk(queue, first, (gridDim.x * blockDim.x) >> 5,
+    const uint32_t frags = fold_queue_walk<uint32_t>(queue, first, (gridDim.x * blockDim.x) >> 5,
                                            [&](uint32_t) -> const FoldFrame & { return f; });
     add_frags_warp(frags, f.fb.fragments);
 }

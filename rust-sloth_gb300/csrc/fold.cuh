@@ -300,19 +300,20 @@ __device__ __forceinline__ uint32_t fold_queued(uint32_t gtri, uint32_t part, ui
 
 // The queued triangles of one frame or many, over the warps of a grid (this is warp `warp` of
 // nwarps): frame_of(q) gives the frame of queue entry q as a pair of its geometry and buffers.
-template <class FrameOf>
+// Index: FoldItems.
+template <class Index, class FrameOf>
 __device__ __forceinline__ uint32_t fold_queue_walk(const FoldQueue &queue, uint32_t warp, uint32_t nwarps,
                                                     FrameOf frame_of)
 {
     const int lane = threadIdx.x & 31;
     const uint32_t large = queue.count[0], mid = queue.count[1];
     const bool whole = mid > nwarps;   // a warp for each of the smaller ones
-    const FoldItems items(large, mid, queue.cap, whole);
+    const FoldItems<Index> items(large, mid, queue.cap, whole);
     const bool filter = large + mid > kFoldFilterMin;
     uint32_t frags = 0;
-    for (uint64_t base = warp; base < items.all; base += 32ull * nwarps) {
+    for (Index base = warp; base < items.all; base += (Index)32 * nwarps) {
         // lane l holds item base + l*nwarps: neighbouring items go to neighbouring warps
-        const uint64_t it = base + (uint64_t)lane * nwarps;
+        const Index it = base + (Index)lane * nwarps;
         uint32_t q = 0, part = 0, tri = 0;
         bool live = it < items.all;
         const bool is_large = it < items.cut;

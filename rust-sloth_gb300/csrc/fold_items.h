@@ -1,9 +1,10 @@
 // fold_items.h -- how the work items of queued triangles are numbered, for the walk of a
 // fold's queue (fold.cuh) and the overflow folds of the tile rasters (raster.cu, batch.cu).
 //
-// The numbers are 64-bit: a context's fold stops at 2^20 triangles, but the frames of a batch
-// share one queue, and from 8,388,608 large triangles on kFoldParts items each are 2^32 or
-// more.  Plain C++, so that the numbering is tested on the host at sizes no test draws.
+// The frames of a batch share one queue, and from 8,388,608 large triangles on kFoldParts items
+// each are 2^32 or more: their numbers are 64-bit.  One draw's fold stops at 2^20 triangles,
+// and 32 bits do (with 64 the sixteen walks of 16 models at 1280x720 took 7 us of 160 more).
+// Plain C++, so that the numbering is tested on the host at sizes no test draws.
 #pragma once
 
 #include <cstdint>
@@ -22,6 +23,7 @@ constexpr uint32_t kFoldParts = 512, kFoldMidParts = 8;
 constexpr uint32_t kOverflowParts = 64;
 
 // n / d; the 64-bit division, many times as long, only for the counts that need it.
+SLOTH_HD uint32_t item_part(uint32_t n, uint32_t d) { return n / d; }
 SLOTH_HD uint32_t item_part(uint64_t n, uint32_t d)
 {
     return n >> 32 ? (uint32_t)(n / d) : (uint32_t)n / d;
@@ -29,18 +31,20 @@ SLOTH_HD uint32_t item_part(uint64_t n, uint32_t d)
 
 // The items of a fold's queue: every part of the large triangles, part after part, then of
 // the others (one item each when `whole`).  The large ones are queued from the front of the
-// cap entries, the others from the back.
+// cap entries, the others from the back.  Index: a type that all + 32 items a warp of the
+// walk's grid fits in.
+template <class Index>
 struct FoldItems {
     uint32_t large, mid, cap;
-    uint64_t cut, all;   // the large ones' items, all items
+    Index cut, all;   // the large ones' items, all items
 
     SLOTH_HD FoldItems(uint32_t large_, uint32_t mid_, uint32_t cap_, bool whole)
-        : large(large_), mid(mid_), cap(cap_), cut((uint64_t)large_ * kFoldParts),
-          all(cut + (uint64_t)mid_ * (whole ? 1u : kFoldMidParts))
+        : large(large_), mid(mid_), cap(cap_), cut((Index)large_ * kFoldParts),
+          all(cut + (Index)mid_ * (whole ? 1u : kFoldMidParts))
     {
     }
     // Queue entry and part of item it (below all).
-    SLOTH_HD uint32_t entry(uint64_t it, uint32_t &part) const
+    SLOTH_HD uint32_t entry(Index it, uint32_t &part) const
     {
         if (it < cut) {
             part = item_part(it, large);

@@ -21,9 +21,14 @@ int main()
     while (scanf("%u %u %u %u %u %llu", &kind, &a, &b, &cap, &whole, &it) == 6) {
         uint32_t part = 0;
         if (kind == 0) {
-            const FoldItems f(a, b, cap, whole != 0);
+            const FoldItems<uint64_t> f(a, b, cap, whole != 0);
             const uint32_t q = f.entry(it, part);
             printf("%llu %llu %u %u\n", (unsigned long long)f.cut, (unsigned long long)f.all, q, part);
+            if ((unsigned long long)a + b <= 1u << 20) {   // a draw's: the same in 32 bits
+                const FoldItems<uint32_t> n(a, b, cap, whole != 0);
+                uint32_t p2 = 0;
+                if (n.entry((uint32_t)it, p2) != q || p2 != part || n.all != f.all || n.cut != f.cut) return 1;
+            }
         } else {
             const OverflowItems f(a, b, cap);
             const uint32_t q = f.entry(it, part);
@@ -52,7 +57,7 @@ def spread(n, rng):
                    *(rng.randrange(n) for _ in range(40))})
 
 
-@pytest.mark.parametrize("large,mid", [(1, 0), (0, 1), (3, 5), (700, 31), (8388312, 10), (8388607, 0), (8388608, 3),
+@pytest.mark.parametrize("large,mid", [(1, 0), (0, 1), (3, 5), (700, 31), (1048576, 0), (0, 1048576), (8388312, 10), (8388607, 0), (8388608, 3),
                                        (8400000, 900000), (20000000, 0), (0, 600000000), (2**31 - 2, 1)])
 @pytest.mark.parametrize("whole", [0, 1])
 def test_fold_items(items, large, mid, whole):
