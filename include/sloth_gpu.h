@@ -285,10 +285,10 @@ sloth_status sloth_batch_set_transforms(sloth_batch *batch, const float *transfo
 /* Render every frame (asynchronous on the context's stream).  The first render sizes the
  * tile-entry buffer (one host synchronisation); later renders replay a CUDA graph.  A render
  * that outgrows the buffer is rasterized by a slower exact fallback on the device, and a
- * later render or read sizes the buffer again. */
+ * later render sizes the buffer again. */
 sloth_status sloth_batch_render(sloth_batch *batch);
-/* Copy one frame's buffers to host memory (any may be NULL); blocks.  If the last render
- * outgrew the tile-entry buffer, it is re-planned and re-rendered first. */
+/* Copy one frame's buffers, as the last render left them, to host memory (any may be NULL);
+ * blocks. */
 sloth_status sloth_batch_read(sloth_batch *batch, uint32_t frame, uint32_t *cells, float *z, int32_t *winner);
 /* Device pointers of one frame's resolved buffers. */
 sloth_status sloth_batch_frame_buffers(sloth_batch *batch, uint32_t frame, const uint32_t **cells,

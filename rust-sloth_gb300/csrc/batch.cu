@@ -253,7 +253,6 @@ __global__ void __launch_bounds__(256) batch_reset_kernel(BatchReset r)
     if (i0 == 0) {
         r.large_count[0] = r.large_count[1] = 0u;
         *r.fill_count = 0u;
-        *r.overflow = 0u;
         *r.fragments = 0ull;
     }
     for (uint64_t i = i0; i < r.ntiles; i += step) {
@@ -428,10 +427,7 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterMinBlocks) batch_raster
     __shared__ uint32_t s_item;
     const uint32_t blk = blockIdx.x;
     if (b.bb.tile_offset[b.total_tiles] > b.bb.capacity) {
-        if (blk == 0 && threadIdx.x == 0) {
-            *b.overflow = 1;
-            b.status[0] = 1;
-        }
+        if (blk == 0 && threadIdx.x == 0) b.status[0] = 1;
         batch_overflow_fold(b);
         return;
     }

@@ -7,8 +7,8 @@
 // pass of each kernel and one persistent raster pass over a device-side (frame, tile)
 // queue.  After the first render (which sizes the tile-entry buffer on the host) the
 // whole sequence is captured in a CUDA graph and replayed.  If a later render's entries
-// outgrow the buffer, the raster folds its triangles without tiles and reports it, and the
-// next read or render sizes the buffer again.
+// outgrow the buffer, the raster folds its triangles without tiles and reports it, and a
+// later render sizes the buffer again.
 #include <cstring>
 #include <string>
 #include <vector>
@@ -81,11 +81,9 @@ struct sloth_batch {
     BinBuffers bb{};
     size_t entries_cap = 0;
     uint32_t *large_frame = nullptr;
-    uint32_t *overflow = nullptr;
     uint32_t *queue = nullptr;                // the persistent raster's item counter
     uint32_t *fill_count = nullptr;           // entries of bb.fill_list
     uint32_t *h_total = nullptr;              // pinned
-    uint32_t *h_overflow = nullptr;           // pinned
     uint32_t *error = nullptr;                // device error word of the raster (sticky)
     uint32_t *h_error = nullptr;              // pinned
     uint32_t *status = nullptr;               // pinned, written by the raster (BatchDev::status)
@@ -181,7 +179,6 @@ void free_layout(sloth_batch *b)
     bfree(b->bb.slice_offset);
     bfree(b->bb.items);
     b->bb.item_capacity = 0;
-    bfree(b->overflow);
     bfree(b->queue);
     bfree(b->bb.fill_list);
     bfree(b->fill_count);
@@ -357,7 +354,6 @@ sloth_status build(sloth_batch *b, int shape)
     b->bb.large_cap = (uint32_t)rec;
     BCU(b, balloc(&b->large_frame, rec));
     BCU(b, balloc(&b->bb.slice_offset, tiles + kSliceExtra));
-    BCU(b, balloc(&b->overflow, 1));
     BCU(b, balloc(&b->queue, 1));
     BCU(b, balloc(&b->bb.fill_list, fill_words16(rec)));
     b->bb.fill_meta = reinterpret_cast<uint32_t *>(b->bb.fill_list + rec);
@@ -406,7 +402,6 @@ BatchDev dev_view(sloth_batch *b)
     d.bb = b->bb;
     d.bb.capacity = (uint32_t)(b->entries_cap > 0xffffffffu ? 0xffffffffu : b->entries_cap);
     d.large_frame = b->large_frame;
-    d.overflow = b->overflow;
     d.status = b->status;
     d.queue = b->queue;
     d.fill_count = b->fill_count;
@@ -435,7 +430,6 @@ cudaError_t enqueue_reset(sloth_batch *b, cudaStream_t s)
     r.nnl = (uint32_t)b->total_nl;
     r.large_count = b->bb.large_count;
     r.fill_count = b->fill_count;
-    r.overflow = b->overflow;
     r.fragments = b->fragments;
     r.mats = reinterpret_cast<float4 *>(b->d_mats);
     r.mats_host = reinterpret_cast<const float4 *>(b->h_mats);
@@ -565,19 +559,16 @@ sloth_status capture(sloth_batch *b)
     return SLOTH_OK;
 }
 
-// After a render: if the entries outgrew their buffer, re-plan and re-render.
+// Waits for the last render and reports its fault.  Its frames are exact whether or not its
+// entries fitted (batch_overflow_fold), and they stay what they are: the transforms or meshes
+// may be others by now, and the caller may hold the device buffers.  The next render of one
+// that did not fit sizes the buffer again (status[0]).
 sloth_status settle(sloth_batch *b)
 {
-    BCU(b, cudaMemcpyAsync(b->h_overflow, b->overflow, 4, cudaMemcpyDeviceToHost, b->stream));
     BCU(b, cudaMemcpyAsync(b->h_error, b->error, 4, cudaMemcpyDeviceToHost, b->stream));
     BCU(b, cudaStreamSynchronize(b->stream));
     if (*b->h_error)
         return sloth_ctx_fail(b->ctx, SLOTH_ERR_DEVICE_FAULT, "a raster block gave up waiting for its tile copy");
-    if (*b->h_overflow) {
-        sloth_status st = render_planned(b);
-        if (st != SLOTH_OK) return st;
-        BCU(b, cudaStreamSynchronize(b->stream));
-    }
     return SLOTH_OK;
 }
 
@@ -626,7 +617,6 @@ void sloth_batch_detach(sloth_batch *b)
     flush_release(b->flush);
     if (b->h_mats) cudaFreeHost(b->h_mats);
     if (b->h_total) cudaFreeHost(b->h_total);
-    if (b->h_overflow) cudaFreeHost(b->h_overflow);
     if (b->h_error) cudaFreeHost(b->h_error);
     if (b->status) cudaFreeHost(b->status);
     bfree(b->error);
@@ -638,7 +628,7 @@ void sloth_batch_detach(sloth_batch *b)
     if (b->nl_s) cudaStreamDestroy(b->nl_s);
     b->nl_s = nullptr;
     b->h_mats = nullptr;
-    b->h_total = b->h_overflow = b->h_error = b->status = nullptr;
+    b->h_total = b->h_error = b->status = nullptr;
     b->ctx = nullptr;
     b->stream = nullptr;
     b->rendered = false;
@@ -682,7 +672,7 @@ sloth_status sloth_batch_create(sloth_ctx *ctx, const sloth_frame_desc *frames, 
         b->transforms.insert(b->transforms.end(), draws[d].transform, draws[d].transform + 16);
     }
     if (cudaMallocHost(&b->h_mats, (ndraws ? ndraws : 1) * sizeof(Mat4)) != cudaSuccess ||
-        cudaMallocHost(&b->h_total, 4) != cudaSuccess || cudaMallocHost(&b->h_overflow, 4) != cudaSuccess ||
+        cudaMallocHost(&b->h_total, 4) != cudaSuccess ||
         cudaMallocHost(&b->h_error, 4) != cudaSuccess || cudaMallocHost(&b->status, 8) != cudaSuccess ||
         cudaMalloc(&b->error, 4) != cudaSuccess ||
         cudaMemset(b->error, 0, 4) != cudaSuccess ||
@@ -739,7 +729,6 @@ sloth_status sloth_batch_render(sloth_batch *b)
         b->graph = nullptr;
     }
     // a render known to have outgrown its entries: the buffer grows before the next one
-    // (settle does the same for a caller that reads)
     const bool tiles = b->folded == FoldForm::none;
     const bool grow = tiles && *(volatile uint32_t *)&b->status[0];
     if (grow || !b->rendered || (tiles && !b->bb.entries)) return render_planned(b);
@@ -901,10 +890,11 @@ sloth_status apply_tune(sloth_batch *b, const BatchTune &t)
 sloth_status time_tune(sloth_batch *b, const BatchTune &t, int reps, cudaEvent_t e0, cudaEvent_t e1, float *ms)
 {
     sloth_status st = apply_tune(b, t);
-    if (st == SLOTH_OK) st = sloth_batch_render(b);     // plan + size the entries
-    if (st == SLOTH_OK) st = settle(b);
-    if (st == SLOTH_OK) st = sloth_batch_render(b);     // capture + warm
-    if (st == SLOTH_OK) st = settle(b);
+    // plan and size the entries (again, if other transforms have outgrown them), capture, warm
+    for (int k = 0; k < 3 && st == SLOTH_OK; ++k) {
+        st = sloth_batch_render(b);
+        if (st == SLOTH_OK) st = settle(b);
+    }
     if (st != SLOTH_OK) return st;
     BCU(b, cudaEventRecord(e0, b->stream));
     for (int i = 0; i < reps && st == SLOTH_OK; ++i) st = sloth_batch_render(b);

@@ -42,7 +42,6 @@ struct BatchDev {
     const uint32_t *frame_tile_off;   // nframes + 1 (for tile -> frame lookups)
     BinBuffers bb;             // global tile arrays and entries
     uint32_t *large_frame;     // frame of each large-queue entry
-    uint32_t *overflow;        // set when the entries outgrew their capacity
     volatile uint32_t *status; // pinned host words: [0] a render's entries outgrew their capacity,
                                // [1] a raster block gave up waiting for its keys
     uint32_t *queue;           // the persistent raster's next item (zeroed by the fill)
@@ -60,7 +59,7 @@ struct BatchReset {
     uint32_t ntiles, gen;      // the generation every tile gets
     int32_t *nltree;
     uint32_t nnl;
-    uint32_t *large_count, *fill_count, *overflow;
+    uint32_t *large_count, *fill_count;
     unsigned long long *fragments;
     float4 *mats;              // device matrices, and the pinned ones they are copied from
     const float4 *mats_host;
