@@ -197,6 +197,11 @@ sloth_status sloth_ctx_flush_device(sloth_ctx *ctx, int format, const char **dev
  *   default), 1024 or 4096; a block has at most 256 threads, each taking its share of the
  *   block's triangles in turn.  Results are identical either way. */
 #define SLOTH_OPTION_TRIANGLES_PER_BLOCK 5
+/* SLOTH_OPTION_KEEP_TILES: a test hook.  1 keeps the tile raster for every draw of the context
+ *   and every render of its batches, also with depth culling on, where those of few samples
+ *   otherwise go without tiles; 0 (the default) is normal operation.  Results are identical
+ *   either way. */
+#define SLOTH_OPTION_KEEP_TILES 6
 sloth_status sloth_ctx_set_option(sloth_ctx *ctx, int option, int64_t value);
 
 /* Autotuner of the single-frame path: renders the frame clear + draw_mesh(meshes[i],

@@ -115,6 +115,7 @@ void sloth_ctx_unregister_batch(sloth_ctx *ctx, sloth_batch *b);
 int sloth_ctx_device(const sloth_ctx *ctx);
 cudaStream_t sloth_ctx_stream(const sloth_ctx *ctx);
 int sloth_ctx_depth_cull(const sloth_ctx *ctx);
+int sloth_ctx_may_fold(const sloth_ctx *ctx);
 int sloth_ctx_direct_samples(const sloth_ctx *ctx);
 struct MeshView {
     const float *x, *y, *z;
@@ -722,7 +723,7 @@ sloth_status sloth_batch_render(sloth_batch *b)
     if (!b || !b->ctx) return SLOTH_ERR_INVALID_ARGUMENT;
     BCU(b, cudaSetDevice(b->device));
     b->vis_valid = false;
-    const FoldForm fold = sloth_ctx_depth_cull(b->ctx) ? b->fold : FoldForm::none;
+    const FoldForm fold = sloth_ctx_may_fold(b->ctx) ? b->fold : FoldForm::none;
     if (fold != b->folded) {
         b->folded = fold;
         if (b->graph) cudaGraphExecDestroy(b->graph);

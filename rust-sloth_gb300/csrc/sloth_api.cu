@@ -91,6 +91,7 @@ struct sloth_ctx {
 
     // instrumentation and options
     int depth_cull = 1;
+    int keep_tiles = 0;            // SLOTH_OPTION_KEEP_TILES
     int tile_shape = 0;
     int direct_max = 0;            // SLOTH_OPTION_DIRECT_SAMPLES (applied at the next clear)
     int tpb = kDefaultTrianglesPerBlock;   // SLOTH_OPTION_TRIANGLES_PER_BLOCK
@@ -371,6 +372,7 @@ void sloth_ctx_unregister_batch(sloth_ctx *ctx, sloth_batch *b)
 int sloth_ctx_device(const sloth_ctx *ctx) { return ctx->device; }
 cudaStream_t sloth_ctx_stream(const sloth_ctx *ctx) { return ctx->stream; }
 int sloth_ctx_depth_cull(const sloth_ctx *ctx) { return ctx->depth_cull; }
+int sloth_ctx_may_fold(const sloth_ctx *ctx) { return ctx->depth_cull && !ctx->keep_tiles; }
 int sloth_ctx_direct_samples(const sloth_ctx *ctx) { return ctx->direct_max; }
 struct MeshView {
     const float *x, *y, *z;
@@ -1053,7 +1055,7 @@ static sloth_status poll_entry_max(sloth_ctx *ctx)
 // test needs its tile loads: both keep it.
 static bool draws_without_tiles(const sloth_ctx *ctx, const sloth_mesh *mesh, const Mat4 &M)
 {
-    if (!ctx->depth_cull || ctx->fb.wait_test || !(mesh->span2 > 0.0f)) return false;
+    if (!sloth_ctx_may_fold(ctx) || ctx->fb.wait_test || !(mesh->span2 > 0.0f)) return false;
     const float cells = (float)ctx->g.w * (float)ctx->g.h;
     if (mesh->ntri > kFoldMaxTriangles &&
         (mesh->updated || mesh->ntri > kFoldMaxTrianglesMade || (float)mesh->ntri > 26.0f * cells ||
@@ -1185,6 +1187,10 @@ sloth_status sloth_ctx_set_option(sloth_ctx *ctx, int option, int64_t value)
     case SLOTH_OPTION_WAIT_TEST:
         if (value != 0 && value != 1) return fail(ctx, SLOTH_ERR_INVALID_ARGUMENT, "wait test is 0 or 1");
         ctx->fb.wait_test = (uint32_t)value;
+        return SLOTH_OK;
+    case SLOTH_OPTION_KEEP_TILES:
+        if (value != 0 && value != 1) return fail(ctx, SLOTH_ERR_INVALID_ARGUMENT, "keep tiles is 0 or 1");
+        ctx->keep_tiles = (int)value;
         return SLOTH_OK;
     case SLOTH_OPTION_DEPTH_CULL:
         if (value != 0 && value != 1) return fail(ctx, SLOTH_ERR_INVALID_ARGUMENT, "depth cull is 0 or 1");

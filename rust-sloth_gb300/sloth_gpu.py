@@ -26,6 +26,7 @@ OPTION_TILE_SHAPE = 2
 OPTION_WAIT_TEST = 3
 OPTION_DIRECT_SAMPLES = 4
 OPTION_TRIANGLES_PER_BLOCK = 5
+OPTION_KEEP_TILES = 6
 STATUS ={0: "OK", 1: "INVALID_ARGUMENT", 2: "OUT_OF_MEMORY", 3: "CUDA", 4: "LIMIT", 5: "DEVICE_FAULT"}
 
 # Every symbol declared in include/sloth_gpu.h, with (restype, argtypes).
@@ -278,6 +279,10 @@ class Context:
     def set_depth_cull(self, on: bool):
         """SLOTH_OPTION_DEPTH_CULL: skip triangles proven hidden (same results)."""
         self._check(self.lib.sloth_ctx_set_option(self.h, OPTION_DEPTH_CULL, 1 if on else 0))
+
+    def set_keep_tiles(self, on: bool):
+        """SLOTH_OPTION_KEEP_TILES, a test hook: every draw and batch keeps the tile raster."""
+        self._check(self.lib.sloth_ctx_set_option(self.h, OPTION_KEEP_TILES, 1 if on else 0))
 
     def set_direct_samples(self, samples: int):
         """SLOTH_OPTION_DIRECT_SAMPLES: triangles of at most this many samples are folded
