@@ -11,6 +11,7 @@
 // later render sizes the buffer again.
 #include <cstring>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "batch_kernels.h"
@@ -40,8 +41,9 @@ struct sloth_batch {
     std::vector<sloth_frame_desc> frames;
     std::vector<const sloth_mesh *> meshes;   // per draw
     std::vector<float> transforms;            // 16 per draw
-    std::vector<uint32_t> draw_ntri;          // per draw: its mesh's triangles and span2
-    std::vector<float> draw_span2;
+    std::vector<uint32_t> draw_ntri, draw_unique;   // per draw: its mesh's triangles, its place in `unique`
+    std::vector<const sloth_mesh *> unique;   // the draws' meshes, each once, and the sums of
+    std::vector<float> span2;                 // squared edges that `fold` was decided with
     int shape = 0;
     int direct_max = 0;                       // FrameGeom::direct_max of every frame
     bool persistent = true;                   // raster over the device queue (else one CTA per item)
@@ -124,9 +126,9 @@ struct MeshView {
     uint32_t nvert, ntri;
     int device;
     const uint32_t *order, *oidx;   // setup's order of an indexed mesh (MeshDev), or null
-    float span2;                    // sum of the triangles' longest edges squared (mesh_span2)
 };
 MeshView sloth_mesh_view(const sloth_mesh *m);
+float sloth_mesh_span2(const sloth_mesh *m);   // sum of the triangles' longest edges squared
 }
 
 namespace {
@@ -208,9 +210,10 @@ FoldForm batch_folds(const sloth_batch *b)
         for (uint32_t k = 0; k < fd.ndraws; ++k) {
             const uint32_t d = fd.first_draw + k, n = b->draw_ntri[d];
             if (n == 0) continue;
-            if (n > kFoldMaxTriangles || !(b->draw_span2[d] > 0.0f)) return FoldForm::none;
+            const float span2 = b->span2[b->draw_unique[d]];
+            if (n > kFoldMaxTriangles || !(span2 > 0.0f)) return FoldForm::none;
             tri += n;
-            frame += fold_estimate(b->draw_span2[d], n, b->h_mats[d], (int)fd.width, (int)fd.height);
+            frame += fold_estimate(span2, n, b->h_mats[d], (int)fd.width, (int)fd.height);
         }
         if (!(frame <= kFoldMaxSamples)) return FoldForm::none;
         est += frame;
@@ -219,6 +222,19 @@ FoldForm batch_folds(const sloth_batch *b)
     if (tri > kFoldTableTriangles) return FoldForm::setup;
     if (tri > kFoldMany4) return each < 4.0 ? FoldForm::setup : FoldForm::warps1;
     return tri >= kFoldMany && each <= 20.0 ? FoldForm::warps1 : FoldForm::warps4;
+}
+
+// Decides again when an update has changed a mesh's edges since (sloth_mesh::span2).
+void follow_updates(sloth_batch *b)
+{
+    bool changed = false;
+    for (size_t k = 0; k < b->unique.size(); ++k) {
+        const float s = sloth_mesh_span2(b->unique[k]);
+        if (s == b->span2[k] || (s != s && b->span2[k] != b->span2[k])) continue;
+        b->span2[k] = s;
+        changed = true;
+    }
+    if (changed) b->fold = batch_folds(b);
 }
 
 void set_mats(sloth_batch *b)
@@ -665,11 +681,16 @@ sloth_status sloth_batch_create(sloth_ctx *ctx, const sloth_frame_desc *frames, 
     b->device = dev;
     b->stream = sloth_ctx_stream(ctx);
     b->frames.assign(frames, frames + nframes);
+    std::unordered_map<const sloth_mesh *, uint32_t> place;
     for (uint32_t d = 0; d < ndraws; ++d) {
-        const MeshView mv = sloth_mesh_view(draws[d].mesh);
         b->meshes.push_back(draws[d].mesh);
-        b->draw_ntri.push_back(mv.ntri);
-        b->draw_span2.push_back(mv.span2);
+        b->draw_ntri.push_back(sloth_mesh_view(draws[d].mesh).ntri);
+        const auto at = place.emplace(draws[d].mesh, (uint32_t)b->unique.size());
+        if (at.second) {
+            b->unique.push_back(draws[d].mesh);
+            b->span2.push_back(sloth_mesh_span2(draws[d].mesh));
+        }
+        b->draw_unique.push_back(at.first->second);
         b->transforms.insert(b->transforms.end(), draws[d].transform, draws[d].transform + 16);
     }
     if (cudaMallocHost(&b->h_mats, (ndraws ? ndraws : 1) * sizeof(Mat4)) != cudaSuccess ||
@@ -723,6 +744,7 @@ sloth_status sloth_batch_render(sloth_batch *b)
     if (!b || !b->ctx) return SLOTH_ERR_INVALID_ARGUMENT;
     BCU(b, cudaSetDevice(b->device));
     b->vis_valid = false;
+    follow_updates(b);
     const FoldForm fold = sloth_ctx_may_fold(b->ctx) ? b->fold : FoldForm::none;
     if (fold != b->folded) {
         b->folded = fold;

@@ -290,14 +290,67 @@ cudaError_t launch_vertex_transform(const MeshDev &mesh, const Mat4 &M, float4 *
     return launch_pdl(vertex_transform_kernel, dim3((quads + 255) / 256), dim3(256), 0, s, mesh, M, tv);
 }
 
+constexpr int kMeshThreads = 1024;
+
+// The sum over a mesh's triangles of their longest edge squared, by one block, as mesh_span2
+// takes it on the host: at most kSpanTriangles of them, four a thread, their loads in flight
+// together.  Triangles with a coordinate that is not finite count nothing.
+template <class Position>
+__device__ __forceinline__ void mesh_span_block(const uint32_t *__restrict__ idx, uint32_t ntri, volatile float *span,
+                                                Position at)
+{
+    __shared__ float ws[kMeshThreads / 32];
+    constexpr int kEach = (int)kSpanTriangles / kMeshThreads;
+    const uint32_t step = (ntri + kSpanTriangles - 1) / kSpanTriangles, n = (ntri + step - 1) / step;
+    float3 v[kEach][3];
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) {
+        const uint32_t k = threadIdx.x + (uint32_t)(j * kMeshThreads), t = (k < n ? k : 0u) * step;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[j][c] = at(idx ? idx[3 * (size_t)t + c] : 3 * t + c);
+    }
+    float sum = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) {
+        float e2 = 0.0f;
+        bool finite = threadIdx.x + (uint32_t)(j * kMeshThreads) < n;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float3 p = v[j][c], q = v[j][(c + 1) % 3];
+            const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+            finite = finite && isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
+            e2 = fmaxf(e2, fminf(dx * dx + dy * dy + dz * dz, kFltMax));
+        }
+        sum += finite ? e2 : 0.0f;
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = sum;
+    block_sync();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < kMeshThreads / 32; ++k) sum += ws[k];
+        *span = sum * ((float)ntri / (float)n);
+    }
+}
+
 // A mesh's arrays from interleaved positions and packed colours: each element once, so bound
 // by its launch at the sizes meshes are refitted at (three strided copies and four memcpys
-// before).  The colours go by words where both ends allow it.
-__global__ void __launch_bounds__(256)
+// before).  The colours go by words where both ends allow it.  The last block sums the new
+// positions' edges beside the others.
+__global__ void __launch_bounds__(kMeshThreads)
 mesh_split_kernel(const float *__restrict__ xyz, const uint8_t *__restrict__ rgb, float *x, float *y, float *z,
-                  uint8_t *rgb_out, uint32_t nvert, uint64_t nbytes, int words)
+                  uint8_t *rgb_out, uint32_t nvert, const uint32_t *__restrict__ idx, uint32_t ntri, int words,
+                  volatile float *span)
 {
-    const uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    const uint32_t nblk = gridDim.x - (span ? 1u : 0u);
+    if (blockIdx.x == nblk) {
+        mesh_span_block(idx, ntri, span, [&](uint32_t i) {
+            return make_float3(xyz[3 * (size_t)i], xyz[3 * (size_t)i + 1], xyz[3 * (size_t)i + 2]);
+        });
+        return;
+    }
+    const uint64_t nbytes = 3ull * ntri;
+    const uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)nblk * blockDim.x;
     for (uint64_t i = i0; i < nvert; i += step) {
         x[i] = xyz[3 * i];
         y[i] = xyz[3 * i + 1];
@@ -310,13 +363,29 @@ mesh_split_kernel(const float *__restrict__ xyz, const uint8_t *__restrict__ rgb
 }
 
 cudaError_t launch_mesh_split(const float *xyz, const uint8_t *rgb, float *x, float *y, float *z, uint8_t *rgb_out,
-                              uint32_t nvert, uint32_t ntri, cudaStream_t s)
+                              uint32_t nvert, const uint32_t *idx, uint32_t ntri, volatile float *span, cudaStream_t s)
 {
     const uint64_t n = std::max<uint64_t>(nvert, ntri);
     if (n == 0) return cudaSuccess;
-    const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, 8ull * (uint64_t)device_sm_count());
-    mesh_split_kernel<<<(unsigned)blocks, 256, 0, s>>>(xyz, rgb, x, y, z, rgb_out, nvert, 3ull * ntri,
-                                                       (reinterpret_cast<uintptr_t>(rgb) & 3u) == 0);
+    if (ntri == 0) span = nullptr;
+    const uint64_t blocks = std::min<uint64_t>((n + kMeshThreads - 1) / kMeshThreads, 2ull * (uint64_t)device_sm_count());
+    mesh_split_kernel<<<(unsigned)blocks + (span ? 1u : 0u), kMeshThreads, 0, s>>>(
+        xyz, rgb, x, y, z, rgb_out, nvert, idx, ntri, (reinterpret_cast<uintptr_t>(rgb) & 3u) == 0, span);
+    return cudaGetLastError();
+}
+
+__global__ void __launch_bounds__(kMeshThreads)
+mesh_span_kernel(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
+                 const uint32_t *__restrict__ idx, uint32_t ntri, volatile float *span)
+{
+    mesh_span_block(idx, ntri, span, [&](uint32_t i) { return make_float3(x[i], y[i], z[i]); });
+}
+
+cudaError_t launch_mesh_span(const float *x, const float *y, const float *z, const uint32_t *idx, uint32_t ntri,
+                             volatile float *span, cudaStream_t s)
+{
+    if (ntri == 0 || !span) return cudaSuccess;
+    mesh_span_kernel<<<1, kMeshThreads, 0, s>>>(x, y, z, idx, ntri, span);
     return cudaGetLastError();
 }
 

@@ -52,7 +52,12 @@ struct sloth_mesh {
     float bbox_max[3] = {0, 0, 0};
     uint32_t *order = nullptr, *oidx = nullptr;   // setup's order of an indexed mesh (spatial_order)
     bool updated = false;   // positions may change on the stream (sloth_mesh_update*)
-    float span2 = 0.0f;   // sum over the triangles of their longest edge squared, when made (mesh_span2)
+    // Sum over the triangles of their longest edge squared, page-locked: of the positions the
+    // mesh was made with (mesh_span2), then of those of the last update that has run
+    // (mesh_span_block); null without memory for it.
+    volatile float *span2 = nullptr;
+
+    float span() const { return span2 ? *span2 : 0.0f; }
 };
 
 struct sloth_ctx {
@@ -381,12 +386,12 @@ struct MeshView {
     uint32_t nvert, ntri;
     int device;
     const uint32_t *order, *oidx;   // setup's order of an indexed mesh (MeshDev), or null
-    float span2;                    // sum of the triangles' longest edges squared (mesh_span2)
 };
 MeshView sloth_mesh_view(const sloth_mesh *m)
 {
-    return MeshView{m->x, m->y, m->z, m->idx, m->rgb, m->nvert, m->ntri, m->device, m->order, m->oidx, m->span2};
+    return MeshView{m->x, m->y, m->z, m->idx, m->rgb, m->nvert, m->ntri, m->device, m->order, m->oidx};
 }
+float sloth_mesh_span2(const sloth_mesh *m) { return m->span(); }
 
 // ---------------------------------------------------------------------------------------
 // host math (restated from the reference and nalgebra 0.22.1; -ffp-contract=off)
@@ -838,11 +843,11 @@ static void spatial_order(const float *x, const float *y, const float *z, const 
     order.swap(src);
 }
 
-// Sum over the triangles of the longest edge squared, from at most 4096 of them spread over
-// the mesh: what draws_without_tiles estimates a draw's samples from.
+// Sum over the triangles of the longest edge squared, from at most kSpanTriangles of them
+// spread over the mesh: what draws_without_tiles and batch_folds estimate a draw's samples from.
 static float mesh_span2(const float *x, const float *y, const float *z, const uint32_t *idx, uint32_t ntri)
 {
-    const uint32_t step = ntri / 4096 + 1;
+    const uint32_t step = (ntri + kSpanTriangles - 1) / kSpanTriangles;
     double sum = 0.0;
     uint32_t n = 0;
     for (uint64_t t = 0; t < ntri; t += step, ++n) {
@@ -898,7 +903,13 @@ sloth_status sloth_mesh_create(sloth_ctx *ctx, const float *x, const float *y, c
     m->device = ctx->device;
     m->nvert = nvert;
     m->ntri = ntri;
-    m->span2 = mesh_span2(x, y, z, idx, ntri);
+    void *span = nullptr;
+    if (cudaMallocHost(&span, sizeof(float)) == cudaSuccess) {
+        m->span2 = static_cast<volatile float *>(span);
+        *m->span2 = mesh_span2(x, y, z, idx, ntri);
+    } else {
+        cudaGetLastError();   // such a mesh keeps the tiles
+    }
     auto cleanup = [&](sloth_status st) {
         sloth_mesh_destroy(m);
         return st;
@@ -974,6 +985,7 @@ void sloth_mesh_destroy(sloth_mesh *m)
     dfree(m->rgb);
     dfree(m->order);
     dfree(m->oidx);
+    if (m->span2) cudaFreeHost(const_cast<float *>(m->span2));   // an update in flight has ended (cudaFree waits)
     delete m;
 }
 
@@ -993,6 +1005,7 @@ sloth_status sloth_mesh_update(sloth_mesh *m, const float *x, const float *y, co
         CU(ctx, cudaMemcpyAsync(m->z, z, nb, cudaMemcpyDefault, ctx->stream));
     }
     if (m->ntri) CU(ctx, cudaMemcpyAsync(m->rgb, rgb, 3 * (size_t)m->ntri, cudaMemcpyDefault, ctx->stream));
+    CU(ctx, launch_mesh_span(m->x, m->y, m->z, m->idx, m->ntri, m->span2, ctx->stream));
     return SLOTH_OK;
 }
 
@@ -1003,7 +1016,7 @@ sloth_status sloth_mesh_update_interleaved(sloth_mesh *m, const float *xyz, cons
     if ((m->nvert && !xyz) || (m->ntri && !rgb)) return fail(ctx, SLOTH_ERR_INVALID_ARGUMENT, "xyz or rgb is NULL");
     CU(ctx, cudaSetDevice(m->device));
     m->updated = true;
-    CU(ctx, launch_mesh_split(xyz, rgb, m->x, m->y, m->z, m->rgb, m->nvert, m->ntri, ctx->stream));
+    CU(ctx, launch_mesh_split(xyz, rgb, m->x, m->y, m->z, m->rgb, m->nvert, m->idx, m->ntri, m->span2, ctx->stream));
     return SLOTH_OK;
 }
 
@@ -1035,8 +1048,10 @@ static sloth_status poll_entry_max(sloth_ctx *ctx)
 }
 
 // Whether a draw goes without tiles (fold.cuh).  The samples it will walk (est) are estimated
-// from the mesh's edges as it was made and the matrix's scale; a mesh of no extent says
-// nothing.  The fold takes about 14 us + 0.3 us per million samples; the tile raster 40 us of
+// from the mesh's edges and the matrix's scale; a mesh of no extent says nothing.  An updated
+// mesh's edges are summed on the device, and the host reads the last sum that has arrived: a
+// draw queued right behind an update that changes the mesh's size goes by the size before,
+// the draws after that update has run by the new one.  The fold takes about 14 us + 0.3 us per million samples; the tile raster 40 us of
 // launches, 0.2 us more per thousand triangles than the fold, and, as its lists grow with
 // them, 0.12 us per sample a cell gets (deep), but next to nothing per sample, which it
 // culls.  Hence the line; us a frame on both sides of it, tiles / fold: 500 triangles at
@@ -1045,8 +1060,8 @@ static sloth_status poll_entry_max(sloth_ctx *ctx)
 // 3840x1426, 1e8, 121 / 97 (tiles kept); 8k at 1921x1079, 1.2e8, 82 / 91; 32k at 1921x1079,
 // 4.1e8, 94 / 170; 262k at 525x371, 3.8e7, 325 / 52; 200k at 1921x1079, 3.7e8, 139 / 190;
 // 500k at 1280x720, 1.6e8, 243 / 222; 1M there, 8.5e8, 466 / 596.  Above kFoldMaxTriangles
-// only for positions as they were made: the estimate of updated ones may be wrong, and the
-// tiles bound what that costs.  There the cells must not be too few for the triangles either,
+// only for positions as they were made: an updated mesh's estimate may be the last update's,
+// and the tiles bound what that costs.  There the cells must not be too few for the triangles either,
 // whose reductions then queue at the same keys (200k at 160x48, 26 a cell, 62 / 55; 262k
 // there, 34, 56 / 70; 1M, 87 / 244); with direct samples on, the tile raster's setup folds the
 // small ones itself (500k fine ones at 1280x720 69 / 89); and the newline rows of a soup in no
@@ -1055,13 +1070,14 @@ static sloth_status poll_entry_max(sloth_ctx *ctx)
 // test needs its tile loads: both keep it.
 static bool draws_without_tiles(const sloth_ctx *ctx, const sloth_mesh *mesh, const Mat4 &M)
 {
-    if (!sloth_ctx_may_fold(ctx) || ctx->fb.wait_test || !(mesh->span2 > 0.0f)) return false;
+    const float span2 = mesh->span();
+    if (!sloth_ctx_may_fold(ctx) || ctx->fb.wait_test || !(span2 > 0.0f)) return false;
     const float cells = (float)ctx->g.w * (float)ctx->g.h;
     if (mesh->ntri > kFoldMaxTriangles &&
         (mesh->updated || mesh->ntri > kFoldMaxTrianglesMade || (float)mesh->ntri > 26.0f * cells ||
          ctx->g.direct_max > 0 || (ctx->g.image && !mesh->order)))
         return false;
-    const float est = fold_estimate(mesh->span2, mesh->ntri, M, ctx->g.w, ctx->g.h);
+    const float est = fold_estimate(span2, mesh->ntri, M, ctx->g.w, ctx->g.h);
     const float deep = std::fmin(est / cells, 2000.0f);
     return est <= 3e7f + 400.0f * (float)mesh->ntri + 2e5f * deep;   // false for NaN
 }

@@ -170,9 +170,17 @@ cudaError_t launch_clear_keys(uint64_t *keys, uint64_t ncells, int tw, bool even
 cudaError_t launch_frame_reset(const FrameBuffers &fb, const BinBuffers &bb, uint32_t nl_nodes, uint32_t ntiles,
                                bool frame, bool draw, bool tiles_current, cudaStream_t s);
 
-// positions split from x, y, z triples and face colours copied into a mesh's arrays.
+// Triangles that the sum of a mesh's longest edges squared is taken from (mesh_span2), spread
+// over the mesh.
+constexpr uint32_t kSpanTriangles = 4096;
+
+// positions split from x, y, z triples and face colours copied into a mesh's arrays; span
+// (page-locked, may be null) gets the sum of the triangles' longest edges squared.
 cudaError_t launch_mesh_split(const float *xyz, const uint8_t *rgb, float *x, float *y, float *z, uint8_t *rgb_out,
-                              uint32_t nvert, uint32_t ntri, cudaStream_t s);
+                              uint32_t nvert, const uint32_t *idx, uint32_t ntri, volatile float *span, cudaStream_t s);
+// that sum alone, from a mesh's own arrays
+cudaError_t launch_mesh_span(const float *x, const float *y, const float *z, const uint32_t *idx, uint32_t ntri,
+                             volatile float *span, cudaStream_t s);
 
 // vertex transform: tv[i] = (M*v_i).xyz (nalgebra order), float4 per vertex.
 cudaError_t launch_vertex_transform(const MeshDev &mesh, const Mat4 &M, float4 *tv,
