@@ -33,6 +33,7 @@ enum { kTabSetup, kTabNewline, kTabResolve, kTabFold, kTables };
 // How a render draws without tiles: not at all, or with the setup of 32 triangles to a block
 // of four warps or of one, or with the batch's own setup kernel (b.tpb a block).
 enum class FoldForm { none, warps4, warps1, setup };
+constexpr int kFoldForms = 4;
 
 struct sloth_batch {
     sloth_ctx *ctx = nullptr;
@@ -49,7 +50,7 @@ struct sloth_batch {
     bool persistent = true;                   // raster over the device queue (else one CTA per item)
     int tpb = kDefaultTrianglesPerBlock;      // triangles per setup block
     FoldForm fold = FoldForm::none;           // what the draws' estimates allow
-    FoldForm folded = FoldForm::none;         // how the graph, and the last render, draw
+    FoldForm folded = FoldForm::none;         // how the last render draws
 
     // layout (per shape)
     std::vector<BatchFrame> hframes;
@@ -94,7 +95,10 @@ struct sloth_batch {
     uint32_t resolve_chunk = kBatchResolveChunk;
     bool any_odd = false;                     // some frame has an odd width
 
-    cudaGraphExec_t graph = nullptr;
+    // the captured renders, one for each form drawn so far (a batch on a line between two would
+    // capture anew every time it crosses), all with depth culling as `graph_cull`
+    cudaGraphExec_t graphs[kFoldForms] = {nullptr, nullptr, nullptr, nullptr};
+    int graph_cull = 1;
     bool rendered = false;
     // a large batch's newline fold beside the rest: forked from and joined into `stream`
     cudaStream_t nl_s = nullptr;
@@ -155,10 +159,17 @@ void bfree(T *&p)
     p = nullptr;
 }
 
+void drop_graphs(sloth_batch *b)
+{
+    for (cudaGraphExec_t &g : b->graphs) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+}
+
 void free_layout(sloth_batch *b)
 {
-    if (b->graph) cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
+    drop_graphs(b);
     bfree(b->d_frames);
     bfree(b->d_draws);
     bfree(b->d_mats);
@@ -538,10 +549,7 @@ sloth_status render_planned(sloth_batch *b)
     BCU(b, cudaStreamSynchronize(s));
     const size_t need = (size_t)*b->h_total;
     if (need > b->entries_cap || !b->bb.entries) {
-        if (b->graph) {
-            cudaGraphExecDestroy(b->graph);
-            b->graph = nullptr;
-        }
+        drop_graphs(b);
         bfree(b->bb.entries);
         bfree(b->bb.items);
         const size_t cap = need + need / 4 + 1024;   // headroom for other transforms
@@ -570,7 +578,7 @@ sloth_status capture(sloth_batch *b)
         if (g) cudaGraphDestroy(g);
         return sloth_ctx_fail(b->ctx, SLOTH_ERR_CUDA, "batch graph capture failed");
     }
-    e = cudaGraphInstantiate(&b->graph, g, 0);
+    e = cudaGraphInstantiate(&b->graphs[(int)b->folded], g, 0);
     cudaGraphDestroy(g);
     BCU(b, e);
     return SLOTH_OK;
@@ -745,22 +753,21 @@ sloth_status sloth_batch_render(sloth_batch *b)
     BCU(b, cudaSetDevice(b->device));
     b->vis_valid = false;
     follow_updates(b);
-    const FoldForm fold = sloth_ctx_may_fold(b->ctx) ? b->fold : FoldForm::none;
-    if (fold != b->folded) {
-        b->folded = fold;
-        if (b->graph) cudaGraphExecDestroy(b->graph);
-        b->graph = nullptr;
-    }
+    b->folded = sloth_ctx_may_fold(b->ctx) ? b->fold : FoldForm::none;
+    const int cull = sloth_ctx_depth_cull(b->ctx);
+    if (cull != b->graph_cull) drop_graphs(b);   // it is an argument of the captured raster
+    b->graph_cull = cull;
     // a render known to have outgrown its entries: the buffer grows before the next one
     const bool tiles = b->folded == FoldForm::none;
     const bool grow = tiles && *(volatile uint32_t *)&b->status[0];
     if (grow || !b->rendered || (tiles && !b->bb.entries)) return render_planned(b);
-    if (!b->graph && b->stream != nullptr) {
+    cudaGraphExec_t &graph = b->graphs[(int)b->folded];
+    if (!graph && b->stream != nullptr) {
         const sloth_status st = capture(b);
         if (st != SLOTH_OK) return st;
     }
-    if (b->graph) {
-        BCU(b, cudaGraphLaunch(b->graph, b->stream));
+    if (graph) {
+        BCU(b, cudaGraphLaunch(graph, b->stream));
         return SLOTH_OK;
     }
     return render_planned(b);
@@ -851,10 +858,7 @@ sloth_status sloth_batch_set_triangles_per_block(sloth_batch *b, int tpb)
     b->nblk[kTabSetup] = (uint32_t)bt.size();
     BCU(b, balloc(&b->blk[kTabSetup], bt.size()));
     if (!bt.empty()) BCU(b, cudaMemcpy(b->blk[kTabSetup], bt.data(), bt.size() * sizeof(int2), cudaMemcpyHostToDevice));
-    if (b->graph) {
-        cudaGraphExecDestroy(b->graph);
-        b->graph = nullptr;
-    }
+    drop_graphs(b);
     return SLOTH_OK;
 }
 
@@ -865,10 +869,7 @@ sloth_status sloth_batch_set_persistent(sloth_batch *b, int persistent)
     BCU(b, cudaStreamSynchronize(b->stream));
     if ((persistent != 0) == b->persistent) return SLOTH_OK;
     b->persistent = persistent != 0;
-    if (b->graph) {
-        cudaGraphExecDestroy(b->graph);   // the raster launch is part of the graph
-        b->graph = nullptr;
-    }
+    drop_graphs(b);   // the raster launch is part of the graph
     return SLOTH_OK;
 }
 
@@ -883,10 +884,7 @@ sloth_status sloth_batch_set_direct_samples(sloth_batch *b, int samples)
     if (b->d_frames)
         BCU(b, cudaMemcpy(b->d_frames, b->hframes.data(), b->hframes.size() * sizeof(BatchFrame),
                           cudaMemcpyHostToDevice));
-    if (b->graph) {
-        cudaGraphExecDestroy(b->graph);   // the key clear of a render depends on the setting
-        b->graph = nullptr;
-    }
+    drop_graphs(b);   // the key clear of a render depends on the setting
     return SLOTH_OK;
 }
 

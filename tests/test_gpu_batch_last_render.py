@@ -47,3 +47,33 @@ def test_read_after_an_overflow_is_the_render_that_overflowed(after, ask):
             for i, f in enumerate(frames):
                 assert_same((*b.read(i), None), oracle_render([m2], Rn, f["w"], f["h"], f["image"], U=f["U"]), f"next {rep}/{i}")
         b.close()
+
+
+def test_a_batch_that_crosses_the_line_keeps_its_graphs():
+    """Transforms on both sides of the line between tiles and none, render after render: every
+    frame exact, from the graph of its own form, and settings that the captured renders depend
+    on capture them again."""
+    m = W.soup(9000, seed=6, n_large=20)
+    R = O.euler_rotation(*W.cli_rotation(yaw=0.8))
+    far = O.mat4_mul(R, np.diag([60.0, 60.0, 60.0, 1.0]).astype(np.float32))
+    w, h = 160, 48
+    U = O.viewport_transform(w, h, O.scene_extent([m["bbox_max"]]))
+    refs = {id(T): oracle_render([m, m], T, w, h, True, U=U) for T in (R, far)}
+    with S.Context(0) as c:
+        dm = S.Mesh(c, m["x"], m["y"], m["z"], m["rgb"], None, m["bbox_max"])
+        b = S.Batch(c, [{"w": w, "h": h, "image": True, "U": U, "draws": [(dm, R), (dm, R)]}])
+
+        def across(n, label):
+            for k in range(n):
+                T = far if k % 2 else R
+                b.set_transforms(np.stack([T, T]))
+                b.render()
+                assert_same((*b.read(0), None), refs[id(T)], f"{label} {k}")
+
+        across(7, "both forms")
+        for change in (lambda: c.set_depth_cull(False), lambda: c.set_depth_cull(True), lambda: b.set_direct_samples(16),
+                       lambda: b.set_triangles_per_block(1024), lambda: b.set_persistent(False),
+                       lambda: b.set_tile_shape(3), lambda: c.set_keep_tiles(True), lambda: c.set_keep_tiles(False)):
+            change()
+            across(4, "after a change of settings")
+        b.close()
