@@ -208,7 +208,8 @@ sloth_status sloth_ctx_set_option(sloth_ctx *ctx, int option, int64_t value);
  * transforms[16*i]) for i < ndraws + resolve, `reps` times per candidate setting, and keeps
  * the fastest (tile shape, direct-sample limit in {0, 4, 16, 64}, triangles per block in
  * {128, 256, 1024, 4096}) as the context's options; reports them and the mean frame time in ms
- * (any output may be NULL).  Needs a viewport and utransform; leaves the context with the
+ * (any output may be NULL).  Where the fastest frame goes without tiles, the settings that do
+ * nothing to it stay as they were.  Needs a viewport and utransform; leaves the context with the
  * last candidate's frame drawn (clear before the next frame). */
 sloth_status sloth_ctx_autotune(sloth_ctx *ctx, const sloth_mesh *const *meshes, const float *transforms,
                                 uint32_t ndraws, int reps, int *best_shape, int *best_direct, int *best_tpb,
@@ -320,7 +321,7 @@ sloth_status sloth_batch_set_triangles_per_block(sloth_batch *batch, int tpb);
  * (tile shape, direct-sample limit in {0, 4, 16, 64}, triangles per block in {128, 256,
  * 1024, 4096}, persistent raster or not), searching one dimension at a time from the current
  * settings, twice over; reports the choice and its mean render time in ms (any output may
- * be NULL).  Every setting renders the same frames. */
+ * be NULL).  A batch that goes without tiles keeps the settings that do nothing to it.  Every setting renders the same frames. */
 sloth_status sloth_batch_autotune(sloth_batch *batch, int reps, int *best_shape, int *best_direct, int *best_tpb,
                                   int *best_persistent, float *best_ms);
 

@@ -944,6 +944,10 @@ sloth_status sloth_batch_autotune(sloth_batch *b, int reps, int *best_shape, int
     sloth_status st = time_tune(b, best, reps, e0, e1, &best_t);
     for (int round = 0; round < 2 && st == SLOTH_OK; ++round) {
         for (int dim = 0; dim < 4 && st == SLOTH_OK; ++dim) {
+            // what a render without tiles does not depend on stays as it is
+            if (b->folded != FoldForm::none &&
+                (dim == 1 || dim == 3 || (dim == 2 && b->folded != FoldForm::setup)))
+                continue;
             const int n = dim == 0 ? kNumTileShapes : dim == 1 ? 4 : dim == 2 ? 4 : 2;
             BatchTune keep = best;
             for (int k = 0; k < n && st == SLOTH_OK; ++k) {

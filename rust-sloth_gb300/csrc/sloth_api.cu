@@ -104,6 +104,7 @@ struct sloth_ctx {
     uint32_t *fold_counts = nullptr;   // queue counters of the draws without tiles (launch_fold_setup)
     bool fold_begun = false;           // they were emptied in this frame
     uint32_t fold_draws = 0;           // such draws of the frame so far
+    uint32_t tiled_draws = 0;          // draws of the frame so far that went through the tiles
     uint64_t fold_last = ~0ull;        // `launches` after the last one's, in its frame
     bool timing = false;
     std::map<std::string, KernelClock> clocks;
@@ -614,6 +615,7 @@ sloth_status sloth_ctx_clear(sloth_ctx *ctx)
     ctx->keys_current = false;
     ctx->fold_begun = false;
     ctx->fold_last = ~0ull;
+    ctx->tiled_draws = 0;
     return SLOTH_OK;
 }
 
@@ -1184,6 +1186,7 @@ sloth_status sloth_draw_mesh(sloth_ctx *ctx, const sloth_mesh *mesh, const float
     CU(ctx, timed(ctx, "raster", [&] {
            return launch_raster(g, ctx->fb, ctx->bb, ctx->depth_cull, ctx->tri_base, s);
        }));
+    ctx->tiled_draws++;
     ctx->tri_base += mesh->ntri;
     ctx->dirty = true;
     return SLOTH_OK;
@@ -1255,8 +1258,12 @@ sloth_status sloth_ctx_autotune(sloth_ctx *ctx, const sloth_mesh *const *meshes,
     };
     int bs = shape0, bd = direct0, bt = tpb0;
     float best = -1.0f;
+    bool best_folded = false;
     sloth_status st = SLOTH_OK;
-    for (int shape = 0; shape < kNumTileShapes && st == SLOTH_OK; ++shape)
+    for (int shape = 0; shape < kNumTileShapes && st == SLOTH_OK; ++shape) {
+        // A frame drawn without tiles throughout does not depend on the other settings: it is
+        // timed once a shape, and they stay as they were if it is the fastest.
+        bool folded = false;
         for (int direct : kCtxDirectCandidates)
             for (int tpb : kTrianglesPerBlockChoices) {
                 if (st != SLOTH_OK) break;
@@ -1265,6 +1272,9 @@ sloth_status sloth_ctx_autotune(sloth_ctx *ctx, const sloth_mesh *const *meshes,
                 ctx->tpb = tpb;
                 st = frame();                          // sizes buffers for this setting
                 if (st == SLOTH_OK) st = sloth_ctx_synchronize(ctx);
+                const bool tiles = ctx->tiled_draws != 0;
+                if (st == SLOTH_OK && folded && !tiles) continue;
+                folded = folded || !tiles;
                 if (st == SLOTH_OK) st = frame();      // warm
                 if (st != SLOTH_OK) break;
                 cudaEventRecord(e0, ctx->stream);
@@ -1279,9 +1289,19 @@ sloth_status sloth_ctx_autotune(sloth_ctx *ctx, const sloth_mesh *const *meshes,
                         bs = shape;
                         bd = direct;
                         bt = tpb;
+                        best_folded = !tiles;
                     }
                 }
             }
+    }
+    if (st == SLOTH_OK && best_folded) {
+        ctx->tile_shape = bs;
+        ctx->direct_max = direct0;
+        ctx->tpb = bt = tpb0;
+        st = frame();
+        if (ctx->tiled_draws == 0) bd = direct0;
+        if (st == SLOTH_OK) st = sloth_ctx_synchronize(ctx);
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     ctx->timing = timing0;
