@@ -79,9 +79,10 @@ class ShadedViews:
 
     def shade_backward(self, vrgb, light, grad_rgb):
         self._check_stream()
-        # one buffer, cleared at once
-        buf = torch.zeros(2 * self.nvert + 1, 3, dtype=torch.float32, device=self.device)
-        gpos, gcol, gl = buf[:self.nvert], buf[self.nvert:2 * self.nvert], buf[2 * self.nvert]
+        # three tensors, not views of one: a caller may keep, detach or resize each by itself
+        gpos = torch.zeros(self.nvert, 3, dtype=torch.float32, device=self.device)
+        gcol = torch.zeros(self.nvert, 3, dtype=torch.float32, device=self.device)
+        gl = torch.zeros(3, dtype=torch.float32, device=self.device)
         self.batch.shade_backward(vrgb.data_ptr(), light.data_ptr(), grad_rgb.data_ptr(), gpos.data_ptr(),
                                   gcol.data_ptr(), gl.data_ptr())
         return gpos, gcol, gl

@@ -1,0 +1,42 @@
+"""What a program may do with ShadedViews beyond a fit: keep one gradient and let the others
+go, detach it in place, and subclass render and shade."""
+import numpy as np
+import pytest
+
+import sloth_gpu as S
+import workloads as W
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+import diff_render as DR  # noqa: E402
+
+
+def views(cls):
+    m = W.displaced_icosphere(2, seed=1)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        ctx = S.Context(0, stream=stream.cuda_stream)
+        U = S.viewport_transform(80, 40, S.scene_extent([m["bbox_max"]]))
+        sv = cls(ctx, m, [{"w": 80, "h": 40, "image": False, "U": U, "R": np.eye(4, dtype=np.float32)}], stream)
+        p = torch.from_numpy(np.stack([m["x"], m["y"], m["z"]], 1)).cuda()
+        v = torch.rand(p.shape[0], 3, device="cuda")
+        light = torch.tensor([0.1, 0.2, 0.9], device="cuda")
+    return ctx, sv, stream, [t.requires_grad_(True) for t in (p, v, light)]
+
+
+def test_each_gradient_stands_by_itself():
+    ctx, sv, stream, leaves = views(DR.ShadedViews)
+    with torch.cuda.stream(stream):
+        DR.shade_views(*leaves, sv).sum().backward()
+        grads = [t.grad for t in leaves]
+        assert all((g != 0).any() for g in grads)
+        assert len({g.untyped_storage().data_ptr() for g in grads}) == 3
+        for t, g in zip(leaves, grads):
+            assert g.untyped_storage().nbytes() == 4 * t.numel() and g.shape == t.shape
+            g.detach_()
+            before = [o._version for o in grads if o is not g]
+            g.zero_()
+            assert [o._version for o in grads if o is not g] == before
+        torch.cuda.synchronize()
+    sv.close()
+    ctx.close()
