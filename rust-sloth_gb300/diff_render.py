@@ -54,9 +54,6 @@ class ShadedViews:
     def render(self, pos: torch.Tensor):
         """Upload (nvert, 3) positions and render every view."""
         self._check_stream()
-        self._render(pos)
-
-    def _render(self, pos: torch.Tensor):
         p = pos.detach().to(torch.float32)
         if p.device == self.device and p.shape == (self.nvert, 3):
             self._keep = p = p.contiguous()     # the kernel reads it asynchronously
@@ -70,9 +67,6 @@ class ShadedViews:
     def shade(self, vrgb: torch.Tensor, light: torch.Tensor) -> torch.Tensor:
         """(ncells, 3) f32 image of the last render."""
         self._check_stream()
-        return self._shade(vrgb, light)
-
-    def _shade(self, vrgb: torch.Tensor, light: torch.Tensor) -> torch.Tensor:
         out = torch.empty(self.ncells, 3, dtype=torch.float32, device=self.device)
         self.batch.shade(vrgb.data_ptr(), light.data_ptr(), out.data_ptr(), self.store_visibility)
         return out
@@ -101,9 +95,8 @@ class _ShadeFn(torch.autograd.Function):
     def forward(ctx, pos, vrgb, light, views: ShadedViews):
         vrgb_c = vrgb.detach().contiguous().to(torch.float32)
         light_c = light.detach().contiguous().to(torch.float32)
-        views._check_stream()
-        views._render(pos)
-        rgb = views._shade(vrgb_c, light_c)
+        views.render(pos)
+        rgb = views.shade(vrgb_c, light_c)
         ctx.views = views
         ctx.save_for_backward(vrgb_c, light_c)
         return rgb

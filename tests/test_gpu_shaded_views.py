@@ -40,3 +40,31 @@ def test_each_gradient_stands_by_itself():
         torch.cuda.synchronize()
     sv.close()
     ctx.close()
+
+
+def test_a_subclass_sees_every_call():
+    calls = []
+
+    class Logged(DR.ShadedViews):
+        def render(self, pos):
+            calls.append("render")
+            super().render(pos)
+
+        def shade(self, vrgb, light):
+            calls.append("shade")
+            return super().shade(vrgb, light) * 2.0
+
+        def shade_backward(self, vrgb, light, grad_rgb):
+            calls.append("shade_backward")
+            return super().shade_backward(vrgb, light, grad_rgb)
+
+    ctx, sv, stream, leaves = views(Logged)
+    with torch.cuda.stream(stream):
+        rgb = DR.shade_views(*leaves, sv)
+        plain = DR.ShadedViews.shade(sv, leaves[1].detach(), leaves[2].detach())
+        assert torch.equal(rgb, 2.0 * plain) and (plain > 0).any()
+        rgb.sum().backward()
+        assert calls == ["render", "shade", "shade_backward"]
+        torch.cuda.synchronize()
+    sv.close()
+    ctx.close()
