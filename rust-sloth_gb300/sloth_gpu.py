@@ -321,9 +321,9 @@ FLUSH_PLAIN, FLUSH_ANSI, FLUSH_HTML = 0, 1, 2
 # A bytes object of a given size to be filled once by the library before anyone else sees it
 # (PyBytes_FromStringAndSize with no source): the text is copied straight into the result.
 # Zeroing a buffer and copying out of it twice took 600 us of an 800 us flush of 8 MB.
-_new_bytes = C.pythonapi.PyBytes_FromStringAndSize
-_new_bytes.restype = C.py_object
-_new_bytes.argtypes = [C.c_void_p, C.c_ssize_t]
+# A function object of this module's own: ctypes.pythonapi's is shared by the whole process, and
+# so would its argument types be.
+_new_bytes = C.PYFUNCTYPE(C.py_object, C.c_void_p, C.c_ssize_t)(("PyBytes_FromStringAndSize", C.pythonapi))
 
 
 def _flush_bytes(call) -> bytes:
