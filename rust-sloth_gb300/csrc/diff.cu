@@ -30,6 +30,9 @@ namespace {
 
 constexpr uint32_t kNoTri = 0xffffffffu;
 constexpr int kDiffThreads = 256;
+// A gradient whose components come to this or more, or are not finite, keeps to its own sample:
+// the sums of a run of 32 (up to 496 times it) stay below the largest float.
+constexpr float kRunMax = 1e35f;
 
 struct Hit {
     uint32_t tri;      // frame-local triangle (draw order), kNoTri when none
@@ -382,8 +385,9 @@ batch_shade_backward_kernel(BatchDev b, const int2 *__restrict__ blocks, const f
         }
         if (!__any_sync(0xffffffffu, h.tri != kNoTri)) continue;
         // a run: one triangle over consecutive samples of a row.  A gradient that is not
-        // finite keeps to its own sample, so that it reaches what it reached by itself.
-        const bool wild = h.tri != kNoTri && !(fabsf(go.x) + fabsf(go.y) + fabsf(go.z) < INFINITY);
+        // finite, or would overflow the run's sums, keeps to its own sample, so that it
+        // reaches what it reached by itself.
+        const bool wild = h.tri != kNoTri && !(fabsf(go.x) + fabsf(go.y) + fabsf(go.z) < kRunMax);
         const bool split = __any_sync(0xffffffffu, wild);
         const uint32_t pt = __shfl_up_sync(0xffffffffu, h.tri, 1);
         const int pxl = __shfl_up_sync(0xffffffffu, h.x, 1), pyl = __shfl_up_sync(0xffffffffu, h.y, 1);
