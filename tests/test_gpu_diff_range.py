@@ -23,13 +23,13 @@ def test_large_finite_gradients(env, w, h, store):
                             & (np.arange(w - 4)[None, :] % 2 == 0))
     big = np.float32(1.5e38)
     checked = 0
-    for k in range(0, rows.size, max(1, rows.size // 12)):
+    for k in range(0, rows.size, max(1, rows.size // 40)):
         g = np.zeros_like(grad)
         at = rows[k] * w + cols[k]
         g[[at, at + 2, at + 4], 0] = big
         want = D.shade_vjp(host_pos(m).astype(np.float64), vrgb.astype(np.float64), np.array(LIGHT), m["idx"], ov,
                            g.astype(np.float64))[1]
-        if not np.abs(want).max() < 2e38:
+        if not 1e37 < np.abs(want).max() < 2e38:    # unlit, or past the largest float itself
             continue
         got = backward(env, sv, m, vrgb, g)[1]
         assert np.isfinite(got).all()
