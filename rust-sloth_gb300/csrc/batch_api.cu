@@ -383,8 +383,6 @@ sloth_status build(sloth_batch *b, int shape)
     BCU(b, balloc(&b->large_frame, rec));
     BCU(b, balloc(&b->bb.slice_offset, tiles + kSliceExtra));
     BCU(b, balloc(&b->queue, 1));
-    BCU(b, balloc(&b->bb.fill_list, fill_words16(rec)));
-    b->bb.fill_meta = reinterpret_cast<uint32_t *>(b->bb.fill_list + rec);
     BCU(b, balloc(&b->fill_count, 1));
     BCU(b, balloc(&b->d_mats, nd));
     for (uint32_t f = 0; f < nf; ++f) {
@@ -537,13 +535,17 @@ cudaError_t enqueue_back(sloth_batch *b, const BatchDev &d, cudaStream_t s)
 sloth_status render_planned(sloth_batch *b)
 {
     cudaStream_t s = b->stream;
-    BatchDev d = dev_view(b);
     b->status[0] = 0;
     if (b->folded != FoldForm::none) {   // no entries to size
-        BCU(b, enqueue_folded(b, d, s));
+        BCU(b, enqueue_folded(b, dev_view(b), s));
         b->rendered = true;
         return SLOTH_OK;
     }
+    if (!b->bb.fill_list) {   // 20 bytes a triangle that a batch without tiles does not need
+        BCU(b, balloc(&b->bb.fill_list, fill_words16(b->total_rec)));
+        b->bb.fill_meta = reinterpret_cast<uint32_t *>(b->bb.fill_list + b->total_rec);
+    }
+    BatchDev d = dev_view(b);
     BCU(b, enqueue_front(b, d, s));
     BCU(b, cudaMemcpyAsync(b->h_total, b->bb.tile_offset + b->total_tiles, 4, cudaMemcpyDeviceToHost, s));
     BCU(b, cudaStreamSynchronize(s));
