@@ -356,7 +356,8 @@ def run_gpu(args):
         step()
     torch.cuda.synchronize()
     kernels = {}
-    for name in ("reset", "vertex", "setup", "newline", "bin_count_large", "bin_scan", "bin_fill", "bin_fill_large", "bin_items", "raster", "resolve"):
+    for name in ("reset", "vertex", "setup", "newline", "bin_count_large", "bin_scan", "bin_fill", "raster", "fold",
+                 "fold_large", "resolve"):
         t, n = ctx.kernel_time(name)
         if n:
             kernels[name] = {"ms_per_launch": t / n, "launches": n}

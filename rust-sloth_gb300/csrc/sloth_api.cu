@@ -337,11 +337,6 @@ static sloth_status report_device_error(sloth_ctx *ctx)
 // The newline fold of a draw's triangles on its own stream, after everything queued so far.
 static sloth_status fork_newline(sloth_ctx *ctx, const MeshDev &md)
 {
-    if (!ctx->nl_stream) {
-        CU(ctx, cudaStreamCreateWithFlags(&ctx->nl_stream, cudaStreamNonBlocking));
-        CU(ctx, cudaEventCreateWithFlags(&ctx->setup_ev, cudaEventDisableTiming));
-        CU(ctx, cudaEventCreateWithFlags(&ctx->nl_ev, cudaEventDisableTiming));
-    }
     CU(ctx, cudaEventRecord(ctx->setup_ev, ctx->stream));
     CU(ctx, cudaStreamWaitEvent(ctx->nl_stream, ctx->setup_ev, 0));
     CU(ctx, timed(ctx, "newline", [&] {
@@ -363,6 +358,18 @@ static sloth_status resolve_pending(sloth_ctx *ctx)
     CU(ctx, timed(ctx, "resolve", [&] { return launch_resolve(ctx->g, ctx->fb, ctx->stream); }));
     ctx->dirty = false;
     return SLOTH_OK;
+}
+
+// Frames of at most kStageCells cells are read through page-locked memory (readback_kernel):
+// 160x48 with all three buffers 71 us a frame with a copy each, 43 so; larger ones keep
+// the copy engine, whose copies need no second pass over the bytes on the host.  Without the
+// memory every frame does.
+constexpr size_t kStageCells = 32768;
+static void stage_memory(sloth_ctx *ctx)
+{
+    if (cudaMallocHost(&ctx->h_stage, (3 * (kStageCells + 4) + 4) * sizeof(uint32_t)) == cudaSuccess) return;
+    cudaGetLastError();
+    ctx->h_stage = nullptr;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -499,12 +506,20 @@ sloth_status sloth_ctx_create(sloth_ctx **out, int device, void *stream)
         cudaMallocHost(&ctx->h_error, sizeof(uint32_t)) != cudaSuccess ||
         cudaMalloc(&ctx->fb.error, sizeof(uint32_t)) != cudaSuccess ||
         cudaMemset(ctx->fb.error, 0, sizeof(uint32_t)) != cudaSuccess ||
-        cudaMallocHost(&ctx->h_outgrew, sizeof(uint32_t)) != cudaSuccess) {
+        cudaMallocHost(&ctx->h_outgrew, sizeof(uint32_t)) != cudaSuccess ||
+        dalloc(&ctx->fold_counts, 2 * kFoldSlots) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&ctx->nl_stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->setup_ev, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->nl_ev, cudaEventDisableTiming) != cudaSuccess) {
         if (ctx->h_total) cudaFreeHost(ctx->h_total);
         if (ctx->h_frags) cudaFreeHost(ctx->h_frags);
         if (ctx->h_error) cudaFreeHost(ctx->h_error);
         if (ctx->fb.error) cudaFree(ctx->fb.error);
         if (ctx->h_outgrew) cudaFreeHost(ctx->h_outgrew);
+        dfree(ctx->fold_counts);
+        if (ctx->nl_stream) cudaStreamDestroy(ctx->nl_stream);
+        if (ctx->setup_ev) cudaEventDestroy(ctx->setup_ev);
+        if (ctx->nl_ev) cudaEventDestroy(ctx->nl_ev);
         if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
         delete ctx;
         return SLOTH_ERR_OUT_OF_MEMORY;
@@ -512,6 +527,7 @@ sloth_status sloth_ctx_create(sloth_ctx **out, int device, void *stream)
     *ctx->h_error = 0;
     *ctx->h_outgrew = 0;
     ctx->bb.outgrew = ctx->h_outgrew;
+    stage_memory(ctx);   // here, not in the first read
     *out = ctx;
     return SLOTH_OK;
 }
@@ -628,18 +644,6 @@ sloth_status sloth_ctx_sizes(const sloth_ctx *ctx, uint64_t *frame_cells, uint64
     return SLOTH_OK;
 }
 
-// Frames of at most kStageCells cells are read through page-locked memory (readback_kernel):
-// 160x48 with all three buffers 71 us a frame with a copy each, 43 so; larger ones keep
-// the copy engine, whose copies need no second pass over the bytes on the host.
-constexpr size_t kStageCells = 32768;
-static bool stage_memory(sloth_ctx *ctx)
-{
-    if (cudaMallocHost(&ctx->h_stage, (3 * (kStageCells + 4) + 4) * sizeof(uint32_t)) == cudaSuccess) return true;
-    cudaGetLastError();
-    ctx->h_stage = nullptr;
-    return false;
-}
-
 static sloth_status read_staged(sloth_ctx *ctx, uint32_t *cells, float *z, int32_t *winner, uint32_t ncells,
                                 uint32_t nz)
 {
@@ -671,7 +675,7 @@ sloth_status sloth_ctx_read(sloth_ctx *ctx, uint32_t *cells, float *z, int32_t *
     if (st != SLOTH_OK) return st;
     const size_t nz = (size_t)ctx->g.w * ctx->g.h;
     const size_t ncells = ctx->g.image ? nz + ctx->g.h : nz;
-    if (ncells <= kStageCells && (ctx->h_stage || stage_memory(ctx)))
+    if (ncells <= kStageCells && ctx->h_stage)
         return read_staged(ctx, cells, z, winner, (uint32_t)ncells, (uint32_t)nz);
     if (cells)
         CU(ctx, cudaMemcpyAsync(cells, ctx->fb.cells_out, ncells * sizeof(uint32_t),
@@ -1090,7 +1094,6 @@ static sloth_status draw_folded(sloth_ctx *ctx, const sloth_mesh *mesh, const Ma
 {
     sloth_status st;
     cudaStream_t s = ctx->stream;
-    if (!ctx->fold_counts) CU(ctx, dalloc(&ctx->fold_counts, 2 * kFoldSlots));
     if (ctx->reset_pending || !ctx->keys_current || !ctx->fold_begun) {
         if ((st = join_newline(ctx)) != SLOTH_OK) return st;   // the last frame's fold into the tree
         const bool frame = ctx->reset_pending;
