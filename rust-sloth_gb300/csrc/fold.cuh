@@ -316,20 +316,20 @@ __device__ __forceinline__ uint32_t fold_queue_walk(const FoldQueue &queue, uint
         const Index it = base + (Index)lane * nwarps;
         uint32_t q = 0, part = 0, tri = 0;
         bool live = it < items.all;
-        const bool is_large = it < items.cut;
         if (live) {
             q = items.entry(it, part);
             tri = queue.tri[q];
             const int4 xr = *(reinterpret_cast<const int4 *>(frame_of(q).fb.records + tri) + 4);
-            live = xr.z + (int)part * (is_large ? kFoldRows : kFoldMidRows) < xr.w;
+            live = xr.z + (int)part * (it < items.cut ? kFoldRows : kFoldMidRows) < xr.w;
+            // a large one's part carries the class (the walk below has no register to spare)
+            if (it < items.cut) part |= 0x80000000u;
         }
-        const unsigned larges = __ballot_sync(0xffffffffu, is_large);
         for (unsigned todo = __ballot_sync(0xffffffffu, live); todo; todo &= todo - 1u) {
             const int src = __ffs(todo) - 1;
             const uint32_t wq = __shfl_sync(0xffffffffu, q, src), wt = __shfl_sync(0xffffffffu, tri, src),
                            wp = __shfl_sync(0xffffffffu, part, src);
             const auto &f = frame_of(wq);
-            if (larges >> src & 1u) frags += fold_queued<kFoldRows>(wt, wp, kFoldParts, filter, f.g, f.fb);
+            if (wp >> 31) frags += fold_queued<kFoldRows>(wt, wp & 0x7fffffffu, kFoldParts, filter, f.g, f.fb);
             else if (!whole) frags += fold_queued<kFoldMidRows>(wt, wp, kFoldMidParts, filter, f.g, f.fb);
             else frags += fold_queued<32>(wt, 0u, 1u, filter, f.g, f.fb);
         }
