@@ -360,6 +360,11 @@ sloth_status sloth_batch_shade(sloth_batch *batch, const float *vertex_rgb, cons
 sloth_status sloth_batch_shade_backward(sloth_batch *batch, const float *vertex_rgb, const float *light,
                                         const float *grad_rgb, float *grad_pos, float *grad_vertex_rgb,
                                         float *grad_light);
+/* sloth_batch_shade_backward with grad_pos, grad_vertex_rgb and grad_light set to the gradients
+ * instead of added to: they are cleared first, by one kernel. */
+sloth_status sloth_batch_shade_gradients(sloth_batch *batch, const float *vertex_rgb, const float *light,
+                                         const float *grad_rgb, float *grad_pos, float *grad_vertex_rgb,
+                                         float *grad_light);
 
 /* ---- one frame without device allocation ------------------------------------------ */
 

@@ -1005,17 +1005,34 @@ sloth_status sloth_batch_shade(sloth_batch *b, const float *vertex_rgb, const fl
     return SLOTH_OK;
 }
 
-sloth_status sloth_batch_shade_backward(sloth_batch *b, const float *vertex_rgb, const float *light,
-                                        const float *grad_rgb, float *grad_pos, float *grad_vertex_rgb,
-                                        float *grad_light)
+static sloth_status shade_backward(sloth_batch *b, const float *vertex_rgb, const float *light, const float *grad_rgb,
+                                   float *grad_pos, float *grad_vertex_rgb, float *grad_light, bool clear)
 {
     if (!b || !b->ctx || !grad_rgb) return SLOTH_ERR_INVALID_ARGUMENT;
     sloth_status st = diff_prepare(b, vertex_rgb, light);
     if (st != SLOTH_OK) return st;
+    if (clear) {
+        const uint32_t nvert = b->meshes.empty() ? 0u : sloth_mesh_view(b->meshes[0]).nvert;
+        BCU(b, launch_clear_gradients(grad_pos, grad_vertex_rgb, grad_light, nvert, b->stream));
+    }
     BCU(b, launch_batch_shade_backward(dev_view(b), b->diff_blk, b->ndiff_blk, vertex_rgb, light, grad_rgb,
                                        b->vis_valid ? b->vis : nullptr, grad_pos, grad_vertex_rgb, grad_light,
                                        b->stream));
     return SLOTH_OK;
+}
+
+sloth_status sloth_batch_shade_backward(sloth_batch *b, const float *vertex_rgb, const float *light,
+                                        const float *grad_rgb, float *grad_pos, float *grad_vertex_rgb,
+                                        float *grad_light)
+{
+    return shade_backward(b, vertex_rgb, light, grad_rgb, grad_pos, grad_vertex_rgb, grad_light, false);
+}
+
+sloth_status sloth_batch_shade_gradients(sloth_batch *b, const float *vertex_rgb, const float *light,
+                                         const float *grad_rgb, float *grad_pos, float *grad_vertex_rgb,
+                                         float *grad_light)
+{
+    return shade_backward(b, vertex_rgb, light, grad_rgb, grad_pos, grad_vertex_rgb, grad_light, true);
 }
 
 sloth_status sloth_tile_shape(int shape, uint32_t *cells, uint32_t *rows)

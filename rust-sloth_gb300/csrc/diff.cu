@@ -428,7 +428,26 @@ batch_shade_backward_kernel(BatchDev b, const int2 *__restrict__ blocks, const f
     }
 }
 
+__global__ void __launch_bounds__(kDiffThreads) clear_gradients_kernel(float *gpos, float *gcol, float *glight, uint64_t n)
+{
+    const uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = i0; i < n; i += step) {
+        if (gpos) gpos[i] = 0.0f;
+        if (gcol) gcol[i] = 0.0f;
+    }
+    if (glight && i0 < 3) glight[i0] = 0.0f;
+}
+
 }  // namespace
+
+cudaError_t launch_clear_gradients(float *gpos, float *gcol, float *glight, uint32_t nvert, cudaStream_t s)
+{
+    const uint64_t n = 3ull * nvert, most = 8ull * (uint64_t)device_sm_count();
+    const uint64_t blocks = (n + kDiffThreads - 1) / kDiffThreads;
+    clear_gradients_kernel<<<(unsigned)(blocks < 1 ? 1 : blocks < most ? blocks : most), kDiffThreads, 0, s>>>(gpos, gcol,
+                                                                                                         glight, n);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_batch_shade(const BatchDev &b, const int2 *blocks, uint32_t nblocks, const float *vrgb,
                                const float *light, float *rgb, uint2 *vis, cudaStream_t s)

@@ -327,9 +327,12 @@ __device__ __forceinline__ void mesh_span_block(const uint32_t *__restrict__ idx
     for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
     if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = sum;
     block_sync();
-    if (threadIdx.x == 0) {
-        for (int k = 1; k < kMeshThreads / 32; ++k) sum += ws[k];
-        *span = sum * ((float)ntri / (float)n);
+    if (threadIdx.x < 32) {
+        static_assert(kMeshThreads == 32 * 32, "a lane per warp");
+        sum = ws[threadIdx.x];
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        if (threadIdx.x == 0) *span = sum * ((float)ntri / (float)n);
     }
 }
 

@@ -1,7 +1,7 @@
 """Differentiable shading of many views of one mesh, as a torch.autograd.Function.
 
 The renderer and both shading passes are the library's (sloth_batch_render,
-sloth_batch_shade, sloth_batch_shade_backward); torch only holds the device tensors,
+sloth_batch_shade, sloth_batch_shade_gradients); torch only holds the device tensors,
 orders the work on one CUDA stream and runs the loss and the optimiser.  The reference
 renderer has no differentiable path (its shading is the normal's z of
 src/rasterizer.rs:76); the image and its adjoint are documented in include/sloth_gpu.h.
@@ -73,12 +73,13 @@ class ShadedViews:
 
     def shade_backward(self, vrgb, light, grad_rgb):
         self._check_stream()
-        # three tensors, not views of one: a caller may keep, detach or resize each by itself
-        gpos = torch.zeros(self.nvert, 3, dtype=torch.float32, device=self.device)
-        gcol = torch.zeros(self.nvert, 3, dtype=torch.float32, device=self.device)
-        gl = torch.zeros(3, dtype=torch.float32, device=self.device)
-        self.batch.shade_backward(vrgb.data_ptr(), light.data_ptr(), grad_rgb.data_ptr(), gpos.data_ptr(),
-                                  gcol.data_ptr(), gl.data_ptr())
+        # three tensors, not views of one: a caller may keep, detach or resize each by itself;
+        # cleared by one kernel of the call (three torch.zeros take the host 32 us)
+        gpos = torch.empty(self.nvert, 3, dtype=torch.float32, device=self.device)
+        gcol = torch.empty(self.nvert, 3, dtype=torch.float32, device=self.device)
+        gl = torch.empty(3, dtype=torch.float32, device=self.device)
+        self.batch.shade_gradients(vrgb.data_ptr(), light.data_ptr(), grad_rgb.data_ptr(), gpos.data_ptr(),
+                                   gcol.data_ptr(), gl.data_ptr())
         return gpos, gcol, gl
 
     def view_image(self, rgb: torch.Tensor, i: int) -> torch.Tensor:

@@ -90,6 +90,7 @@ SIGNATURES = {
     "sloth_batch_flush": (C.c_int, [_vp, C.c_uint32, C.c_int, C.c_char_p, C.c_uint64, _u64p]),
     "sloth_batch_shade": (C.c_int, [_vp, _vp, _vp, _vp, C.c_int]),
     "sloth_batch_shade_backward": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "sloth_batch_shade_gradients": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "sloth_ctx_set_timing": (C.c_int, [_vp, C.c_int]),
     "sloth_ctx_kernel_time": (C.c_int, [_vp, C.c_char_p, C.POINTER(C.c_double), _u64p]),
     "sloth_ctx_launch_count": (C.c_uint64, [_vp]),
@@ -518,6 +519,13 @@ class Batch:
     def shade_backward(self, vertex_rgb: int, light: int, grad_rgb: int, grad_pos: int = 0,
                        grad_vertex_rgb: int = 0, grad_light: int = 0):
         self.ctx._check(self.lib.sloth_batch_shade_backward(
+            self.h, C.c_void_p(vertex_rgb), C.c_void_p(light), C.c_void_p(grad_rgb),
+            C.c_void_p(grad_pos or None), C.c_void_p(grad_vertex_rgb or None), C.c_void_p(grad_light or None)))
+
+    def shade_gradients(self, vertex_rgb: int, light: int, grad_rgb: int, grad_pos: int = 0,
+                        grad_vertex_rgb: int = 0, grad_light: int = 0):
+        """shade_backward into buffers of any content: set to the gradients, not added to."""
+        self.ctx._check(self.lib.sloth_batch_shade_gradients(
             self.h, C.c_void_p(vertex_rgb), C.c_void_p(light), C.c_void_p(grad_rgb),
             C.c_void_p(grad_pos or None), C.c_void_p(grad_vertex_rgb or None), C.c_void_p(grad_light or None)))
 
