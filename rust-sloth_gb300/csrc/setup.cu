@@ -290,70 +290,64 @@ cudaError_t launch_vertex_transform(const MeshDev &mesh, const Mat4 &M, float4 *
     return launch_pdl(vertex_transform_kernel, dim3((quads + 255) / 256), dim3(256), 0, s, mesh, M, tv);
 }
 
-constexpr int kMeshThreads = 1024;
+constexpr int kMeshThreads = 256;
+static_assert(kSpanParts * kMeshThreads == kSpanTriangles, "a triangle a thread");
 
-// The sum over a mesh's triangles of their longest edge squared, by one block, as mesh_span2
-// takes it on the host: at most kSpanTriangles of them, four a thread, their loads in flight
-// together.  Triangles with a coordinate that is not finite count nothing.
+// Part `part` of the sum over a mesh's triangles of their longest edge squared, as mesh_span2
+// takes it on the host, by a block: a triangle a thread, at most kSpanTriangles in all.
+// Triangles with a coordinate that is not finite count nothing.
 template <class Position>
-__device__ __forceinline__ void mesh_span_block(const uint32_t *__restrict__ idx, uint32_t ntri, volatile float *span,
-                                                Position at)
+__device__ __forceinline__ void mesh_span_block(uint32_t part, const uint32_t *__restrict__ idx, uint32_t ntri,
+                                                volatile float *span, Position at)
 {
     __shared__ float ws[kMeshThreads / 32];
-    constexpr int kEach = (int)kSpanTriangles / kMeshThreads;
     const uint32_t step = (ntri + kSpanTriangles - 1) / kSpanTriangles, n = (ntri + step - 1) / step;
-    float3 v[kEach][3];
-#pragma unroll
-    for (int j = 0; j < kEach; ++j) {
-        const uint32_t k = threadIdx.x + (uint32_t)(j * kMeshThreads), t = (k < n ? k : 0u) * step;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) v[j][c] = at(idx ? idx[3 * (size_t)t + c] : 3 * t + c);
-    }
+    const uint32_t k = part * kMeshThreads + threadIdx.x;
     float sum = 0.0f;
+    if (k < n) {
+        const uint32_t t = k * step;
+        float3 v[3];
 #pragma unroll
-    for (int j = 0; j < kEach; ++j) {
-        float e2 = 0.0f;
-        bool finite = threadIdx.x + (uint32_t)(j * kMeshThreads) < n;
+        for (int c = 0; c < 3; ++c) v[c] = at(idx ? idx[3 * (size_t)t + c] : 3 * t + c);
+        bool finite = true;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const float3 p = v[j][c], q = v[j][(c + 1) % 3];
+            const float3 p = v[c], q = v[(c + 1) % 3];
             const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
             finite = finite && isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
-            e2 = fmaxf(e2, fminf(dx * dx + dy * dy + dz * dz, kFltMax));
+            sum = fmaxf(sum, fminf(dx * dx + dy * dy + dz * dz, kFltMax));
         }
-        sum += finite ? e2 : 0.0f;
+        if (!finite) sum = 0.0f;
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
     if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = sum;
     block_sync();
-    if (threadIdx.x < 32) {
-        static_assert(kMeshThreads == 32 * 32, "a lane per warp");
-        sum = ws[threadIdx.x];
+    if (threadIdx.x == 0) {
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
-        if (threadIdx.x == 0) *span = sum * ((float)ntri / (float)n);
+        for (int w = 1; w < kMeshThreads / 32; ++w) sum += ws[w];
+        span[part] = sum * ((float)ntri / (float)n);
     }
 }
 
 // A mesh's arrays from interleaved positions and packed colours: each element once, so bound
 // by its launch at the sizes meshes are refitted at (three strided copies and four memcpys
-// before).  The colours go by words where both ends allow it.  The last block sums the new
-// positions' edges beside the others.
+// before).  The colours go by words where both ends allow it.  The first kSpanParts blocks sum
+// the new positions' edges beside the others.
 __global__ void __launch_bounds__(kMeshThreads)
 mesh_split_kernel(const float *__restrict__ xyz, const uint8_t *__restrict__ rgb, float *x, float *y, float *z,
                   uint8_t *rgb_out, uint32_t nvert, const uint32_t *__restrict__ idx, uint32_t ntri, int words,
                   volatile float *span)
 {
-    const uint32_t nblk = gridDim.x - (span ? 1u : 0u);
-    if (blockIdx.x == nblk) {
-        mesh_span_block(idx, ntri, span, [&](uint32_t i) {
+    const uint32_t parts = span ? kSpanParts : 0u;
+    if (blockIdx.x < parts) {
+        mesh_span_block(blockIdx.x, idx, ntri, span, [&](uint32_t i) {
             return make_float3(xyz[3 * (size_t)i], xyz[3 * (size_t)i + 1], xyz[3 * (size_t)i + 2]);
         });
         return;
     }
-    const uint64_t nbytes = 3ull * ntri;
-    const uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)nblk * blockDim.x;
+    const uint64_t nbytes = 3ull * ntri, step = (uint64_t)(gridDim.x - parts) * blockDim.x;
+    const uint64_t i0 = (blockIdx.x - parts) * (uint64_t)blockDim.x + threadIdx.x;
     for (uint64_t i = i0; i < nvert; i += step) {
         x[i] = xyz[3 * i];
         y[i] = xyz[3 * i + 1];
@@ -371,8 +365,8 @@ cudaError_t launch_mesh_split(const float *xyz, const uint8_t *rgb, float *x, fl
     const uint64_t n = std::max<uint64_t>(nvert, ntri);
     if (n == 0) return cudaSuccess;
     if (ntri == 0) span = nullptr;
-    const uint64_t blocks = std::min<uint64_t>((n + kMeshThreads - 1) / kMeshThreads, 2ull * (uint64_t)device_sm_count());
-    mesh_split_kernel<<<(unsigned)blocks + (span ? 1u : 0u), kMeshThreads, 0, s>>>(
+    const uint64_t blocks = std::min<uint64_t>((n + kMeshThreads - 1) / kMeshThreads, 8ull * (uint64_t)device_sm_count());
+    mesh_split_kernel<<<(unsigned)blocks + (span ? kSpanParts : 0u), kMeshThreads, 0, s>>>(
         xyz, rgb, x, y, z, rgb_out, nvert, idx, ntri, (reinterpret_cast<uintptr_t>(rgb) & 3u) == 0, span);
     return cudaGetLastError();
 }
@@ -381,14 +375,14 @@ __global__ void __launch_bounds__(kMeshThreads)
 mesh_span_kernel(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
                  const uint32_t *__restrict__ idx, uint32_t ntri, volatile float *span)
 {
-    mesh_span_block(idx, ntri, span, [&](uint32_t i) { return make_float3(x[i], y[i], z[i]); });
+    mesh_span_block(blockIdx.x, idx, ntri, span, [&](uint32_t i) { return make_float3(x[i], y[i], z[i]); });
 }
 
 cudaError_t launch_mesh_span(const float *x, const float *y, const float *z, const uint32_t *idx, uint32_t ntri,
                              volatile float *span, cudaStream_t s)
 {
     if (ntri == 0 || !span) return cudaSuccess;
-    mesh_span_kernel<<<1, kMeshThreads, 0, s>>>(x, y, z, idx, ntri, span);
+    mesh_span_kernel<<<kSpanParts, kMeshThreads, 0, s>>>(x, y, z, idx, ntri, span);
     return cudaGetLastError();
 }
 

@@ -52,12 +52,17 @@ struct sloth_mesh {
     float bbox_max[3] = {0, 0, 0};
     uint32_t *order = nullptr, *oidx = nullptr;   // setup's order of an indexed mesh (spatial_order)
     bool updated = false;   // positions may change on the stream (sloth_mesh_update*)
-    // Sum over the triangles of their longest edge squared, page-locked: of the positions the
-    // mesh was made with (mesh_span2), then of those of the last update that has run
-    // (mesh_span_block); null without memory for it.
+    // Sum over the triangles of their longest edge squared, in kSpanParts page-locked parts: of
+    // the positions the mesh was made with (mesh_span2, all in the first), then of those of the
+    // last update that has run (mesh_span_block); null without memory for it.
     volatile float *span2 = nullptr;
 
-    float span() const { return span2 ? *span2 : 0.0f; }
+    float span() const
+    {
+        float sum = 0.0f;
+        for (uint32_t k = 0; span2 && k < kSpanParts; ++k) sum += span2[k];
+        return sum;
+    }
 };
 
 struct sloth_ctx {
@@ -910,9 +915,10 @@ sloth_status sloth_mesh_create(sloth_ctx *ctx, const float *x, const float *y, c
     m->nvert = nvert;
     m->ntri = ntri;
     void *span = nullptr;
-    if (cudaMallocHost(&span, sizeof(float)) == cudaSuccess) {
+    if (cudaMallocHost(&span, kSpanParts * sizeof(float)) == cudaSuccess) {
         m->span2 = static_cast<volatile float *>(span);
-        *m->span2 = mesh_span2(x, y, z, idx, ntri);
+        for (uint32_t k = 0; k < kSpanParts; ++k) m->span2[k] = 0.0f;
+        m->span2[0] = mesh_span2(x, y, z, idx, ntri);
     } else {
         cudaGetLastError();   // such a mesh keeps the tiles
     }

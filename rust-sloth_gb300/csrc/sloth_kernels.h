@@ -173,9 +173,12 @@ cudaError_t launch_frame_reset(const FrameBuffers &fb, const BinBuffers &bb, uin
 // Triangles that the sum of a mesh's longest edges squared is taken from (mesh_span2), spread
 // over the mesh.
 constexpr uint32_t kSpanTriangles = 4096;
+// On the device by this many blocks, whose parts of the sum are kept apart (one block alone
+// took 5 us for its gathers, longer than the rest of an update).
+constexpr uint32_t kSpanParts = 16;
 
 // positions split from x, y, z triples and face colours copied into a mesh's arrays; span
-// (page-locked, may be null) gets the sum of the triangles' longest edges squared.
+// (kSpanParts page-locked words, may be null) gets the sum of the triangles' longest edges squared.
 cudaError_t launch_mesh_split(const float *xyz, const uint8_t *rgb, float *x, float *y, float *z, uint8_t *rgb_out,
                               uint32_t nvert, const uint32_t *idx, uint32_t ntri, volatile float *span, cudaStream_t s);
 // that sum alone, from a mesh's own arrays
