@@ -149,7 +149,9 @@ sloth_status sloth_ctx_device_buffers(sloth_ctx *ctx, const uint32_t **cells, co
 
 /* Covered samples (all three edge functions >= 0, src/rasterizer.rs:75) since the last
  * clear, counted by the raster kernels over what depth culling left (triangles, or samples
- * where a draw goes without tiles): every covered sample when SLOTH_OPTION_DEPTH_CULL is 0.  Blocks until pending work completes. */
+ * where a draw goes without tiles; how many that are depends on the order in which the
+ * device's warps run): every covered sample when SLOTH_OPTION_DEPTH_CULL is 0.  Blocks until
+ * pending work completes. */
 sloth_status sloth_ctx_fragments(sloth_ctx *ctx, uint64_t *fragments);
 
 /* The bytes Context::flush(color, webify) prints for the frame (src/context.rs:50-92),
@@ -349,7 +351,9 @@ sloth_status sloth_batch_autotune(sloth_batch *batch, int reps, int *best_shape,
  * the context's stream.  With store_visibility = 1 the forward call also keeps the
  * winning (triangle, sample) of every cell (8 bytes per depth cell) for the next backward
  * call; otherwise the backward call decodes it again from the depth keys.  Either way the
- * backward call must follow the render it differentiates, before the next render. */
+ * backward call must follow the render it differentiates, before the next render.  The calls
+ * do not wait for the render: a device fault of one still in flight (SLOTH_ERR_DEVICE_FAULT)
+ * comes from a later call on the batch, and from every one after that. */
 sloth_status sloth_batch_depth_cells(sloth_batch *batch, uint32_t frame, uint64_t *first, uint64_t *count);
 sloth_status sloth_batch_shade(sloth_batch *batch, const float *vertex_rgb, const float *light, float *rgb,
                                int store_visibility);

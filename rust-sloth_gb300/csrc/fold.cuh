@@ -2,8 +2,8 @@
 // frame's global depth keys.
 //
 // The tile raster (raster_common.cuh) pays for itself when the samples are many: a tile
-// count, a scan, an entry per triangle and tile, a sort and a walk per tile, in nine
-// launches that each wait for the one before.  A draw of a few thousand triangles over few
+// count, a scan, an entry per triangle and tile, a sort and a walk per tile, in six or
+// seven launches that each wait for the one before.  A draw of a few thousand triangles over few
 // samples is all launches.  Here it takes two: fold_triangles sets up 32 triangles per
 // block and walks their samples (direct.cuh) with every warp of the block, and queues the
 // triangles of more than kFoldBlockSamples samples; fold_queue_walk walks those with the

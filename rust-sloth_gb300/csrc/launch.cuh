@@ -44,7 +44,9 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 
 // An ordinary launch with the same arguments: what the kernels of a captured graph use, where
 // the edges between dependents cost what they save (uneven batch 1583 us a pass with them,
-// 1561 without; 24 views of 160x48 38.4 and 36.0).
+// 1561 without; 24 views of 160x48 38.4 and 36.0).  Two are dependent there all the same: the
+// setup of 32 triangles a block, behind the reset (24 views 29.3 us, plain 29.5), and the scan,
+// whose launcher contexts share (1557 us either way).
 template <class... K, class... A>
 cudaError_t launch(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
 {
