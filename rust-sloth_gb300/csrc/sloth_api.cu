@@ -649,6 +649,18 @@ sloth_status sloth_ctx_sizes(const sloth_ctx *ctx, uint64_t *frame_cells, uint64
     return SLOTH_OK;
 }
 
+// Whether the host can write there (null: nothing to write).  The copies go wherever a pointer
+// leads, and a program that gives them device memory goes on with them.
+static bool host_memory(const void *p)
+{
+    cudaPointerAttributes a{};
+    if (p && cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return !p || a.type != cudaMemoryTypeDevice;
+}
+
 static sloth_status read_staged(sloth_ctx *ctx, uint32_t *cells, float *z, int32_t *winner, uint32_t ncells,
                                 uint32_t nz)
 {
@@ -680,7 +692,7 @@ sloth_status sloth_ctx_read(sloth_ctx *ctx, uint32_t *cells, float *z, int32_t *
     if (st != SLOTH_OK) return st;
     const size_t nz = (size_t)ctx->g.w * ctx->g.h;
     const size_t ncells = ctx->g.image ? nz + ctx->g.h : nz;
-    if (ncells <= kStageCells && ctx->h_stage)
+    if (ncells <= kStageCells && ctx->h_stage && host_memory(cells) && host_memory(z) && host_memory(winner))
         return read_staged(ctx, cells, z, winner, (uint32_t)ncells, (uint32_t)nz);
     if (cells)
         CU(ctx, cudaMemcpyAsync(cells, ctx->fb.cells_out, ncells * sizeof(uint32_t),
