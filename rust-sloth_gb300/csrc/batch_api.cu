@@ -426,7 +426,7 @@ BatchDev dev_view(sloth_batch *b)
     d.total_tiles = b->total_tiles;
     d.frame_tile_off = b->frame_tile_off;
     d.bb = b->bb;
-    d.bb.capacity = (uint32_t)(b->entries_cap > 0xffffffffu ? 0xffffffffu : b->entries_cap);
+    d.bb.capacity = entry_capacity(b->entries_cap);
     d.large_frame = b->large_frame;
     d.status = b->status;
     d.queue = b->queue;

@@ -118,8 +118,8 @@ __global__ void __launch_bounds__(1024) bin_scan_kernel(uint32_t n, BinBuffers b
     }
     if (tid < kV) carry[tid] = 0;
     block_sync();
+    unsigned long long te = 0;   // thread 0: all entries
     if (tid == 0) {
-        unsigned long long te = 0;
         uint32_t tt = 0;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
             te += red_e[w];
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(1024) bin_scan_kernel(uint32_t n, BinBuffers b
         block_sync();
     }
     if (tid == 0) {
-        bb.tile_offset[n] = carry[0];
+        bb.tile_offset[n] = entry_total(te);   // carry[0] where that fits
         bb.slice_offset[n] = carry[1] + carry[2] + carry[3];
         bb.slice_offset[n + 1] = sp.threshold;
         bb.slice_offset[n + 2] = sp.slice;

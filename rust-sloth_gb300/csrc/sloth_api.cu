@@ -1063,11 +1063,11 @@ sloth_status sloth_mesh_info(const sloth_mesh *m, uint32_t *ntri, float bbox_max
 static sloth_status poll_entry_max(sloth_ctx *ctx)
 {
     const uint32_t most = *(volatile uint32_t *)ctx->h_outgrew;
-    if (!ctx->bb.entries || most <= ctx->bb.capacity) return SLOTH_OK;
+    if (!ctx->bb.entries || most <= ctx->bb.capacity || ctx->bb.capacity == entry_capacity(most)) return SLOTH_OK;
     size_t ecap = ctx->bb.capacity;
     sloth_status st = ensure_scratch(ctx, &ctx->bb.entries, &ecap, most);
     if (st != SLOTH_OK) return st;
-    ctx->bb.capacity = (uint32_t)(ecap > 0xffffffffu ? 0xffffffffu : ecap);
+    ctx->bb.capacity = entry_capacity(ecap);
     return SLOTH_OK;
 }
 
@@ -1196,7 +1196,7 @@ sloth_status sloth_draw_mesh(sloth_ctx *ctx, const sloth_mesh *mesh, const float
         bound = *ctx->h_total;
         size_t ecap = ctx->bb.capacity;
         if ((st = ensure_scratch(ctx, &ctx->bb.entries, &ecap, bound)) != SLOTH_OK) return st;
-        ctx->bb.capacity = (uint32_t)(ecap > 0xffffffffu ? 0xffffffffu : ecap);
+        ctx->bb.capacity = entry_capacity(ecap);
     }
     size_t icap = ctx->bb.item_capacity;
     if ((st = ensure_scratch(ctx, &ctx->bb.items, &icap, raster_item_bound(ntiles, bound))) != SLOTH_OK) return st;

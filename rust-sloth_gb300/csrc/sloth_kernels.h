@@ -104,6 +104,23 @@ __host__ __device__ inline uint32_t item_offset(const uint32_t *so, uint32_t nti
     return so[t] + base;
 }
 
+// A draw's entries as the scan reports them: slots are 32-bit, so 2^32 entries or more (33,000
+// triangles over all of 16384x16384 cells) are all kEntriesBeyond, which no capacity reaches:
+// they outgrow every buffer, and nobody reads the offsets, which have wrapped.
+constexpr uint32_t kEntriesBeyond = 0xffffffffu;
+__host__ __device__ constexpr uint32_t entry_total(uint64_t entries)
+{
+    return entries < kEntriesBeyond ? (uint32_t)entries : kEntriesBeyond;
+}
+constexpr uint32_t entry_capacity(uint64_t entries)
+{
+    return entries < kEntriesBeyond ? (uint32_t)entries : kEntriesBeyond - 1u;
+}
+static_assert(entry_total(0) == 0 && entry_total(4294967294u) == 4294967294u && entry_total(4294967295u) == kEntriesBeyond &&
+                  entry_total(1ull << 32) > entry_capacity(1ull << 32) && entry_total(~0ull) > entry_capacity(~0ull) &&
+                  entry_total(4294967295u) > entry_capacity(4294967295u),
+              "what does not fit 32 bits outgrows every buffer");
+
 // Raster CTAs needed for ntiles tiles holding at most `capacity` entries in total.
 inline uint32_t raster_item_bound(uint32_t ntiles, size_t capacity)
 {
