@@ -23,14 +23,14 @@ __global__ void __launch_bounds__(256, 8) resolve_kernel(FrameGeom g, FrameBuffe
     if (kEven) {
         const uint32_t npairs = ncells / 2 + (ncells & 1u), span = blockDim.x * kEvenPairs;
         for (uint64_t base = (uint64_t)blockIdx.x * span; base < npairs; base += (uint64_t)gridDim.x * span)
-            resolve_even<kEvenPairs>(g, fb, (uint32_t)base + tid, blockDim.x, npairs, vec != 0);
+            resolve_even<kEvenPairs, true>(g, fb, (uint32_t)base + tid, blockDim.x, npairs, vec != 0);
         return;
     }
     const uint32_t nruns = ncells / kRun + (ncells % kRun != 0);
     const int lane = threadIdx.x & 31;
     for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < nruns; base += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t p = (uint32_t)base + tid;
-        resolve_run<kRun>(g, fb, p, p < nruns, lane, vec != 0);
+        resolve_run<kRun, true>(g, fb, p, p < nruns, lane, vec != 0);
     }
 }
 

@@ -32,6 +32,10 @@ __device__ __forceinline__ bool later(const Cand &a, const Cand &b)
     return a.x > b.x;
 }
 
+// kDependent: the kernel was launched by launch_pdl right behind one that writes keys and
+// generations, and reads them by plain loads (launch.cuh).  Elsewhere read-only loads, which the
+// compiler moves past the stores of the cells before (59 views of 151x81: 94 us for 99).
+template <bool kDependent = false>
 __device__ __forceinline__ uint64_t key_at(const FrameGeom &g, const FrameBuffers &fb, int r, int cc)
 {
     // no sample writes an odd column of an even-width frame, and its key is not kept
@@ -39,9 +43,11 @@ __device__ __forceinline__ uint64_t key_at(const FrameGeom &g, const FrameBuffer
     // tile sides are powers of two; both reads issued before either is tested (the key
     // of a tile of an older generation is in bounds, only stale)
     const int tile = (r >> (__ffs(g.th) - 1)) * g.ntx + (cc >> (__ffs(g.tw) - 1));
-    // (plain loads: the kernel before may have written both, launch.cuh)
-    const uint32_t gen = fb.tile_gen[tile];
-    const uint64_t k = fb.keys[(size_t)r * g.pitch + key_col(cc, g.tw)];
+    const uint32_t *gp = fb.tile_gen + tile;
+    const unsigned long long *kp =
+        reinterpret_cast<const unsigned long long *>(fb.keys) + (size_t)r * g.pitch + key_col(cc, g.tw);
+    const uint32_t gen = kDependent ? *gp : __ldg(gp);
+    const uint64_t k = kDependent ? *kp : __ldg(kp);
     return gen == fb.gen ? k : kEmptyKey;
 }
 
@@ -130,7 +136,7 @@ __device__ __forceinline__ Cand shfl_up_cand(const Cand &c)
 // lane order; lanes with valid false (past the end) write nothing.  Depth cell c0-1's
 // winner is the previous lane's last depth cell (lane 0 decodes it itself).  With vec the
 // outputs are 4K-byte aligned and a lane's K cells go out in one store per buffer.
-template <int K>
+template <int K, bool kDependent = false>
 __device__ __forceinline__ void resolve_run(const FrameGeom &g, const FrameBuffers &fb, uint32_t p, bool valid,
                                             int lane, bool vec)
 {
@@ -147,7 +153,7 @@ __device__ __forceinline__ void resolve_run(const FrameGeom &g, const FrameBuffe
     for (int j = 0; j < K; ++j) {
         rj[j] = j == 0 ? r0 : (cj[j - 1] + 1 == g.w ? rj[j - 1] + 1 : rj[j - 1]);
         cj[j] = j == 0 ? cc0 : (cj[j - 1] + 1 == g.w ? 0 : cj[j - 1] + 1);
-        key[j] = valid && c0 + j < nz ? key_at(g, fb, rj[j], cj[j]) : kEmptyKey;
+        key[j] = valid && c0 + j < nz ? key_at<kDependent>(g, fb, rj[j], cj[j]) : kEmptyKey;
     }
     Cand kc[K];
     bool hc[K];
@@ -173,7 +179,7 @@ __device__ __forceinline__ void resolve_run(const FrameGeom &g, const FrameBuffe
                 rm = g.h - 1;
                 cm = g.w - 1;
             }
-            const uint64_t k = key_at(g, fb, rm, cm);
+            const uint64_t k = key_at<kDependent>(g, fb, rm, cm);
             if (k != kEmptyKey) {
                 km = decode(g, fb, k, rm, cm, nullptr);
                 hm = true;
@@ -237,7 +243,7 @@ __device__ __forceinline__ void resolve_run(const FrameGeom &g, const FrameBuffe
 // pairs p0 + j*stride below pend, issuing every key load first, then every winner's record
 // loads, then the arithmetic and stores: J independent chains in flight instead of one.
 // With vec the outputs are 8-byte aligned and a pair goes out in one store per buffer.
-template <int J>
+template <int J, bool kDependent = false>
 __device__ __forceinline__ void resolve_even(const FrameGeom &g, const FrameBuffers &fb, uint32_t p0, uint32_t stride,
                                              uint32_t pend, bool vec)
 {
@@ -253,7 +259,7 @@ __device__ __forceinline__ void resolve_even(const FrameGeom &g, const FrameBuff
         if (p < pend && c0 < nz) {
             rr[j] = (int)(c0 / (uint32_t)g.w);
             cc[j] = (int)(c0 - (uint32_t)rr[j] * (uint32_t)g.w);
-            key[j] = key_at(g, fb, rr[j], cc[j]);
+            key[j] = key_at<kDependent>(g, fb, rr[j], cc[j]);
         }
     }
     float4 q0[J], q1[J];
