@@ -260,6 +260,15 @@ void set_mats(sloth_batch *b)
     b->fold = batch_folds(b);
 }
 
+// The fill list and its metas: 20 bytes a triangle that a batch without tiles does not need.
+sloth_status ensure_fill_list(sloth_batch *b)
+{
+    if (b->bb.fill_list) return SLOTH_OK;
+    BCU(b, balloc(&b->bb.fill_list, fill_words16(b->total_rec)));
+    b->bb.fill_meta = reinterpret_cast<uint32_t *>(b->bb.fill_list + b->total_rec);
+    return SLOTH_OK;
+}
+
 // Lay out every frame for tile shape `shape` and allocate the batch's buffers.
 sloth_status build(sloth_batch *b, int shape)
 {
@@ -384,6 +393,10 @@ sloth_status build(sloth_batch *b, int shape)
     BCU(b, balloc(&b->bb.slice_offset, tiles + kSliceExtra));
     BCU(b, balloc(&b->queue, 1));
     BCU(b, balloc(&b->fill_count, 1));
+    if (b->fold == FoldForm::none) {   // its first render takes tiles: not then
+        const sloth_status st = ensure_fill_list(b);
+        if (st != SLOTH_OK) return st;
+    }
     BCU(b, balloc(&b->d_mats, nd));
     for (uint32_t f = 0; f < nf; ++f) {
         BatchFrame &bf = b->hframes[f];
@@ -541,10 +554,8 @@ sloth_status render_planned(sloth_batch *b)
         b->rendered = true;
         return SLOTH_OK;
     }
-    if (!b->bb.fill_list) {   // 20 bytes a triangle that a batch without tiles does not need
-        BCU(b, balloc(&b->bb.fill_list, fill_words16(b->total_rec)));
-        b->bb.fill_meta = reinterpret_cast<uint32_t *>(b->bb.fill_list + b->total_rec);
-    }
+    const sloth_status st = ensure_fill_list(b);
+    if (st != SLOTH_OK) return st;
     BatchDev d = dev_view(b);
     BCU(b, enqueue_front(b, d, s));
     BCU(b, cudaMemcpyAsync(b->h_total, b->bb.tile_offset + b->total_tiles, 4, cudaMemcpyDeviceToHost, s));
