@@ -199,8 +199,7 @@ struct DirectWalk {
 // triangle needs no proven tight bound nor depth bounds.  A finite triangle with an edge
 // of dy > 0 is sized by its unproven right end floor(max.x)+1 (xe) and walked with early
 // row exits up to the reference's bound; any other triangle is sized and walked by its
-// stored range.  A triangle is direct exactly when is_direct(x0, xe, y0, y1, direct_max)
-// holds for the stored range, so later kernels recognise it from row 4 alone.
+// stored range.
 __device__ __forceinline__ TriRecord build_record(float4 p1, float4 p2, float4 p3, uint32_t rgb, int w, int h,
                                                   int direct_max = 0, DirectWalk *dw = nullptr)
 {
