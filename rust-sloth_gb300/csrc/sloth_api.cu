@@ -651,16 +651,16 @@ sloth_status sloth_ctx_sizes(const sloth_ctx *ctx, uint64_t *frame_cells, uint64
     return SLOTH_OK;
 }
 
-// Whether the host can write there (null: nothing to write).  The copies go wherever a pointer
-// leads, and a program that gives them device memory goes on with them.
+// Whether the host can write there.  The copies go wherever a pointer leads, and a program that
+// gives them device memory goes on with them.
 static bool host_memory(const void *p)
 {
     cudaPointerAttributes a{};
-    if (p && cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return true;
     }
-    return !p || a.type != cudaMemoryTypeDevice;
+    return a.type != cudaMemoryTypeDevice;
 }
 
 static sloth_status read_staged(sloth_ctx *ctx, uint32_t *cells, float *z, int32_t *winner, uint32_t ncells,
@@ -679,9 +679,15 @@ static sloth_status read_staged(sloth_ctx *ctx, uint32_t *cells, float *z, int32
         at += (r.n[k] + 3u) & ~3u;
     }
     CU(ctx, timed(ctx, "readback", [&] { return launch_readback(r, ctx->stream); }));
+    bool host[3];   // looked up while the kernels run
+    for (int k = 0; k < 3; ++k) {
+        host[k] = !r.n[k] || host_memory(to[k]);
+        if (!host[k])
+            CU(ctx, cudaMemcpyAsync(to[k], in[k], r.n[k] * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    }
     CU(ctx, cudaStreamSynchronize(ctx->stream));
     for (int k = 0; k < 3; ++k)
-        if (r.n[k]) memcpy(to[k], r.out[k], r.n[k] * sizeof(uint32_t));
+        if (r.n[k] && host[k]) memcpy(to[k], r.out[k], r.n[k] * sizeof(uint32_t));
     *ctx->h_error = ctx->h_stage[0];
     return report_device_error(ctx);
 }
@@ -694,7 +700,7 @@ sloth_status sloth_ctx_read(sloth_ctx *ctx, uint32_t *cells, float *z, int32_t *
     if (st != SLOTH_OK) return st;
     const size_t nz = (size_t)ctx->g.w * ctx->g.h;
     const size_t ncells = ctx->g.image ? nz + ctx->g.h : nz;
-    if (ncells <= kStageCells && ctx->h_stage && host_memory(cells) && host_memory(z) && host_memory(winner))
+    if (ncells <= kStageCells && ctx->h_stage)
         return read_staged(ctx, cells, z, winner, (uint32_t)ncells, (uint32_t)nz);
     if (cells)
         CU(ctx, cudaMemcpyAsync(cells, ctx->fb.cells_out, ncells * sizeof(uint32_t),
